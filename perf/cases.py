@@ -220,3 +220,70 @@ def tolerance(case):
     if case["dtype"] == "f16":
         return {"rel": 1.2e-2, "max": 6e-2}
     return {"rel": 1e-5, "max": 6e-5}
+
+
+def _scores64(q, k):
+    """[source, query, head] of one batch item; q, k [token, head, width] in float64."""
+    step = max(1, (1 << 26) // q.numel())
+    return torch.cat([(q[None] - k[s:s + step, None]).abs_().sum(-1) for s in range(0, k.shape[0], step)]) / -q.shape[-1] ** 0.5
+
+
+def _gradients64(q, k, g):
+    """Both gradients of _scores64 under g [source, query, head], with sign(0) = 0."""
+    step = max(1, (1 << 26) // q.numel())
+    dq, dk = torch.zeros_like(q), []
+    for s in range(0, k.shape[0], step):
+        terms = (q[None] - k[s:s + step, None]).sign_().mul_(g[s:s + step, :, :, None])
+        dq += terms.sum(0)
+        dk.append(terms.sum(1))
+    scale = q.shape[-1] ** -0.5
+    return dq * -scale, torch.cat(dk) * scale
+
+
+def exact(case, seed):
+    """What `run` returns for the inputs of this seed, in float64 from the definitions of the operators."""
+    st = prepare(case, seed)
+    q, k, v, vb, grad = (st[name].detach().double() if name in st else None for name in ("q", "k", "v", "vb", "grad"))
+    bs, n = q.shape[:2]
+    scale = -q.shape[-1] ** -0.5
+    if case["kind"] == "dense":
+        each = [(_scores64(q[b], k[b]), *_gradients64(q[b], k[b], grad[b])) for b in range(bs)]
+        return [torch.stack(x) for x in zip(*each)]
+    if case["kind"] == "fused":
+        each = []
+        for b in range(bs):
+            x = _scores64(q[b], k[b])
+            if case["mode"] == "softmax":
+                p = x.softmax(0)
+            else:
+                p = x.exp()
+                p = p / (1 + p.sum(0)) if case["mode"] == "softmax_plus_one" else p
+            dp = torch.einsum("shc,thc->sth", v[b], grad[b])
+            delta = 0 if case["mode"] == "exp" else (p * dp).sum(0)
+            each.append((torch.einsum("sth,shc->thc", p, v[b]), *_gradients64(q[b], k[b], p * (dp - delta)), torch.einsum("sth,thc->shc", p, grad[b])))
+        return [torch.stack(x) for x in zip(*each)]
+    edges = st["edges"] if case["kind"] == "graph" else st["coo"][:, :2].long()
+    dst, src = edges[:, 0], edges[:, 1]
+    each = []
+    for b in range(bs):
+        diff = q[b][dst] - k[b][src]
+        e = (diff.abs().sum(-1) * scale).exp()
+        a = e / (1 + torch.zeros_like(q[b, :, :, 0]).index_add_(0, dst, e))[dst] if case.get("softmax", True) else e
+        vo = torch.zeros_like(v[b]).index_add_(0, dst, a[..., None] * v[b][src])
+        if case.get("bidi"):
+            vo.index_add_(0, src, a[..., None] * vb[b][dst])
+        if case["dtype"] in ("f16", "bf16"):
+            each.append((vo,))
+            continue
+        da = (v[b][src] * grad[b][dst]).sum(-1)
+        dv = torch.zeros_like(v[b]).index_add_(0, src, a[..., None] * grad[b][dst])
+        dvb = ()
+        if case.get("bidi"):
+            da += (vb[b][dst] * grad[b][src]).sum(-1)
+            dvb = (torch.zeros_like(v[b]).index_add_(0, dst, a[..., None] * grad[b][src]),)
+        if case.get("softmax", True):
+            da = da - torch.zeros_like(q[b, :, :, 0]).index_add_(0, dst, a * da)[dst]
+        d = diff.sign_() * (a * da * scale)[..., None]
+        each.append((vo, dv, *dvb, torch.zeros_like(q[b]).index_add_(0, dst, d), torch.zeros_like(k[b]).index_add_(0, src, -d)))
+    out = [torch.stack(x) for x in zip(*each)]
+    return out + [None, None, None] if case["kind"] == "graph" else out  # whole numbers: the expanded list and its lengths
