@@ -350,3 +350,34 @@ def test_expandcoo_edge_cases():
         coo, dm, sm = cabi.expand_coo_host(co)
         rcoo, rdm, rsm = oracle.expand_coo(co)
         assert np.array_equal(coo, rcoo) and (dm, sm) == (rdm, rsm)
+
+
+@pytest.mark.parametrize("cl,keys", [(31, 40), (300, 2400), (300, 2401), (513, 1), (4095, 4096), (4097, 3), (20011, 3001), (9000, 13312),
+                                     (9000, 13313), (9000, 26624), (9000, 26625)])
+def test_ranks_by_cluster_bit_exact(cl, keys):
+    """Row and id counts on both sides of the switch to the cluster kernel, chunks that end inside a row group, chunks without rows; ids
+    up to the most that two and one counter arrays hold, and one more.  The index is built from rows that partly fall
+    outside its range: they are reported, and the others keep the list order."""
+    from oracle import oracle
+    cabi = _cabi()
+    rng = np.random.RandomState(cl + keys)
+    co = np.stack([rng.randint(0, keys, cl), (rng.random_sample(cl) ** 3 * keys).astype(np.int64)], 1) - 7
+    co[0], co[-1] = -7, keys - 8
+    coo, dm, sm = cabi.expand_coo_host(co)
+    rcoo, rdm, rsm = oracle.expand_coo(co)
+    assert np.array_equal(coo, rcoo) and (dm, sm) == (rdm, rsm)
+
+    n_tok, dm = keys + 3, max(1, dm - 1)  # one slot too few: the rows of the longest lists are out of range
+    rows = rcoo.copy()
+    rows[:, :2] += 7
+    ix = cabi.SparseIndex(_dev(rows), n_tok, dm)
+    ok = rows[:, 2] < dm
+    assert (int(ix.status.item()) == 0) == bool(ok.all())
+    pad = lambda n: (n + 3) // 4 * 4
+    buf, at = _host(ix.buf), pad(n_tok * dm)
+    off = buf[at:at + n_tok + 1]
+    slot = buf[at + pad(n_tok + 1):][:cl]
+    kept = rows[ok]
+    assert np.array_equal(off, np.concatenate([[0], np.cumsum(np.bincount(kept[:, 1], minlength=n_tok))]))
+    order = np.argsort(kept[:, 1], kind="stable")
+    assert np.array_equal(slot[:kept.shape[0]], kept[order, 0] * dm + kept[order, 2])
