@@ -18,6 +18,8 @@
 namespace l1b {
 namespace {
 
+constexpr int CTA = 128; // threads: the warps are independent, and small CTAs fill the register file with any register count
+
 struct SparseArgs {
 	int bs, n_tok, n_heads, width, v_width, dm; // dm = dst_mxlen
 	int lph;                                     // lanes per head (power of two <= 32)
@@ -130,21 +132,27 @@ template <int LPHC> __device__ __forceinline__ bool decode(const SparseArgs &a, 
 // any of them is used, so U row fetches (L2 latency each) are in flight per warp instead of one.
 constexpr int U = 4;
 
-// Walk of this lane's vectors of a row: x = li*VEC, += lanes-per-head * VEC.  With NX > 0 the trip count
-// is a compile-time constant (width == NX * lanes-per-head * VEC) and the walk unrolls completely.
-#define L1B_XLOOP(WIDTH) _Pragma("unroll") for (int it_ = 0, x = w.li * VEC; (NX > 0 ? it_ < NX : x < (WIDTH)); it_++, x += step)
+// Generic branches (NX == 0, rows of more than 4 * 32 vectors): this lane's vectors of a row, x = li*VEC, += lanes-per-head * VEC.
+#define L1B_XLOOP(WIDTH) for (int x = w.li * VEC; x < (WIDTH); x += step)
 
-// Edge-outer walk for the widths whose vector count per lane is a compile-time constant (NX > 0): every
+// Does vector `it` of this lane lie inside a row of `width` elements?  EX: the row is exactly NX vectors on every
+// lane, and so is the value row; otherwise vectors past the end are not loaded (zeros, which add nothing) nor stored.
+template <int VEC, bool EX> __device__ __forceinline__ bool in_row(int li, int it, int step, int width)
+{
+	return EX || li * VEC + it * step < width;
+}
+
+// Edge-outer walk for rows of at most NX vectors per lane (NX > 0, compile time): every
 // list entry (a slot of the destination or an incoming edge of the source) is decoded ONCE -- index,
 // weight, row address -- and its NX vectors are fetched at immediate offsets, instead of walking the whole
 // list once per vector (which repeated the decoding, and in the source lists an integer division, NX times).
-//   MODE 0: acc += weight * row      MODE 1: acc += sign(own - row) * weight      MODE 2: acc += sign(row - own) * weight
+//   acc += weight * row
 // entry(i, ptr, weight) fills the row pointer of entry i (already at this lane's first vector; any valid
 // address when the entry is absent: the row is then loaded but not used, which is cheaper than a
 // predicated load plus zero fill) and its weight, and returns whether the entry exists.
 constexpr int UE = 2; // entries in flight per lane: UE * NX 16-byte loads
-template <typename S, typename T, int VEC, int NX, int MODE, typename F>
-__device__ __forceinline__ void walk_list(Pack<T, VEC> (&acc)[NX], const Pack<T, VEC> (&own)[NX], int n, int step, F entry)
+template <typename S, typename T, int VEC, int NX, bool EX, typename F>
+__device__ __forceinline__ void walk_list(Pack<T, VEC> (&acc)[NX], int n, int li, int step, int width, F entry)
 {
 	for (int e0 = 0; e0 < n; e0 += UE) {
 		T wgt[UE];
@@ -162,21 +170,15 @@ __device__ __forceinline__ void walk_list(Pack<T, VEC> (&acc)[NX], const Pack<T,
 		for (int u = 0; u < UE; u++)
 #pragma unroll
 			for (int it = 0; it < NX; it++)
-				row[u][it] = ldc<S, T, VEC>(ptr[u] + it * step, true);
+				row[u][it] = ldc<S, T, VEC>(ptr[u] + it * step, in_row<VEC, EX>(li, it, step, width));
 #pragma unroll
 		for (int u = 0; u < UE; u++)
 			if (ok[u])
 #pragma unroll
 			for (int it = 0; it < NX; it++)
 #pragma unroll
-				for (int i = 0; i < VEC; i++) {
-					if (MODE == 0)
-						acc[it].v[i] += wgt[u] * row[u][it].v[i];
-					else if (MODE == 1)
-						acc[it].v[i] += sign_apply(own[it].v[i] - row[u][it].v[i], wgt[u]);
-					else
-						acc[it].v[i] += sign_apply(row[u][it].v[i] - own[it].v[i], wgt[u]);
-				}
+				for (int i = 0; i < VEC; i++)
+					acc[it].v[i] += wgt[u] * row[u][it].v[i];
 	}
 }
 template <typename T, int VEC, int NX> __device__ __forceinline__ void zero_acc(Pack<T, VEC> (&acc)[NX])
@@ -189,8 +191,11 @@ template <typename T, int VEC, int NX> __device__ __forceinline__ void zero_acc(
 }
 
 // ---- forward, dst pass: scores -> exp -> (+1)-softmax -> attn, vo[dst] = sum_r a_r v[src_r] ----
-template <typename S, typename T, int VEC, int LPHC, int NX>
-__global__ void __launch_bounds__(256) sparse_fwd_dst_kernel(SparseArgs a, const S *__restrict__ v,
+// With NX > 0 ONE walk over the slots does all of it: k[src] and v[src] of a slot are gathered together.  The weights
+// have no maximum to subtract, so vo = (sum_r e_r v[src_r]) / denom needs no second walk (two walks: the v rows waited
+// for the last score, and every weight went through memory).
+template <typename S, typename T, int VEC, int LPHC, int NX, bool EX>
+__global__ void __launch_bounds__(CTA) sparse_fwd_dst_kernel(SparseArgs a, const S *__restrict__ v,
 							      const S *__restrict__ q, const S *__restrict__ k,
 							      S *__restrict__ vo, S *attn, T scale)
 {
@@ -206,6 +211,71 @@ __global__ void __launch_bounds__(256) sparse_fwd_dst_kernel(SparseArgs a, const
 	const int lph = LPHC > 0 ? LPHC : a.lph;
 	const int step = lph * VEC;
 
+	if constexpr (NX > 0) {
+		constexpr int FU = NX > 2 ? 1 : 2; // slots in flight per lane: FU * NX vectors each of k and v
+		Pack<T, VEC> qv[NX], acc[NX];
+#pragma unroll
+		for (int it = 0; it < NX; it++)
+			qv[it] = ldc<S, T, VEC>(qrow + w.li * VEC + it * step, in_row<VEC, EX>(w.li, it, step, W));
+		zero_acc(acc);
+		const S *kbase = k + (tokrow * H + hh) * W + w.li * VEC, *vbase = v + (tokrow * H + hh) * Wv + w.li * VEC;
+		T denom = T(1);
+		for (int r0 = 0; r0 < dm; r0 += FU) {
+			int src[FU];
+			Pack<T, VEC> kr[FU][NX], vr[FU][NX];
+#pragma unroll
+			for (int u = 0; u < FU; u++) {
+				src[u] = r0 + u < dm ? slots[r0 + u] : -1;
+				// rows of absent slots / heads past the end are read from a valid address and not used
+				const size_t so = size_t(src[u] < 0 ? 0 : src[u]) * H;
+#pragma unroll
+				for (int it = 0; it < NX; it++)
+					kr[u][it] = ldc<S, T, VEC>(kbase + so * W + it * step, in_row<VEC, EX>(w.li, it, step, W));
+#pragma unroll
+				for (int it = 0; it < NX; it++)
+					vr[u][it] = ldc<S, T, VEC>(vbase + so * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
+			}
+#pragma unroll
+			for (int u = 0; u < FU; u++) {
+				T part = T(0);
+#pragma unroll
+				for (int it = 0; it < NX; it++)
+#pragma unroll
+					for (int i = 0; i < VEC; i++)
+						part += absdiff(qv[it].v[i], kr[u][it].v[i]);
+				part = group_sum<LPHC>(part, lph);
+				const T e = src[u] >= 0 ? exp_t(part * scale) : T(0);
+				denom += e;
+				if (w.li == 0 && w.head_ok && r0 + u < dm)
+					st1<S, T>(arow + size_t(r0 + u) * H, e);
+				if (src[u] >= 0)
+#pragma unroll
+					for (int it = 0; it < NX; it++)
+#pragma unroll
+						for (int i = 0; i < VEC; i++)
+							acc[it].v[i] += e * vr[u][it].v[i];
+			}
+		}
+		__syncwarp();
+		if (!w.head_ok)
+			return;
+		T inv = T(1);
+		if (a.use_softmax) {
+			inv = T(1) / denom;
+			for (int r = w.li; r < dm; r += lph)
+				st1<S, T>(arow + size_t(r) * H, ld1<S, T>(arow + size_t(r) * H) / denom);
+		}
+		S *orow = vo + ((tokrow + dst) * H + hh) * Wv + w.li * VEC;
+#pragma unroll
+		for (int it = 0; it < NX; it++) {
+#pragma unroll
+			for (int i = 0; i < VEC; i++)
+				acc[it].v[i] *= inv;
+			if (in_row<VEC, EX>(w.li, it, step, Wv))
+				stc<S, T, VEC>(orow + it * step, acc[it]);
+		}
+		return;
+	}
 	T denom = T(1);
 	for (int r0 = 0; r0 < dm; r0 += U) {
 		int src[U];
@@ -247,25 +317,6 @@ __global__ void __launch_bounds__(256) sparse_fwd_dst_kernel(SparseArgs a, const
 	__syncwarp();
 
 	S *orow = vo + ((tokrow + dst) * H + hh) * Wv;
-	if constexpr (NX > 0) {
-		Pack<T, VEC> acc[NX];
-		zero_acc(acc);
-		const S *vbase = v + (tokrow * H + hh) * Wv + w.li * VEC;
-		walk_list<S, T, VEC, NX, 0>(acc, acc, dm, step, [&](int r, const S *&ptr, T &wgt) {
-			const int src = slots[r];
-			const bool ok = w.head_ok && src >= 0;
-			ptr = vbase + size_t(ok ? src : 0) * H * Wv;
-			if (ok)
-				wgt = ld1<S, T>(arow + size_t(r) * H);
-			return ok;
-		});
-		if (w.head_ok) {
-#pragma unroll
-			for (int it = 0; it < NX; it++)
-				stc<S, T, VEC>(orow + w.li * VEC + it * step, acc[it]);
-		}
-		return;
-	}
 	L1B_XLOOP(Wv) {
 		Pack<T, VEC> acc = ldv<T, VEC>(nullptr, false);
 		for (int r0 = 0; r0 < dm; r0 += U) {
@@ -290,8 +341,8 @@ __global__ void __launch_bounds__(256) sparse_fwd_dst_kernel(SparseArgs a, const
 }
 
 // ---- forward, src pass (bidi only): vo[src] += sum_{incoming (dst,r)} a[dst][r] * vb[dst] ----
-template <typename S, typename T, int VEC, int LPHC, int NX>
-__global__ void __launch_bounds__(256) sparse_fwd_src_kernel(SparseArgs a, const S *__restrict__ vb,
+template <typename S, typename T, int VEC, int LPHC, int NX, bool EX>
+__global__ void __launch_bounds__(CTA) sparse_fwd_src_kernel(SparseArgs a, const S *__restrict__ vb,
 							      const S *__restrict__ attn, S *vo)
 {
 	Who w;
@@ -310,7 +361,7 @@ __global__ void __launch_bounds__(256) sparse_fwd_src_kernel(SparseArgs a, const
 		zero_acc(acc);
 		const S *bbase = vb + (tokrow * H + w.h) * Wv + w.li * VEC;
 		const S *abase = attn + (tokrow * dm) * H + w.h;
-		walk_list<S, T, VEC, NX, 0>(acc, acc, e1 - e0, step, [&](int e, const S *&ptr, T &wgt) {
+		walk_list<S, T, VEC, NX, EX>(acc, e1 - e0, w.li, step, Wv, [&](int e, const S *&ptr, T &wgt) {
 			const int slot = a.csc_slot[e0 + e];
 			ptr = bbase + size_t(slot / dm) * H * Wv;
 			wgt = ld1<S, T>(abase + size_t(slot) * H);
@@ -318,6 +369,8 @@ __global__ void __launch_bounds__(256) sparse_fwd_src_kernel(SparseArgs a, const
 		});
 #pragma unroll
 		for (int it = 0; it < NX; it++) {
+			if (!in_row<VEC, EX>(w.li, it, step, Wv))
+				continue;
 			Pack<T, VEC> cur = ldc<S, T, VEC>(orow + w.li * VEC + it * step, true);
 #pragma unroll
 			for (int i = 0; i < VEC; i++)
@@ -357,10 +410,11 @@ __global__ void __launch_bounds__(256) sparse_fwd_src_kernel(SparseArgs a, const
 //   softmax: dx_r = a_r (ds_r - sum_j a_j ds_j)   [same as the reference's Jacobian product,
 //            cuda/l1attn_sparse_cuda_kernel.cu:256-295, without its O(dst_mxlen^2) loop]
 //   else:    dx_r = a_r ds_r
-// For the common widths ONE walk over the slots does all of it (see the NX > 0 branch): 121 registers, two CTAs
-// per SM.  The generic branch walks the list once per quantity and is capped at three CTAs per SM.
-template <typename T, int VEC, int LPHC, int NX, bool BIDI>
-__global__ void __launch_bounds__(256, NX == 4 ? 2 : 3) sparse_bwd_dst_kernel(SparseArgs a, const T *__restrict__ dvo,
+// Rows of at most four vectors per lane: ONE walk over the slots does all of it (see the NX > 0 branch), 121 registers
+// with four vectors (up to 168 when bidirectional: dvo[src] and d_vb come on top).  The generic branch walks the
+// list once per quantity and is capped at 24 warps per SM.
+template <typename T, int VEC, int LPHC, int NX, bool EX, bool BIDI>
+__global__ void __launch_bounds__(CTA, (NX == 4 ? 4 : 6) - (BIDI && NX > 0 ? 1 : 0)) sparse_bwd_dst_kernel(SparseArgs a, const T *__restrict__ dvo,
 							      const T *__restrict__ v, const T *__restrict__ vb,
 							      const T *__restrict__ q, const T *__restrict__ k,
 							      const T *__restrict__ attn, T *dx, T *__restrict__ d_q,
@@ -390,9 +444,10 @@ __global__ void __launch_bounds__(256, NX == 4 ? 2 : 3) sparse_bwd_dst_kernel(Sp
 		const T *qrow = q + ((tokrow + dst) * H + hh) * W + w.li * VEC;
 #pragma unroll
 		for (int it = 0; it < NX; it++) {
-			qv[it] = ldv<T, VEC>(qrow + it * step, w.head_ok);
-			gd[it] = ldv<T, VEC>(gdst + w.li * VEC + it * step, true);
-			bd[it] = ldv<T, VEC>(BIDI ? bdst + w.li * VEC + it * step : gdst, BIDI);
+			const bool okw = in_row<VEC, EX>(w.li, it, step, W), okv = in_row<VEC, EX>(w.li, it, step, Wv);
+			qv[it] = ldv<T, VEC>(qrow + it * step, w.head_ok && okw);
+			gd[it] = ldv<T, VEC>(gdst + w.li * VEC + it * step, okv);
+			bd[it] = ldv<T, VEC>(BIDI ? bdst + w.li * VEC + it * step : gdst, BIDI && okv);
 		}
 		zero_acc(acc1);
 		zero_acc(acc2);
@@ -407,13 +462,13 @@ __global__ void __launch_bounds__(256, NX == 4 ? 2 : 3) sparse_bwd_dst_kernel(Sp
 			Pack<T, VEC> vr[NX], kr[NX], gr[NX];
 #pragma unroll
 			for (int it = 0; it < NX; it++) {
-				vr[it] = ldv<T, VEC>(vbase + so * Wv + it * step, true);
-				kr[it] = ldv<T, VEC>(kbase + so * W + it * step, true);
+				vr[it] = ldv<T, VEC>(vbase + so * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
+				kr[it] = ldv<T, VEC>(kbase + so * W + it * step, in_row<VEC, EX>(w.li, it, step, W));
 			}
 			if (BIDI) {
 #pragma unroll
 				for (int it = 0; it < NX; it++)
-					gr[it] = ldv<T, VEC>(gbase + so * Wv + it * step, true);
+					gr[it] = ldv<T, VEC>(gbase + so * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
 			}
 			const T ar = ok ? arow[size_t(r) * H] : T(0);
 			T part = T(0);
@@ -467,13 +522,15 @@ __global__ void __launch_bounds__(256, NX == 4 ? 2 : 3) sparse_bwd_dst_kernel(Sp
 #pragma unroll
 				for (int i = 0; i < VEC; i++)
 					acc1[it].v[i] = (acc1[it].v[i] - sfac * acc2[it].v[i]) * scale;
-				*reinterpret_cast<Pack<T, VEC> *>(orow + it * step) = acc1[it];
+				if (in_row<VEC, EX>(w.li, it, step, W))
+					*reinterpret_cast<Pack<T, VEC> *>(orow + it * step) = acc1[it];
 			}
 			if (BIDI) { // d_vb[dst] = sum_r a_r dvo[src_r]
 				T *brow = d_vb + ((tokrow + dst) * H + hh) * Wv + w.li * VEC;
 #pragma unroll
 				for (int it = 0; it < NX; it++)
-					*reinterpret_cast<Pack<T, VEC> *>(brow + it * step) = accb[it];
+					if (in_row<VEC, EX>(w.li, it, step, Wv))
+						*reinterpret_cast<Pack<T, VEC> *>(brow + it * step) = accb[it];
 			}
 		}
 		return;
@@ -590,8 +647,8 @@ __global__ void __launch_bounds__(256, NX == 4 ? 2 : 3) sparse_bwd_dst_kernel(Sp
 }
 
 // ---- backward, src pass: d_v[src] = sum a dvo[dst];  d_k[src] = -scale sum sign(q[dst]-k[src]) dx ----
-template <typename T, int VEC, int LPHC, int NX>
-__global__ void __launch_bounds__(256) sparse_bwd_src_kernel(SparseArgs a, const T *__restrict__ dvo,
+template <typename T, int VEC, int LPHC, int NX, bool EX>
+__global__ void __launch_bounds__(CTA, NX == 4 ? 4 : 6) sparse_bwd_src_kernel(SparseArgs a, const T *__restrict__ dvo,
 							      const T *__restrict__ q, const T *__restrict__ k,
 							      const T *__restrict__ attn, const T *__restrict__ dx,
 							      T *__restrict__ d_v, T *__restrict__ d_k, T scale)
@@ -615,7 +672,7 @@ __global__ void __launch_bounds__(256) sparse_bwd_src_kernel(SparseArgs a, const
 		const T *krow = k + ((tokrow + src) * H + w.h) * W + w.li * VEC;
 #pragma unroll
 		for (int it = 0; it < NX; it++)
-			kv[it] = ldv<T, VEC>(krow + it * step, true);
+			kv[it] = ldv<T, VEC>(krow + it * step, in_row<VEC, EX>(w.li, it, step, W));
 		const T *gbase = dvo + (tokrow * H + w.h) * Wv + w.li * VEC, *qbase = q + (tokrow * H + w.h) * W + w.li * VEC;
 		const T *abase = attn + (tokrow * dm) * H + w.h, *xbase = dx + (tokrow * dm) * H + w.h;
 		for (int e = e0; e < e1; e++) {
@@ -624,8 +681,8 @@ __global__ void __launch_bounds__(256) sparse_bwd_src_kernel(SparseArgs a, const
 			Pack<T, VEC> gr[NX], qr[NX];
 #pragma unroll
 			for (int it = 0; it < NX; it++) {
-				gr[it] = ldv<T, VEC>(gbase + d * Wv + it * step, true);
-				qr[it] = ldv<T, VEC>(qbase + d * W + it * step, true);
+				gr[it] = ldv<T, VEC>(gbase + d * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
+				qr[it] = ldv<T, VEC>(qbase + d * W + it * step, in_row<VEC, EX>(w.li, it, step, W));
 			}
 			const T ar = abase[size_t(slot) * H], dxr = xbase[size_t(slot) * H];
 #pragma unroll
@@ -639,11 +696,13 @@ __global__ void __launch_bounds__(256) sparse_bwd_src_kernel(SparseArgs a, const
 		T *orow = d_k + ((tokrow + src) * H + w.h) * W + w.li * VEC;
 #pragma unroll
 		for (int it = 0; it < NX; it++) {
-			*reinterpret_cast<Pack<T, VEC> *>(vrow + w.li * VEC + it * step) = accv[it];
+			if (in_row<VEC, EX>(w.li, it, step, Wv))
+				*reinterpret_cast<Pack<T, VEC> *>(vrow + w.li * VEC + it * step) = accv[it];
 #pragma unroll
 			for (int i = 0; i < VEC; i++)
 				acck[it].v[i] *= -scale;
-			*reinterpret_cast<Pack<T, VEC> *>(orow + it * step) = acck[it];
+			if (in_row<VEC, EX>(w.li, it, step, W))
+				*reinterpret_cast<Pack<T, VEC> *>(orow + it * step) = acck[it];
 		}
 		return;
 	}
@@ -696,14 +755,6 @@ __global__ void __launch_bounds__(256) sparse_bwd_src_kernel(SparseArgs a, const
 	}
 }
 
-// Lanes per head.  Four 16-byte vectors per lane is the fastest walk (fewer shuffle rounds, less index math per
-// term), but a warp then covers 32 / lph heads, and with fewer heads than that (a head-group shard of a multi-GPU
-// run, a model with few heads) the other lanes idle.  `idle_den`: more lanes share a head when at least
-// (idle_den - 1) / idle_den of them would idle otherwise.  Measured at 4096 tokens, 131072 edges, width 64, one batch item:
-// forward 4 heads 0.038 ms against 0.055 ms, 2 heads 0.030 / 0.050; backward 4 heads 0.124 against 0.107 (the
-// unrolled four-vector walk wins although half its lanes idle), 2 heads 0.073 / 0.104 -- so the forward asks
-// with idle_den 2 and the backward with 4.
-int lanes_per_head(int mw, int n_heads, int vec, int idle_den);
 int pow2_ceil(int x)
 {
 	int p = 1;
@@ -712,24 +763,37 @@ int pow2_ceil(int x)
 	return p;
 }
 
-int lanes_per_head(int mw, int n_heads, int vec, int idle_den)
+// Lanes per head and vectors per lane (nx: 1, 2 or 4; 0: the row is longer than 4 vectors on 32 lanes, generic walk).
+// Four vectors per lane is the fastest walk (fewer shuffle rounds, less index math per term), at least four lanes to a
+// head so that a head's loads are whole 64-byte pieces.  A warp covers 32 / lph heads; with fewer heads than that (a
+// head-group shard of a multi-GPU run, a model with few heads) the other lanes idle, and more lanes share a head when at
+// least (idle_den - 1) / idle_den of them would.  Measured at 4096 tokens, 131072 edges, width 64, one batch item:
+// forward 4 heads 0.038 ms against 0.055 ms, 2 heads 0.030 / 0.050; backward 4 heads 0.124 against 0.107 (the
+// unrolled four-vector walk wins although half its lanes idle), 2 heads 0.073 / 0.104 -- so the forward asks
+// with idle_den 2 and the backward with 4.  Rows that are not whole lanes of vectors used to take the generic walk, once
+// per vector and quantity; forward + backward, start and now: 256 tokens, 17 edges each, 64 items of 8 x 32 columns,
+// bidirectional 629 / 259 us; 3001 tokens, 75000 edges, 2 items of 6 x 40 columns (values 24) 578 / 346 us.
+struct RowPlan {
+	int lph, nx;
+	bool exact; // width == v_width == nx * lph vectors: no vector of any lane lies past the end of a row
+};
+RowPlan plan_rows(int width, int v_width, int n_heads, int vec, int idle_den)
 {
-	int lph = pow2_ceil((mw + 4 * vec - 1) / (4 * vec));
-	if (lph > 32)
-		lph = 32;
-	{
-		const int hpw = 32 / lph, slots = hpw * ((n_heads + hpw - 1) / hpw);
-		if (idle_den * (slots - n_heads) < (idle_den - 1) * slots)
-			return lph; // few enough idle lanes as it is
-	}
-	static const bool no_fill = getenv("L1ATTN_SPARSE_NO_FILL") != nullptr; // debugging aid: keep four vectors per lane
-	while (!no_fill && lph < 32 && mw >= 2 * lph * vec) {
-		const int hpw = 32 / lph, slots = hpw * ((n_heads + hpw - 1) / hpw);
-		if (2 * n_heads > slots)
-			break; // more than half the lanes busy
-		lph *= 2;
-	}
-	return lph;
+	const int mw = width > v_width ? width : v_width, nv = (mw + vec - 1) / vec;
+	RowPlan p;
+	p.lph = pow2_ceil((nv + 3) / 4);
+	p.lph = p.lph < 4 ? 4 : p.lph > 32 ? 32 : p.lph;
+	int hpw = 32 / p.lph, slots = hpw * ((n_heads + hpw - 1) / hpw);
+	if (idle_den * (slots - n_heads) >= (idle_den - 1) * slots)
+		while (p.lph < 32 && nv >= 2 * p.lph && 2 * n_heads <= slots) {
+			p.lph *= 2;
+			hpw = 32 / p.lph;
+			slots = hpw * ((n_heads + hpw - 1) / hpw);
+		}
+	const int need = (nv + p.lph - 1) / p.lph;
+	p.nx = need > 4 ? 0 : need > 2 ? 4 : need;
+	p.exact = width == v_width && width == p.nx * p.lph * vec;
+	return p;
 }
 
 struct Grid {
@@ -740,50 +804,51 @@ Grid grid_for(const SparseArgs &a)
 {
 	const int hpw = 32 / a.lph;
 	const long long warps = (long long)a.bs * a.n_tok * ((a.n_heads + hpw - 1) / hpw);
-	const long long blocks = (warps + 7) / 8;
+	const long long blocks = (warps + CTA / 32 - 1) / (CTA / 32);
 	return {unsigned(blocks), blocks <= 0x7fffffffLL};
 }
 
 template <typename S, typename T, int VEC>
 int fwd_t(SparseArgs a, const S *v, const S *vb, const S *q, const S *k, S *vo, S *attn, cudaStream_t st)
 {
-	const int mw = a.width > a.v_width ? a.width : a.v_width;
-	a.lph = lanes_per_head(mw, a.n_heads, VEC, 2);
+	RowPlan p = plan_rows(a.width, a.v_width, a.n_heads, VEC, 2);
+	p.exact = p.exact && VEC > 1;
+	a.lph = p.lph;
 	const Grid g = grid_for(a);
 	if (!g.ok)
 		return L1ATTN_ERR_SHAPE;
 	const T scale = T(-1.0 / sqrt(double(a.width)));
-	// lanes per head as a compile-time constant for the common widths (16-byte vectors, 32..128+ columns)
-#define L1B_FWD(LP, NXV)                                                                                      \
-	do {                                                                                             \
-		sparse_fwd_dst_kernel<S, T, VEC, LP, NXV><<<g.blocks, 256, 0, st>>>(a, v, q, k, vo, attn, scale); \
-		L1B_LAUNCH_CHECK();                                                                      \
-		if (a.bidi) {                                                                            \
-			sparse_fwd_src_kernel<S, T, VEC, LP, NXV><<<g.blocks, 256, 0, st>>>(a, vb, attn, vo);     \
-			L1B_LAUNCH_CHECK();                                                              \
-		}                                                                                        \
+#define L1B_RUN(LP, NXV, EX)                                                                                         \
+	do {                                                                                                         \
+		sparse_fwd_dst_kernel<S, T, VEC, LP, NXV, EX><<<g.blocks, CTA, 0, st>>>(a, v, q, k, vo, attn, scale); \
+		L1B_LAUNCH_CHECK();                                                                                  \
+		if (a.bidi) {                                                                                        \
+			sparse_fwd_src_kernel<S, T, VEC, LP, NXV, EX><<<g.blocks, CTA, 0, st>>>(a, vb, attn, vo);     \
+			L1B_LAUNCH_CHECK();                                                                          \
+		}                                                                                                    \
 	} while (0)
-	// four vectors per lane exactly (width == v_width == 16 * lanes-per-head elements of 16-byte vectors): unrolled walk
-	const bool nx4 = VEC > 1 && a.width == a.v_width && a.width == 4 * a.lph * VEC;
-	if (nx4 && a.lph == 4)
-		L1B_FWD(4, 4);
-	else if (nx4 && a.lph == 8)
-		L1B_FWD(8, 4);
-	else if (nx4 && a.lph == 16)
-		L1B_FWD(16, 4);
-	else if (nx4 && a.lph == 32)
-		L1B_FWD(32, 4);
-	else if (VEC > 1 && a.lph == 4)
-		L1B_FWD(4, 0);
-	else if (VEC > 1 && a.lph == 8)
-		L1B_FWD(8, 0);
-	else if (VEC > 1 && a.lph == 16)
-		L1B_FWD(16, 0);
-	else if (VEC > 1 && a.lph == 32)
-		L1B_FWD(32, 0);
-	else
-		L1B_FWD(0, 0);
-#undef L1B_FWD
+	// (lanes per head, vectors per lane) as compile-time constants; rows that are not whole lanes of vectors take the
+	// two- and four-vector walks with their ends masked, and only those exist for single-element loads (odd widths)
+	if (p.nx == 0)
+		L1B_RUN(0, 0, false);
+#define L1B_PICK(LP, NXV)                                  \
+	else if (p.lph == LP && p.nx == NXV && p.exact)    \
+		L1B_RUN(LP, NXV, true);
+#define L1B_PICKM(LP, NXV)                                 \
+	else if (p.lph == LP && p.nx <= NXV && !p.exact)   \
+		L1B_RUN(LP, NXV, false);
+	L1B_PICKM(4, 2) L1B_PICKM(8, 2) L1B_PICKM(16, 2) L1B_PICKM(32, 2)
+	L1B_PICKM(4, 4) L1B_PICKM(8, 4) L1B_PICKM(16, 4) L1B_PICKM(32, 4)
+	else if constexpr (VEC > 1) {
+		if (false)
+			;
+		L1B_PICK(4, 1) L1B_PICK(8, 1) L1B_PICK(16, 1) L1B_PICK(32, 1)
+		L1B_PICK(4, 2) L1B_PICK(8, 2) L1B_PICK(16, 2) L1B_PICK(32, 2)
+		L1B_PICK(4, 4) L1B_PICK(8, 4) L1B_PICK(16, 4) L1B_PICK(32, 4)
+	}
+#undef L1B_PICK
+#undef L1B_PICKM
+#undef L1B_RUN
 	return L1ATTN_OK;
 }
 
@@ -791,44 +856,46 @@ template <typename T, int VEC>
 int bwd_t(SparseArgs a, const T *dvo, const T *v, const T *vb, const T *q, const T *k, const T *attn, T *d_v,
 	  T *d_vb, T *d_q, T *d_k, T *dx, cudaStream_t st)
 {
-	const int mw = a.width > a.v_width ? a.width : a.v_width;
 	// (two vectors per lane, twice the warps at ~75 registers, measured 2 % slower than four at 8 heads)
-	a.lph = lanes_per_head(mw, a.n_heads, VEC, 4);
+	RowPlan p = plan_rows(a.width, a.v_width, a.n_heads, VEC, 4);
+	p.exact = p.exact && VEC > 1;
+	a.lph = p.lph;
 	const Grid g = grid_for(a);
 	if (!g.ok)
 		return L1ATTN_ERR_SHAPE;
 	const T scale = T(-1.0 / sqrt(double(a.width)));
-#define L1B_BWD(LP, NXV)                                                                                                       \
-	do {                                                                                                              \
-		if (a.bidi)                                                                                               \
-			sparse_bwd_dst_kernel<T, VEC, LP, NXV, true><<<g.blocks, 256, 0, st>>>(a, dvo, v, vb, q, k, attn, dx, d_q, d_vb, scale); \
-		else                                                                                                      \
-			sparse_bwd_dst_kernel<T, VEC, LP, NXV, false><<<g.blocks, 256, 0, st>>>(a, dvo, v, vb, q, k, attn, dx, d_q, d_vb, scale); \
-		L1B_LAUNCH_CHECK();                                                                                       \
-		sparse_bwd_src_kernel<T, VEC, LP, NXV><<<g.blocks, 256, 0, st>>>(a, dvo, q, k, attn, dx, d_v, d_k, scale);        \
-		L1B_LAUNCH_CHECK();                                                                                       \
+#define L1B_RUN(LP, NXV, EX)                                                                                                      \
+	do {                                                                                                                      \
+		if (a.bidi)                                                                                                       \
+			sparse_bwd_dst_kernel<T, VEC, LP, NXV, EX, true><<<g.blocks, CTA, 0, st>>>(a, dvo, v, vb, q, k, attn, dx, d_q, d_vb, scale); \
+		else                                                                                                              \
+			sparse_bwd_dst_kernel<T, VEC, LP, NXV, EX, false><<<g.blocks, CTA, 0, st>>>(a, dvo, v, vb, q, k, attn, dx, d_q, d_vb, scale); \
+		L1B_LAUNCH_CHECK();                                                                                               \
+		sparse_bwd_src_kernel<T, VEC, LP, NXV, EX><<<g.blocks, CTA, 0, st>>>(a, dvo, q, k, attn, dx, d_v, d_k, scale);         \
+		L1B_LAUNCH_CHECK();                                                                                               \
 	} while (0)
-	// four vectors per lane exactly (width == v_width == 16 * lanes-per-head elements of 16-byte vectors): unrolled walk
-	const bool nx4 = VEC > 1 && a.width == a.v_width && a.width == 4 * a.lph * VEC;
-	if (nx4 && a.lph == 4)
-		L1B_BWD(4, 4);
-	else if (nx4 && a.lph == 8)
-		L1B_BWD(8, 4);
-	else if (nx4 && a.lph == 16)
-		L1B_BWD(16, 4);
-	else if (nx4 && a.lph == 32)
-		L1B_BWD(32, 4);
-	else if (VEC > 1 && a.lph == 4)
-		L1B_BWD(4, 0);
-	else if (VEC > 1 && a.lph == 8)
-		L1B_BWD(8, 0);
-	else if (VEC > 1 && a.lph == 16)
-		L1B_BWD(16, 0);
-	else if (VEC > 1 && a.lph == 32)
-		L1B_BWD(32, 0);
-	else
-		L1B_BWD(0, 0);
-#undef L1B_BWD
+	// (lanes per head, vectors per lane) as compile-time constants; rows that are not whole lanes of vectors take the
+	// two- and four-vector walks with their ends masked, and only those exist for single-element loads (odd widths)
+	if (p.nx == 0)
+		L1B_RUN(0, 0, false);
+#define L1B_PICK(LP, NXV)                                  \
+	else if (p.lph == LP && p.nx == NXV && p.exact)    \
+		L1B_RUN(LP, NXV, true);
+#define L1B_PICKM(LP, NXV)                                 \
+	else if (p.lph == LP && p.nx <= NXV && !p.exact)   \
+		L1B_RUN(LP, NXV, false);
+	L1B_PICKM(4, 2) L1B_PICKM(8, 2) L1B_PICKM(16, 2) L1B_PICKM(32, 2)
+	L1B_PICKM(4, 4) L1B_PICKM(8, 4) L1B_PICKM(16, 4) L1B_PICKM(32, 4)
+	else if constexpr (VEC > 1) {
+		if (false)
+			;
+		L1B_PICK(4, 1) L1B_PICK(8, 1) L1B_PICK(16, 1) L1B_PICK(32, 1)
+		L1B_PICK(4, 2) L1B_PICK(8, 2) L1B_PICK(16, 2) L1B_PICK(32, 2)
+		L1B_PICK(4, 4) L1B_PICK(8, 4) L1B_PICK(16, 4) L1B_PICK(32, 4)
+	}
+#undef L1B_PICK
+#undef L1B_PICKM
+#undef L1B_RUN
 	return L1ATTN_OK;
 }
 
@@ -887,17 +954,22 @@ extern "C" int l1attn_sparse_fwd(const void *v, const void *vb, const void *q, c
 		     ix.slot_src, ix.csc_off, ix.csc_slot};
 	const bool a16 = all_aligned16({v, vb, q, k, vo});
 	if (dtype == L1ATTN_F16 || dtype == L1ATTN_BF16) {
-		// 16-bit storage, float arithmetic: four elements (8 bytes) per load when rows allow it
+		// 16-bit storage, float arithmetic: eight elements (16 bytes) per load, or four, when rows allow it
+		const bool a16h = a16 && width % 8 == 0 && v_width % 8 == 0;
 		bool a8 = width % 4 == 0 && v_width % 4 == 0;
 		for (const void *p : {v, vb, q, k, (const void *)vo})
 			a8 = a8 && (!p || aligned(p, 8));
 		if (dtype == L1ATTN_F16) {
 			using H = __half;
+			if (a16h)
+				return fwd_t<H, float, 8>(a, (const H *)v, (const H *)vb, (const H *)q, (const H *)k, (H *)vo, (H *)attn, st);
 			if (a8)
 				return fwd_t<H, float, 4>(a, (const H *)v, (const H *)vb, (const H *)q, (const H *)k, (H *)vo, (H *)attn, st);
 			return fwd_t<H, float, 1>(a, (const H *)v, (const H *)vb, (const H *)q, (const H *)k, (H *)vo, (H *)attn, st);
 		}
 		using B = __nv_bfloat16;
+		if (a16h)
+			return fwd_t<B, float, 8>(a, (const B *)v, (const B *)vb, (const B *)q, (const B *)k, (B *)vo, (B *)attn, st);
 		if (a8)
 			return fwd_t<B, float, 4>(a, (const B *)v, (const B *)vb, (const B *)q, (const B *)k, (B *)vo, (B *)attn, st);
 		return fwd_t<B, float, 1>(a, (const B *)v, (const B *)vb, (const B *)q, (const B *)k, (B *)vo, (B *)attn, st);

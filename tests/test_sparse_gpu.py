@@ -88,6 +88,27 @@ def test_vs_oracle(case, usm, bidi, dtype):
         assert_close(x, r, tol, name)
 
 
+# the walks' lanes per head and vectors per lane: one, two, four vectors exactly; rows that end inside a lane's vectors, k and
+# v rows of different length among them; few heads (more lanes to a head); rows of more than four vectors on 32 lanes
+ROW_CASES = [(2, 24, 8, 16, 16, 6), (2, 24, 8, 32, 32, 6), (1, 30, 2, 32, 32, 5), (1, 30, 5, 48, 48, 5), (2, 26, 6, 40, 24, 7),
+             (1, 26, 3, 96, 96, 5), (1, 26, 1, 20, 36, 5), (1, 18, 2, 128, 128, 4), (1, 12, 1, 520, 516, 3), (1, 20, 9, 12, 8, 4),
+             (1, 20, 3, 72, 64, 4), (1, 16, 2, 141, 47, 4)]
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("bidi", [False, True])
+@pytest.mark.parametrize("case", ROW_CASES)
+def test_row_plans_vs_oracle(case, bidi, dtype):
+    test_vs_oracle(case, bool(case[3] % 3), bidi, dtype)
+
+
+@pytest.mark.parametrize("tdtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("bidi", [False, True])
+@pytest.mark.parametrize("case", ROW_CASES)
+def test_row_plans_16bit(case, bidi, tdtype):
+    test_forward_16bit_storage(case, bool(case[3] % 3), bidi, tdtype)
+
+
 @pytest.mark.parametrize("tdtype", ["float16", "bfloat16"])
 @pytest.mark.parametrize("bidi", [False, True])
 @pytest.mark.parametrize("usm", [True, False])
