@@ -14,9 +14,10 @@
 // Two kernels:
 //   * softmax_v_kernel: any shape, fp32/fp64.  One CTA per (b, t, h) keeps the n_tok scores of its row
 //     in shared memory: scores, max, exp/sum, value product, each in a fixed order.
-//   * softmax_v_tma_kernel (fp32, width 32..128 in steps of 32, v_width 32/64/128): one CTA per
-//     (b, h, tile of 64 or 128 query rows) streams the keys and values of its head in tiles of 64
-//     through a TMA ring and keeps running max / sum / output rows in registers (online softmax).
+//   * softmax_v_tile_kernel (fp32, width and v_width up to 128): one CTA per (b, h, tile of 64 or 128 query
+//     rows) streams the keys and values of its head in tiles of 64 through a ring and keeps running
+//     max / sum / output rows in registers (online softmax).  The ring is filled by TMA where rows are whole
+//     16-byte vectors, else by 4-byte asynchronous copies of all threads; columns past the end of a row read as zeros.
 #include <math.h>
 #include <stdlib.h>
 #include "common.cuh"
@@ -135,15 +136,42 @@ constexpr int PP = TS + 4; // row pitch (floats) of the weight tile: the two hal
 constexpr int MAX_STAGE = 3;
 
 struct SvShape {
-	int n_tok, n_heads, nwb, nstage, ntt, mode;
+	int n_tok, n_heads, width, v_width, nwb, nstage, ntt, mode;
 	float scale;
 };
 
-template <int NV, int TI, int NW>
+// Rows that TMA cannot address (a row pitch or base that is no multiple of 16 bytes): the CTA's warps copy `rows` token
+// rows, 32 columns at a time, with 4-byte asynchronous copies into the place and order a TMA box would leave them in.
+// `base` is the head's row of token 0.  Slices of 32 columns: [slice][row] of 128 bytes, SWZ: 16-byte chunk ^= row & 7;
+// !SWZ: [row][32 * slices].  Columns >= width and tokens >= n_tok become zeros.  The copies are ~16 per thread and tile against
+// ~2500 instructions of math: [4,300,5,33], values 21 wide, takes 31 us forward and 38 us backward (dx, dv), [4,333,6,48],
+// values 40 wide, through TMA 34 and 48 us; the any-shape kernels took about 290 and 740 us for the latter.
+template <int NW, bool SWZ>
+__device__ __forceinline__ void copy_rows(unsigned char *dst, const float *base, size_t pitch, int t0, int rows, int nslice, int width, int n_tok)
+{
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	for (int sl = 0; sl < nslice; sl++) {
+		const int col = sl * 32 + lane;
+		for (int r = warp; r < rows; r += NW) {
+			const bool ok = col < width && t0 + r < n_tok;
+			const float *src = base + (ok ? size_t(t0 + r) * pitch + col : 0);
+			const uint32_t d = smem_u32(dst) + (SWZ ? (sl * rows + r) * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4
+								: (r * nslice * 32 + col) * 4);
+			asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(ok ? 4 : 0) : "memory");
+		}
+	}
+}
+// this thread's arrival on `bar` once its asynchronous copies so far have landed
+__device__ __forceinline__ void copy_arrive(uint64_t *bar)
+{
+	asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+template <int NV, int TI, int NW, bool TMA, bool FULL>
 __global__ void __launch_bounds__(NW * 32, 1)
-softmax_v_tma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
-		     const __grid_constant__ CUtensorMap vmap, float *__restrict__ vo, float *__restrict__ lse, SvShape sh,
-		     int *err)
+softmax_v_tile_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
+		      const __grid_constant__ CUtensorMap vmap, const float *__restrict__ q, const float *__restrict__ k,
+		      const float *__restrict__ v, float *__restrict__ vo, float *__restrict__ lse, SvShape sh, int *err)
 {
 	constexpr int TT = 2 * NW * TI; // query rows of the CTA: a half-warp owns TI of them (t = i*2*NW + tg)
 	constexpr int NTH = NW * 32;
@@ -166,28 +194,42 @@ softmax_v_tma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
 	const int ns = (sh.n_tok + TS - 1) / TS;
 
 	if (tid == 0) {
-		mbar_init(&q_bar, 1);
+		mbar_init(&q_bar, TMA ? 1 : NTH);
 		for (int s = 0; s < MAX_STAGE; s++) {
-			mbar_init(&full_bar[s], 1);
+			mbar_init(&full_bar[s], TMA ? 1 : NTH);
 			mbar_init(&empty_bar[s], NTH / 32);
 		}
 		mbar_fence_init();
 	}
 	__syncthreads();
 
-	// key/value tile m goes to stage m % nstage; the caller has made sure the stage is free
+	const size_t krow = size_t(sh.n_heads) * sh.width, vrow = size_t(sh.n_heads) * sh.v_width;
+	const size_t qk0 = size_t(b) * sh.n_tok * krow + size_t(h) * sh.width, v0 = size_t(b) * sh.n_tok * vrow + size_t(h) * sh.v_width;
+	// key/value tile m goes to stage m % nstage; the caller has made sure the stage is free (TMA: one thread asks;
+	// otherwise every thread copies its part and arrives when it has landed)
 	auto load_tile = [&](int m) {
 		const int st = m % sh.nstage;
 		unsigned char *dst = stages + size_t(st) * stage_bytes;
+		if (!TMA) {
+			copy_rows<NW, true>(dst, k + qk0, krow, m * TS, TS, sh.nwb, sh.width, sh.n_tok);
+			copy_rows<NW, false>(dst + k_bytes, v + v0, vrow, m * TS, TS, VW / 32, sh.v_width, sh.n_tok);
+			copy_arrive(&full_bar[st]);
+			return;
+		}
 		mbar_expect_tx(&full_bar[st], uint32_t(stage_bytes));
 		for (int wb = 0; wb < sh.nwb; wb++)
 			tma_load_4d(dst + wb * TS * 128, &kmap, &full_bar[st], wb * 32, h, m * TS, b);
 		tma_load_4d(dst + k_bytes, &vmap, &full_bar[st], 0, h, m * TS, b);
 	};
-	if (tid == 0) {
-		mbar_expect_tx(&q_bar, uint32_t(q_bytes));
-		for (int wb = 0; wb < sh.nwb; wb++)
-			tma_load_4d(Qs + wb * TT * 128, &qmap, &q_bar, wb * 32, h, t0, b);
+	if (!TMA || tid == 0) {
+		if (TMA) {
+			mbar_expect_tx(&q_bar, uint32_t(q_bytes));
+			for (int wb = 0; wb < sh.nwb; wb++)
+				tma_load_4d(Qs + wb * TT * 128, &qmap, &q_bar, wb * 32, h, t0, b);
+		} else {
+			copy_rows<NW, true>(Qs, q + qk0, krow, t0, TT, sh.nwb, sh.width, sh.n_tok);
+			copy_arrive(&q_bar);
+		}
 		for (int m = 0; m < sh.nstage - 1 && m < ns; m++)
 			load_tile(m);
 	}
@@ -211,7 +253,7 @@ softmax_v_tma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
 	for (int m = 0; m < ns; m++) {
 		// one lane asks for the tile that will be needed nstage-1 tiles from now; its stage held tile
 		// m-1, which every warp must have released (the duty rotates so that no warp is always late)
-		if (warp == m % NW && lane == 0 && m + sh.nstage - 1 < ns && !dead) {
+		if ((!TMA || (warp == m % NW && lane == 0)) && m + sh.nstage - 1 < ns && !dead) {
 			const int mm = m + sh.nstage - 1;
 			if (mbar_wait(&empty_bar[mm % sh.nstage], ((unsigned(mm) / unsigned(sh.nstage)) & 1u) ^ 1u, err))
 				load_tile(mm);
@@ -235,8 +277,9 @@ softmax_v_tma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
 		for (int wb = 0; wb < sh.nwb; wb++) {
 			const ulonglong2 *Qb = reinterpret_cast<const ulonglong2 *>(Qs + wb * TT * 128);
 			const ulonglong2 *Kb = reinterpret_cast<const ulonglong2 *>(Ks + wb * TS * 128);
+			const int nc = FULL ? 8 : min(8, ((sh.width - wb * 32 + 7) >> 3) * 2); // 16-byte chunks of this slice, to a pair
 #pragma unroll 2
-			for (int c = 0; c < 8; c++) {
+			for (int c = 0; c < nc; c++) {
 				ulonglong2 kv[4];
 #pragma unroll
 				for (int j = 0; j < 4; j++) // row j*16+sg, chunk c ^ (row & 7)
@@ -339,7 +382,6 @@ softmax_v_tma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
 			mbar_arrive(&empty_bar[st]);
 	}
 
-	const size_t vrow = size_t(sh.n_heads) * VW;
 #pragma unroll
 	for (int i = 0; i < TI; i++) {
 		const int t = t0 + i * (2 * NW) + tg;
@@ -348,27 +390,28 @@ softmax_v_tma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_cons
 		const float inv = sh.mode == L1ATTN_SV_EXP ? 1.f : 1.f / lrow[i];
 		if (lse && sg == 0) // weight of (s, t) = exp(x - lse)
 			lse[(size_t(b) * sh.n_tok + t) * sh.n_heads + h] = sh.mode == L1ATTN_SV_EXP ? 0.f : mrow[i] + logf(lrow[i]);
-		float *op = vo + (size_t(b) * sh.n_tok + t) * vrow + size_t(h) * VW + sg * NV;
+		float *op = vo + v0 + size_t(t) * vrow + sg * NV;
 #pragma unroll
 		for (int e = 0; e < NV; e++)
-			op[e] = o[i][e] * inv;
+			if (FULL || sg * NV + e < sh.v_width)
+				op[e] = o[i][e] * inv;
 	}
 }
 
-template <int NV, int TI, int NW>
-int launch_tma(const float *q, const float *k, const float *v, float *vo, float *lse, int bs, int n_tok, int n_heads,
-	       int width, int mode, int nstage, size_t smem, cudaStream_t st)
+template <int NV, int TI, int NW, bool TMA, bool FULL>
+int launch_tile(const float *q, const float *k, const float *v, float *vo, float *lse, int bs, int n_tok, int n_heads,
+		int width, int v_width, int mode, int nstage, size_t smem, cudaStream_t st)
 {
 	constexpr int TT = 2 * NW * TI, VW = 16 * NV, NTH = NW * 32;
 	const uint64_t dims[4] = {uint64_t(width), uint64_t(n_heads), uint64_t(n_tok), uint64_t(bs)};
 	const uint64_t str[3] = {uint64_t(width) * 4, uint64_t(n_heads) * width * 4, uint64_t(n_tok) * n_heads * width * 4};
-	const uint64_t vdims[4] = {uint64_t(VW), uint64_t(n_heads), uint64_t(n_tok), uint64_t(bs)};
-	const uint64_t vstr[3] = {uint64_t(VW) * 4, uint64_t(n_heads) * VW * 4, uint64_t(n_tok) * n_heads * VW * 4};
+	const uint64_t vdims[4] = {uint64_t(v_width), uint64_t(n_heads), uint64_t(n_tok), uint64_t(bs)};
+	const uint64_t vstr[3] = {uint64_t(v_width) * 4, uint64_t(n_heads) * v_width * 4, uint64_t(n_tok) * n_heads * v_width * 4};
 	const uint32_t qbox[4] = {32, 1, TT, 1}, kbox[4] = {32, 1, TS, 1}, vbox[4] = {VW, 1, TS, 1};
-	CUtensorMap qmap, kmap, vmap;
-	if (!encode_tmap_4d(&qmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, q, dims, str, qbox, CU_TENSOR_MAP_SWIZZLE_128B) ||
+	CUtensorMap qmap{}, kmap{}, vmap{};
+	if (TMA && (!encode_tmap_4d(&qmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, q, dims, str, qbox, CU_TENSOR_MAP_SWIZZLE_128B) ||
 	    !encode_tmap_4d(&kmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, k, dims, str, kbox, CU_TENSOR_MAP_SWIZZLE_128B) ||
-	    !encode_tmap_4d(&vmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, v, vdims, vstr, vbox, CU_TENSOR_MAP_SWIZZLE_NONE))
+	    !encode_tmap_4d(&vmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, v, vdims, vstr, vbox, CU_TENSOR_MAP_SWIZZLE_NONE)))
 		return 1;
 	int *err = device_error_word();
 	if (!err)
@@ -376,7 +419,9 @@ int launch_tma(const float *q, const float *k, const float *v, float *vo, float 
 	SvShape sh;
 	sh.n_tok = n_tok;
 	sh.n_heads = n_heads;
-	sh.nwb = width / 32;
+	sh.width = width;
+	sh.v_width = v_width;
+	sh.nwb = (width + 31) / 32;
 	sh.nstage = nstage;
 	sh.ntt = (n_tok + TT - 1) / TT;
 	sh.mode = mode;
@@ -384,9 +429,9 @@ int launch_tma(const float *q, const float *k, const float *v, float *vo, float 
 	const long long grid = (long long)bs * n_heads * sh.ntt;
 	if (grid > 0x7fffffffLL)
 		return L1ATTN_ERR_SHAPE;
-	auto kern = softmax_v_tma_kernel<NV, TI, NW>;
+	auto kern = softmax_v_tile_kernel<NV, TI, NW, TMA, FULL>;
 	L1B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-	kern<<<unsigned(grid), NTH, smem, st>>>(qmap, kmap, vmap, vo, lse, sh, err);
+	kern<<<unsigned(grid), NTH, smem, st>>>(qmap, kmap, vmap, q, k, v, vo, lse, sh, err);
 	L1B_LAUNCH_CHECK();
 	return L1ATTN_OK;
 }
@@ -398,40 +443,62 @@ size_t sv_smem(int nwb, int nv, int tt_rows, int nstage)
 	return size_t(nwb) * tt * 128 + size_t(nstage) * (size_t(nwb) * TS * 128 + size_t(TS) * nv * 64) + tt * PP * 4 + 1024;
 }
 
-// Returns L1ATTN_OK, a negative error, or 1 when the shape is outside this kernel's set.
-int softmax_v_tma(const float *q, const float *k, const float *v, float *vo, float *lse, int bs, int n_tok, int n_heads,
-		  int width, int v_width, int mode, cudaStream_t st)
+// (query rows per half-warp, warps, ring stages) of the tiled kernels.  4 x 16 and 8 x 8 make a 128-row CTA, 4 x 8 a 64-row
+// one.  Sixteen warps of 128 registers measured 7 % faster than eight of 168 (four warps per scheduler hide the
+// shared-memory and arithmetic latencies); with 128 value columns the thread state does not fit 128 registers.  A 64-row CTA
+// takes SHORT_CTA of the time of a 128-row one; it is taken where the rows do not fit shared memory otherwise, or where its
+// finer grid fills the SMs better (few rows in all, or few left over for the last wave).
+struct TilePlan {
+	int ti, nw, nstage; // nstage 0: no form fits
+	size_t smem;
+};
+constexpr double SHORT_CTA = 0.6;
+template <typename F> TilePlan plan_tile(int nv, long long groups, int n_tok, F smem_of)
 {
-	if (width % 32 != 0 || width > 128 || (v_width != 32 && v_width != 64 && v_width != 128))
-		return 1;
-	for (const void *p : {(const void *)q, (const void *)k, (const void *)v, (const void *)vo})
-		if (!aligned(p, 16))
-			return 1;
-	const int nwb = width / 32, nv = v_width / 16;
 	const size_t limit = 227 * 1024 - 256; // per-CTA maximum minus the static barriers
-	// (rows per half-warp, warps): 4 x 16 and 8 x 8 give 128-row CTAs, 4 x 8 a 64-row CTA for the widest rows.
-	// Sixteen warps of 128 registers measured 7 % faster than eight of 168 (four warps per scheduler hide
-	// the shared-memory and arithmetic latencies); with 128 value columns the thread state does not fit 128 registers.
 	const bool nw16 = nv <= 4;
 	const int cand[2][2] = {{nw16 ? 4 : 8, nw16 ? 16 : 8}, {4, 8}};
-	int ti = 0, nw = 0, nstage = 0;
-	for (const auto &c : cand) {
-		for (int cand_ns : {3, 2})
-			if (!ti && sv_smem(nwb, nv, 2 * c[0] * c[1], cand_ns) <= limit) {
-				ti = c[0];
-				nw = c[1];
-				nstage = cand_ns;
+	TilePlan best{0, 0, 0, 0};
+	double best_cost = 0;
+	for (const auto &c : cand)
+		for (int ns : {3, 2}) {
+			const int tt = 2 * c[0] * c[1];
+			const size_t smem = smem_of(tt, ns);
+			if (smem > limit)
+				continue;
+			const long long ctas = groups * ((n_tok + tt - 1) / tt);
+			const double cost = double((ctas + 147) / 148) * (tt == 64 ? SHORT_CTA : 1.0);
+			if (!best.nstage || cost < best_cost) {
+				best = {c[0], c[1], ns, smem};
+				best_cost = cost;
 			}
-	}
-	if (!ti)
+			break; // the deeper ring that fits
+		}
+	return best;
+}
+
+// Returns L1ATTN_OK, a negative error, or 1 when the shape is outside this kernel's set.
+int softmax_v_tile(const float *q, const float *k, const float *v, float *vo, float *lse, int bs, int n_tok, int n_heads,
+		   int width, int v_width, int mode, cudaStream_t st)
+{
+	if (width > 128 || v_width > 128)
 		return 1;
-	const size_t smem = sv_smem(nwb, nv, 2 * ti * nw, nstage);
-#define L1B_SV(NV_, TI_, NW_)                       \
-	if (nv == NV_ && ti == TI_ && nw == NW_)    \
-		return launch_tma<NV_, TI_, NW_>(q, k, v, vo, lse, bs, n_tok, n_heads, width, mode, nstage, smem, st);
-	L1B_SV(2, 8, 8) L1B_SV(4, 8, 8) L1B_SV(8, 8, 8) L1B_SV(2, 4, 8) L1B_SV(4, 4, 8) L1B_SV(8, 4, 8)
-	L1B_SV(2, 4, 16) L1B_SV(4, 4, 16) L1B_SV(8, 4, 16)
+	const bool tma = width % 4 == 0 && v_width % 4 == 0 && aligned(q, 16) && aligned(k, 16) && aligned(v, 16);
+	const int nwb = (width + 31) / 32, nv = v_width <= 32 ? 2 : v_width <= 64 ? 4 : 8;
+	const bool full = width % 32 == 0 && v_width == 16 * nv; // no padded columns
+	const TilePlan p = plan_tile(nv, (long long)bs * n_heads, n_tok, [&](int tt, int ns) { return sv_smem(nwb, nv, tt, ns); });
+	if (!p.nstage)
+		return 1;
+#define L1B_SV_RUN(NV_, TI_, NW_, TMA_, FULL_) \
+	launch_tile<NV_, TI_, NW_, TMA_, FULL_>(q, k, v, vo, lse, bs, n_tok, n_heads, width, v_width, mode, p.nstage, p.smem, st)
+#define L1B_SV(NV_, TI_, NW_)                                                                                                  \
+	if (nv == NV_ && p.ti == TI_ && p.nw == NW_) {                                                                         \
+		const int rc = !tma ? 1 : full ? L1B_SV_RUN(NV_, TI_, NW_, true, true) : L1B_SV_RUN(NV_, TI_, NW_, true, false); \
+		return rc <= 0 ? rc : L1B_SV_RUN(NV_, TI_, NW_, false, false);                                                  \
+	}
+	L1B_SV(2, 4, 8) L1B_SV(4, 4, 8) L1B_SV(8, 4, 8) L1B_SV(8, 8, 8) L1B_SV(2, 4, 16) L1B_SV(4, 4, 16)
 #undef L1B_SV
+#undef L1B_SV_RUN
 	return 1;
 }
 
@@ -509,16 +576,17 @@ int launch_bwd_generic(const T *q, const T *k, const T *v, const T *dvo, const T
 	return L1ATTN_OK;
 }
 
-// TMA variant: the forward kernel with the roles swapped.  The CTA owns TT source rows (their key and
+// Tiled variant: the forward kernel with the roles swapped.  The CTA owns TT source rows (their key and
 // value rows stay in shared memory) and streams the query and dvo rows in tiles of 64; a half-warp
 // owns TI source rows, a lane 4 query columns for the scores and the <v, dvo> products, and NV value
 // columns for dv.  Every operand row is kept as 128-byte slices with the 128-byte swizzle.
-template <int NV, int TI, int NW>
+template <int NV, int TI, int NW, bool TMA, bool FULL>
 __global__ void __launch_bounds__(NW * 32, 1)
-softmax_v_bwd_tma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
+softmax_v_bwd_tile_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
 			 const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap gmap,
-			 const float *__restrict__ lse, const float *__restrict__ delta, float *__restrict__ dx,
-			 float *__restrict__ dv, SvShape sh, int *err)
+			 const float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v,
+			 const float *__restrict__ dvo, const float *__restrict__ lse, const float *__restrict__ delta,
+			 float *__restrict__ dx, float *__restrict__ dv, SvShape sh, int *err)
 {
 	constexpr int TT = 2 * NW * TI; // source rows of the CTA
 	constexpr int NTH = NW * 32;
@@ -542,30 +610,44 @@ softmax_v_bwd_tma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 	const int nt = (sh.n_tok + TS - 1) / TS;
 
 	if (tid == 0) {
-		mbar_init(&own_bar, 1);
+		mbar_init(&own_bar, TMA ? 1 : NTH);
 		for (int s = 0; s < MAX_STAGE; s++) {
-			mbar_init(&full_bar[s], 1);
+			mbar_init(&full_bar[s], TMA ? 1 : NTH);
 			mbar_init(&empty_bar[s], NTH / 32);
 		}
 		mbar_fence_init();
 	}
 	__syncthreads();
 
+	const size_t krow = size_t(sh.n_heads) * sh.width, vrow = size_t(sh.n_heads) * sh.v_width;
+	const size_t qk0 = size_t(b) * sh.n_tok * krow + size_t(h) * sh.width, v0 = size_t(b) * sh.n_tok * vrow + size_t(h) * sh.v_width;
 	auto load_tile = [&](int m) {
 		const int st = m % sh.nstage;
 		unsigned char *dst = stages + size_t(st) * stage_bytes;
+		if (!TMA) {
+			copy_rows<NW, true>(dst, q + qk0, krow, m * TS, TS, sh.nwb, sh.width, sh.n_tok);
+			copy_rows<NW, true>(dst + q_bytes, dvo + v0, vrow, m * TS, TS, NVB, sh.v_width, sh.n_tok);
+			copy_arrive(&full_bar[st]);
+			return;
+		}
 		mbar_expect_tx(&full_bar[st], uint32_t(stage_bytes));
 		for (int wb = 0; wb < sh.nwb; wb++)
 			tma_load_4d(dst + wb * TS * 128, &qmap, &full_bar[st], wb * 32, h, m * TS, b);
 		for (int vb = 0; vb < NVB; vb++)
 			tma_load_4d(dst + q_bytes + vb * TS * 128, &gmap, &full_bar[st], vb * 32, h, m * TS, b);
 	};
-	if (tid == 0) {
-		mbar_expect_tx(&own_bar, uint32_t(k_bytes + v_bytes));
-		for (int wb = 0; wb < sh.nwb; wb++)
-			tma_load_4d(Ks + wb * TT * 128, &kmap, &own_bar, wb * 32, h, s0, b);
-		for (int vb = 0; vb < NVB; vb++)
-			tma_load_4d(Vs + vb * TT * 128, &vmap, &own_bar, vb * 32, h, s0, b);
+	if (!TMA || tid == 0) {
+		if (TMA) {
+			mbar_expect_tx(&own_bar, uint32_t(k_bytes + v_bytes));
+			for (int wb = 0; wb < sh.nwb; wb++)
+				tma_load_4d(Ks + wb * TT * 128, &kmap, &own_bar, wb * 32, h, s0, b);
+			for (int vb = 0; vb < NVB; vb++)
+				tma_load_4d(Vs + vb * TT * 128, &vmap, &own_bar, vb * 32, h, s0, b);
+		} else {
+			copy_rows<NW, true>(Ks, k + qk0, krow, s0, TT, sh.nwb, sh.width, sh.n_tok);
+			copy_rows<NW, true>(Vs, v + v0, vrow, s0, TT, NVB, sh.v_width, sh.n_tok);
+			copy_arrive(&own_bar);
+		}
 		for (int m = 0; m < sh.nstage - 1 && m < nt; m++)
 			load_tile(m);
 	}
@@ -584,7 +666,7 @@ softmax_v_bwd_tma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 	const size_t hstride = size_t(sh.n_heads);
 
 	for (int m = 0; m < nt; m++) {
-		if (warp == m % NW && lane == 0 && m + sh.nstage - 1 < nt && !dead) {
+		if ((!TMA || (warp == m % NW && lane == 0)) && m + sh.nstage - 1 < nt && !dead) {
 			const int mm = m + sh.nstage - 1;
 			if (mbar_wait(&empty_bar[mm % sh.nstage], ((unsigned(mm) / unsigned(sh.nstage)) & 1u) ^ 1u, err))
 				load_tile(mm);
@@ -619,8 +701,9 @@ softmax_v_bwd_tma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 		for (int wb = 0; wb < sh.nwb; wb++) {
 			const ulonglong2 *Kb = reinterpret_cast<const ulonglong2 *>(Ks + wb * TT * 128);
 			const ulonglong2 *Qb = reinterpret_cast<const ulonglong2 *>(Qs + wb * TS * 128);
+			const int nc = FULL ? 8 : min(8, ((sh.width - wb * 32 + 7) >> 3) * 2);
 #pragma unroll 2
-			for (int c = 0; c < 8; c++) {
+			for (int c = 0; c < nc; c++) {
 				ulonglong2 qv[4];
 #pragma unroll
 				for (int j = 0; j < 4; j++)
@@ -648,8 +731,9 @@ softmax_v_bwd_tma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 		for (int vb = 0; vb < NVB; vb++) {
 			const float4 *Vb = reinterpret_cast<const float4 *>(Vs + vb * TT * 128);
 			const float4 *Gb = reinterpret_cast<const float4 *>(Gs + vb * TS * 128);
+			const int nc = FULL ? 8 : min(8, ((sh.v_width - vb * 32 + 7) >> 3) * 2);
 #pragma unroll 2
-			for (int c = 0; c < 8; c++) {
+			for (int c = 0; c < nc; c++) {
 				float4 gv[4];
 #pragma unroll
 				for (int j = 0; j < 4; j++)
@@ -725,16 +809,16 @@ softmax_v_bwd_tma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_
 			mbar_arrive(&empty_bar[st]);
 	}
 
-	const size_t vrow = size_t(sh.n_heads) * VW;
 #pragma unroll
 	for (int i = 0; i < TI; i++) {
 		const int s = s0 + i * (2 * NW) + tg;
 		if (s >= sh.n_tok)
 			continue;
-		float *op = dv + (size_t(b) * sh.n_tok + s) * vrow + size_t(h) * VW + sg * NV;
+		float *op = dv + v0 + size_t(s) * vrow + sg * NV;
 #pragma unroll
 		for (int e = 0; e < NV; e++)
-			op[e] = o[i][e];
+			if (FULL || sg * NV + e < sh.v_width)
+				op[e] = o[i][e];
 	}
 }
 
@@ -744,21 +828,21 @@ size_t sv_bwd_smem(int nwb, int nv, int tt_rows, int nstage)
 	return (size_t(nwb) + nvb) * tt * 128 + size_t(nstage) * (size_t(nwb) + nvb) * TS * 128 + tt * PP * 4 + 1024;
 }
 
-template <int NV, int TI, int NW>
-int launch_bwd_tma(const float *q, const float *k, const float *v, const float *dvo, const float *lse, const float *delta,
-		   float *dx, float *dv, int bs, int n_tok, int n_heads, int width, int nstage, size_t smem, cudaStream_t st)
+template <int NV, int TI, int NW, bool TMA, bool FULL>
+int launch_bwd_tile(const float *q, const float *k, const float *v, const float *dvo, const float *lse, const float *delta,
+		    float *dx, float *dv, int bs, int n_tok, int n_heads, int width, int v_width, int nstage, size_t smem, cudaStream_t st)
 {
-	constexpr int TT = 2 * NW * TI, VW = 16 * NV, NTH = NW * 32;
+	constexpr int TT = 2 * NW * TI, NTH = NW * 32;
 	const uint64_t dims[4] = {uint64_t(width), uint64_t(n_heads), uint64_t(n_tok), uint64_t(bs)};
 	const uint64_t str[3] = {uint64_t(width) * 4, uint64_t(n_heads) * width * 4, uint64_t(n_tok) * n_heads * width * 4};
-	const uint64_t vdims[4] = {uint64_t(VW), uint64_t(n_heads), uint64_t(n_tok), uint64_t(bs)};
-	const uint64_t vstr[3] = {uint64_t(VW) * 4, uint64_t(n_heads) * VW * 4, uint64_t(n_tok) * n_heads * VW * 4};
+	const uint64_t vdims[4] = {uint64_t(v_width), uint64_t(n_heads), uint64_t(n_tok), uint64_t(bs)};
+	const uint64_t vstr[3] = {uint64_t(v_width) * 4, uint64_t(n_heads) * v_width * 4, uint64_t(n_tok) * n_heads * v_width * 4};
 	const uint32_t own[4] = {32, 1, TT, 1}, stream[4] = {32, 1, TS, 1};
-	CUtensorMap qmap, kmap, vmap, gmap;
+	CUtensorMap qmap{}, kmap{}, vmap{}, gmap{};
 	const auto f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
 	const auto swz = CU_TENSOR_MAP_SWIZZLE_128B;
-	if (!encode_tmap_4d(&qmap, f32, q, dims, str, stream, swz) || !encode_tmap_4d(&kmap, f32, k, dims, str, own, swz) ||
-	    !encode_tmap_4d(&vmap, f32, v, vdims, vstr, own, swz) || !encode_tmap_4d(&gmap, f32, dvo, vdims, vstr, stream, swz))
+	if (TMA && (!encode_tmap_4d(&qmap, f32, q, dims, str, stream, swz) || !encode_tmap_4d(&kmap, f32, k, dims, str, own, swz) ||
+	    !encode_tmap_4d(&vmap, f32, v, vdims, vstr, own, swz) || !encode_tmap_4d(&gmap, f32, dvo, vdims, vstr, stream, swz)))
 		return 1;
 	int *err = device_error_word();
 	if (!err)
@@ -766,7 +850,9 @@ int launch_bwd_tma(const float *q, const float *k, const float *v, const float *
 	SvShape sh;
 	sh.n_tok = n_tok;
 	sh.n_heads = n_heads;
-	sh.nwb = width / 32;
+	sh.width = width;
+	sh.v_width = v_width;
+	sh.nwb = (width + 31) / 32;
 	sh.nstage = nstage;
 	sh.ntt = (n_tok + TT - 1) / TT;
 	sh.mode = 0;
@@ -774,43 +860,34 @@ int launch_bwd_tma(const float *q, const float *k, const float *v, const float *
 	const long long grid = (long long)bs * n_heads * sh.ntt;
 	if (grid > 0x7fffffffLL)
 		return L1ATTN_ERR_SHAPE;
-	auto kern = softmax_v_bwd_tma_kernel<NV, TI, NW>;
+	auto kern = softmax_v_bwd_tile_kernel<NV, TI, NW, TMA, FULL>;
 	L1B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-	kern<<<unsigned(grid), NTH, smem, st>>>(qmap, kmap, vmap, gmap, lse, delta, dx, dv, sh, err);
+	kern<<<unsigned(grid), NTH, smem, st>>>(qmap, kmap, vmap, gmap, q, k, v, dvo, lse, delta, dx, dv, sh, err);
 	L1B_LAUNCH_CHECK();
 	return L1ATTN_OK;
 }
 
-int softmax_v_bwd_tma(const float *q, const float *k, const float *v, const float *dvo, const float *lse, const float *delta,
-		      float *dx, float *dv, int bs, int n_tok, int n_heads, int width, int v_width, cudaStream_t st)
+int softmax_v_bwd_tile(const float *q, const float *k, const float *v, const float *dvo, const float *lse, const float *delta,
+		       float *dx, float *dv, int bs, int n_tok, int n_heads, int width, int v_width, cudaStream_t st)
 {
-	if (width % 32 != 0 || width > 128 || (v_width != 32 && v_width != 64 && v_width != 128))
+	if (width > 128 || v_width > 128)
 		return 1;
-	for (const void *p : {(const void *)q, (const void *)k, (const void *)v, (const void *)dvo})
-		if (!aligned(p, 16))
-			return 1;
-	const int nwb = width / 32, nv = v_width / 16;
-	const size_t limit = 227 * 1024 - 256;
-	const bool nw16 = nv <= 4; // see softmax_v_tma
-	const int cand[2][2] = {{nw16 ? 4 : 8, nw16 ? 16 : 8}, {4, 8}};
-	int ti = 0, nw = 0, nstage = 0;
-	for (const auto &c : cand) {
-		for (int cand_ns : {3, 2})
-			if (!ti && sv_bwd_smem(nwb, nv, 2 * c[0] * c[1], cand_ns) <= limit) {
-				ti = c[0];
-				nw = c[1];
-				nstage = cand_ns;
-			}
+	const bool tma = width % 4 == 0 && v_width % 4 == 0 && aligned(q, 16) && aligned(k, 16) && aligned(v, 16) && aligned(dvo, 16);
+	const int nwb = (width + 31) / 32, nv = v_width <= 32 ? 2 : v_width <= 64 ? 4 : 8;
+	const bool full = width % 32 == 0 && v_width == 16 * nv; // no padded columns
+	const TilePlan p = plan_tile(nv, (long long)bs * n_heads, n_tok, [&](int tt, int ns) { return sv_bwd_smem(nwb, nv, tt, ns); });
+	if (!p.nstage)
+		return 1;
+#define L1B_SVB_RUN(NV_, TI_, NW_, TMA_, FULL_) \
+	launch_bwd_tile<NV_, TI_, NW_, TMA_, FULL_>(q, k, v, dvo, lse, delta, dx, dv, bs, n_tok, n_heads, width, v_width, p.nstage, p.smem, st)
+#define L1B_SVB(NV_, TI_, NW_)                                                                                                   \
+	if (nv == NV_ && p.ti == TI_ && p.nw == NW_) {                                                                           \
+		const int rc = !tma ? 1 : full ? L1B_SVB_RUN(NV_, TI_, NW_, true, true) : L1B_SVB_RUN(NV_, TI_, NW_, true, false); \
+		return rc <= 0 ? rc : L1B_SVB_RUN(NV_, TI_, NW_, false, false);                                                   \
 	}
-	if (!ti)
-		return 1;
-	const size_t smem = sv_bwd_smem(nwb, nv, 2 * ti * nw, nstage);
-#define L1B_SVB(NV_, TI_, NW_)                      \
-	if (nv == NV_ && ti == TI_ && nw == NW_)    \
-		return launch_bwd_tma<NV_, TI_, NW_>(q, k, v, dvo, lse, delta, dx, dv, bs, n_tok, n_heads, width, nstage, smem, st);
-	L1B_SVB(2, 8, 8) L1B_SVB(4, 8, 8) L1B_SVB(8, 8, 8) L1B_SVB(2, 4, 8) L1B_SVB(4, 4, 8) L1B_SVB(8, 4, 8)
-	L1B_SVB(2, 4, 16) L1B_SVB(4, 4, 16) L1B_SVB(8, 4, 16)
+	L1B_SVB(2, 4, 8) L1B_SVB(4, 4, 8) L1B_SVB(8, 4, 8) L1B_SVB(8, 8, 8) L1B_SVB(2, 4, 16) L1B_SVB(4, 4, 16)
 #undef L1B_SVB
+#undef L1B_SVB_RUN
 	return 1;
 }
 
@@ -823,7 +900,7 @@ int dense_softmax_v_launch(const void *q, const void *k, const void *v, void *vo
 		return L1ATTN_OK;
 	static const bool no_tma = getenv("L1ATTN_NO_TMA") != nullptr; // debugging aid: force the generic kernel
 	if (dtype == L1ATTN_F32 && !no_tma && width > 0) {
-		const int rc = softmax_v_tma((const float *)q, (const float *)k, (const float *)v, (float *)vo, (float *)lse, bs, n_tok,
+		const int rc = softmax_v_tile((const float *)q, (const float *)k, (const float *)v, (float *)vo, (float *)lse, bs, n_tok,
 					     n_heads, width, v_width, mode, st);
 		if (rc <= 0)
 			return rc;
@@ -843,7 +920,7 @@ int dense_softmax_v_bwd_dx_launch(const void *q, const void *k, const void *v, c
 		return L1ATTN_OK;
 	static const bool no_tma = getenv("L1ATTN_NO_TMA") != nullptr;
 	if (dtype == L1ATTN_F32 && !no_tma && width > 0) {
-		const int rc = softmax_v_bwd_tma((const float *)q, (const float *)k, (const float *)v, (const float *)dvo,
+		const int rc = softmax_v_bwd_tile((const float *)q, (const float *)k, (const float *)v, (const float *)dvo,
 						 (const float *)lse, (const float *)delta, (float *)dx, (float *)dv, bs, n_tok, n_heads,
 						 width, v_width, st);
 		if (rc <= 0)

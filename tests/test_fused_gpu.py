@@ -13,10 +13,13 @@ pytestmark = pytest.mark.gpu
 TOL = {np.float32: 1e-5, np.float64: 1e-12}
 MODES = ["softmax", "softmax_plus_one", "exp"]
 
-# (bs, n, h, w, wv); the fp32 cases with w in {32, 64, 96, 128} and wv in {32, 64, 128} take the TMA kernel,
-# the others (and all fp64 cases) the generic one
+# (bs, n, h, w, wv); the fp32 cases with widths up to 128 take the tiled kernels (RAGGED: rows that end inside a slice of 32
+# columns, filled by TMA and by element-wise copies, value rows of every padding), the others (and all fp64 cases) the generic ones
 SHAPES = [(1, 1, 1, 1, 1), (2, 3, 4, 8, 8), (1, 9, 2, 7, 5), (2, 70, 3, 32, 32), (1, 130, 2, 64, 64),
           (1, 200, 2, 128, 128), (1, 64, 4, 96, 64), (2, 129, 2, 64, 128), (1, 257, 1, 32, 64), (1, 40, 3, 64, 48)]
+
+RAGGED = [(2, 70, 3, 40, 24), (1, 130, 2, 33, 21), (1, 100, 2, 48, 40), (1, 200, 5, 100, 7), (1, 65, 1, 127, 128), (2, 66, 2, 64, 100),
+          (1, 64, 3, 1, 64), (1, 33, 2, 129, 64)]
 
 
 def _cabi():
@@ -38,7 +41,7 @@ def _dev(a):
 
 @pytest.mark.parametrize("mode", MODES)
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
-@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("shape", SHAPES + RAGGED)
 def test_fwd_vs_oracle(shape, dtype, mode):
     from oracle import oracle
     q, k, v = _rand(shape, dtype, sum(shape), spread=0.3)  # scores of order -1: weights of order 1/n
@@ -92,7 +95,7 @@ def test_host_entry_point():
 @pytest.mark.parametrize("mode", MODES)
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
 @pytest.mark.parametrize("dims", [(2, 37, 3, 32, 32), (1, 150, 2, 64, 64), (1, 70, 2, 128, 128), (2, 66, 1, 64, 128),
-                                  (1, 20, 2, 7, 5)])
+                                  (1, 20, 2, 7, 5)] + RAGGED[:7])
 def test_autograd_matches_the_unfused_chain(mode, dtype, dims):
     """Gradients of the fused module against torch autograd through the chain the reference's callers
     write (README.md:64-66), built here on pure-PyTorch scores."""
