@@ -142,45 +142,11 @@ template <int VEC, bool EX> __device__ __forceinline__ bool in_row(int li, int i
 	return EX || li * VEC + it * step < width;
 }
 
-// Edge-outer walk for rows of at most NX vectors per lane (NX > 0, compile time): every
-// list entry (a slot of the destination or an incoming edge of the source) is decoded ONCE -- index,
-// weight, row address -- and its NX vectors are fetched at immediate offsets, instead of walking the whole
-// list once per vector (which repeated the decoding, and in the source lists an integer division, NX times).
-//   acc += weight * row
-// entry(i, ptr, weight) fills the row pointer of entry i (already at this lane's first vector; any valid
-// address when the entry is absent: the row is then loaded but not used, which is cheaper than a
-// predicated load plus zero fill) and its weight, and returns whether the entry exists.
-constexpr int UE = 2; // entries in flight per lane: UE * NX 16-byte loads
-template <typename S, typename T, int VEC, int NX, bool EX, typename F>
-__device__ __forceinline__ void walk_list(Pack<T, VEC> (&acc)[NX], int n, int li, int step, int width, F entry)
-{
-	for (int e0 = 0; e0 < n; e0 += UE) {
-		T wgt[UE];
-		const S *ptr[UE];
-		bool ok[UE];
-#pragma unroll
-		for (int u = 0; u < UE; u++) {
-			wgt[u] = T(0);
-			ok[u] = entry(e0 + u < n ? e0 + u : e0, ptr[u], wgt[u]) && e0 + u < n;
-			if (!ok[u])
-				wgt[u] = T(0);
-		}
-		Pack<T, VEC> row[UE][NX];
-#pragma unroll
-		for (int u = 0; u < UE; u++)
-#pragma unroll
-			for (int it = 0; it < NX; it++)
-				row[u][it] = ldc<S, T, VEC>(ptr[u] + it * step, in_row<VEC, EX>(li, it, step, width));
-#pragma unroll
-		for (int u = 0; u < UE; u++)
-			if (ok[u])
-#pragma unroll
-			for (int it = 0; it < NX; it++)
-#pragma unroll
-				for (int i = 0; i < VEC; i++)
-					acc[it].v[i] += wgt[u] * row[u][it].v[i];
-	}
-}
+// Walks with NX > 0 go over a list ONCE: every entry (a slot of the destination or an incoming edge of the source) is decoded
+// once -- index, weight, row addresses -- and its vectors are fetched at immediate offsets.  The entries' indices are
+// loaded by the lanes of the warp together and handed out by shuffles, 32 at a time (as many as lanes are left): with one
+// load per entry the row fetches of every entry waited for an index first, and the lists of incoming edges cost an
+// integer division per entry instead of one per lane.
 template <typename T, int VEC, int NX> __device__ __forceinline__ void zero_acc(Pack<T, VEC> (&acc)[NX])
 {
 #pragma unroll
@@ -202,7 +168,7 @@ __global__ void __launch_bounds__(CTA) sparse_fwd_dst_kernel(SparseArgs a, const
 	Who w;
 	if (!decode<LPHC>(a, w))
 		return;
-	const int dst = w.tok, H = a.n_heads, W = a.width, Wv = a.v_width, dm = a.dm;
+	const int dst = w.tok, H = a.n_heads, W = a.width, Wv = a.v_width, dm = a.dm, lane = threadIdx.x & 31;
 	const int hh = w.head_ok ? w.h : 0;
 	const size_t tokrow = size_t(w.b) * a.n_tok;
 	const S *qrow = q + ((tokrow + dst) * H + hh) * W;
@@ -220,12 +186,15 @@ __global__ void __launch_bounds__(CTA) sparse_fwd_dst_kernel(SparseArgs a, const
 		zero_acc(acc);
 		const S *kbase = k + (tokrow * H + hh) * W + w.li * VEC, *vbase = v + (tokrow * H + hh) * Wv + w.li * VEC;
 		T denom = T(1);
+		int mine = -1; // slot (r0 & ~31) + lane of the list
 		for (int r0 = 0; r0 < dm; r0 += FU) {
+			if (r0 % 32 == 0)
+				mine = r0 + lane < dm ? slots[r0 + lane] : -1;
 			int src[FU];
 			Pack<T, VEC> kr[FU][NX], vr[FU][NX];
 #pragma unroll
 			for (int u = 0; u < FU; u++) {
-				src[u] = r0 + u < dm ? slots[r0 + u] : -1;
+				src[u] = __shfl_sync(0xffffffffu, mine, (r0 + u) & 31);
 				// rows of absent slots / heads past the end are read from a valid address and not used
 				const size_t so = size_t(src[u] < 0 ? 0 : src[u]) * H;
 #pragma unroll
@@ -348,8 +317,10 @@ __global__ void __launch_bounds__(CTA) sparse_fwd_src_kernel(SparseArgs a, const
 	Who w;
 	if (!decode<LPHC>(a, w))
 		return;
+	const unsigned act = __ballot_sync(0xffffffffu, w.head_ok); // the first nact lanes (a multiple of four, or all)
 	if (!w.head_ok)
 		return;
+	const int lane = threadIdx.x & 31, nact = __popc(act);
 	const int src = w.tok, H = a.n_heads, Wv = a.v_width, dm = a.dm;
 	const size_t tokrow = size_t(w.b) * a.n_tok;
 	const int e0 = a.csc_off[src], e1 = a.csc_off[src + 1];
@@ -359,14 +330,37 @@ __global__ void __launch_bounds__(CTA) sparse_fwd_src_kernel(SparseArgs a, const
 	if constexpr (NX > 0) {
 		Pack<T, VEC> acc[NX];
 		zero_acc(acc);
+		constexpr int UE = 2; // entries in flight per lane
 		const S *bbase = vb + (tokrow * H + w.h) * Wv + w.li * VEC;
 		const S *abase = attn + (tokrow * dm) * H + w.h;
-		walk_list<S, T, VEC, NX, EX>(acc, e1 - e0, w.li, step, Wv, [&](int e, const S *&ptr, T &wgt) {
-			const int slot = a.csc_slot[e0 + e];
-			ptr = bbase + size_t(slot / dm) * H * Wv;
-			wgt = ld1<S, T>(abase + size_t(slot) * H);
-			return true;
-		});
+		int slot_l = 0, dst_l = 0;
+		for (int e = e0, i = 0; e < e1; e += UE, i += UE) {
+			if (i == nact)
+				i = 0;
+			if (i == 0) {
+				slot_l = e + lane < e1 ? a.csc_slot[e + lane] : 0;
+				dst_l = slot_l / dm;
+			}
+			T ar[UE];
+			Pack<T, VEC> row[UE][NX];
+#pragma unroll
+			for (int u = 0; u < UE; u++) { // past the end of the list: slot 0, read but not used
+				const int slot = __shfl_sync(act, slot_l, i + u);
+				const size_t d = size_t(__shfl_sync(act, dst_l, i + u)) * H;
+				ar[u] = ld1<S, T>(abase + size_t(slot) * H);
+#pragma unroll
+				for (int it = 0; it < NX; it++)
+					row[u][it] = ldc<S, T, VEC>(bbase + d * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
+			}
+#pragma unroll
+			for (int u = 0; u < UE; u++)
+				if (e + u < e1)
+#pragma unroll
+					for (int it = 0; it < NX; it++)
+#pragma unroll
+						for (int j = 0; j < VEC; j++)
+							acc[it].v[j] += ar[u] * row[u][it].v[j];
+		}
 #pragma unroll
 		for (int it = 0; it < NX; it++) {
 			if (!in_row<VEC, EX>(w.li, it, step, Wv))
@@ -423,7 +417,7 @@ __global__ void __launch_bounds__(CTA, (NX == 4 ? 4 : 6) - (BIDI && NX > 0 ? 1 :
 	Who w;
 	if (!decode<LPHC>(a, w))
 		return;
-	const int dst = w.tok, H = a.n_heads, W = a.width, Wv = a.v_width, dm = a.dm;
+	const int dst = w.tok, H = a.n_heads, W = a.width, Wv = a.v_width, dm = a.dm, lane = threadIdx.x & 31;
 	const int hh = w.head_ok ? w.h : 0;
 	const size_t tokrow = size_t(w.b) * a.n_tok;
 	const size_t aoff = ((tokrow + dst) * dm) * H + hh;
@@ -455,8 +449,11 @@ __global__ void __launch_bounds__(CTA, (NX == 4 ? 4 : 6) - (BIDI && NX > 0 ? 1 :
 		const T *vbase = v + (tokrow * H + hh) * Wv + w.li * VEC, *kbase = k + (tokrow * H + hh) * W + w.li * VEC;
 		const T *gbase = dvo + (tokrow * H + hh) * Wv + w.li * VEC;
 		T S = T(0);
+		int mine = -1; // slot (r & ~31) + lane of the list
 		for (int r = 0; r < dm; r++) {
-			const int src = slots[r];
+			if (r % 32 == 0)
+				mine = r + lane < dm ? slots[r + lane] : -1;
+			const int src = __shfl_sync(0xffffffffu, mine, r & 31);
 			const bool ok = w.head_ok && src >= 0;
 			const size_t so = size_t(ok ? src : 0) * H;
 			Pack<T, VEC> vr[NX], kr[NX], gr[NX];
@@ -656,8 +653,10 @@ __global__ void __launch_bounds__(CTA, NX == 4 ? 4 : 6) sparse_bwd_src_kernel(Sp
 	Who w;
 	if (!decode<LPHC>(a, w))
 		return;
+	const unsigned act = __ballot_sync(0xffffffffu, w.head_ok); // the first nact lanes (a multiple of four, or all)
 	if (!w.head_ok)
 		return;
+	const int lane = threadIdx.x & 31, nact = __popc(act);
 	const int src = w.tok, H = a.n_heads, W = a.width, Wv = a.v_width, dm = a.dm;
 	const size_t tokrow = size_t(w.b) * a.n_tok;
 	const int e0 = a.csc_off[src], e1 = a.csc_off[src + 1];
@@ -675,9 +674,16 @@ __global__ void __launch_bounds__(CTA, NX == 4 ? 4 : 6) sparse_bwd_src_kernel(Sp
 			kv[it] = ldv<T, VEC>(krow + it * step, in_row<VEC, EX>(w.li, it, step, W));
 		const T *gbase = dvo + (tokrow * H + w.h) * Wv + w.li * VEC, *qbase = q + (tokrow * H + w.h) * W + w.li * VEC;
 		const T *abase = attn + (tokrow * dm) * H + w.h, *xbase = dx + (tokrow * dm) * H + w.h;
-		for (int e = e0; e < e1; e++) {
-			const int slot = a.csc_slot[e];
-			const size_t d = size_t(slot / dm) * H;
+		int slot_l = 0, dst_l = 0;
+		for (int e = e0, i = 0; e < e1; e++, i++) {
+			if (i == nact)
+				i = 0;
+			if (i == 0) {
+				slot_l = e + lane < e1 ? a.csc_slot[e + lane] : 0;
+				dst_l = slot_l / dm;
+			}
+			const int slot = __shfl_sync(act, slot_l, i);
+			const size_t d = size_t(__shfl_sync(act, dst_l, i)) * H;
 			Pack<T, VEC> gr[NX], qr[NX];
 #pragma unroll
 			for (int it = 0; it < NX; it++) {
@@ -772,7 +778,8 @@ int pow2_ceil(int x)
 // unrolled four-vector walk wins although half its lanes idle), 2 heads 0.073 / 0.104 -- so the forward asks
 // with idle_den 2 and the backward with 4.  Rows that are not whole lanes of vectors used to take the generic walk, once
 // per vector and quantity; forward + backward, start and now: 256 tokens, 17 edges each, 64 items of 8 x 32 columns,
-// bidirectional 629 / 259 us; 3001 tokens, 75000 edges, 2 items of 6 x 40 columns (values 24) 578 / 346 us.
+// bidirectional 629 / 259 us; 3001 tokens, 75000 edges, 2 items of 6 x 40 columns (values 24), a new list in
+// every pass (its index included) 718 / 502 us.
 struct RowPlan {
 	int lph, nx;
 	bool exact; // width == v_width == nx * lph vectors: no vector of any lane lies past the end of a row
