@@ -75,6 +75,11 @@ int l1attn_device_status(void);
  * No counterpart in the reference, whose kernels have no waits and whose launchers check no errors.
  */
 int l1attn_device_status_async(int *host_word, void *stream);
+
+/* The current device's word in pinned host memory that a kernel of this library sets to 1 when it gives up a bounded wait: nothing
+ * to enqueue, the caller looks at it when it likes and clears it (l1attn_device_status() clears the device's word).  NULL
+ * when it cannot be set up at that moment; every later call may try again. */
+int *l1attn_device_status_word(void);
 /*
  * Test hook, not an operator: launches one warp that waits at most limit_us (1..100000) microseconds on a
  * barrier nothing completes.  The wait gives up, l1attn_device_status() then reports L1ATTN_ERR_TIMEOUT once

@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
+#include <mutex>
 #include "l1attn_b200.h"
 
 namespace l1b {
@@ -18,6 +20,40 @@ int cuda_fail(cudaError_t e);
 
 // After a kernel launch: pick up configuration errors without synchronising.
 #define L1B_LAUNCH_CHECK() L1B_CUDA(cudaGetLastError())
+
+// Lets `kern` be launched with `bytes` of dynamic shared memory on the current device.  The runtime call costs about a
+// microsecond and a dense backward launches up to five kernels, so every place that launches one remembers, per
+// device, the most it has asked for (the attribute only ever grows: any smaller launch is allowed by it too).
+struct SharedMemoryLimit {
+	static constexpr int MAX_DEVICES = 64;
+	std::atomic<int> granted[MAX_DEVICES] = {};
+	std::mutex mu;
+	int ask(const void *kern, int bytes)
+	{
+		int dev = 0;
+		L1B_CUDA(cudaGetDevice(&dev));
+		if (dev >= 0 && dev < MAX_DEVICES && granted[dev].load(std::memory_order_acquire) >= bytes)
+			return L1ATTN_OK;
+		std::lock_guard<std::mutex> lock(mu);
+		if (dev >= 0 && dev < MAX_DEVICES && granted[dev].load(std::memory_order_relaxed) >= bytes)
+			return L1ATTN_OK;
+		L1B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+		if (dev >= 0 && dev < MAX_DEVICES)
+			granted[dev].store(bytes, std::memory_order_release);
+		return L1ATTN_OK;
+	}
+};
+// (one instance per kernel: a launcher template launches one kernel per instantiation)
+#define L1B_SHARED_MEMORY(kern, bytes)                                                          \
+	do {                                                                                    \
+		static ::l1b::SharedMemoryLimit limit__;                                        \
+		const int rc__ = limit__.ask(reinterpret_cast<const void *>(kern), int(bytes)); \
+		if (rc__)                                                                       \
+			return rc__;                                                            \
+	} while (0)
+
+// Multiprocessors of the current device (asked for once per device).
+int multiprocessors(int *out);
 
 inline bool aligned(const void *p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 

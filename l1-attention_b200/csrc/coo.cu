@@ -322,7 +322,7 @@ int launch_rank(const K *keys, int stride, int n, long long key_lo, long long n_
 		const int fit = int(RANK_SMEM / (n_keys * 4)) - 1, nwarp = fit < RANK_THREADS / 32 ? fit : RANK_THREADS / 32;
 		const size_t smem = size_t(nwarp + 1) * n_keys * 4;
 		auto kern = rank_cluster_kernel<K>;
-		L1B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+		L1B_SHARED_MEMORY(kern, int(smem));
 		kern<<<ncol * RC, RANK_THREADS, smem, st>>>(keys, stride, n, key_lo, int(n_keys), rank_out, rstride, counts, max_out,
 							    col_step, nwarp, key_out);
 		L1B_LAUNCH_CHECK();
@@ -334,7 +334,7 @@ int launch_rank(const K *keys, int stride, int n, long long key_lo, long long n_
 	auto kern = rank_by_key_kernel<K>;
 	size_t smem = use_smem ? size_t(n_keys) * 4 : 0;
 	if (smem > 48 * 1024)
-		L1B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+		L1B_SHARED_MEMORY(kern, int(smem));
 	if (!use_smem)
 		L1B_CUDA(cudaMemsetAsync(counts, 0, size_t(ncol) * n_keys * 4, st));
 	kern<<<ncol, 32, smem, st>>>(keys, stride, n, key_lo, n_keys, rank_out, rstride, counts, max_out, col_step,

@@ -416,11 +416,11 @@ int dense_bwd_sv_launch(const void *d_attn, const void *q, const void *k, void *
 		return 1;
 	wk.total = unsigned(total);
 	wk.nt = ((n_tok + SV_TY - 1) / SV_TY + ns - 1) / ns; // per item; the last range may reach past the end (zero-filled loads, no stores)
-	int dev = 0, sms = 0;
-	L1B_CUDA(cudaGetDevice(&dev));
-	L1B_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+	int sms = 0;
+	if (const int rc = multiprocessors(&sms))
+		return rc;
 	const unsigned grid = wk.total < unsigned(sms) ? wk.total : unsigned(sms);
-	L1B_CUDA(cudaFuncSetAttribute(dense_bwd_sv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SV_SMEM)));
+	L1B_SHARED_MEMORY(dense_bwd_sv_kernel, int(SV_SMEM));
 	const float scale = float(-1.0 / sqrt(double(width)));
 	const size_t n4 = size_t(bs) * n_tok * n_heads * width / 4;
 	dense_bwd_sv_kernel<<<grid, SV_THREADS, SV_SMEM, st>>>(kmap, gmap, (const float *)q, ns > 1 ? (float *)dq_part : (float *)d_q,

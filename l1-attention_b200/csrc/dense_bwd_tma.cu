@@ -351,12 +351,12 @@ int dense_bwd_tma_launch(const void *d_attn, const void *q, const void *k, void 
 	wk.per_pass = unsigned(per_pass);
 	wk.total = unsigned(2 * per_pass);
 	wk.ny = (n_tok + TY - 1) / TY;
-	int dev = 0, sms = 0;
-	L1B_CUDA(cudaGetDevice(&dev));
-	L1B_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+	int sms = 0;
+	if (const int rc = multiprocessors(&sms))
+		return rc;
 	const unsigned grid = wk.total < unsigned(sms) ? wk.total : unsigned(sms);
 	const size_t smem = size_t(NSTAGE) * STAGE_BYTES + 1024;
-	L1B_CUDA(cudaFuncSetAttribute(dense_bwd_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+	L1B_SHARED_MEMORY(dense_bwd_tma_kernel, int(smem));
 	const float scale = float(-1.0 / sqrt(double(width)));
 	const BwdFlagLayout fl = bwd_flag_layout(bs, n_tok, n_heads, width);
 	dense_bwd_tma_kernel<<<grid, NTHREADS, smem, st>>>(qmap, kmap, gmap0, gmap1, (const float *)q, (const float *)k,

@@ -142,7 +142,7 @@ int launch(const T *q, const T *k, T *attn, int bs, int n_tok, int n_heads, int 
 		return L1ATTN_ERR_SHAPE;
 	const size_t smem = 2 * size_t(TT + TS) * HG * CH * 16;
 	auto kern = dense_fwd_kernel<T, TM, TN, NWARP>;
-	L1B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+	L1B_SHARED_MEMORY(kern, int(smem));
 	const int vec_ok = (width % VEC == 0) && aligned(q, 16) && aligned(k, 16);
 	const T scale = T(-1.0 / sqrt(double(width)));
 	kern<<<unsigned(nblk), NWARP * 32, smem, st>>>(q, k, attn, n_tok, n_heads, width, scale, vec_ok, ntt, nst, nhg);

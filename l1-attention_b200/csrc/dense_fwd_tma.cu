@@ -259,13 +259,13 @@ int launch(const T *q, const T *k, T *attn, int bs, int n_tok, int n_heads, int 
 	if (total > 0x7fffffffLL)
 		return L1ATTN_ERR_SHAPE;
 	wk.total = unsigned(total);
-	int dev = 0, sms = 0;
-	L1B_CUDA(cudaGetDevice(&dev));
-	L1B_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+	int sms = 0;
+	if (const int rc = multiprocessors(&sms))
+		return rc;
 	const unsigned grid = wk.total < unsigned(sms) ? wk.total : unsigned(sms);
 	const size_t smem = size_t(NSTAGE) * STAGE_BYTES + OUT_BYTES + 1024;
 	auto kern = dense_fwd_tma_kernel<T, HG>;
-	L1B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+	L1B_SHARED_MEMORY(kern, int(smem));
 	const T scale = T(-1.0 / sqrt(double(width)));
 	kern<<<unsigned(grid), NTHREADS, smem, st>>>(qmap, kmap, omap, tma_store, attn, n_tok, n_heads, width, scale, wk, err);
 	L1B_LAUNCH_CHECK();

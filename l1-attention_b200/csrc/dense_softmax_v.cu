@@ -114,7 +114,7 @@ int launch_generic(const T *q, const T *k, const T *v, T *vo, T *lse, int bs, in
 	if (grid > 0x7fffffffLL || smem > 200 * 1024)
 		return L1ATTN_ERR_SHAPE;
 	auto kern = softmax_v_kernel<T>;
-	L1B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+	L1B_SHARED_MEMORY(kern, int(smem));
 	kern<<<unsigned(grid), GEN_NT, smem, st>>>(q, k, v, vo, lse, n_tok, n_heads, width, v_width,
 						    T(-1.0 / sqrt(double(width))), mode);
 	L1B_LAUNCH_CHECK();
@@ -430,7 +430,7 @@ int launch_tile(const float *q, const float *k, const float *v, float *vo, float
 	if (grid > 0x7fffffffLL)
 		return L1ATTN_ERR_SHAPE;
 	auto kern = softmax_v_tile_kernel<NV, TI, NW, TMA, FULL>;
-	L1B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+	L1B_SHARED_MEMORY(kern, int(smem));
 	kern<<<unsigned(grid), NTH, smem, st>>>(qmap, kmap, vmap, q, k, v, vo, lse, sh, err);
 	L1B_LAUNCH_CHECK();
 	return L1ATTN_OK;
@@ -569,7 +569,7 @@ int launch_bwd_generic(const T *q, const T *k, const T *v, const T *dvo, const T
 	if (grid > 0x7fffffffLL || smem > 200 * 1024)
 		return L1ATTN_ERR_SHAPE;
 	auto kern = softmax_v_bwd_kernel<T>;
-	L1B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+	L1B_SHARED_MEMORY(kern, int(smem));
 	kern<<<unsigned(grid), GEN_NT, smem, st>>>(q, k, v, dvo, lse, delta, dx, dv, n_tok, n_heads, width, v_width,
 						    T(-1.0 / sqrt(double(width))));
 	L1B_LAUNCH_CHECK();
@@ -861,7 +861,7 @@ int launch_bwd_tile(const float *q, const float *k, const float *v, const float 
 	if (grid > 0x7fffffffLL)
 		return L1ATTN_ERR_SHAPE;
 	auto kern = softmax_v_bwd_tile_kernel<NV, TI, NW, TMA, FULL>;
-	L1B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+	L1B_SHARED_MEMORY(kern, int(smem));
 	kern<<<unsigned(grid), NTH, smem, st>>>(qmap, kmap, vmap, gmap, q, k, v, dvo, lse, delta, dx, dv, sh, err);
 	L1B_LAUNCH_CHECK();
 	return L1ATTN_OK;

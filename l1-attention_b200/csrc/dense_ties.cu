@@ -212,7 +212,7 @@ int launch_nc(const float *q, const float *k, unsigned char *flags, int bs, int 
 	if (grid > 0x7fffffffLL)
 		return 1;
 	const size_t smem = size_t(NC) * (size_t(1) << log2bits) / 8;
-	L1B_CUDA(cudaFuncSetAttribute(dense_ties_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+	L1B_SHARED_MEMORY(dense_ties_kernel<NC>, int(smem));
 	int nt = 256;
 	while (nt < NT_MAX && nt * TB < n_tok)
 		nt *= 2;
@@ -328,7 +328,7 @@ int dense_tiefix_launch(const void *d_attn, void *d_q, void *d_k, const unsigned
 {
 	const BwdScratchLayout sl = bwd_scratch_layout(bs, n_tok, n_heads, width);
 	const size_t smem = size_t(BWD_TIE_CAP) * (16 + 8);
-	L1B_CUDA(cudaFuncSetAttribute(dense_tiefix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+	L1B_SHARED_MEMORY(dense_tiefix_kernel, int(smem));
 	dense_tiefix_kernel<<<1, 1024, smem, st>>>(reinterpret_cast<const int *>(scratch + sl.hdr),
 						   reinterpret_cast<const uint4 *>(scratch + sl.ties), (const float *)d_attn,
 						   (float *)d_q, (float *)d_k, n_tok, n_heads, width,

@@ -92,6 +92,7 @@ inline std::vector<torch::Tensor> l1b_sparse_forward(torch::Tensor v, torch::Ten
 	TORCH_CHECK(dst_mxlen >= 0, "dst_mxlen must be >= 0");
 	const int dt = l1b_dtype(q, "l1attnSparse forward", true);
 	const c10::cuda::CUDAGuard guard(q.device());
+	l1b_check_pending("l1attnSparse forward");
 	const int bs = q.size(0), n = q.size(1), h = q.size(2), w = q.size(3), wv = v.size(3), cl = coo.size(0);
 	auto index = l1b_index_for(coo, n, dst_mxlen);
 	auto opts = q.options().requires_grad(false);
@@ -122,6 +123,7 @@ inline std::vector<torch::Tensor> l1b_sparse_backward(torch::Tensor dvo, torch::
 			    attn.size(3) == h,
 		    "attn must be [batch, n_tokens, dst_mxlen, heads] as returned by forward");
 	const c10::cuda::CUDAGuard guard(q.device());
+	l1b_check_pending("l1attnSparse backward");
 	auto index = l1b_index_for(coo, n, dst_mxlen);
 	auto d_v = torch::empty_like(v), d_q = torch::empty_like(q), d_k = torch::empty_like(k);
 	torch::Tensor d_vb;

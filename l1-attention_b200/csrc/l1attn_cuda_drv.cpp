@@ -8,24 +8,22 @@
 
 std::vector<torch::Tensor> l1attn_forward(torch::Tensor q, torch::Tensor k)
 {
-	l1b_check_pending("l1attn forward");
 	CHECK_INPUT(q);
 	CHECK_INPUT(k);
 	TORCH_CHECK(q.dim() == 4, "q must be [batch, n_tokens, heads, width]");
 	l1b_same(q, k, "q", "k");
 	const int dt = l1b_dtype(q, "l1attn forward");
 	const c10::cuda::CUDAGuard guard(q.device());
+	l1b_check_pending("l1attn forward");
 	const int bs = q.size(0), n = q.size(1), h = q.size(2), w = q.size(3);
 	auto attn = torch::empty({bs, n, n, h}, q.options().requires_grad(false));
 	l1b_status(l1attn_dense_fwd(q.data_ptr(), k.data_ptr(), attn.data_ptr(), bs, n, h, w, dt, l1b_stream()),
 		   "l1attn_dense_fwd");
-	l1b_poll_status();
 	return {attn};
 }
 
 std::vector<torch::Tensor> l1attn_backward(torch::Tensor d_attn, torch::Tensor q, torch::Tensor k)
 {
-	l1b_check_pending("l1attn backward");
 	CHECK_INPUT(d_attn);
 	CHECK_INPUT(q);
 	CHECK_INPUT(k);
@@ -38,13 +36,13 @@ std::vector<torch::Tensor> l1attn_backward(torch::Tensor d_attn, torch::Tensor q
 			    d_attn.size(3) == h,
 		    "d_attn must be [batch, n_tokens, n_tokens, heads]");
 	const c10::cuda::CUDAGuard guard(q.device());
+	l1b_check_pending("l1attn backward");
 	auto d_q = torch::empty_like(q), d_k = torch::empty_like(k);
 	auto scratch = torch::empty({(long)l1attn_dense_bwd_scratch_bytes(bs, n, h, w, dt)},
 				    torch::TensorOptions().dtype(torch::kUInt8).device(q.device()));
 	l1b_status(l1attn_dense_bwd(d_attn.data_ptr(), q.data_ptr(), k.data_ptr(), d_q.data_ptr(), d_k.data_ptr(),
 				    scratch.data_ptr(), bs, n, h, w, dt, l1b_stream()),
 		   "l1attn_dense_bwd");
-	l1b_poll_status();
 	return {d_q, d_k};
 }
 

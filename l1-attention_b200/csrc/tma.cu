@@ -1,5 +1,7 @@
 // Host side of the TMA helpers: tensor-map encoding through the driver entry point (no link
 // against libcuda), and the sticky device error word.
+#include <atomic>
+#include <cstddef>
 #include <mutex>
 #include "common.cuh"
 #include "tma.cuh"
@@ -7,7 +9,16 @@
 namespace l1b {
 
 namespace {
-__device__ int l1b_kernel_error = 0;
+struct KernelError {
+	int word, pad;
+	int *host;
+};
+__device__ KernelError l1b_kernel_error;
+static_assert(offsetof(KernelError, host) == ERROR_HOST_WORD * sizeof(int), "layout");
+constexpr int MAX_DEVICES = 64;
+std::atomic<int *> g_error_addr[MAX_DEVICES], g_error_host[MAX_DEVICES];
+std::atomic<int> g_sms[MAX_DEVICES];
+std::mutex g_error_mu;
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
 				  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -48,12 +59,36 @@ bool encode_tmap_4d(CUtensorMap *out, CUtensorMapDataType dt, const void *base, 
 
 int *device_error_word()
 {
-	int *p = nullptr;
+	int dev = 0;
+	KernelError *p = nullptr;
+	if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) {
+		(void)cudaGetLastError();
+		return nullptr;
+	}
+	if (int *known = g_error_addr[dev].load(std::memory_order_acquire))
+		return known;
 	if (cudaGetSymbolAddress(reinterpret_cast<void **>(&p), l1b_kernel_error) != cudaSuccess) {
 		(void)cudaGetLastError();
 		return nullptr;
 	}
-	return p;
+	g_error_addr[dev].store(&p->word, std::memory_order_release);
+	return &p->word;
+}
+
+int multiprocessors(int *out)
+{
+	int dev = 0, n = 0;
+	L1B_CUDA(cudaGetDevice(&dev));
+	const bool slot = dev >= 0 && dev < MAX_DEVICES;
+	if (slot && (n = g_sms[dev].load(std::memory_order_relaxed)) > 0) {
+		*out = n;
+		return L1ATTN_OK;
+	}
+	L1B_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+	if (slot)
+		g_sms[dev].store(n, std::memory_order_relaxed);
+	*out = n;
+	return L1ATTN_OK;
 }
 
 } // namespace l1b
@@ -71,6 +106,46 @@ extern "C" int l1attn_device_status(void)
 		return L1ATTN_ERR_TIMEOUT;
 	}
 	return L1ATTN_OK;
+}
+
+// The current device's host word: pinned memory that a kernel of this library sets to 1 when it gives up a bounded wait, at once and
+// without a copy on any stream.  The caller clears it.  Null when it cannot be had now (the first call on a device needs
+// to allocate and copy: not while a stream of the process captures in global mode).
+extern "C" int *l1attn_device_status_word(void)
+{
+	using namespace l1b;
+	int dev = 0, *err = device_error_word(), *host = nullptr;
+	if (!err || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES)
+		return nullptr;
+	if ((host = g_error_host[dev].load(std::memory_order_acquire)))
+		return host;
+	std::lock_guard<std::mutex> lock(g_error_mu);
+	if ((host = g_error_host[dev].load(std::memory_order_relaxed)))
+		return host;
+	cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed; // this thread's calls below belong to no capture
+	cudaStream_t st = nullptr;
+	if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
+		(void)cudaGetLastError();
+		return nullptr;
+	}
+	bool ok = cudaHostAlloc(reinterpret_cast<void **>(&host), 64, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess;
+	if (ok) {
+		*host = 0;
+		ok = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess &&
+		     cudaMemcpyAsync(err + ERROR_HOST_WORD, &host, sizeof host, cudaMemcpyHostToDevice, st) == cudaSuccess &&
+		     cudaStreamSynchronize(st) == cudaSuccess;
+		if (st)
+			(void)cudaStreamDestroy(st);
+		if (!ok)
+			(void)cudaFreeHost(host);
+	}
+	(void)cudaThreadExchangeStreamCaptureMode(&mode);
+	if (!ok) {
+		(void)cudaGetLastError();
+		return nullptr;
+	}
+	g_error_host[dev].store(host, std::memory_order_release);
+	return host;
 }
 
 // Copies the error word to *host_word on `stream` without waiting and without clearing it.  With host_word in

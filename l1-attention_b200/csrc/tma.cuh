@@ -17,7 +17,10 @@ namespace l1b {
 
 // Address (on the current device) of the sticky error word: 0 = no error; a kernel whose bounded
 // wait ran out stores a non-zero code there.  Read and cleared by l1attn_device_status().
+// Behind it (ERROR_HOST_WORD ints further) lies the address of a word in pinned host memory that the same kernel sets too,
+// or null: whoever asked for it (l1attn_device_status_word) learns of a timeout without a copy.
 int *device_error_word();
+constexpr int ERROR_HOST_WORD = 2;
 
 constexpr uint64_t WAIT_LIMIT_NS = 2000000000ull; // two seconds: orders of magnitude beyond any copy these kernels wait for
 
@@ -70,8 +73,11 @@ static __device__ __noinline__ bool mbar_wait_timed(uint64_t *bar, uint32_t pari
 		n++;
 	if (polls)
 		*polls = n;
-	if (!ok)
+	if (!ok) {
 		*err = 1;
+		if (int *host = *reinterpret_cast<int **>(err + ERROR_HOST_WORD))
+			*reinterpret_cast<volatile int *>(host) = 1;
+	}
 	return ok;
 }
 
