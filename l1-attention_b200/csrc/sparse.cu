@@ -156,6 +156,16 @@ template <typename T, int VEC, int NX> __device__ __forceinline__ void zero_acc(
 			acc[it].v[i] = T(0);
 }
 
+// Slots [rb, rb + 32) of a destination, one per lane (-1: empty); returns how many of them a walk has to look at: empty ones at the end --
+// the rule, slots fill from the front -- are not.  (In the forward the same bound cost the full lists of a kept graph
+// more than it saved elsewhere.)
+__device__ __forceinline__ int next_slots(const int32_t *slots, int rb, int dm, int &mine)
+{
+	const int lane = threadIdx.x & 31;
+	mine = rb + lane < dm ? slots[rb + lane] : -1;
+	return 32 - __clz(__ballot_sync(0xffffffffu, mine >= 0));
+}
+
 // ---- forward, dst pass: scores -> exp -> (+1)-softmax -> attn, vo[dst] = sum_r a_r v[src_r] ----
 // With NX > 0 ONE walk over the slots does all of it: k[src] and v[src] of a slot are gathered together.  The weights
 // have no maximum to subtract, so vo = (sum_r e_r v[src_r]) / denom needs no second walk (two walks: the v rows waited
@@ -449,59 +459,60 @@ __global__ void __launch_bounds__(CTA, (NX == 4 ? 4 : 6) - (BIDI && NX > 0 ? 1 :
 		const T *vbase = v + (tokrow * H + hh) * Wv + w.li * VEC, *kbase = k + (tokrow * H + hh) * W + w.li * VEC;
 		const T *gbase = dvo + (tokrow * H + hh) * Wv + w.li * VEC;
 		T S = T(0);
-		int mine = -1; // slot (r & ~31) + lane of the list
-		for (int r = 0; r < dm; r++) {
-			if (r % 32 == 0)
-				mine = r + lane < dm ? slots[r + lane] : -1;
-			const int src = __shfl_sync(0xffffffffu, mine, r & 31);
-			const bool ok = w.head_ok && src >= 0;
-			const size_t so = size_t(ok ? src : 0) * H;
-			Pack<T, VEC> vr[NX], kr[NX], gr[NX];
+		for (int rb = 0; rb < dm; rb += 32) {
+			int mine;
+			const int n = next_slots(slots, rb, dm, mine);
+			for (int i = 0; i < n; i++) {
+				const int src = __shfl_sync(0xffffffffu, mine, i), r = rb + i;
+				const bool ok = w.head_ok && src >= 0;
+				const size_t so = size_t(ok ? src : 0) * H;
+				Pack<T, VEC> vr[NX], kr[NX], gr[NX];
 #pragma unroll
-			for (int it = 0; it < NX; it++) {
-				vr[it] = ldv<T, VEC>(vbase + so * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
-				kr[it] = ldv<T, VEC>(kbase + so * W + it * step, in_row<VEC, EX>(w.li, it, step, W));
-			}
-			if (BIDI) {
-#pragma unroll
-				for (int it = 0; it < NX; it++)
-					gr[it] = ldv<T, VEC>(gbase + so * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
-			}
-			const T ar = ok ? arow[size_t(r) * H] : T(0);
-			T part = T(0);
-#pragma unroll
-			for (int it = 0; it < NX; it++)
-#pragma unroll
-				for (int i = 0; i < VEC; i++)
-					part += vr[it].v[i] * gd[it].v[i];
-			if (BIDI) {
-#pragma unroll
-				for (int it = 0; it < NX; it++)
-#pragma unroll
-					for (int i = 0; i < VEC; i++)
-						part += bd[it].v[i] * gr[it].v[i];
-			}
-			part = group_sum<LPHC>(part, lph);
-			if (!ok)
-				continue; // (uniform over the lanes of a head; the shuffles above ran for the whole warp)
-			S += ar * part;
-			if (w.li == 0)
-				xrow[size_t(r) * H] = part;
-			const T w1 = ar * part;
-#pragma unroll
-			for (int it = 0; it < NX; it++)
-#pragma unroll
-				for (int i = 0; i < VEC; i++) {
-					const T sg = sign_apply(qv[it].v[i] - kr[it].v[i], T(1));
-					acc1[it].v[i] += sg * w1;
-					acc2[it].v[i] += sg * ar;
+				for (int it = 0; it < NX; it++) {
+					vr[it] = ldv<T, VEC>(vbase + so * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
+					kr[it] = ldv<T, VEC>(kbase + so * W + it * step, in_row<VEC, EX>(w.li, it, step, W));
 				}
-			if (BIDI) {
+				if (BIDI) {
+#pragma unroll
+					for (int it = 0; it < NX; it++)
+						gr[it] = ldv<T, VEC>(gbase + so * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
+				}
+				const T ar = ok ? arow[size_t(r) * H] : T(0);
+				T part = T(0);
 #pragma unroll
 				for (int it = 0; it < NX; it++)
 #pragma unroll
 					for (int i = 0; i < VEC; i++)
-						accb[it].v[i] += ar * gr[it].v[i];
+						part += vr[it].v[i] * gd[it].v[i];
+				if (BIDI) {
+#pragma unroll
+					for (int it = 0; it < NX; it++)
+#pragma unroll
+						for (int i = 0; i < VEC; i++)
+							part += bd[it].v[i] * gr[it].v[i];
+				}
+				part = group_sum<LPHC>(part, lph);
+				if (!ok)
+					continue; // (uniform over the lanes of a head; the shuffles above ran for the whole warp)
+				S += ar * part;
+				if (w.li == 0)
+					xrow[size_t(r) * H] = part;
+				const T w1 = ar * part;
+#pragma unroll
+				for (int it = 0; it < NX; it++)
+#pragma unroll
+					for (int i = 0; i < VEC; i++) {
+						const T sg = sign_apply(qv[it].v[i] - kr[it].v[i], T(1));
+						acc1[it].v[i] += sg * w1;
+						acc2[it].v[i] += sg * ar;
+					}
+				if (BIDI) {
+#pragma unroll
+					for (int it = 0; it < NX; it++)
+#pragma unroll
+						for (int i = 0; i < VEC; i++)
+							accb[it].v[i] += ar * gr[it].v[i];
+				}
 			}
 		}
 		__syncwarp();
@@ -961,8 +972,9 @@ extern "C" int l1attn_sparse_fwd(const void *v, const void *vb, const void *q, c
 		     ix.slot_src, ix.csc_off, ix.csc_slot};
 	const bool a16 = all_aligned16({v, vb, q, k, vo});
 	if (dtype == L1ATTN_F16 || dtype == L1ATTN_BF16) {
-		// 16-bit storage, float arithmetic: eight elements (16 bytes) per load, or four, when rows allow it
-		const bool a16h = a16 && width % 8 == 0 && v_width % 8 == 0;
+		// 16-bit storage, float arithmetic: eight elements (16 bytes) per load, or four, when rows allow it (eight only where
+		// they keep a head's four lanes busy: from 32 columns on)
+		const bool a16h = a16 && width % 8 == 0 && v_width % 8 == 0 && (width >= 32 || v_width >= 32);
 		bool a8 = width % 4 == 0 && v_width % 4 == 0;
 		for (const void *p : {v, vb, q, k, (const void *)vo})
 			a8 = a8 && (!p || aligned(p, 8));
