@@ -240,6 +240,11 @@ int l1attn_sparse_bwd_static(const void *dvo, const void *v, const void *vb, con
 size_t l1attn_expand_coo_scratch_bytes(long long n_keys);
 int l1attn_expand_coo(const int64_t *co, int cl, int32_t *coo, int32_t *mxlen,
 		      long long key_lo, long long n_keys, void *counters, void *stream);
+
+/* The same with the id range found on the way, in one kernel: result (device, 4 x int64) receives the lowest and the highest id, dst_mxlen and
+ * src_mxlen.  Both lengths are 0 and coo is untouched when the ids do not fit int32 or span more than the kernel's counters hold
+ * (26624 ids): the caller then goes on with l1attn_expand_coo.  cl >= 1. */
+int l1attn_expand_coo_once(const int64_t *co, int cl, int32_t *coo, int64_t *result, void *stream);
 int l1attn_i64_minmax(const int64_t *x, long long n, int64_t *out, void *stream);
 
 /* ------------------------------------------------------------------ host buffers -------- */

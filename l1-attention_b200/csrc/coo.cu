@@ -91,15 +91,12 @@ constexpr int RANK_THREADS = 512; // 16 warps; the first `nwarp` of them own a c
 constexpr int RANK_SMEM = 208 * 1024;
 
 template <typename K>
-__global__ void __cluster_dims__(RC, 1, 1) __launch_bounds__(RANK_THREADS)
-rank_cluster_kernel(const K *keys, int stride, int n, long long key_lo, int n_keys, int32_t *rank_out, int rstride,
+__device__ __forceinline__ void rank_chunks(int32_t *rsm, int32_t &smax, int col, const K *keys, int stride, int n, long long key_lo, int n_keys, int32_t *rank_out, int rstride,
 		    int32_t *counts, int32_t *max_out, int col_step, int nwarp, int32_t *key_out)
 {
-	extern __shared__ int32_t rsm[];
-	__shared__ int32_t smax;
 	cg::cluster_group cluster = cg::this_cluster();
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	const int crank = int(cluster.block_rank()), col = int(blockIdx.x) / RC;
+	const int crank = int(cluster.block_rank());
 	keys += size_t(col) * col_step;
 	rank_out += size_t(col) * col_step;
 	if (key_out)
@@ -180,6 +177,83 @@ rank_cluster_kernel(const K *keys, int stride, int n, long long key_lo, int n_ke
 			if (key_out)
 				key_out[size_t(i) * rstride] = int32_t(key + key_lo);
 		}
+	}
+}
+
+template <typename K>
+__global__ void __cluster_dims__(RC, 1, 1) __launch_bounds__(RANK_THREADS)
+rank_cluster_kernel(const K *keys, int stride, int n, long long key_lo, int n_keys, int32_t *rank_out, int rstride,
+		    int32_t *counts, int32_t *max_out, int col_step, int nwarp, int32_t *key_out)
+{
+	extern __shared__ int32_t rsm[];
+	__shared__ int32_t smax;
+	rank_chunks(rsm, smax, int(blockIdx.x) / RC, keys, stride, n, key_lo, n_keys, rank_out, rstride, counts, max_out, col_step, nwarp,
+		    key_out);
+}
+
+__host__ __device__ inline int rank_warps(long long n_keys) // chunks per CTA whose counters fit, one array for the sums left over
+{
+	const long long fit = RANK_SMEM / (n_keys * 4) - 1;
+	return int(fit < RANK_THREADS / 32 ? fit : RANK_THREADS / 32);
+}
+
+// expandCoo as ONE kernel: the range of the ids, then (where it fits) the ranks of both columns, a cluster each.  The host learns range
+// and list lengths from one copy; with the range found first, by a kernel of its own, it had to wait for the device twice.
+// result: lowest id, highest id, length of the longest dst list, of the longest src list -- or 0, 0 when the counters of so
+// many ids (or ids beyond int32) do not fit and nothing else was written.
+__global__ void __cluster_dims__(RC, 1, 1) __launch_bounds__(RANK_THREADS)
+expand_cluster_kernel(const int64_t *co, int n, int32_t *coo, long long *result)
+{
+	extern __shared__ int32_t rsm[];
+	__shared__ int32_t smax;
+	__shared__ int32_t longest[2];
+	__shared__ long long slo[RANK_THREADS / 32], shi[RANK_THREADS / 32], range[2];
+	cg::cluster_group cluster = cg::this_cluster();
+	const int tid = threadIdx.x, crank = int(cluster.block_rank()), col = int(blockIdx.x) / RC;
+	long long lo = INT64_MAX, hi = INT64_MIN;
+#pragma unroll 4
+	for (long long i = (long long)crank * RANK_THREADS + tid; i < 2LL * n; i += RC * RANK_THREADS) {
+		const long long v = co[i];
+		lo = min(lo, v);
+		hi = max(hi, v);
+	}
+	for (int o = 16; o > 0; o >>= 1) {
+		lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+		hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+	}
+	if ((tid & 31) == 0) {
+		slo[tid >> 5] = lo;
+		shi[tid >> 5] = hi;
+	}
+	__syncthreads();
+	if (tid == 0) {
+		for (int w = 1; w < RANK_THREADS / 32; w++) {
+			lo = min(lo, slo[w]);
+			hi = max(hi, shi[w]);
+		}
+		range[0] = lo;
+		range[1] = hi;
+	}
+	cluster.sync();
+	for (int r = 0; r < RC; r++) {
+		const long long *other = cluster.map_shared_rank(range, r);
+		lo = min(lo, other[0]);
+		hi = max(hi, other[1]);
+	}
+	const bool fits = lo >= INT32_MIN && hi <= INT32_MAX && 2 * (hi - lo + 1) * 4 <= RANK_SMEM; // the same in every thread
+	if (fits) {
+		const int n_keys = int(hi - lo + 1);
+		// (max_out: shared memory of this CTA, written by the last CTA of the cluster only)
+		rank_chunks(rsm, smax, col, co, 2, n, lo, n_keys, coo + 2, 4, nullptr, longest, 1, rank_warps(n_keys), coo);
+	} else {
+		cluster.sync(); // shared memory must outlive the others' reads (rank_chunks has such a barrier too)
+	}
+	if (crank == RC - 1 && tid == 0) {
+		if (col == 0) {
+			result[0] = lo;
+			result[1] = hi;
+		}
+		result[2 + col] = fits ? longest[col] : 0;
 	}
 }
 
@@ -319,7 +393,7 @@ int launch_rank(const K *keys, int stride, int n, long long key_lo, long long n_
 	// 8192 ids 18.5 / 19.2 us, 2048 rows 32.8 / 20.5; 2048 rows of 20000 ids 33.9 / 36.9, 8192 rows 116 / 47;
 	// 64 rows of 1024 ids 11.3 / 6.7.
 	if (8LL * n >= n_keys && n > 0 && n_keys > 0 && 2 * n_keys * 4 <= RANK_SMEM) {
-		const int fit = int(RANK_SMEM / (n_keys * 4)) - 1, nwarp = fit < RANK_THREADS / 32 ? fit : RANK_THREADS / 32;
+		const int nwarp = rank_warps(n_keys);
 		const size_t smem = size_t(nwarp + 1) * n_keys * 4;
 		auto kern = rank_cluster_kernel<K>;
 		L1B_SHARED_MEMORY(kern, int(smem));
@@ -422,6 +496,16 @@ extern "C" int l1attn_expand_coo(const int64_t *co, int cl, int32_t *coo, int32_
 	// column 0 -> ranks into coo[:,2], column 1 -> coo[:,3]; with cl == 0 the kernel still writes mxlen = 1
 	int32_t *cnt = n_keys > SMEM_KEYS ? static_cast<int32_t *>(counters) : nullptr;
 	return launch_rank<int64_t>(co, 2, cl, key_lo, n_keys, coo ? coo + 2 : nullptr, 4, cnt, mxlen, 1, 2, coo, st);
+}
+
+extern "C" int l1attn_expand_coo_once(const int64_t *co, int cl, int32_t *coo, int64_t *result, void *stream)
+{
+	if (cl < 1 || !co || !coo || !result)
+		return L1ATTN_ERR_ARG;
+	L1B_SHARED_MEMORY(expand_cluster_kernel, RANK_SMEM);
+	expand_cluster_kernel<<<2 * RC, RANK_THREADS, RANK_SMEM, static_cast<cudaStream_t>(stream)>>>(co, cl, coo, reinterpret_cast<long long *>(result));
+	L1B_LAUNCH_CHECK();
+	return L1ATTN_OK;
 }
 
 extern "C" int l1attn_i64_minmax(const int64_t *x, long long n, int64_t *out, void *stream)

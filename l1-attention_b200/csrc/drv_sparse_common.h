@@ -56,7 +56,7 @@ inline torch::Tensor l1b_index_for(const torch::Tensor &coo, int n_tok, int dst_
 	const size_t bytes = l1attn_sparse_index_bytes(cl, n_tok, dst_mxlen);
 	auto opts = torch::TensorOptions().dtype(torch::kInt32).device(coo.device());
 	auto index = torch::empty({(long)((bytes + 3) / 4)}, opts);
-	auto status = torch::zeros({1}, opts);
+	auto status = torch::empty({1}, opts); // (cleared by the build)
 	l1b_status(l1attn_sparse_build_index(coo.data_ptr<int>(), cl, n_tok, dst_mxlen, index.data_ptr(),
 					     status.data_ptr<int>(), l1b_stream()),
 		   "l1attn_sparse_build_index");
@@ -153,20 +153,22 @@ inline std::tuple<torch::Tensor, int, int> l1b_expand_coo(torch::Tensor co)
 	auto cog = co.slice(1, 0, 2).to(dev, torch::kInt64).contiguous();
 	const int cl = cog.size(0);
 	auto i32 = torch::TensorOptions().dtype(torch::kInt32).device(dev);
-	auto coo = torch::zeros({cl, 4}, i32);
-	auto mx = torch::ones({2}, i32);
+	auto coo = torch::empty({cl, 4}, i32);
 	long long lo = 0, nkeys = 0;
 	torch::Tensor counters;
 	void *cnt = nullptr;
 	if (cl > 0) {
-		auto mm = torch::empty({2}, torch::TensorOptions().dtype(torch::kInt64).device(dev));
-		l1b_status(l1attn_i64_minmax(cog.data_ptr<int64_t>(), 2LL * cl, mm.data_ptr<int64_t>(), l1b_stream()),
-			   "l1attn_i64_minmax");
-		auto mmh = mm.cpu();
-		lo = mmh[0].item<int64_t>();
-		const long long hi = mmh[1].item<int64_t>();
+		auto result = torch::empty({4}, torch::TensorOptions().dtype(torch::kInt64).device(dev));
+		l1b_status(l1attn_expand_coo_once(cog.data_ptr<int64_t>(), cl, coo.data_ptr<int>(), result.data_ptr<int64_t>(), l1b_stream()),
+			   "l1attn_expand_coo_once");
+		const auto host = result.cpu();
+		const int64_t *r = host.data_ptr<int64_t>();
+		lo = r[0];
+		const long long hi = r[1];
 		// the expanded list is int32 (as the reference's is); the rank counters take memory proportional to hi - lo
 		TORCH_CHECK(lo >= INT32_MIN && hi <= INT32_MAX, "expandCoo: token ids must fit in int32, got [", lo, ", ", hi, "]");
+		if (r[2] > 0)
+			return {coo.to(home), int(r[2]), int(r[3])};
 		nkeys = hi - lo + 1;
 		const size_t nb = l1attn_expand_coo_scratch_bytes(nkeys);
 		if (nb) {
@@ -174,6 +176,7 @@ inline std::tuple<torch::Tensor, int, int> l1b_expand_coo(torch::Tensor co)
 			cnt = counters.data_ptr();
 		}
 	}
+	auto mx = torch::ones({2}, i32);
 	l1b_status(l1attn_expand_coo(cl ? cog.data_ptr<int64_t>() : nullptr, cl, cl ? coo.data_ptr<int>() : nullptr,
 				     mx.data_ptr<int>(), lo, nkeys, cnt, l1b_stream()),
 		   "l1attn_expand_coo");

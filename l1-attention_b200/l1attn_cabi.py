@@ -40,6 +40,7 @@ SIGNATURES = {
     "l1attn_sparse_bwd": (_i, [_vp] * 12 + [_i] * 10 + [_vp]),
     "l1attn_sparse_bwd_static_capacity": (_sz, []),
     "l1attn_sparse_bwd_static": (_i, [_vp] * 11 + [_i] * 10 + [_vp]),
+    "l1attn_expand_coo_once": (_i, [_vp, _i, _vp, _vp, _vp]),
     "l1attn_expand_coo_scratch_bytes": (_sz, [_ll]),
     "l1attn_expand_coo": (_i, [_vp, _i, _vp, _vp, _ll, _ll, _vp, _vp]),
     "l1attn_i64_minmax": (_i, [_vp, _ll, _vp, _vp]),

@@ -338,6 +338,27 @@ def test_full_size_config(bidi, qk_scale):
         assert_close(x, r, 1e-5, "grad")
 
 
+@pytest.mark.parametrize("bidi", [False, True])
+@pytest.mark.parametrize("case", [(2, 70, 8, 64, 64), (1, 60, 2, 32, 32), (1, 40, 5, 33, 9), (1, 50, 3, 40, 24)])
+def test_long_and_short_lists_vs_oracle(case, bidi):
+    """Sources with 64, 65 and several hundred incoming edges beside sources with none (long lists are shared by the warps of a
+    CTA), destinations whose slots end early, and a hole in the middle of a list."""
+    bs, n, h, w, wv = case
+    rng = np.random.RandomState(sum(case))
+    rows = [[rng.randint(n), s] for s, c in ((0, 64), (1, 65), (2, 333), (n - 1, 130)) for _ in range(c)] + [[5, s] for s in range(3, 40)]
+    from oracle import oracle
+    coo, dm, _ = oracle.expand_coo(np.array(rows, dtype=np.int64)[rng.permutation(len(rows))])
+    coo = coo[~((coo[:, 0] == 5) & (coo[:, 2] == 7))]  # slot 7 of destination 5 stays empty
+    mk = lambda width: rng.standard_normal((bs, n, h, width)).astype(np.float32)
+    q, k, v, vb, dvo = 0.3 * mk(w), 0.3 * mk(w), mk(wv), (mk(wv) if bidi else None), mk(wv)
+    vo, attn, grads = run_gpu(v, vb, q, k, dvo, coo, dm, True)
+    rvo, rattn, rgrads = run_oracle(v, vb, q, k, dvo, coo, dm, True)
+    assert_close(vo, rvo, 1e-5, "vo")
+    assert_close(attn, rattn, 1e-5, "attn")
+    for x, r in zip(grads, rgrads):
+        assert_close(x, r, 1e-5, "gradients")
+
+
 # ------------------------------------------------------------------ expandCoo
 
 def test_expandcoo_golden(golden):
@@ -387,6 +408,10 @@ def test_ranks_by_cluster_bit_exact(cl, keys):
     coo, dm, sm = cabi.expand_coo_host(co)
     rcoo, rdm, rsm = oracle.expand_coo(co)
     assert np.array_equal(coo, rcoo) and (dm, sm) == (rdm, rsm)
+    import l1attn_sparse_cuda  # the modules' path: range and ranks in one kernel, the other kernels where the counters do not fit
+    for t in (torch.from_numpy(co), torch.from_numpy(co).cuda()):
+        tcoo, tdm, tsm = l1attn_sparse_cuda.expandCoo(t)
+        assert tcoo.device == t.device and np.array_equal(tcoo.cpu().numpy(), rcoo) and (tdm, tsm) == (rdm, rsm)
 
     n_tok, dm = keys + 3, max(1, dm - 1)  # one slot too few: the rows of the longest lists are out of range
     rows = rcoo.copy()
