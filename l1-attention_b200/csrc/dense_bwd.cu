@@ -20,6 +20,60 @@ constexpr int LW = 4;  // lanes along the width (16-byte vectors)
 constexpr int TY = 16; // y rows per shared-memory tile
 constexpr int NCH = 8; // 16-byte chunks per shared row (both tiles)
 
+// one element, global -> shared, asynchronously; !ok: zero
+template <typename T> __device__ __forceinline__ void copy_element(T *dst, const T *src, bool ok)
+{
+	const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+	asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(sizeof(T)), "r"(ok ? int(sizeof(T)) : 0) : "memory");
+}
+
+// One source-side row for a thread: acc[i][e] += sign(a[i][e] - b[e]) * g[i].
+template <int TM, int VEC>
+__device__ __forceinline__ void row_terms(const float (&a)[TM][VEC], const float (&b)[VEC], const float (&g)[TM], float (&acc)[TM][VEC], bool)
+{
+#pragma unroll
+	for (int i = 0; i < TM; i++)
+#pragma unroll
+		for (int e = 0; e < VEC; e++)
+			acc[i][e] += sign_apply(a[i][e] - b[e], g[i]);
+}
+// fp64: two instructions of the FP64 pipe per term (subtract, add) instead of four -- the comparisons of the exact sign run on that
+// pipe too, and it takes two cycles each.  The sign bit of the difference flips g's in the integer pipe, and the high words of
+// a thread's eight differences are searched for a zero (a tie, or a difference below 2^-1042); then, and where an operand is
+// not finite (odd), the row's terms take the exact form.  a holds no negative zeros, so equal values differ by +0.
+template <int TM, int VEC>
+__device__ __forceinline__ void row_terms(const double (&a)[TM][VEC], const double (&b)[VEC], const double (&g)[TM], double (&acc)[TM][VEC], bool odd)
+{
+	double d[TM][VEC];
+	unsigned least = 0xffffffffu;
+	bool exact = odd;
+#pragma unroll
+	for (int e = 0; e < VEC; e++)
+		exact = exact || (__double2hiint(b[e]) & 0x7ff00000) == 0x7ff00000;
+#pragma unroll
+	for (int i = 0; i < TM; i++)
+#pragma unroll
+		for (int e = 0; e < VEC; e++) {
+			d[i][e] = a[i][e] - b[e];
+			least = min(least, unsigned(__double2hiint(d[i][e])));
+		}
+	if (exact || least == 0u) {
+#pragma unroll
+		for (int i = 0; i < TM; i++)
+#pragma unroll
+			for (int e = 0; e < VEC; e++)
+				acc[i][e] += sign_apply(d[i][e], g[i]);
+		return;
+	}
+#pragma unroll
+	for (int i = 0; i < TM; i++)
+#pragma unroll
+		for (int e = 0; e < VEC; e++)
+			acc[i][e] += __hiloint2double(__double2hiint(g[i]) ^ (__double2hiint(d[i][e]) & int(0x80000000)), __double2loint(g[i]));
+}
+__device__ __forceinline__ bool not_finite(float) { return false; }
+__device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
+
 template <typename T, int TM, int NWX, int NWW>
 __global__ void __launch_bounds__(NWX *NWW * 32, 2)
 dense_bwd_kernel(const T *__restrict__ g, const T *__restrict__ q, const T *__restrict__ k,
@@ -33,8 +87,8 @@ dense_bwd_kernel(const T *__restrict__ g, const T *__restrict__ q, const T *__re
 	static_assert(TX / VEC == NCH && WR / VEC == NCH, "tile rows must be 8 chunks of 16 bytes");
 	static_assert(TM % VEC == 0, "TM must be whole vectors");
 	using V = Pack<T, VEC>;
-	__shared__ __align__(16) V Bt[TY * HG * NCH]; // b[y][h][w chunk], chunk ^= h
-	__shared__ __align__(16) V Gt[TY * HG * NCH]; // G[y][h][x chunk], chunk ^= h
+	extern __shared__ __align__(16) unsigned char smem_raw[];
+	V *stages = reinterpret_cast<V *>(smem_raw); // [2]: b[y][h][w chunk], chunk ^= h; then G[y][h][x chunk], chunk ^= h
 
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int lane_h = lane & 7, lane_w = lane >> 3;
@@ -62,33 +116,35 @@ dense_bwd_kernel(const T *__restrict__ g, const T *__restrict__ q, const T *__re
 	const int w = w0 + wv * VEC;
 
 	T a[TM][VEC], acc[TM][VEC];
+	bool odd = false; // a value of a is not finite
 #pragma unroll
 	for (int i = 0; i < TM; i++) {
 		const int x = x0 + wx * TM + i;
 #pragma unroll
 		for (int e = 0; e < VEC; e++) {
 			const bool ok = x < n_tok && h < n_heads && w + e < width;
-			a[i][e] = ok ? av[size_t(x) * row + size_t(h) * width + w + e] : T(0);
+			a[i][e] = ok ? av[size_t(x) * row + size_t(h) * width + w + e] + T(0) : T(1); // (past the end: anything that ties with nothing)
+			odd = odd || not_finite(a[i][e]);
 			acc[i][e] = T(0);
 		}
 	}
 
-	for (int y0 = 0; y0 < n_tok; y0 += TY) {
+	// one tile's copies, asynchronous: they land while the tile before is worked on
+	auto load_tile = [&](int y0) {
+		V *Bt = stages + (y0 / TY & 1) * (2 * TY * HG * NCH), *Gt = Bt + TY * HG * NCH;
 		// b tile: [TY][HG][WR]
 		for (int v = tid; v < TY * HG * NCH; v += NT) {
 			const int c = v % NCH, hh = (v / NCH) % HG, y = v / (NCH * HG);
 			const int gy = y0 + y, gh = h0 + hh, gw = w0 + c * VEC;
 			V *dst = &Bt[(y * HG + hh) * NCH + (c ^ hh)];
-			const T *src = bv + size_t(gy) * row + size_t(gh) * width + gw;
 			const bool ok = gy < n_tok && gh < n_heads;
+			const T *src = ok ? bv + size_t(gy) * row + size_t(gh) * width + gw : bv;
 			if (ok && vec_ok && gw + VEC <= width) {
-				*dst = *reinterpret_cast<const V *>(src);
+				cp_async16(dst, src);
 			} else {
-				V z;
 #pragma unroll
 				for (int e = 0; e < VEC; e++)
-					z.v[e] = (ok && gw + e < width) ? src[e] : T(0);
-				*dst = z;
+					copy_element(&dst->v[e], ok && gw + e < width ? src + e : bv, ok && gw + e < width);
 			}
 		}
 		// G tile: [TY][HG][TX], heads fastest in global memory
@@ -104,12 +160,20 @@ dense_bwd_kernel(const T *__restrict__ g, const T *__restrict__ q, const T *__re
 				x = idx / (HG * TY);
 			}
 			const int gx = x0 + x, gy = y0 + y, gh = h0 + hh;
-			T val = T(0);
-			if (gx < n_tok && gy < n_tok && gh < n_heads)
-				val = gb[size_t(gx) * gsx + size_t(gy) * gsy + gh];
-			Gs[((y * HG + hh) * NCH + ((x / VEC) ^ hh)) * VEC + (x % VEC)] = val;
+			const bool ok = gx < n_tok && gy < n_tok && gh < n_heads;
+			copy_element(&Gs[((y * HG + hh) * NCH + ((x / VEC) ^ hh)) * VEC + (x % VEC)],
+				     ok ? gb + size_t(gx) * gsx + size_t(gy) * gsy + gh : gb, ok);
 		}
+	};
+	load_tile(0);
+	cp_async_commit();
+	for (int y0 = 0; y0 < n_tok; y0 += TY) {
+		if (y0 + TY < n_tok)
+			load_tile(y0 + TY);
+		cp_async_commit();
+		cp_async_wait<1>();
 		__syncthreads();
+		const V *Bt = stages + (y0 / TY & 1) * (2 * TY * HG * NCH), *Gt = Bt + TY * HG * NCH;
 #pragma unroll 4
 		for (int y = 0; y < TY; y++) {
 			const V bvec = Bt[(y * HG + lane_h) * NCH + (wv ^ lane_h)];
@@ -121,11 +185,7 @@ dense_bwd_kernel(const T *__restrict__ g, const T *__restrict__ q, const T *__re
 				for (int e = 0; e < VEC; e++)
 					gv[m * VEC + e] = t.v[e];
 			}
-#pragma unroll
-			for (int i = 0; i < TM; i++)
-#pragma unroll
-				for (int e = 0; e < VEC; e++)
-					acc[i][e] += sign_apply(a[i][e] - bvec.v[e], gv[i]);
+			row_terms<TM, VEC>(a, bvec.v, gv, acc, odd);
 		}
 		__syncthreads();
 	}
@@ -165,7 +225,10 @@ int launch(const T *g, const T *q, const T *k, T *d_q, T *d_k, int bs, int n_tok
 		return L1ATTN_ERR_SHAPE;
 	const int vec_ok = (width % VEC == 0) && aligned(q, 16) && aligned(k, 16) && aligned(d_q, 16) && aligned(d_k, 16);
 	const T scale = T(-1.0 / sqrt(double(width)));
-	dense_bwd_kernel<T, TM, NWX, NWW><<<unsigned(nblk), NWX * NWW * 32, 0, st>>>(
+	auto kern = dense_bwd_kernel<T, TM, NWX, NWW>;
+	constexpr int smem = 2 * 2 * TY * HG * NCH * 16;
+	L1B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+	kern<<<unsigned(nblk), NWX * NWW * 32, smem, st>>>(
 		g, q, k, d_q, d_k, n_tok, n_heads, width, scale, vec_ok, nxt, nwt, nhg, bs);
 	L1B_LAUNCH_CHECK();
 	return L1ATTN_OK;
