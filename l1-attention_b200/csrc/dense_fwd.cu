@@ -158,11 +158,18 @@ int dense_fwd_launch(const void *q, const void *k, void *attn, int bs, int n_tok
 	if (bs == 0 || n_tok == 0 || n_heads == 0)
 		return L1ATTN_OK;
 	static const bool no_tma = getenv("L1ATTN_NO_TMA") != nullptr; // debugging aid: force the generic kernel
-	if (!no_tma) {
+	// Sets of at most 16 tokens: a 16 x 16 tile per CTA.  The TMA kernel's 64 x 32 items would be an eighth full, and there
+	// is no ring to fill ahead with one item per set.
+	const bool tiny = n_tok <= 16;
+	if (!no_tma && !tiny) {
 		const int rc = dense_fwd_tma_launch(q, k, attn, bs, n_tok, n_heads, width, dtype, st);
 		if (rc <= 0)
 			return rc;
 	}
+	if (tiny && dtype == L1ATTN_F32)
+		return launch<float, 4, 4, 4>((const float *)q, (const float *)k, (float *)attn, bs, n_tok, n_heads, width, st);
+	if (tiny)
+		return launch<double, 4, 4, 4>((const double *)q, (const double *)k, (double *)attn, bs, n_tok, n_heads, width, st);
 	if (dtype == L1ATTN_F32)
 		return launch<float, 8, 8, 8>((const float *)q, (const float *)k, (float *)attn, bs, n_tok, n_heads, width, st);
 	return launch<double, 4, 4, 8>((const double *)q, (const double *)k, (double *)attn, bs, n_tok, n_heads, width, st);
