@@ -111,13 +111,20 @@ int dense_fwd_tma_launch(const void *q, const void *k, void *attn, int bs, int n
 int dense_bwd_tma_launch(const void *d_attn, const void *q, const void *k, void *d_q, void *d_k, int bs, int n_tok,
 			 int n_heads, int width, int dtype, const unsigned char *exact_flags, const int *tie_hdr,
 			 int only_on_overflow, cudaStream_t st);
-int dense_bwd_sv_launch(const void *d_attn, const void *q, const void *k, void *d_q, void *d_k, const int *tie_hdr,
-			void *part, void *dq_part, int ns, int bs, int n_tok, int n_heads, int width, int dtype, cudaStream_t st);
+int dense_bwd_sv_launch(const void *d_attn, const void *q, const void *k, void *d_q, void *d_k, void *scratch, int bs, int n_tok,
+			int n_heads, int width, int dtype, cudaStream_t st);
+int dense_bwd_small_launch(const void *d_attn, const void *q, const void *k, void *d_q, void *d_k, int bs, int n_tok, int n_heads,
+			   int width, int dtype, cudaStream_t st);
+int dense_bwd_partsum_launch(void *d_q, void *d_k, void *scratch, int bs, int n_tok, int n_heads, int width, cudaStream_t st);
+int dense_bwd_svr_launch(const void *d_attn, int g_pitch, int only_zeros, const void *q, const void *k, void *d_q, void *d_k, void *scratch, int bs,
+			 int n_tok, int n_heads, int width, cudaStream_t st);
+int dense_bwd_listed_launch(const void *d_attn, int g_pitch, const void *q, const void *k, void *d_q, void *d_k, void *scratch, int bs,
+			    int n_tok, int n_heads, int width, cudaStream_t st);
 // dk_sign: +1 after the two-pass kernel (a tie counted as -scale g in d_k), -1 after the single-visit kernel (+scale g)
-int dense_tiefix_launch(const void *d_attn, void *d_q, void *d_k, const unsigned char *scratch, int bs, int n_tok,
+int dense_tiefix_launch(const void *d_attn, int g_pitch, void *d_q, void *d_k, const unsigned char *scratch, int bs, int n_tok,
 			int n_heads, int width, int dk_sign, cudaStream_t st);
-int dense_ties_launch(const float *q, const float *k, unsigned char *scratch, int bs, int n_tok, int n_heads, int width,
-		      cudaStream_t st);
+int dense_ties_launch(const float *q, const float *k, unsigned char *scratch, void *d_k, int bs, int n_tok, int n_heads, int width,
+		      int drop_zero_rows, cudaStream_t st);
 // scratch: dense_bwd_scratch_bytes() bytes of device memory, or nullptr (then every tile runs the exact loop)
 int dense_bwd_launch(const void *d_attn, const void *q, const void *k, void *d_q, void *d_k, void *scratch, int bs,
 		     int n_tok, int n_heads, int width, int dtype, cudaStream_t st);
@@ -127,6 +134,11 @@ int dense_softmax_v_launch(const void *q, const void *k, const void *v, void *vo
 int dense_softmax_v_bwd_dx_launch(const void *q, const void *k, const void *v, const void *dvo, const void *lse,
 				  const void *delta, void *dx, void *dv, int bs, int n_tok, int n_heads, int width, int v_width,
 				  int dtype, cudaStream_t st);
+// the whole backward; work: dense_softmax_v_bwd_bytes() bytes of device memory, 256-byte aligned
+size_t dense_softmax_v_bwd_bytes(int bs, int n_tok, int n_heads, int width, int v_width, int dtype);
+int dense_softmax_v_bwd_launch(const void *q, const void *k, const void *v, const void *dvo, const void *lse, const void *delta,
+			       void *dq, void *dk, void *dv, void *work, int bs, int n_tok, int n_heads, int width, int v_width,
+			       int dtype, cudaStream_t st);
 
 // Layout of the sparse edge index (all int32, each array padded to 16 bytes):
 //   slot_src [n_tok*dst_mxlen]  src token of slot (dst, r), or -1

@@ -41,6 +41,7 @@ __device__ __forceinline__ void row_terms(const float (&a)[TM][VEC], const float
 // pipe too, and it takes two cycles each.  The sign bit of the difference flips g's in the integer pipe, and the high words of
 // a thread's eight differences are searched for a zero (a tie, or a difference below 2^-1042); then, and where an operand is
 // not finite (odd), the row's terms take the exact form.  a holds no negative zeros, so equal values differ by +0.
+// [2,512,8,128]: 420 us for the backward, 558 with the exact sign everywhere and tiles loaded one after the other.
 template <int TM, int VEC>
 __device__ __forceinline__ void row_terms(const double (&a)[TM][VEC], const double (&b)[VEC], const double (&g)[TM], double (&acc)[TM][VEC], bool odd)
 {
@@ -78,8 +79,10 @@ template <typename T, int TM, int NWX, int NWW>
 __global__ void __launch_bounds__(NWX *NWW * 32, 2)
 dense_bwd_kernel(const T *__restrict__ g, const T *__restrict__ q, const T *__restrict__ k,
 		 T *__restrict__ d_q, T *__restrict__ d_k, int n_tok, int n_heads, int width, T scale,
-		 int vec_ok, int nxt, int nwt, int nhg, int bs)
-{
+		 int vec_ok, int nxt, int nwt, int nhg, int bs, const int *__restrict__ tie_hdr, int g_pitch)
+{ // g_pitch: 0, or g lies [b][h][s][t] in rows of that many elements
+	if (tie_hdr && tie_hdr[BWD_HDR_OVERFLOW] == 0)
+		return; // the single-visit kernel (dense_bwd_svr.cu) has computed this call
 	constexpr int VEC = 16 / sizeof(T);
 	constexpr int TX = NWX * TM;       // x tile
 	constexpr int WR = NWW * LW * VEC; // width slice per CTA
@@ -107,9 +110,10 @@ dense_bwd_kernel(const T *__restrict__ g, const T *__restrict__ q, const T *__re
 	const T *av = (pass == 0 ? q : k) + size_t(b) * n_tok * row;
 	const T *bv = (pass == 0 ? k : q) + size_t(b) * n_tok * row;
 	T *out = (pass == 0 ? d_q : d_k) + size_t(b) * n_tok * row;
-	const T *gb = g + size_t(b) * n_tok * n_tok * n_heads;
-	const size_t gsx = pass == 0 ? size_t(n_heads) : size_t(n_tok) * n_heads;
-	const size_t gsy = pass == 0 ? size_t(n_tok) * n_heads : size_t(n_heads);
+	const T *gb = g + size_t(b) * n_tok * n_heads * (g_pitch > 0 ? g_pitch : n_tok);
+	const size_t gst = g_pitch > 0 ? 1 : n_heads, gss = g_pitch > 0 ? size_t(g_pitch) : size_t(n_tok) * n_heads;
+	const size_t gsh = g_pitch > 0 ? size_t(n_tok) * g_pitch : 1;
+	const size_t gsx = pass == 0 ? gst : gss, gsy = pass == 0 ? gss : gst;
 
 	const int h = h0 + lane_h;
 	const int wv = ww * LW + lane_w; // this thread's 16-byte chunk within the slice
@@ -162,7 +166,7 @@ dense_bwd_kernel(const T *__restrict__ g, const T *__restrict__ q, const T *__re
 			const int gx = x0 + x, gy = y0 + y, gh = h0 + hh;
 			const bool ok = gx < n_tok && gy < n_tok && gh < n_heads;
 			copy_element(&Gs[((y * HG + hh) * NCH + ((x / VEC) ^ hh)) * VEC + (x % VEC)],
-				     ok ? gb + size_t(gx) * gsx + size_t(gy) * gsy + gh : gb, ok);
+				     ok ? gb + size_t(gx) * gsx + size_t(gy) * gsy + gh * gsh : gb, ok);
 		}
 	};
 	load_tile(0);
@@ -215,7 +219,7 @@ dense_bwd_kernel(const T *__restrict__ g, const T *__restrict__ q, const T *__re
 
 template <typename T, int TM, int NWX, int NWW>
 int launch(const T *g, const T *q, const T *k, T *d_q, T *d_k, int bs, int n_tok, int n_heads, int width,
-	   cudaStream_t st)
+	   const int *tie_hdr, int g_pitch, cudaStream_t st)
 {
 	constexpr int VEC = 16 / sizeof(T);
 	constexpr int TX = NWX * TM, WR = NWW * LW * VEC;
@@ -227,9 +231,9 @@ int launch(const T *g, const T *q, const T *k, T *d_q, T *d_k, int bs, int n_tok
 	const T scale = T(-1.0 / sqrt(double(width)));
 	auto kern = dense_bwd_kernel<T, TM, NWX, NWW>;
 	constexpr int smem = 2 * 2 * TY * HG * NCH * 16;
-	L1B_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+	L1B_SHARED_MEMORY(kern, smem);
 	kern<<<unsigned(nblk), NWX * NWW * 32, smem, st>>>(
-		g, q, k, d_q, d_k, n_tok, n_heads, width, scale, vec_ok, nxt, nwt, nhg, bs);
+		g, q, k, d_q, d_k, n_tok, n_heads, width, scale, vec_ok, nxt, nwt, nhg, bs, tie_hdr, g_pitch);
 	L1B_LAUNCH_CHECK();
 	return L1ATTN_OK;
 }
@@ -243,52 +247,77 @@ size_t dense_bwd_scratch_bytes(int bs, int n_tok, int n_heads, int width, int dt
 	return bwd_scratch_layout(bs, n_tok, n_heads, width).bytes; // tie flags, tie header, tie list, shares of d_k
 }
 
+// The single-visit kernel for rows of any pitch, between the tie detector and the repair of the listed ties, and the exact kernel in
+// case the list overflowed.  Returns 1 when nothing was computed (token index beyond 24 bits, too many items).
+int dense_bwd_listed_launch(const void *d_attn, int g_pitch, const void *q, const void *k, void *d_q, void *d_k, void *scratch, int bs,
+			    int n_tok, int n_heads, int width, cudaStream_t st)
+{
+	const float *g = (const float *)d_attn, *qf = (const float *)q, *kf = (const float *)k;
+	int rc = dense_ties_launch(qf, kf, (unsigned char *)scratch, d_k, bs, n_tok, n_heads, width, 1, st);
+	if (!rc)
+		rc = dense_bwd_svr_launch(d_attn, g_pitch, 0, q, k, d_q, d_k, scratch, bs, n_tok, n_heads, width, st);
+	if (!rc)
+		rc = dense_bwd_partsum_launch(d_q, d_k, scratch, bs, n_tok, n_heads, width, st);
+	if (rc)
+		return rc;
+	const int *tie_hdr = (const int *)((const unsigned char *)scratch + bwd_scratch_layout(bs, n_tok, n_heads, width).hdr);
+	rc = launch<float, 8, 4, 2>(g, qf, kf, (float *)d_q, (float *)d_k, bs, n_tok, n_heads, width, tie_hdr, g_pitch, st);
+	return rc ? rc : dense_tiefix_launch(d_attn, g_pitch, d_q, d_k, (const unsigned char *)scratch, bs, n_tok, n_heads, width, -1, st);
+}
+
 int dense_bwd_launch(const void *d_attn, const void *q, const void *k, void *d_q, void *d_k, void *scratch, int bs,
 		     int n_tok, int n_heads, int width, int dtype, cudaStream_t st)
 {
 	if (bs == 0 || n_tok == 0 || n_heads == 0 || width == 0)
 		return L1ATTN_OK;
+	if (n_tok <= BWD_SMALL_TOK)
+		return dense_bwd_small_launch(d_attn, q, k, d_q, d_k, bs, n_tok, n_heads, width, dtype, st);
 	static const bool no_tma = getenv("L1ATTN_NO_TMA") != nullptr; // debugging aid: force the generic kernel
 	static const bool no_sv = getenv("L1ATTN_NO_SV") != nullptr;   // debugging aid: force the two-pass kernel
-	if (!no_tma) {
-		// With scratch the tie detector runs first: it lists every exact tie q == k (and marks tiles, for the case
-		// that the list overflows -- a device-side fact, no host round trip).  Then the single-visit kernel computes
-		// both gradients with the compare form and the listed terms are repaired afterwards.  If the list overflowed
-		// that kernel returns at once and the two-pass kernel, gated on the same word, runs its exact loop where
-		// flagged tiles meet.  Without scratch (or when the detector does not apply) the two-pass kernel runs every
-		// tile with the exact loop.
+	// With scratch the tie detector runs first: it lists every exact tie q == k (and marks tiles, for the case
+	// that the list overflows -- a device-side fact, no host round trip).  Then a single-visit kernel computes
+	// both gradients with the compare form and the listed terms are repaired afterwards.  If the list overflowed
+	// that kernel returns at once and an exact one, gated on the same word, does the call: the two-pass kernel with its
+	// exact loop where flagged tiles meet, or the any-shape kernel.  Without scratch (or when the detector does not apply)
+	// every tile takes the exact loop.
+	const bool listed = scratch && dtype == L1ATTN_F32 && aligned(scratch, 256);
+	bool tma = !no_tma && dtype == L1ATTN_F32 && width % 4 == 0 && n_heads % 4 == 0; // row pitches that TMA can address
+	for (const void *p : {d_attn, q, k, (const void *)d_q, (const void *)d_k})
+		tma = tma && aligned(p, 16);
+	const float *qf = (const float *)q, *kf = (const float *)k;
+	if (tma) {
 		unsigned char *flags = nullptr;
 		const int *tie_hdr = nullptr;
 		int sv = 0;
-		if (scratch && dtype == L1ATTN_F32 && width % 4 == 0 && n_heads % 4 == 0 && aligned(scratch, 256)) {
-			const int trc = dense_ties_launch((const float *)q, (const float *)k, (unsigned char *)scratch, bs, n_tok,
-							  n_heads, width, st);
+		if (listed) {
+			const BwdScratchLayout sl = bwd_scratch_layout(bs, n_tok, n_heads, width);
+			// Both fast kernels are persistent with equal-sized work items, so the last wave of items decides how
+			// full the GPU stays: the single-visit kernel (4 heads x 32 columns x 128 query rows per item, ~8 %
+			// faster per term) runs unless its item count leaves the SMs markedly emptier than the two-pass
+			// kernel's (8 heads x 64 columns x 32 rows per item and gradient) would.
+			int sms = 148;
+			if (const int rc = multiprocessors(&sms))
+				return rc;
+			auto fill = [&](double items) { return bwd_wave_fill(items, sms); };
+			const double it_sv = double(bs) * ((n_heads + 3) / 4) * ((width + 31) / 32) * ((n_tok + 127) / 128) * sl.ns;
+			const double it_tp = 2.0 * bs * ((n_heads + 7) / 8) * ((width + 63) / 64) * ((n_tok + 31) / 32);
+			// (and an item of either kernel is only as busy as its head group is full: 4 heads leave half of an
+			// 8-head item's lanes idle)
+			const double hf_sv = double(n_heads) / (4.0 * ((n_heads + 3) / 4)), hf_tp = double(n_heads) / (8.0 * ((n_heads + 7) / 8));
+			const bool want_sv = !no_sv && 1.08 * fill(it_sv) * hf_sv >= fill(it_tp) * hf_tp;
+			const int trc = dense_ties_launch(qf, kf, (unsigned char *)scratch, d_k, bs, n_tok, n_heads, width, want_sv, st);
 			if (trc < 0)
 				return trc;
 			if (trc == 0) {
-				const BwdScratchLayout sl = bwd_scratch_layout(bs, n_tok, n_heads, width);
-				unsigned char *sc = (unsigned char *)scratch;
-				flags = sc + sl.flags;
-				tie_hdr = (const int *)(sc + sl.hdr);
-				// Both fast kernels are persistent with equal-sized work items, so the last wave of items decides how
-				// full the GPU stays: the single-visit kernel (4 heads x 32 columns x 128 query rows per item, ~8 %
-				// faster per term) runs unless its item count leaves the SMs markedly emptier than the two-pass
-				// kernel's (8 heads x 64 columns x 32 rows per item and gradient) would.
-				int dev = 0, sms = 148;
-				(void)cudaGetDevice(&dev);
-				(void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-				auto fill = [&](double items) { return bwd_wave_fill(items, sms); };
-				const double it_sv = double(bs) * ((n_heads + 3) / 4) * ((width + 31) / 32) * ((n_tok + 127) / 128) * sl.ns;
-				const double it_tp = 2.0 * bs * ((n_heads + 7) / 8) * ((width + 63) / 64) * ((n_tok + 31) / 32);
-				// (and an item of either kernel is only as busy as its head group is full: 4 heads leave half of an
-				// 8-head item's lanes idle)
-				const double hf_sv = double(n_heads) / (4.0 * ((n_heads + 3) / 4)), hf_tp = double(n_heads) / (8.0 * ((n_heads + 7) / 8));
-				if (!no_sv && 1.08 * fill(it_sv) * hf_sv >= fill(it_tp) * hf_tp) {
-					const int frc = dense_bwd_sv_launch(d_attn, q, k, d_q, d_k, tie_hdr, sc + sl.part, sl.ns > 1 ? sc + sl.dqpart : nullptr,
-									    sl.ns, bs, n_tok, n_heads, width, dtype, st);
+				flags = (unsigned char *)scratch + sl.flags;
+				tie_hdr = (const int *)((unsigned char *)scratch + sl.hdr);
+				if (want_sv) {
+					const int frc = dense_bwd_sv_launch(d_attn, q, k, d_q, d_k, scratch, bs, n_tok, n_heads, width, dtype, st);
 					if (frc < 0)
 						return frc;
 					sv = frc == 0;
+					if (!sv) // zero rows are not in the list: the exact loops everywhere
+						flags = nullptr, tie_hdr = nullptr;
 				}
 			}
 		}
@@ -296,17 +325,20 @@ int dense_bwd_launch(const void *d_attn, const void *q, const void *k, void *d_q
 		if (rc < 0)
 			return rc;
 		if (rc == 0)
-			return tie_hdr ? dense_tiefix_launch(d_attn, d_q, d_k, (const unsigned char *)scratch, bs, n_tok, n_heads,
+			return tie_hdr ? dense_tiefix_launch(d_attn, 0, d_q, d_k, (const unsigned char *)scratch, bs, n_tok, n_heads,
 							     width, sv ? -1 : 1, st)
 				       : L1ATTN_OK;
 		if (sv)
 			return L1ATTN_ERR_CUDA; // cannot happen: both fast kernels accept the same shapes and alignments
+	} else if (listed && !no_tma && !no_sv) {
+		const int rc = dense_bwd_listed_launch(d_attn, 0, q, k, d_q, d_k, scratch, bs, n_tok, n_heads, width, st);
+		if (rc <= 0)
+			return rc;
 	}
 	if (dtype == L1ATTN_F32)
-		return launch<float, 8, 4, 2>((const float *)d_attn, (const float *)q, (const float *)k, (float *)d_q,
-					      (float *)d_k, bs, n_tok, n_heads, width, st);
+		return launch<float, 8, 4, 2>((const float *)d_attn, qf, kf, (float *)d_q, (float *)d_k, bs, n_tok, n_heads, width, nullptr, 0, st);
 	return launch<double, 4, 4, 2>((const double *)d_attn, (const double *)q, (const double *)k, (double *)d_q,
-				       (double *)d_k, bs, n_tok, n_heads, width, st);
+				       (double *)d_k, bs, n_tok, n_heads, width, nullptr, 0, st);
 }
 
 } // namespace l1b

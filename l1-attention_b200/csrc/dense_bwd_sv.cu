@@ -141,8 +141,10 @@ dense_bwd_sv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
 		    const float *__restrict__ q, float *__restrict__ d_q, size_t dq_stride, float *__restrict__ part,
 		    const int *__restrict__ tie_hdr, int bs, int n_tok, int n_heads, int width, float scale, SvWork wk, int *err)
 { // d_q, dq_stride: the gradient itself and 0, or (source rows split over wk.ns items) the partial sums' buffer and the size of one
-	if (tie_hdr[1] != 0)
-		return; // too many ties to list: the two-pass kernel computes this call
+	// too many ties to list: the two-pass kernel computes this call; pairs of zero rows to drop: dense_bwd_svr_kernel does (the test and the
+	// dropping in here, even out of line, made calls without padding 1-3 % slower)
+	if (tie_hdr[BWD_HDR_OVERFLOW] != 0 || (tie_hdr[BWD_HDR_ZERO_Q] != 0 && tie_hdr[BWD_HDR_ZERO_K] != 0))
+		return;
 	extern __shared__ __align__(1024) unsigned char smem_raw[];
 	// aligned by OFFSET into the shared array so that the pointers stay in the shared address space
 	unsigned char *base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -352,7 +354,7 @@ __global__ void __launch_bounds__(256)
 dense_bwd_sv_partsum_kernel(const float4 *__restrict__ part, float4 *__restrict__ d_k, const float4 *__restrict__ dq_part,
 			    float4 *__restrict__ d_q, const int *__restrict__ tie_hdr, size_t n4, int ntb, int ns, float scale)
 {
-	if (tie_hdr[1] != 0)
+	if (tie_hdr[BWD_HDR_OVERFLOW] != 0)
 		return;
 	for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += size_t(gridDim.x) * blockDim.x) {
 		float4 s = part[i];
@@ -378,18 +380,41 @@ dense_bwd_sv_partsum_kernel(const float4 *__restrict__ part, float4 *__restrict_
 	}
 }
 
+// As dense_bwd_sv_partsum_kernel, element by element.
+__global__ void __launch_bounds__(256)
+dense_bwd_svr_partsum_kernel(const float *__restrict__ part, float *__restrict__ d_k, const float *__restrict__ dq_part,
+			     float *__restrict__ d_q, const int *__restrict__ tie_hdr, size_t n, int ntb, int ns, float scale)
+{
+	if (tie_hdr[BWD_HDR_OVERFLOW] != 0)
+		return;
+	for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
+		float s = part[i];
+		for (int r = 1; r < ntb; r++)
+			s += part[size_t(r) * n + i];
+		d_k[i] = -scale * s;
+		if (ns > 1) {
+			float t = dq_part[i];
+			for (int r = 1; r < ns; r++)
+				t += dq_part[size_t(r) * n + i];
+			d_q[i] = t;
+		}
+	}
+}
+
 } // namespace
 
 // Returns L1ATTN_OK, a negative error, or 1 when this path does not apply (then nothing was launched).
-// tie_hdr: filled by dense_ties_launch() earlier on the same stream; part, dq_part: the d_k shares and the partial
-// d_q of bwd_scratch_layout() (dq_part is used only when that layout splits the source rows: ns > 1).
-int dense_bwd_sv_launch(const void *d_attn, const void *q, const void *k, void *d_q, void *d_k, const int *tie_hdr,
-			void *part, void *dq_part, int ns, int bs, int n_tok, int n_heads, int width, int dtype, cudaStream_t st)
+// scratch: laid out by bwd_scratch_layout(), its header and lists filled by dense_ties_launch() earlier on the same stream.
+int dense_bwd_sv_launch(const void *d_attn, const void *q, const void *k, void *d_q, void *d_k, void *scratch, int bs, int n_tok,
+			int n_heads, int width, int dtype, cudaStream_t st)
 {
+	const BwdScratchLayout sl = bwd_scratch_layout(bs, n_tok, n_heads, width);
+	unsigned char *sc = static_cast<unsigned char *>(scratch);
+	const int ns = sl.ns;
+	const int *tie_hdr = reinterpret_cast<const int *>(sc + sl.hdr);
+	void *part = sc + sl.part, *dq_part = ns > 1 ? sc + sl.dqpart : nullptr;
 	if (dtype != L1ATTN_F32 || width % 4 != 0 || n_heads % 4 != 0)
 		return 1; // row pitches of k and of d_attn must be multiples of 16 bytes for the tensor maps
-	if (ns < 1 || (ns > 1 && !dq_part))
-		return 1;
 	for (const void *p : {d_attn, q, k, (const void *)d_q, (const void *)d_k, (const void *)part, (const void *)dq_part})
 		if (!aligned(p, 16))
 			return 1;
@@ -427,10 +452,30 @@ int dense_bwd_sv_launch(const void *d_attn, const void *q, const void *k, void *
 							       ns > 1 ? n4 * 4 : size_t(0), (float *)part, tie_hdr, bs, n_tok, n_heads,
 							       width, scale, wk, err);
 	L1B_LAUNCH_CHECK();
-	const size_t want = (n4 + 255) / 256;
-	const unsigned pgrid = unsigned(want < size_t(sms) * 16 ? want : size_t(sms) * 16);
-	dense_bwd_sv_partsum_kernel<<<pgrid, 256, 0, st>>>((const float4 *)part, (float4 *)d_k, (const float4 *)dq_part, (float4 *)d_q,
-							   tie_hdr, n4, int(wk.ntb), ns, scale);
+	if (const int rc = dense_bwd_svr_launch(d_attn, 0, 1, q, k, d_q, d_k, scratch, bs, n_tok, n_heads, width, st))
+		return rc < 0 ? rc : L1ATTN_ERR_SHAPE; // (cannot happen: as many items)
+	return dense_bwd_partsum_launch(d_q, d_k, scratch, bs, n_tok, n_heads, width, st);
+}
+
+// d_k (and, where the source rows are split, d_q) from the shares of either single-visit kernel.
+int dense_bwd_partsum_launch(void *d_q, void *d_k, void *scratch, int bs, int n_tok, int n_heads, int width, cudaStream_t st)
+{
+	const BwdScratchLayout sl = bwd_scratch_layout(bs, n_tok, n_heads, width);
+	const unsigned char *sc = static_cast<const unsigned char *>(scratch);
+	const int *tie_hdr = reinterpret_cast<const int *>(sc + sl.hdr);
+	const float scale = float(-1.0 / sqrt(double(width)));
+	const size_t n = size_t(bs) * n_tok * n_heads * width;
+	const bool vec = n % 4 == 0 && aligned(d_q, 16) && aligned(d_k, 16); // (shares and partial sums start on 256 bytes)
+	const size_t want = (n / (vec ? 4 : 1) + 255) / 256;
+	const unsigned grid = unsigned(want < 148 * 16 ? want : 148 * 16);
+	if (vec)
+		dense_bwd_sv_partsum_kernel<<<grid, 256, 0, st>>>(reinterpret_cast<const float4 *>(sc + sl.part), (float4 *)d_k,
+								  reinterpret_cast<const float4 *>(sc + sl.dqpart), (float4 *)d_q, tie_hdr, n / 4,
+								  sl.ntb, sl.ns, scale);
+	else
+		dense_bwd_svr_partsum_kernel<<<grid, 256, 0, st>>>(reinterpret_cast<const float *>(sc + sl.part), (float *)d_k,
+								   reinterpret_cast<const float *>(sc + sl.dqpart), (float *)d_q, tie_hdr, n, sl.ntb,
+								   sl.ns, scale);
 	L1B_LAUNCH_CHECK();
 	return L1ATTN_OK;
 }

@@ -3,6 +3,7 @@
 #pragma once
 #include <stddef.h>
 #include <cuda_runtime.h>
+#include <stdint.h>
 namespace l1b {
 constexpr int BWD_HG = 8;  // heads per work item
 constexpr int BWD_TX = 32; // x rows (tokens) per work item
@@ -51,9 +52,9 @@ inline double bwd_wave_fill(double items, int sms)
 	const double waves = double((long long)((items + sms - 1) / sms));
 	return waves > 0 ? items / (waves * sms) : 0.0;
 }
-inline int bwd_sv_splits(int bs, int n_tok, int n_heads, int width)
+inline int bwd_sv_splits(int bs, int n_tok, int n_heads, int width, int hg)
 {
-	const double items = double(bs) * ((n_heads + 3) / 4) * ((width + 31) / 32) * ((n_tok + BWD_SV_TX - 1) / BWD_SV_TX);
+	const double items = double(bs) * ((n_heads + hg - 1) / hg) * ((width + 31) / 32) * ((n_tok + 512 / hg - 1) / (512 / hg));
 	const int tiles = (n_tok + 15) / 16;
 	int best = 1;
 	double best_eff = bwd_wave_fill(items, BWD_SV_SMS) * tiles / (tiles + 0.4);
@@ -70,12 +71,33 @@ inline int bwd_sv_splits(int bs, int n_tok, int n_heads, int width)
 	return best;
 }
 
+// Heads per work item of the single-visit kernels: 4 x 128 query rows where TMA reads d_attn and k (both row pitches are
+// multiples of 16 bytes), else 4 x 128, 2 x 256 or 1 x 512, whichever pads the head and the token count least.
+inline int bwd_heads_per_item(int n_tok, int n_heads, int width)
+{
+	if (n_heads % 4 == 0 && width % 4 == 0)
+		return 4;
+	int best = 4;
+	long long least = 0;
+	for (int hg = 4; hg >= 1; hg /= 2) {
+		const long long tx = 512 / hg, padded = ((n_heads + hg - 1) / hg * (long long)hg) * ((n_tok + tx - 1) / tx * tx);
+		if (hg == 4 || padded < least) {
+			best = hg;
+			least = padded;
+		}
+	}
+	return best;
+}
+
+// The tie header: listed ties; set when not every tie is listed; set when some q (k) row is zero in every column
+constexpr int BWD_HDR_COUNT = 0, BWD_HDR_OVERFLOW = 1, BWD_HDR_ZERO_Q = 2, BWD_HDR_ZERO_K = 3;
+
 // Caller-provided scratch of the dense backward, in this order (every part 256-byte aligned):
-//   tie flags | tie header {count, overflow} | tie list uint4[BWD_TIE_CAP] | shares of d_k | partial d_q (if split)
+//   tie flags | tie header | tie list uint4[BWD_TIE_CAP] | shares of d_k | partial d_q (if split)
 // The flags and the header are adjacent so that one memset clears both.
 struct BwdScratchLayout {
 	size_t flags, hdr, ties, part, dqpart, bytes; // offsets, total
-	int ntb, ns;
+	int ntb, ns, hg;
 };
 inline BwdScratchLayout bwd_scratch_layout(int bs, int n_tok, int n_heads, int width)
 {
@@ -85,11 +107,41 @@ inline BwdScratchLayout bwd_scratch_layout(int bs, int n_tok, int n_heads, int w
 	l.hdr = pad(bwd_flag_layout(bs, n_tok, n_heads, width).bytes());
 	l.ties = l.hdr + 256;
 	l.part = l.ties + size_t(BWD_TIE_CAP) * 16;
-	l.ntb = (n_tok + BWD_SV_TX - 1) / BWD_SV_TX;
-	l.ns = bwd_sv_splits(bs, n_tok, n_heads, width);
+	l.hg = bwd_heads_per_item(n_tok, n_heads, width);
+	l.ntb = (n_tok + 512 / l.hg - 1) / (512 / l.hg);
+	l.ns = bwd_sv_splits(bs, n_tok, n_heads, width, l.hg);
 	const size_t n = size_t(bs) * n_tok * n_heads * width * 4;
 	l.dqpart = l.part + pad(size_t(l.ntb) * n);
 	l.bytes = l.dqpart + (l.ns > 1 ? pad(size_t(l.ns) * n) : 0);
 	return l;
 }
+
+// Which rows of q and k are zero in every column (padded tokens), a byte per (batch, token, head) of q, then of k: the detector
+// leaves them in d_k, which nothing writes before the single-visit kernel is through (its shares are summed into d_k
+// by the kernel behind it).  2 bytes a row, where d_k has width * 4.
+struct BwdZeroRows {
+	unsigned char *q, *k;
+};
+inline BwdZeroRows bwd_zero_rows_in(void *d_k, int bs, int n_tok, int n_heads)
+{
+	unsigned char *p = static_cast<unsigned char *>(d_k);
+	return BwdZeroRows{p, p + size_t(bs) * n_tok * n_heads};
+}
+
+constexpr int BWD_SMALL_TOK = 32; // token counts up to here: one exact kernel without scratch (dense_bwd_small.cu)
+
+#ifdef __CUDACC__
+// Four terms of the single-visit backward: four compares, then the eight predicated adds they feed -- the query rows'
+// sums and p, the source row's.
+__device__ __forceinline__ void bwd_sv_terms(float &acc0, float &acc1, float &acc2, float &acc3, float &p, float a0, float a1, float a2,
+					     float a3, float bv, const float4 &g)
+{
+	asm("{\n\t.reg .pred p0, p1, p2, p3;\n\t"
+	    "setp.gt.f32 p0, %5, %9;\n\tsetp.gt.f32 p1, %6, %9;\n\tsetp.gt.f32 p2, %7, %9;\n\tsetp.gt.f32 p3, %8, %9;\n\t"
+	    "@p0 add.f32 %0, %0, %10;\n\t@p1 add.f32 %1, %1, %11;\n\t@p2 add.f32 %2, %2, %12;\n\t@p3 add.f32 %3, %3, %13;\n\t"
+	    "@p0 add.f32 %4, %4, %10;\n\t@p1 add.f32 %4, %4, %11;\n\t@p2 add.f32 %4, %4, %12;\n\t@p3 add.f32 %4, %4, %13;\n\t}"
+	    : "+f"(acc0), "+f"(acc1), "+f"(acc2), "+f"(acc3), "+f"(p)
+	    : "f"(a0), "f"(a1), "f"(a2), "f"(a3), "f"(bv), "f"(g.x), "f"(g.y), "f"(g.z), "f"(g.w));
+}
+#endif
 } // namespace l1b

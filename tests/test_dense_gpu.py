@@ -50,6 +50,20 @@ def test_fwd_bwd_vs_oracle(shape, dtype):
     assert_close(dk, rk, TOL[dtype], "dk %s" % (shape,))
 
 
+# rows that TMA cannot address: groups of 8, 4, 2 and 1 heads, last tiles and last 16-byte pieces of every fill, source rows
+# that are split over several items; and 16-byte rows whose width ends inside a stage or whose heads come in groups of 2 and 1
+RAGGED = [(2, 201, 6, 65), (1, 130, 3, 33), (1, 520, 1, 17), (1, 270, 2, 47), (1, 257, 5, 64), (1, 600, 3, 66), (2, 129, 8, 30),
+          (1, 48, 9, 20), (2, 33, 7, 130), (1, 1040, 1, 7), (1, 513, 1, 48), (1, 300, 2, 36), (2, 70, 8, 40)]
+# sets of at most 32 tokens: both sides of 16, more than eight heads, widths on both sides of 32
+SMALL = [(3, 1, 2, 5), (5, 2, 9, 33), (4, 15, 3, 64), (4, 16, 8, 32), (3, 17, 8, 40), (2, 31, 5, 65), (2, 32, 17, 96)]
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("shape", RAGGED + SMALL)
+def test_ragged_and_small_vs_oracle(shape, dtype):
+    test_fwd_bwd_vs_oracle(shape, dtype)
+
+
 def test_golden_fixtures(golden):
     """Reference outputs (pure-PyTorch and compiled CPU extension) on seeded inputs, incl. the
     tie-heavy and zero-padded cases: sign(0) must be exactly 0."""
@@ -135,6 +149,56 @@ def test_fast_backward_tie_handling(kind, shape):
     dq2, dk2 = (x.cpu().numpy() for x in cabi.dense_bwd(_dev(g), _dev(q), _dev(k), scratch=None))
     assert_close(dq2, rq, 1e-5, "dq exact " + kind)
     assert_close(dk2, rk, 1e-5, "dk exact " + kind)
+
+
+@pytest.mark.parametrize("shape", [(2, 90, 6, 33), (1, 300, 5, 20), (1, 540, 7, 9), (3, 24, 5, 36), (3, 16, 8, 32)])
+@pytest.mark.parametrize("kind", ["sparse_ties", "padded", "q_is_k", "grid"])
+def test_ragged_and_small_tie_handling(kind, shape):
+    test_fast_backward_tie_handling(kind, shape)
+
+
+def test_many_listed_ties_are_repaired():
+    """A few zeros among the values of k rows and several hundred padded q rows: runs of listed ties on one element of d_k,
+    close to as many as the list holds, on rows that stay on the fast path."""
+    from oracle import oracle
+    cabi = _cabi()
+    q, k, g = _rand((1, 1000, 4, 32), np.float32, 35)
+    q[:, 600:] = 0
+    k[0, 7, 0, 3] = k[0, 8, 0, 3] = k[0, 9, 1, 31] = k[0, 500, 3, 0] = k[0, 501, 3, 5] = k[0, 650, 2, 16] = 0
+    k[0, 700:] = 0  # (and padded k rows, so that the fast path drops pairs: 6 x 400 ties are left to the list)
+    rq, rk = oracle.dense_bwd(g.astype(np.float64), q.astype(np.float64), k.astype(np.float64))
+    dq, dk = (x.cpu().numpy() for x in cabi.dense_bwd(_dev(g), _dev(q), _dev(k)))
+    assert_close(dq, rq, 1e-5, "dq")
+    assert_close(dk, rk, 1e-5, "dk")
+    again = cabi.dense_bwd(_dev(g), _dev(q), _dev(k))
+    assert np.array_equal(again[0].cpu().numpy(), dq) and np.array_equal(again[1].cpu().numpy(), dk)
+
+
+@pytest.mark.parametrize("shape", [(2, 200, 8, 64), (1, 1040, 4, 32), (2, 90, 6, 33), (1, 540, 1, 20)])
+def test_zero_rows_beside_zero_values(shape):
+    """Padded tokens, and zeros among the values of other rows: those tie with the padded rows one by one, and with each
+    other; a row that is zero but for its last column is not a padded one.  Non-finite gradients of padded pairs
+    reach nothing."""
+    from oracle import oracle
+    cabi = _cabi()
+    rng = np.random.RandomState(33)
+    bs, n, nh, nw = shape
+    q, k, g = _rand(shape, np.float32, 34)
+    q[:, n - 5:], k[:, n - 9:] = 0, 0
+    q[0, n - 5, 0, nw - 1], k[0, n - 9, 0, nw - 1] = 1e-30, -1e-30
+    q[0, n - 4, 0, 0] = -0.0
+    for x in (q, k):
+        for _ in range(5):
+            x[rng.randint(bs), rng.randint(n - 9), rng.randint(nh), rng.randint(nw)] = 0
+    q[0, 3, nh - 1, 0] = k[0, 4, nh - 1, 0] = 0
+    g2 = g.copy()
+    g2[:, n - 8:, n - 4:] = np.nan
+    g[:, n - 8:, n - 4:] = 0
+    rq, rk = oracle.dense_bwd(g.astype(np.float64), q.astype(np.float64), k.astype(np.float64))
+    for grad in (g, g2):
+        dq, dk = (x.cpu().numpy() for x in cabi.dense_bwd(_dev(grad), _dev(q), _dev(k)))
+        assert_close(dq, rq, 1e-5, "dq")
+        assert_close(dk, rk, 1e-5, "dk")
 
 
 def test_deterministic():
