@@ -107,12 +107,13 @@ int l1attn_dense_fwd(const void *q, const void *k, void *attn,
  * `scratch`: device buffer of l1attn_dense_bwd_scratch_bytes() bytes (256-byte aligned), or NULL.
  * In fp32 a detector kernel proves every exact tie q == k -- the one case the fast inner loop (compare +
  * predicated adds) gets wrong -- and writes them there as a list, which a fix kernel applies after the
- * backward, plus one flag per tile for the case that the list overflows (zero-padded tokens, q == k:
- * flagged tiles then take an exact loop).  The rest of the buffer receives the shares of d_k that the
- * single-visit kernel leaves per block of 128 query rows: ceil(n_tok / 128) * sizeof(d_k) bytes, i.e.
- * about width / 128 times the size of d_attn (plus 2 or 4 times sizeof(d_q) for shapes whose work items
+ * backward, plus one flag per tile for the case that the list overflows (q == k, a coarse grid of values:
+ * flagged tiles then take an exact loop); pairs of rows that are zero in every column (padded tokens) are dropped
+ * without being listed.  The rest of the buffer receives the shares of d_k that the
+ * single-visit kernels leave per block of 128 (256, 512) query rows: ceil(n_tok / 128) * sizeof(d_k) bytes, i.e.
+ * about width / 128 times the size of d_attn (plus 2, 4 or 8 times sizeof(d_q) for shapes whose work items
  * split their source rows: long context with a small batch).  With NULL every tile takes the exact loop and no scratch is
- * needed (same results, about 2.7 times the time in fp32).  Contents need no initialisation and mean
+ * needed (same results, about 2.7 times the time in fp32).  Sets of at most 32 tokens, and fp64, take an exact kernel in any case.  Contents need no initialisation and mean
  * nothing after the call; calls that share a scratch buffer must not overlap on the GPU.
  * Replaces l1attn_cuda_drv.backward (cuda/l1attn_cuda_drv.cpp:67-104) and
  * l1attn_cuda_backward{,32,64} (cuda/l1attn_cuda_kernel.cu:559-685).
@@ -154,6 +155,18 @@ int l1attn_dense_softmax_v_bwd_dx(const void *q, const void *k, const void *v, c
 				  const void *lse, const void *delta, void *dx, void *dv,
 				  int bs, int n_tok, int n_heads, int width, int v_width,
 				  int dtype, void *stream);
+
+/*
+ * The whole backward of l1attn_dense_softmax_v_fwd: dv as above, and dq, dk of the scores.  The gradients of the scores stay in `work`, a
+ * device buffer of l1attn_dense_softmax_v_bwd_bytes() bytes (256-byte aligned; contents need no initialisation and mean nothing
+ * after the call), in whatever order suits the kernels.  Chunks of the batch as above; calls that share a buffer must
+ * not overlap on the GPU.
+ */
+size_t l1attn_dense_softmax_v_bwd_bytes(int bs, int n_tok, int n_heads, int width, int v_width, int dtype);
+int l1attn_dense_softmax_v_bwd(const void *q, const void *k, const void *v, const void *dvo,
+			       const void *lse, const void *delta, void *dq, void *dk, void *dv, void *work,
+			       int bs, int n_tok, int n_heads, int width, int v_width,
+			       int dtype, void *stream);
 
 /* ------------------------------------------------------------------ sparse -------------- */
 

@@ -236,6 +236,29 @@ extern "C" int l1attn_dense_softmax_v_bwd_dx(const void *q, const void *k, const
 					     static_cast<cudaStream_t>(stream));
 }
 
+extern "C" size_t l1attn_dense_softmax_v_bwd_bytes(int bs, int n_tok, int n_heads, int width, int v_width, int dtype)
+{
+	if (bs < 1 || n_tok < 1 || n_heads < 1 || width < 1 || v_width < 1 || (dtype != L1ATTN_F32 && dtype != L1ATTN_F64))
+		return 256;
+	return dense_softmax_v_bwd_bytes(bs, n_tok, n_heads, width, v_width, dtype);
+}
+
+extern "C" int l1attn_dense_softmax_v_bwd(const void *q, const void *k, const void *v, const void *dvo, const void *lse,
+					   const void *delta, void *dq, void *dk, void *dv, void *work, int bs, int n_tok,
+					   int n_heads, int width, int v_width, int dtype, void *stream)
+{
+	const void *ptrs[] = {q, k, v, dvo, lse, delta, dq, dk, dv, work};
+	int rc = check_dense(ptrs, 10, bs, n_tok, n_heads, width, dtype);
+	if (rc)
+		return rc;
+	if (v_width < 1)
+		return L1ATTN_ERR_ARG;
+	if (work && !aligned(work, 256))
+		return L1ATTN_ERR_ALIGN;
+	return dense_softmax_v_bwd_launch(q, k, v, dvo, lse, delta, dq, dk, dv, work, bs, n_tok, n_heads, width, v_width, dtype,
+					  static_cast<cudaStream_t>(stream));
+}
+
 extern "C" size_t l1attn_dense_bwd_scratch_bytes(int bs, int n_tok, int n_heads, int width, int dtype)
 {
 	return dense_bwd_scratch_bytes(bs, n_tok, n_heads, width, dtype);

@@ -22,6 +22,7 @@
 #include <stdlib.h>
 #include "common.cuh"
 #include "tma.cuh"
+#include "dense_bwd_tiles.h"
 
 namespace l1b {
 namespace {
@@ -137,6 +138,7 @@ constexpr int MAX_STAGE = 3;
 
 struct SvShape {
 	int n_tok, n_heads, width, v_width, nwb, nstage, ntt, mode;
+	int dx_pitch; // backward: 0 = dx as d_attn lies, [b][s][t][h]; else [b][h][s][t] in rows of that many floats
 	float scale;
 };
 
@@ -145,7 +147,7 @@ struct SvShape {
 // `base` is the head's row of token 0.  Slices of 32 columns: [slice][row] of 128 bytes, SWZ: 16-byte chunk ^= row & 7;
 // !SWZ: [row][32 * slices].  Columns >= width and tokens >= n_tok become zeros.  The copies are ~16 per thread and tile against
 // ~2500 instructions of math: [4,300,5,33], values 21 wide, takes 31 us forward and 38 us backward (dx, dv), [4,333,6,48],
-// values 40 wide, through TMA 34 and 48 us; the any-shape kernels took about 290 and 740 us for the latter.
+// values 40 wide, through TMA 34 and 48 us (the whole pass with the any-shape kernels 1633 us, with these 373).
 template <int NW, bool SWZ>
 __device__ __forceinline__ void copy_rows(unsigned char *dst, const float *base, size_t pitch, int t0, int rows, int nslice, int width, int n_tok)
 {
@@ -446,7 +448,8 @@ size_t sv_smem(int nwb, int nv, int tt_rows, int nstage)
 // (query rows per half-warp, warps, ring stages) of the tiled kernels.  4 x 16 and 8 x 8 make a 128-row CTA, 4 x 8 a 64-row
 // one.  Sixteen warps of 128 registers measured 7 % faster than eight of 168 (four warps per scheduler hide the
 // shared-memory and arithmetic latencies); with 128 value columns the thread state does not fit 128 registers.  A 64-row CTA
-// takes SHORT_CTA of the time of a 128-row one; it is taken where the rows do not fit shared memory otherwise, or where its
+// takes SHORT_CTA of the time of a 128-row one (forward 41 / 66 us at [4,333,6,64], 97 / 164 at [1,1024,8,64]; 56 / 88 with 128 value
+// columns; two waves of it against one 1.13-1.17); it is taken where the rows do not fit shared memory otherwise, or where its
 // finer grid fills the SMs better (few rows in all, or few left over for the last wave).
 struct TilePlan {
 	int ti, nw, nstage; // nstage 0: no form fits
@@ -664,6 +667,8 @@ softmax_v_bwd_tile_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
 		dead = true;
 	float *Pw = Ps + tg * PP;
 	const size_t hstride = size_t(sh.n_heads);
+	const size_t dx_t = sh.dx_pitch > 0 ? 1 : hstride, dx_s = sh.dx_pitch > 0 ? size_t(sh.dx_pitch) : hstride * sh.n_tok;
+	const size_t dx0 = sh.dx_pitch > 0 ? (size_t(b) * sh.n_heads + h) * sh.n_tok * sh.dx_pitch : size_t(b) * sh.n_tok * sh.n_tok * hstride + h;
 
 	for (int m = 0; m < nt; m++) {
 		if ((!TMA || (warp == m % NW && lane == 0)) && m + sh.nstage - 1 < nt && !dead) {
@@ -756,14 +761,15 @@ softmax_v_bwd_tile_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
 #pragma unroll
 		for (int i = 0; i < TI; i++) {
 			const int s = s0 + i * (2 * NW) + tg;
-			float *dxr = dx + ((size_t(b) * sh.n_tok + (s < sh.n_tok ? s : 0)) * sh.n_tok) * hstride + h;
+			float *dxr = dx + dx0 + size_t(s < sh.n_tok ? s : 0) * dx_s;
 #pragma unroll
 			for (int j = 0; j < 4; j++) {
 				const int t = m * TS + j * 16 + sg;
 				const float p = expf(acc[i][j] * sh.scale - lj[j]);
 				Pw[i * (2 * NW) * PP + j * 16 + sg] = p;
+				// (equal rows: the distance has no slope in any column, so its gradient reaches neither)
 				if (s < sh.n_tok && t < sh.n_tok)
-					dxr[size_t(t) * hstride] = p * (dp[i][j] - dj[j]);
+					dxr[size_t(t) * dx_t] = sh.dx_pitch > 0 && acc[i][j] == 0.f ? 0.f : p * (dp[i][j] - dj[j]);
 			}
 		}
 		__syncwarp();
@@ -830,7 +836,8 @@ size_t sv_bwd_smem(int nwb, int nv, int tt_rows, int nstage)
 
 template <int NV, int TI, int NW, bool TMA, bool FULL>
 int launch_bwd_tile(const float *q, const float *k, const float *v, const float *dvo, const float *lse, const float *delta,
-		    float *dx, float *dv, int bs, int n_tok, int n_heads, int width, int v_width, int nstage, size_t smem, cudaStream_t st)
+		    float *dx, int dx_pitch, float *dv, int bs, int n_tok, int n_heads, int width, int v_width, int nstage, size_t smem,
+		    cudaStream_t st)
 {
 	constexpr int TT = 2 * NW * TI, NTH = NW * 32;
 	const uint64_t dims[4] = {uint64_t(width), uint64_t(n_heads), uint64_t(n_tok), uint64_t(bs)};
@@ -856,6 +863,7 @@ int launch_bwd_tile(const float *q, const float *k, const float *v, const float 
 	sh.nstage = nstage;
 	sh.ntt = (n_tok + TT - 1) / TT;
 	sh.mode = 0;
+	sh.dx_pitch = dx_pitch;
 	sh.scale = float(-1.0 / sqrt(double(width)));
 	const long long grid = (long long)bs * n_heads * sh.ntt;
 	if (grid > 0x7fffffffLL)
@@ -868,7 +876,7 @@ int launch_bwd_tile(const float *q, const float *k, const float *v, const float 
 }
 
 int softmax_v_bwd_tile(const float *q, const float *k, const float *v, const float *dvo, const float *lse, const float *delta,
-		       float *dx, float *dv, int bs, int n_tok, int n_heads, int width, int v_width, cudaStream_t st)
+		       float *dx, int dx_pitch, float *dv, int bs, int n_tok, int n_heads, int width, int v_width, cudaStream_t st)
 {
 	if (width > 128 || v_width > 128)
 		return 1;
@@ -879,7 +887,7 @@ int softmax_v_bwd_tile(const float *q, const float *k, const float *v, const flo
 	if (!p.nstage)
 		return 1;
 #define L1B_SVB_RUN(NV_, TI_, NW_, TMA_, FULL_) \
-	launch_bwd_tile<NV_, TI_, NW_, TMA_, FULL_>(q, k, v, dvo, lse, delta, dx, dv, bs, n_tok, n_heads, width, v_width, p.nstage, p.smem, st)
+	launch_bwd_tile<NV_, TI_, NW_, TMA_, FULL_>(q, k, v, dvo, lse, delta, dx, dx_pitch, dv, bs, n_tok, n_heads, width, v_width, p.nstage, p.smem, st)
 #define L1B_SVB(NV_, TI_, NW_)                                                                                                   \
 	if (nv == NV_ && p.ti == TI_ && p.nw == NW_) {                                                                           \
 		const int rc = !tma ? 1 : full ? L1B_SVB_RUN(NV_, TI_, NW_, true, true) : L1B_SVB_RUN(NV_, TI_, NW_, true, false); \
@@ -921,7 +929,7 @@ int dense_softmax_v_bwd_dx_launch(const void *q, const void *k, const void *v, c
 	static const bool no_tma = getenv("L1ATTN_NO_TMA") != nullptr;
 	if (dtype == L1ATTN_F32 && !no_tma && width > 0) {
 		const int rc = softmax_v_bwd_tile((const float *)q, (const float *)k, (const float *)v, (const float *)dvo,
-						 (const float *)lse, (const float *)delta, (float *)dx, (float *)dv, bs, n_tok, n_heads,
+						 (const float *)lse, (const float *)delta, (float *)dx, 0, (float *)dv, bs, n_tok, n_heads,
 						 width, v_width, st);
 		if (rc <= 0)
 			return rc;
@@ -933,6 +941,41 @@ int dense_softmax_v_bwd_dx_launch(const void *q, const void *k, const void *v, c
 	return launch_bwd_generic((const double *)q, (const double *)k, (const double *)v, (const double *)dvo,
 				  (const double *)lse, (const double *)delta, (double *)dx, (double *)dv, bs, n_tok, n_heads, width,
 				  v_width, st);
+}
+
+// Workspace of the whole backward: dx, then the dense backward's scratch.
+static size_t sv_dx_bytes(int bs, int n_tok, int n_heads, int dtype)
+{
+	const size_t es = dtype == L1ATTN_F64 ? 8 : 4, pitch = (size_t(n_tok) + 3) / 4 * 4; // rows of dx as the tiled kernels write them
+	return (size_t(bs) * n_heads * n_tok * pitch * es + 255) / 256 * 256;
+}
+size_t dense_softmax_v_bwd_bytes(int bs, int n_tok, int n_heads, int width, int, int dtype)
+{
+	return sv_dx_bytes(bs, n_tok, n_heads, dtype) + dense_bwd_scratch_bytes(bs, n_tok, n_heads, width, dtype);
+}
+
+// dx lies [b][h][s][t] between its two kernels: the tiled kernel that makes it owns one head, and in d_attn's order, heads innermost, each of
+// its 4-byte stores touched a sector of its own (32 sectors per warp store, about as many cycles of the load/store pipe as its shared
+// reads take); the kernel that consumes it reads 16 bytes of a row at once and has nothing to transpose.
+int dense_softmax_v_bwd_launch(const void *q, const void *k, const void *v, const void *dvo, const void *lse, const void *delta,
+			       void *dq, void *dk, void *dv, void *work, int bs, int n_tok, int n_heads, int width, int v_width,
+			       int dtype, cudaStream_t st)
+{
+	if (bs == 0 || n_tok == 0 || n_heads == 0)
+		return L1ATTN_OK;
+	static const bool no_tma = getenv("L1ATTN_NO_TMA") != nullptr, no_sv = getenv("L1ATTN_NO_SV") != nullptr;
+	void *scratch = static_cast<unsigned char *>(work) + sv_dx_bytes(bs, n_tok, n_heads, dtype);
+	if (dtype == L1ATTN_F32 && !no_tma && !no_sv && n_tok > BWD_SMALL_TOK && n_tok < (1 << 24)) {
+		const int pitch = (n_tok + 3) / 4 * 4;
+		int rc = softmax_v_bwd_tile((const float *)q, (const float *)k, (const float *)v, (const float *)dvo, (const float *)lse,
+					    (const float *)delta, (float *)work, pitch, (float *)dv, bs, n_tok, n_heads, width, v_width, st);
+		if (!rc)
+			rc = dense_bwd_listed_launch(work, pitch, q, k, dq, dk, scratch, bs, n_tok, n_heads, width, st);
+		if (rc <= 0)
+			return rc;
+	}
+	const int rc = dense_softmax_v_bwd_dx_launch(q, k, v, dvo, lse, delta, work, dv, bs, n_tok, n_heads, width, v_width, dtype, st);
+	return rc ? rc : dense_bwd_launch(work, q, k, dq, dk, scratch, bs, n_tok, n_heads, width, dtype, st);
 }
 
 } // namespace l1b

@@ -30,6 +30,8 @@ SIGNATURES = {
     "l1attn_test_wait_timeout": (_i, [_i, _vp, _vp]),
     "l1attn_dense_fwd": (_i, [_vp] * 3 + [_i] * 5 + [_vp]),
     "l1attn_dense_softmax_v_fwd": (_i, [_vp] * 5 + [_i] * 7 + [_vp]),
+    "l1attn_dense_softmax_v_bwd_bytes": (_sz, [_i] * 6),
+    "l1attn_dense_softmax_v_bwd": (_i, [_vp] * 10 + [_i] * 6 + [_vp]),
     "l1attn_dense_softmax_v_bwd_dx": (_i, [_vp] * 8 + [_i] * 6 + [_vp]),
     "l1attn_dense_bwd_scratch_bytes": (_sz, [_i] * 5),
     "l1attn_dense_bwd": (_i, [_vp] * 6 + [_i] * 5 + [_vp]),
@@ -268,6 +270,23 @@ def dense_softmax_v_bwd_dx(q, k, v, dvo, lse, delta, dx, dv):
     assert dx.shape == (bs, n, n, h) and dv.shape == v.shape and lse.shape == (bs, n, h) and delta.shape == (bs, n, h)
     _check(lib().l1attn_dense_softmax_v_bwd_dx(_dp(q), _dp(k), _dp(v), _dp(dvo), _dp(lse), _dp(delta), _dp(dx), _dp(dv),
                                                bs, n, h, w, v.shape[3], _tdt(q), _stream()), "l1attn_dense_softmax_v_bwd_dx")
+
+
+def dense_softmax_v_bwd_work(q, v, items):
+    """Device buffer for dense_softmax_v_bwd on up to `items` batch items of q, v."""
+    import torch
+    _, n, h, w = q.shape
+    nb = lib().l1attn_dense_softmax_v_bwd_bytes(items, n, h, w, v.shape[3], _tdt(q))
+    return torch.empty(nb, dtype=torch.uint8, device=q.device)
+
+
+def dense_softmax_v_bwd(q, k, v, dvo, lse, delta, dq, dk, dv, work):
+    """Whole backward of dense_softmax_v_fwd; fills dq, dk, dv.  work: dense_softmax_v_bwd_work()."""
+    bs, n, h, w = q.shape
+    for t in (q, k, v, dvo, lse, delta, dq, dk, dv):
+        assert t.is_cuda and t.is_contiguous() and t.dtype == q.dtype
+    _check(lib().l1attn_dense_softmax_v_bwd(_dp(q), _dp(k), _dp(v), _dp(dvo), _dp(lse), _dp(delta), _dp(dq), _dp(dk), _dp(dv),
+                                            _dp(work), bs, n, h, w, v.shape[3], _tdt(q), _stream()), "l1attn_dense_softmax_v_bwd")
 
 
 def dense_bwd(d_attn, q, k, out=None, scratch="auto"):

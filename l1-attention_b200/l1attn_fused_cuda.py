@@ -13,8 +13,8 @@ all-zero source row, or plain exp).  `l1attn_cuda.L1Attn` itself is unchanged.
 
 Forward: one kernel (`l1attn_dense_softmax_v_fwd`), nothing of size n x n is stored; it keeps the log
 of every query row's normaliser ([bs, n, h]) for the backward.
-Backward, a few batch items at a time: `l1attn_dense_softmax_v_bwd_dx` recomputes the weights and
-writes the score gradients dx [c, n, n, h] and dv; the library's dense backward turns dx into dq, dk.
+Backward, a few batch items at a time (`l1attn_dense_softmax_v_bwd`): one kernel recomputes the weights and
+writes the score gradients dx and dv; the library's dense backward turns dx into dq, dk.
 The only n x n tensor alive is that one chunk of dx (256 MB by default).
 """
 import torch
@@ -55,12 +55,10 @@ class L1AttnSoftmaxVFn(torch.autograd.Function):
         delta = torch.zeros_like(lse) if ctx.mode == "exp" else (dvo * vo).sum(-1)
         step = max(1, min(bs, _CHUNK_BYTES // max(1, n * n * h * q.element_size())))
         with torch.cuda.device(q.device):
-            dx = torch.empty((step, n, n, h), dtype=q.dtype, device=q.device)
+            work = _c.dense_softmax_v_bwd_work(q, v, step)
             for b0 in range(0, bs, step):
                 sl = slice(b0, min(bs, b0 + step))  # leading-dimension slices of contiguous tensors stay contiguous
-                c = sl.stop - sl.start
-                _c.dense_softmax_v_bwd_dx(q[sl], k[sl], v[sl], dvo[sl], lse[sl], delta[sl], dx[:c], dv[sl])
-                _c.dense_bwd(dx[:c], q[sl], k[sl], out=(dq[sl], dk[sl]))
+                _c.dense_softmax_v_bwd(q[sl], k[sl], v[sl], dvo[sl], lse[sl], delta[sl], dq[sl], dk[sl], dv[sl], work)
         return dq, dk, dv, None
 
 

@@ -125,6 +125,32 @@ def test_autograd_matches_the_unfused_chain(mode, dtype, dims):
         assert_close(a_.cpu().numpy(), b_.cpu().numpy(), tol, "%s %s" % (name, mode))
 
 
+@pytest.mark.parametrize("dims", [(2, 70, 4, 32, 32), (1, 45, 3, 40, 24), (1, 90, 2, 33, 20), (2, 20, 2, 32, 32)])
+@pytest.mark.parametrize("kind", ["equal_rows", "padded", "grid"])
+def test_backward_with_equal_rows_and_ties(dims, kind):
+    """Equal query and key rows (the distance has no slope in any column), padded tokens, and ties everywhere (more than
+    the list holds), against torch's own chain in float64, whose |x| has slope 0 at 0."""
+    import l1attn_fused_cuda
+    torch.manual_seed(3)
+    bs, n, h, w, wv = dims
+    q, k = (0.3 * torch.randn(bs, n, h, w, device="cuda") for _ in range(2))
+    if kind == "equal_rows":
+        k[:, 3:9] = q[:, 5:11]
+    elif kind == "padded":
+        q[:, n - 7:], k[:, n - 7:] = 0, 0
+        k[0, 2, 0, 1] = 0
+    else:
+        q, k = (q * 4).round() / 4, (k * 4).round() / 4
+    v, g = torch.randn(bs, n, h, wv, device="cuda"), torch.randn(bs, n, h, wv, device="cuda")
+    got = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    l1attn_fused_cuda.L1AttnSoftmaxV()(*got).backward(g)
+    ref = [t.double().requires_grad_(True) for t in (q, k, v)]
+    x = -(ref[0][:, None] - ref[1][:, :, None]).abs().sum(-1) / w ** 0.5
+    torch.einsum("bsdh,bshw->bdhw", torch.softmax(x, 1), ref[2]).backward(g.double())
+    for name, a, b in zip(("dq", "dk", "dv"), got, ref):
+        assert_close(a.grad.cpu().numpy(), b.grad.cpu().numpy(), 1e-5, name)
+
+
 def test_backward_chunks_over_the_batch(monkeypatch):
     """The backward walks the batch in chunks; a chunk size of one item must give the same gradients."""
     import l1attn_fused_cuda
