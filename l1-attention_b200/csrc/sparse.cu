@@ -147,6 +147,11 @@ template <int VEC, bool EX> __device__ __forceinline__ bool in_row(int li, int i
 // loaded by the lanes of the warp together and handed out by shuffles, 32 at a time (as many as lanes are left): with one
 // load per entry the row fetches of every entry waited for an index first, and the lists of incoming edges cost an
 // integer division per entry instead of one per lane.
+// The entries whose rows a lane has under way at a time, of the backward's walks (two rows per entry): short rows come several at a time, so that
+// a lane has four vectors of either row in flight whatever the width (one entry at a time: the bidirectional case below 258 us,
+// these 250).
+constexpr int entries_in_flight(int nx) { return nx >= 4 ? 1 : 4 / (nx > 0 ? nx : 1); }
+
 template <typename T, int VEC, int NX> __device__ __forceinline__ void zero_acc(Pack<T, VEC> (&acc)[NX])
 {
 #pragma unroll
@@ -188,7 +193,7 @@ __global__ void __launch_bounds__(CTA) sparse_fwd_dst_kernel(SparseArgs a, const
 	const int step = lph * VEC;
 
 	if constexpr (NX > 0) {
-		constexpr int FU = NX > 2 ? 1 : 2; // slots in flight per lane: FU * NX vectors each of k and v
+		constexpr int FU = NX > 2 ? 1 : 2; // slots in flight per lane (four of one vector measured 106 us against 94 at 2 heads)
 		Pack<T, VEC> qv[NX], acc[NX];
 #pragma unroll
 		for (int it = 0; it < NX; it++)
@@ -340,7 +345,7 @@ __global__ void __launch_bounds__(CTA) sparse_fwd_src_kernel(SparseArgs a, const
 	if constexpr (NX > 0) {
 		Pack<T, VEC> acc[NX];
 		zero_acc(acc);
-		constexpr int UE = 2; // entries in flight per lane
+		constexpr int UE = NX > 2 || VEC * sizeof(T) > 16 ? 2 : 4; // entries in flight per lane (one row each)
 		const S *bbase = vb + (tokrow * H + w.h) * Wv + w.li * VEC;
 		const S *abase = attn + (tokrow * dm) * H + w.h;
 		int slot_l = 0, dst_l = 0;
@@ -418,7 +423,7 @@ __global__ void __launch_bounds__(CTA) sparse_fwd_src_kernel(SparseArgs a, const
 // with four vectors (up to 168 when bidirectional: dvo[src] and d_vb come on top).  The generic branch walks the
 // list once per quantity and is capped at 24 warps per SM.
 template <typename T, int VEC, int LPHC, int NX, bool EX, bool BIDI>
-__global__ void __launch_bounds__(CTA, (NX == 4 ? 4 : 6) - (BIDI && NX > 0 ? 1 : 0)) sparse_bwd_dst_kernel(SparseArgs a, const T *__restrict__ dvo,
+__global__ void __launch_bounds__(CTA, (NX == 4 ? 4 : NX > 0 ? 5 : 6) - (BIDI && NX > 0 ? 1 : 0)) sparse_bwd_dst_kernel(SparseArgs a, const T *__restrict__ dvo,
 							      const T *__restrict__ v, const T *__restrict__ vb,
 							      const T *__restrict__ q, const T *__restrict__ k,
 							      const T *__restrict__ attn, T *dx, T *__restrict__ d_q,
@@ -462,56 +467,68 @@ __global__ void __launch_bounds__(CTA, (NX == 4 ? 4 : 6) - (BIDI && NX > 0 ? 1 :
 		for (int rb = 0; rb < dm; rb += 32) {
 			int mine;
 			const int n = next_slots(slots, rb, dm, mine);
-			for (int i = 0; i < n; i++) {
-				const int src = __shfl_sync(0xffffffffu, mine, i), r = rb + i;
-				const bool ok = w.head_ok && src >= 0;
-				const size_t so = size_t(ok ? src : 0) * H;
-				Pack<T, VEC> vr[NX], kr[NX], gr[NX];
+			constexpr int FU = entries_in_flight(NX);
+			for (int i = 0; i < n; i += FU) {
+				Pack<T, VEC> vr[FU][NX], kr[FU][NX], gr[FU][BIDI ? NX : 1];
+				T ar[FU], part[FU];
+				bool ok[FU];
 #pragma unroll
-				for (int it = 0; it < NX; it++) {
-					vr[it] = ldv<T, VEC>(vbase + so * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
-					kr[it] = ldv<T, VEC>(kbase + so * W + it * step, in_row<VEC, EX>(w.li, it, step, W));
-				}
-				if (BIDI) {
+				for (int u = 0; u < FU; u++) { // (FU divides 32; past n: empty)
+					const int src = __shfl_sync(0xffffffffu, mine, i + u);
+					ok[u] = w.head_ok && src >= 0;
+					const size_t so = size_t(ok[u] ? src : 0) * H;
 #pragma unroll
-					for (int it = 0; it < NX; it++)
-						gr[it] = ldv<T, VEC>(gbase + so * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
-				}
-				const T ar = ok ? arow[size_t(r) * H] : T(0);
-				T part = T(0);
-#pragma unroll
-				for (int it = 0; it < NX; it++)
-#pragma unroll
-					for (int i = 0; i < VEC; i++)
-						part += vr[it].v[i] * gd[it].v[i];
-				if (BIDI) {
-#pragma unroll
-					for (int it = 0; it < NX; it++)
-#pragma unroll
-						for (int i = 0; i < VEC; i++)
-							part += bd[it].v[i] * gr[it].v[i];
-				}
-				part = group_sum<LPHC>(part, lph);
-				if (!ok)
-					continue; // (uniform over the lanes of a head; the shuffles above ran for the whole warp)
-				S += ar * part;
-				if (w.li == 0)
-					xrow[size_t(r) * H] = part;
-				const T w1 = ar * part;
-#pragma unroll
-				for (int it = 0; it < NX; it++)
-#pragma unroll
-					for (int i = 0; i < VEC; i++) {
-						const T sg = sign_apply(qv[it].v[i] - kr[it].v[i], T(1));
-						acc1[it].v[i] += sg * w1;
-						acc2[it].v[i] += sg * ar;
+					for (int it = 0; it < NX; it++) {
+						vr[u][it] = ldv<T, VEC>(vbase + so * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
+						kr[u][it] = ldv<T, VEC>(kbase + so * W + it * step, in_row<VEC, EX>(w.li, it, step, W));
 					}
-				if (BIDI) {
+					if constexpr (BIDI) {
+#pragma unroll
+						for (int it = 0; it < NX; it++)
+							gr[u][it] = ldv<T, VEC>(gbase + so * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
+					}
+					ar[u] = ok[u] ? arow[size_t(rb + i + u) * H] : T(0);
+				}
+#pragma unroll
+				for (int u = 0; u < FU; u++) {
+					part[u] = T(0);
 #pragma unroll
 					for (int it = 0; it < NX; it++)
 #pragma unroll
-						for (int i = 0; i < VEC; i++)
-							accb[it].v[i] += ar * gr[it].v[i];
+						for (int j = 0; j < VEC; j++)
+							part[u] += vr[u][it].v[j] * gd[it].v[j];
+					if constexpr (BIDI) {
+#pragma unroll
+						for (int it = 0; it < NX; it++)
+#pragma unroll
+							for (int j = 0; j < VEC; j++)
+								part[u] += bd[it].v[j] * gr[u][it].v[j];
+					}
+					part[u] = group_sum<LPHC>(part[u], lph);
+				}
+#pragma unroll
+				for (int u = 0; u < FU; u++) {
+					if (!ok[u])
+						continue; // (uniform over the lanes of a head; the shuffles above ran for the whole warp)
+					const T w1 = ar[u] * part[u];
+					S += w1;
+					if (w.li == 0)
+						xrow[size_t(rb + i + u) * H] = part[u];
+#pragma unroll
+					for (int it = 0; it < NX; it++)
+#pragma unroll
+						for (int j = 0; j < VEC; j++) {
+							const T sg = sign_apply(qv[it].v[j] - kr[u][it].v[j], T(1));
+							acc1[it].v[j] += sg * w1;
+							acc2[it].v[j] += sg * ar[u];
+						}
+					if constexpr (BIDI) {
+#pragma unroll
+						for (int it = 0; it < NX; it++)
+#pragma unroll
+							for (int j = 0; j < VEC; j++)
+								accb[it].v[j] += ar[u] * gr[u][it].v[j];
+					}
 				}
 			}
 		}
@@ -656,7 +673,7 @@ __global__ void __launch_bounds__(CTA, (NX == 4 ? 4 : 6) - (BIDI && NX > 0 ? 1 :
 
 // ---- backward, src pass: d_v[src] = sum a dvo[dst];  d_k[src] = -scale sum sign(q[dst]-k[src]) dx ----
 template <typename T, int VEC, int LPHC, int NX, bool EX>
-__global__ void __launch_bounds__(CTA, NX == 4 ? 4 : 6) sparse_bwd_src_kernel(SparseArgs a, const T *__restrict__ dvo,
+__global__ void __launch_bounds__(CTA, NX == 4 ? 4 : NX > 0 ? 5 : 6) sparse_bwd_src_kernel(SparseArgs a, const T *__restrict__ dvo,
 							      const T *__restrict__ q, const T *__restrict__ k,
 							      const T *__restrict__ attn, const T *__restrict__ dx,
 							      T *__restrict__ d_v, T *__restrict__ d_k, T scale)
@@ -686,29 +703,38 @@ __global__ void __launch_bounds__(CTA, NX == 4 ? 4 : 6) sparse_bwd_src_kernel(Sp
 		const T *gbase = dvo + (tokrow * H + w.h) * Wv + w.li * VEC, *qbase = q + (tokrow * H + w.h) * W + w.li * VEC;
 		const T *abase = attn + (tokrow * dm) * H + w.h, *xbase = dx + (tokrow * dm) * H + w.h;
 		int slot_l = 0, dst_l = 0;
-		for (int e = e0, i = 0; e < e1; e++, i++) {
+		constexpr int FU = entries_in_flight(NX);
+		for (int e = e0, i = 0; e < e1; e += FU, i += FU) {
 			if (i == nact)
 				i = 0;
 			if (i == 0) {
 				slot_l = e + lane < e1 ? a.csc_slot[e + lane] : 0;
 				dst_l = slot_l / dm;
 			}
-			const int slot = __shfl_sync(act, slot_l, i);
-			const size_t d = size_t(__shfl_sync(act, dst_l, i)) * H;
-			Pack<T, VEC> gr[NX], qr[NX];
+			Pack<T, VEC> gr[FU][NX], qr[FU][NX];
+			T ar[FU], dxr[FU];
 #pragma unroll
-			for (int it = 0; it < NX; it++) {
-				gr[it] = ldv<T, VEC>(gbase + d * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
-				qr[it] = ldv<T, VEC>(qbase + d * W + it * step, in_row<VEC, EX>(w.li, it, step, W));
-			}
-			const T ar = abase[size_t(slot) * H], dxr = xbase[size_t(slot) * H];
+			for (int u = 0; u < FU; u++) { // past the end of the list: slot 0, read but not used (nact is a multiple of four)
+				const int slot = __shfl_sync(act, slot_l, i + u);
+				const size_t d = size_t(__shfl_sync(act, dst_l, i + u)) * H;
 #pragma unroll
-			for (int it = 0; it < NX; it++)
-#pragma unroll
-				for (int i = 0; i < VEC; i++) {
-					accv[it].v[i] += ar * gr[it].v[i];
-					acck[it].v[i] += sign_apply(qr[it].v[i] - kv[it].v[i], dxr);
+				for (int it = 0; it < NX; it++) {
+					gr[u][it] = ldv<T, VEC>(gbase + d * Wv + it * step, in_row<VEC, EX>(w.li, it, step, Wv));
+					qr[u][it] = ldv<T, VEC>(qbase + d * W + it * step, in_row<VEC, EX>(w.li, it, step, W));
 				}
+				ar[u] = abase[size_t(slot) * H];
+				dxr[u] = xbase[size_t(slot) * H];
+			}
+#pragma unroll
+			for (int u = 0; u < FU; u++)
+				if (e + u < e1)
+#pragma unroll
+					for (int it = 0; it < NX; it++)
+#pragma unroll
+						for (int j = 0; j < VEC; j++) {
+							accv[it].v[j] += ar[u] * gr[u][it].v[j];
+							acck[it].v[j] += sign_apply(qr[u][it].v[j] - kv[it].v[j], dxr[u]);
+						}
 		}
 		T *orow = d_k + ((tokrow + src) * H + w.h) * W + w.li * VEC;
 #pragma unroll
