@@ -650,9 +650,10 @@ def roofline_of(wl, t, pk, clocks, l2_gbs=None):
     return roof, None
 
 
-# kernels of this library per dense step: forward; tie detector; single-visit backward; sum of the d_k shares;
-# two-pass kernel (returns at once unless the tie list overflowed); tie fix
-DENSE_LAUNCHES_PER_STEP = 6
+# kernels of this library per dense step: forward; tie detector; single-visit backward; its form for inputs with zero rows
+# (returns at once unless there are pairs of them); sum of the d_k shares; two-pass kernel (returns at once unless
+# the tie list overflowed); tie fix
+DENSE_LAUNCHES_PER_STEP = 7
 # ncu dram__bytes_read.sum + dram__bytes_write.sum per launch at the profiling sizes (profiles/*.md)
 DENSE_BWD_TRAFFIC_B2 = 198.8e6
 SPARSE_TRAFFIC_B2 = 226.9e6
