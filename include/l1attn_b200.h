@@ -114,7 +114,8 @@ int l1attn_dense_fwd(const void *q, const void *k, void *attn,
  * about width / 128 times the size of d_attn (plus 2, 4 or 8 times sizeof(d_q) for shapes whose work items
  * split their source rows: long context with a small batch).  With NULL every tile takes the exact loop and no scratch is
  * needed (same results, about 2.7 times the time in fp32).  Sets of at most 32 tokens, and fp64, take an exact kernel in any case.  Contents need no initialisation and mean
- * nothing after the call; calls that share a scratch buffer must not overlap on the GPU.
+ * nothing after the call; calls that share a scratch buffer must not overlap on the GPU.  A smaller batch may need more
+ * (its source rows may be split over more ranges): a buffer that serves several batch sizes has the largest of their sizes.
  * Replaces l1attn_cuda_drv.backward (cuda/l1attn_cuda_drv.cpp:67-104) and
  * l1attn_cuda_backward{,32,64} (cuda/l1attn_cuda_kernel.cu:559-685).
  */
@@ -159,8 +160,8 @@ int l1attn_dense_softmax_v_bwd_dx(const void *q, const void *k, const void *v, c
 /*
  * The whole backward of l1attn_dense_softmax_v_fwd: dv as above, and dq, dk of the scores.  The gradients of the scores stay in `work`, a
  * device buffer of l1attn_dense_softmax_v_bwd_bytes() bytes (256-byte aligned; contents need no initialisation and mean nothing
- * after the call), in whatever order suits the kernels.  Chunks of the batch as above; calls that share a buffer must
- * not overlap on the GPU.
+ * after the call), in whatever order suits the kernels.  Chunks of the batch as above: the size stated for bs items serves every
+ * call of 1 .. bs items.  Calls that share a buffer must not overlap on the GPU.
  */
 size_t l1attn_dense_softmax_v_bwd_bytes(int bs, int n_tok, int n_heads, int width, int v_width, int dtype);
 int l1attn_dense_softmax_v_bwd(const void *q, const void *k, const void *v, const void *dvo,

@@ -410,7 +410,7 @@ extern "C" int l1attn_dense_bwd_host_async(const void *d_attn, const void *q, co
 	if (!ar)
 		return rc;
 	const int G = host_group(bs, na);
-	const size_t nsc = dense_bwd_scratch_bytes(G, n_tok, n_heads, width, dtype);
+	const size_t nsc = dense_bwd_scratch_bytes_upto(G, n_tok, n_heads, width, dtype); // (the last group may be smaller)
 	int deferred;
 	if ((rc = arena_reserve(ar, size_t(bs) * (4 * pad256(nqk) + pad256(na)) + size_t((bs + G - 1) / G) * pad256(nsc) + 4096, &deferred)))
 		return rc;

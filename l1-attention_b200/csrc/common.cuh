@@ -129,6 +129,8 @@ int dense_ties_launch(const float *q, const float *k, unsigned char *scratch, vo
 int dense_bwd_launch(const void *d_attn, const void *q, const void *k, void *d_q, void *d_k, void *scratch, int bs,
 		     int n_tok, int n_heads, int width, int dtype, cudaStream_t st);
 size_t dense_bwd_scratch_bytes(int bs, int n_tok, int n_heads, int width, int dtype);
+// for every call of 1 .. bs items: what a buffer needs that calls of several sizes use
+size_t dense_bwd_scratch_bytes_upto(int bs, int n_tok, int n_heads, int width, int dtype);
 int dense_softmax_v_launch(const void *q, const void *k, const void *v, void *vo, void *lse, int bs, int n_tok, int n_heads,
 			   int width, int v_width, int mode, int dtype, cudaStream_t st);
 int dense_softmax_v_bwd_dx_launch(const void *q, const void *k, const void *v, const void *dvo, const void *lse,

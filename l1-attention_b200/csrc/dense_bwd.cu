@@ -247,6 +247,13 @@ size_t dense_bwd_scratch_bytes(int bs, int n_tok, int n_heads, int width, int dt
 	return bwd_scratch_layout(bs, n_tok, n_heads, width).bytes; // tie flags, tie header, tie list, shares of d_k
 }
 
+size_t dense_bwd_scratch_bytes_upto(int bs, int n_tok, int n_heads, int width, int dtype)
+{
+	if (dtype != L1ATTN_F32 || bs < 1 || n_tok < 1 || n_heads < 1 || width < 1)
+		return dense_bwd_scratch_bytes(bs, n_tok, n_heads, width, dtype);
+	return bwd_scratch_bytes_upto(bs, n_tok, n_heads, width);
+}
+
 // The single-visit kernel for rows of any pitch, between the tie detector and the repair of the listed ties, and the exact kernel in
 // case the list overflowed.  Returns 1 when nothing was computed (token index beyond 24 bits, too many items).
 int dense_bwd_listed_launch(const void *d_attn, int g_pitch, const void *q, const void *k, void *d_q, void *d_k, void *scratch, int bs,

@@ -116,6 +116,23 @@ inline BwdScratchLayout bwd_scratch_layout(int bs, int n_tok, int n_heads, int w
 	return l;
 }
 
+// Scratch for any call of 1 .. bs items.  That can be more than a call of bs items needs: fewer items may split their source rows
+// over more ranges, and every range has a partial d_q of its own (600 tokens, 16 heads, 64 columns: 135 MB for 11 items,
+// 221 MB for 10).
+inline size_t bwd_scratch_bytes_upto(int bs, int n_tok, int n_heads, int width)
+{
+	size_t most = bwd_scratch_layout(bs, n_tok, n_heads, width).bytes;
+	if ((n_tok + 15) / 16 <= 14)
+		return most; // too few tiles to be split: the layout grows with the items
+	for (int c = bs - 1; c >= 1; c--) {
+		const BwdScratchLayout l = bwd_scratch_layout(c, n_tok, n_heads, width);
+		most = l.bytes > most ? l.bytes : most;
+		if (most >= l.dqpart + size_t(8) * c * n_tok * n_heads * width * 4 + 256)
+			break; // as much as c items in eight ranges need, and fewer items need less than that
+	}
+	return most;
+}
+
 // Which rows of q and k are zero in every column (padded tokens), a byte per (batch, token, head) of q, then of k: the detector
 // leaves them in d_k, which nothing writes before the single-visit kernel is through (its shares are summed into d_k
 // by the kernel behind it).  2 bytes a row, where d_k has width * 4.

@@ -943,7 +943,8 @@ int dense_softmax_v_bwd_dx_launch(const void *q, const void *k, const void *v, c
 				  v_width, st);
 }
 
-// Workspace of the whole backward: dx, then the dense backward's scratch.
+// Workspace of the whole backward: dx, then the dense backward's scratch.  Its size serves every call of up to bs items (a batch is
+// walked in chunks, the last of them smaller).
 static size_t sv_dx_bytes(int bs, int n_tok, int n_heads, int dtype)
 {
 	const size_t es = dtype == L1ATTN_F64 ? 8 : 4, pitch = (size_t(n_tok) + 3) / 4 * 4; // rows of dx as the tiled kernels write them
@@ -951,7 +952,7 @@ static size_t sv_dx_bytes(int bs, int n_tok, int n_heads, int dtype)
 }
 size_t dense_softmax_v_bwd_bytes(int bs, int n_tok, int n_heads, int width, int, int dtype)
 {
-	return sv_dx_bytes(bs, n_tok, n_heads, dtype) + dense_bwd_scratch_bytes(bs, n_tok, n_heads, width, dtype);
+	return sv_dx_bytes(bs, n_tok, n_heads, dtype) + dense_bwd_scratch_bytes_upto(bs, n_tok, n_heads, width, dtype);
 }
 
 // dx lies [b][h][s][t] between its two kernels: the tiled kernel that makes it owns one head, and in d_attn's order, heads innermost, each of

@@ -285,6 +285,7 @@ def dense_softmax_v_bwd(q, k, v, dvo, lse, delta, dq, dk, dv, work):
     bs, n, h, w = q.shape
     for t in (q, k, v, dvo, lse, delta, dq, dk, dv):
         assert t.is_cuda and t.is_contiguous() and t.dtype == q.dtype
+    assert work.numel() * work.element_size() >= lib().l1attn_dense_softmax_v_bwd_bytes(bs, n, h, w, v.shape[3], _tdt(q))
     _check(lib().l1attn_dense_softmax_v_bwd(_dp(q), _dp(k), _dp(v), _dp(dvo), _dp(lse), _dp(delta), _dp(dq), _dp(dk), _dp(dv),
                                             _dp(work), bs, n, h, w, v.shape[3], _tdt(q), _stream()), "l1attn_dense_softmax_v_bwd")
 
@@ -299,6 +300,8 @@ def dense_bwd(d_attn, q, k, out=None, scratch="auto"):
     if isinstance(scratch, str):
         scratch = torch.empty(lib().l1attn_dense_bwd_scratch_bytes(bs, n, h, w, _tdt(q)), dtype=torch.uint8,
                               device=q.device)
+    elif scratch is not None:
+        assert scratch.numel() * scratch.element_size() >= lib().l1attn_dense_bwd_scratch_bytes(bs, n, h, w, _tdt(q))
     _check(lib().l1attn_dense_bwd(_dp(d_attn), _dp(q), _dp(k), _dp(dq), _dp(dk), _dp(scratch), bs, n, h, w, _tdt(q),
                                   _stream()), "l1attn_dense_bwd")
     return dq, dk

@@ -3,6 +3,7 @@ include/l1attn_b200.h declares, the ctypes table covers the same set, and argume
 answers before any CUDA call is made (so these run on a box without a GPU)."""
 import ctypes
 import os
+import random
 import re
 
 import pytest
@@ -92,6 +93,24 @@ def test_size_queries():
     assert lib.l1attn_dense_bwd_scratch_bytes(16, 1024, 16, 64, 1) == 16  # float64 needs none
     assert lib.l1attn_expand_coo_scratch_bytes(4096) == 0
     assert lib.l1attn_expand_coo_scratch_bytes(1 << 20) == (1 << 20) * 8
+
+
+def test_workspace_of_a_chunk_serves_smaller_chunks():
+    """A call of fewer items may split its source rows over more ranges and lay out more scratch than one of more items; the
+    fused backward's workspace is one for all chunks of a batch, so the size for `step` items covers every count below."""
+    lib = l1attn_cabi.lib()
+    rng = random.Random(1)
+    shapes = [(11, 600, 16, 64), (17, 688, 8, 64), (18, 470, 16, 64), (12, 960, 6, 64), (28, 547, 8, 64), (24, 1135, 4, 96), (10, 520, 1, 33)]
+    shapes += [(rng.randint(2, 40), rng.randint(33, 1200), rng.randint(1, 16), rng.choice([16, 32, 33, 64, 96, 128])) for _ in range(300)]
+    larger = 0
+    for step, n, h, w in shapes:
+        work = lib.l1attn_dense_softmax_v_bwd_bytes(step, n, h, w, w, 0)
+        for c in range(1, step + 1):
+            dx = (c * h * n * ((n + 3) // 4 * 4) * 4 + 255) // 256 * 256
+            scratch = lib.l1attn_dense_bwd_scratch_bytes(c, n, h, w, 0)
+            assert dx + scratch <= work, (step, c, n, h, w)
+            larger += scratch > lib.l1attn_dense_bwd_scratch_bytes(step, n, h, w, 0)
+    assert larger > 100  # (such counts are among them)
 
 
 def test_no_cpu_fallback_in_product():

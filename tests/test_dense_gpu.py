@@ -210,6 +210,19 @@ def test_deterministic():
     assert torch.equal(f[0], f[1])
 
 
+def test_host_buffers_with_a_smaller_last_group(monkeypatch):
+    """The last group of batch items may need more scratch than the others (its source rows are split over more ranges)."""
+    cabi = _cabi()
+    monkeypatch.setenv("L1ATTN_HOST_GROUP", "10")
+    q, k, g = _rand((18, 520, 1, 33), np.float32, 36)
+    dq, dk = cabi.dense_bwd_host(g, q, k)
+    for b in (0, 9, 10, 17):
+        rq, rk = cabi.dense_bwd(_dev(g[b:b + 1]), _dev(q[b:b + 1]), _dev(k[b:b + 1]))
+        assert_close(dq[b:b + 1], rq.cpu().numpy(), 1e-5, "dq")
+        assert_close(dk[b:b + 1], rk.cpu().numpy(), 1e-5, "dk")
+    assert cabi.lib().l1attn_host_release() == 0
+
+
 def test_host_buffer_entry_points():
     from oracle import oracle
     cabi = _cabi()

@@ -167,6 +167,28 @@ def test_backward_chunks_over_the_batch(monkeypatch):
         assert torch.equal(a, b.grad)
 
 
+@pytest.mark.parametrize("dims,step", [((18, 520, 1, 33, 33), 10), ((21, 600, 16, 64, 64), 11)])
+def test_smaller_last_chunk(monkeypatch, dims, step):
+    """A last chunk of fewer items splits its source rows over more ranges than the others: every item's gradients are what
+    the item gives alone (the sums over ranges round differently)."""
+    import l1attn_fused_cuda
+    torch.manual_seed(4)
+    bs, n, h, w, wv = dims
+    q, k = (0.3 * torch.randn(bs, n, h, w, device="cuda") for _ in range(2))
+    v, g = torch.randn(bs, n, h, wv, device="cuda"), torch.randn(bs, n, h, wv, device="cuda")
+    monkeypatch.setattr(l1attn_fused_cuda, "_CHUNK_BYTES", step * n * n * h * 4)
+
+    def gradients(sl):
+        leaves = [t[sl].clone().requires_grad_(True) for t in (q, k, v)]
+        l1attn_fused_cuda.L1AttnSoftmaxV()(*leaves).backward(g[sl])
+        return [t.grad for t in leaves]
+
+    whole = gradients(slice(None))
+    for b in (0, step - 1, step, bs - 1):
+        for name, x, r in zip(("dq", "dk", "dv"), whole, gradients(slice(b, b + 1))):
+            assert_close(x[b:b + 1].cpu().numpy(), r.cpu().numpy(), 1e-5, name)
+
+
 def test_module_argument_checks():
     import l1attn_fused_cuda
     q = torch.randn(1, 4, 2, 8, device="cuda")
