@@ -145,6 +145,25 @@ inline BwdZeroRows bwd_zero_rows_in(void *d_k, int bs, int n_tok, int n_heads)
 	return BwdZeroRows{p, p + size_t(bs) * n_tok * n_heads};
 }
 
+// The tie detector's bitmaps, one for each of the BWD_TIE_COLS columns of a CTA: 64 bits per token, 32 Kbit at least (a false candidate
+// costs a small set more than clearing does: with 4 Kbit at least the detector took 17 us instead of 12 at [8,256,8,64];
+// 32 KiB per CTA at 1024 tokens: seven CTAs per SM hide the load latency; 128 bits per token held three and took twice the time for
+// 1/4 of the false candidates) up to 4096 tokens, fewer beyond: more false candidates to prove, and past ~16k tokens the list
+// overflows into the conservative marking.
+constexpr int BWD_TIE_COLS = 4;
+inline int bwd_bitmap_log2bits(int n_tok)
+{
+	int log2bits = 15;
+	while (log2bits < 18 && (1 << log2bits) < 64 * n_tok)
+		log2bits++;
+	return log2bits;
+}
+inline size_t bwd_bitmap_bytes(int n_tok) { return size_t(BWD_TIE_COLS) << bwd_bitmap_log2bits(n_tok) >> 3; }
+// The detector's pass over the zeros keeps two mask bytes per token where the bitmaps were, in whole 8-byte entries: up to 65536 tokens
+// fit.  Beyond, zeros are candidates like any other value.
+inline size_t bwd_zero_mask_bytes(int n_tok) { return (2 * size_t(n_tok) + 7) / 8 * 8; }
+inline bool bwd_zeros_apart(int n_tok) { return bwd_zero_mask_bytes(n_tok) <= bwd_bitmap_bytes(n_tok); }
+
 constexpr int BWD_SMALL_TOK = 32; // token counts up to here: one exact kernel without scratch (dense_bwd_small.cu)
 
 #ifdef __CUDACC__

@@ -75,6 +75,7 @@ struct ZeroArgs {
 	int *hdr;
 	BwdFlagLayout fl;
 	int n_tok, n_heads, width, ncg; // ncg: CTAs (groups of NC columns) per (batch, head)
+	int apart;                      // zeros have a pass of their own (bwd_zeros_apart())
 };
 
 // The ties between zeros in the CTA's columns, where both q and k hold some: padded tokens tie with one another in every column, and each
@@ -83,7 +84,7 @@ struct ZeroArgs {
 //   1. per token: which columns are zero, and is the whole row?  (the CTAs of the first columns write the tables)
 //   2. the zeros of rows that are not zero throughout, a short list on either side
 //   3. every q zero against the k zeros of that list, every q zero of that list against the zero k rows.
-// smem: `room` uint2, of which the first (2 n_tok + 7) / 8 hold the tokens' masks.
+// smem: `room` uint2, of which the first (2 n_tok + 7) / 8 hold the tokens' masks (bwd_zeros_apart(): they fit).
 template <int NC>
 __device__ __noinline__ void zero_ties(const ZeroArgs &z, uint2 *smem, int room, uint4 *tie_list, int &n_hits, int &hit_base)
 {
@@ -247,8 +248,8 @@ __global__ void __launch_bounds__(NT_MAX) dense_ties_kernel(const __grid_constan
 					if (t < n_tok && j < ncol && x == x) {
 						const unsigned bits = canon(x), want = hash_bits(bits);
 						if ((bitmap[j * words + hash_word(bits, sh)] & want) == want) {
-							if (bits == 0u) {
-								zero_cand = 1; // zeros have a pass of their own
+							if (bits == 0u && z.apart) {
+								zero_cand = 1;
 							} else {
 								const int idx = atomicAdd(&n_cand, 1);
 								if (idx < CAP) {
@@ -349,11 +350,12 @@ __global__ void __launch_bounds__(NT_MAX) dense_ties_kernel(const __grid_constan
 template <int NC>
 int launch_nc(ZeroArgs z, int bs, int log2bits, uint4 *tie_list, int vec_ok, cudaStream_t st)
 {
+	static_assert(NC == BWD_TIE_COLS, "bwd_bitmap_bytes() counts that many bitmaps");
 	z.ncg = (z.width + NC - 1) / NC;
 	const long long grid = (long long)bs * z.n_heads * z.ncg;
 	if (grid > 0x7fffffffLL)
 		return 1;
-	const size_t smem = size_t(NC) * (size_t(1) << log2bits) / 8;
+	const size_t smem = bwd_bitmap_bytes(z.n_tok);
 	L1B_SHARED_MEMORY(dense_ties_kernel<NC>, int(smem));
 	int nt = 256;
 	while (nt < NT_MAX && nt * TB < z.n_tok)
@@ -445,14 +447,7 @@ int dense_ties_launch(const float *q, const float *k, unsigned char *scratch, vo
 		return 1;
 	// four columns as one 16-byte vector where the rows are made of such; the C ABI only promises element alignment
 	const int vec_ok = width % 4 == 0 && aligned(q, 16) && aligned(k, 16);
-	// 64 bits per token, 32 Kbit at least (a false candidate costs a small set more than clearing does: with 4 Kbit at least the
-	// detector took 17 us instead of 12 at [8,256,8,64]; 32 KiB per CTA at 1024 tokens: seven CTAs per SM hide the load latency; 128 bits per
-	// token held three and took twice the time for 1/4 of the false candidates) up to 4096 tokens, fewer
-	// beyond: more false candidates to prove, and past ~16k tokens the list overflows into the
-	// conservative marking.  Four columns per CTA keep the global loads 16 bytes wide.
-	int log2bits = 15;
-	while (log2bits < 18 && (1 << log2bits) < 64 * n_tok)
-		log2bits++;
+	// four columns per CTA keep the global loads 16 bytes wide
 	if ((unsigned long long)bs * n_heads * width > 0xffffffffull)
 		return 1; // a tie entry holds the (batch, head, column) index in 32 bits
 	const BwdFlagLayout fl = bwd_flag_layout(bs, n_tok, n_heads, width);
@@ -460,8 +455,8 @@ int dense_ties_launch(const float *q, const float *k, unsigned char *scratch, vo
 	L1B_CUDA(cudaMemsetAsync(scratch, 0, sl.hdr + 256, st)); // flags and header
 	const BwdZeroRows zr = bwd_zero_rows_in(d_k, bs, n_tok, n_heads);
 	const ZeroArgs z{q, k, drop_zero_rows ? zr.q : nullptr, drop_zero_rows ? zr.k : nullptr, scratch + sl.flags,
-			 reinterpret_cast<int *>(scratch + sl.hdr), fl, n_tok, n_heads, width, 0};
-	return launch_nc<4>(z, bs, log2bits, reinterpret_cast<uint4 *>(scratch + sl.ties), vec_ok, st);
+			 reinterpret_cast<int *>(scratch + sl.hdr), fl, n_tok, n_heads, width, 0, bwd_zeros_apart(n_tok)};
+	return launch_nc<BWD_TIE_COLS>(z, bs, bwd_bitmap_log2bits(n_tok), reinterpret_cast<uint4 *>(scratch + sl.ties), vec_ok, st);
 }
 
 // Enqueue after the compare-form backward: adds the listed ties' terms back (no-op when the list overflowed).

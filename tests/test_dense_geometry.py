@@ -1,0 +1,39 @@
+"""Host-side geometry of the dense backward's kernels (csrc/dense_bwd_tiles.h), compiled for the CPU: what a kernel lays out has to
+fit the memory that its launch gives it."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from conftest import PKG
+
+
+@pytest.fixture(scope="module")
+def tiles(tmp_path_factory):
+    gxx, nvcc = shutil.which("g++"), shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    if not gxx or not os.path.isfile(os.path.join(include, "cuda_runtime.h")):
+        pytest.skip("needs g++ and the CUDA headers")
+    d = tmp_path_factory.mktemp("tiles")
+    (d / "t.cpp").write_text('#include "dense_bwd_tiles.h"\nextern "C" {\n'
+                             'size_t bitmap_bytes(int n) { return l1b::bwd_bitmap_bytes(n); }\n'
+                             'size_t zero_mask_bytes(int n) { return l1b::bwd_zero_mask_bytes(n); }\n'
+                             'int zeros_apart(int n) { return l1b::bwd_zeros_apart(n); }\n}\n')
+    subprocess.run([gxx, "-shared", "-fPIC", "-O1", "-std=c++17", "-I", os.path.join(PKG, "csrc"), "-I", include,
+                    str(d / "t.cpp"), "-o", str(d / "t.so")], check=True)
+    lib = ctypes.CDLL(str(d / "t.so"))
+    lib.bitmap_bytes.restype = lib.zero_mask_bytes.restype = ctypes.c_size_t
+    return lib
+
+
+def test_zero_masks_fit_the_bitmaps(tiles):
+    """Two bytes per token in the memory of the bitmaps, which stop growing at 128 KiB; more tokens than that go without."""
+    assert tiles.bitmap_bytes(1 << 23) == tiles.bitmap_bytes(4096) == 4 * (1 << 18) // 8
+    for n in [1, 3, 33, 1000, 4096, 32768, 65533, 65535, 65536, 65537, 65540, 100000, (1 << 24) - 1]:
+        assert tiles.zero_mask_bytes(n) >= 2 * n
+        assert bool(tiles.zeros_apart(n)) == (n <= 65536)
+        assert not tiles.zeros_apart(n) or tiles.zero_mask_bytes(n) <= tiles.bitmap_bytes(n)
+    source = open(os.path.join(PKG, "csrc", "dense_ties.cu")).read()
+    assert "z.apart" in source and "bwd_zeros_apart(n_tok)" in source  # the pass is entered by this rule
