@@ -397,7 +397,7 @@ dense_tiefix_kernel(const int *__restrict__ tie_hdr, const uint4 *__restrict__ t
 	FixEntry *sorted = reinterpret_cast<FixEntry *>(fix_smem + size_t(BWD_TIE_CAP) * sizeof(uint4)); // used in the first two CTAs
 	for (int i = threadIdx.x; i < n; i += FIX_THREADS)
 		e[i] = ties[i];
-	__syncthreads();
+	cluster.sync(); // the list is complete, and the first two CTAs run: their shared memory may be written from now on
 	const unsigned hwn = unsigned(n_heads) * unsigned(width);
 	// entry i of this thread: spread over the CTAs first, so that short lists use all of them
 	const int i = int(threadIdx.x) * FIX_CTAS + int(cluster.block_rank());

@@ -2,6 +2,7 @@
 fit the memory that its launch gives it."""
 import ctypes
 import os
+import re
 import shutil
 import subprocess
 
@@ -37,3 +38,13 @@ def test_zero_masks_fit_the_bitmaps(tiles):
         assert not tiles.zeros_apart(n) or tiles.zero_mask_bytes(n) <= tiles.bitmap_bytes(n)
     source = open(os.path.join(PKG, "csrc", "dense_ties.cu")).read()
     assert "z.apart" in source and "bwd_zeros_apart(n_tok)" in source  # the pass is entered by this rule
+
+
+@pytest.mark.parametrize("name", ["coo.cu", "dense_ties.cu"])
+def test_cluster_barrier_before_remote_shared_memory(name):
+    """Shared memory of another CTA of the cluster may be accessed only behind a cluster barrier: before it that CTA need not run yet."""
+    source = re.sub(r"//.*", "", open(os.path.join(PKG, "csrc", name)).read())
+    bodies = [b for b in re.split(r"\n}\n", source) if "map_shared_rank" in b]
+    assert bodies
+    for body in bodies:
+        assert "cluster.sync()" in body[:body.index("map_shared_rank")], body[:300]

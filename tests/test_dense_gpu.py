@@ -201,6 +201,21 @@ def test_zero_rows_beside_zero_values(shape):
         assert_close(dk, rk, 1e-5, "dk")
 
 
+@pytest.mark.parametrize("count", [1, 2, 7, 8, 9, 33])
+def test_few_listed_ties_are_repaired(count):
+    """Lists shorter than the repair's CTAs, and one more."""
+    from oracle import oracle
+    cabi = _cabi()
+    q, k, g = _rand((1, 160, 4, 32), np.float32, 37)
+    for i in range(count):
+        k[0, 150 - i, i % 4, i % 32] = q[0, 3 * i, i % 4, i % 32]
+    rq, rk = oracle.dense_bwd(g.astype(np.float64), q.astype(np.float64), k.astype(np.float64))
+    for _ in range(20):
+        dq, dk = (x.cpu().numpy() for x in cabi.dense_bwd(_dev(g), _dev(q), _dev(k)))
+        assert_close(dq, rq, 1e-5, "dq")
+        assert_close(dk, rk, 1e-5, "dk")
+
+
 def test_deterministic():
     cabi = _cabi()
     q, k, g = _rand((2, 96, 16, 64), np.float32, 11)
