@@ -64,7 +64,7 @@ const char *l1attn_strerror(int code);
 int l1attn_last_cuda_error(void);
 /*
  * Synchronises with the device and reports whether any kernel of this library gave up a bounded
- * wait since the last call (L1ATTN_ERR_TIMEOUT, cleared by the call) -- the kernels that stage
+ * wait since the last call (L1ATTN_ERR_TIMEOUT, cleared by the call, in the host word below too) -- the kernels that stage
  * tiles with asynchronous bulk copies never spin without a limit.  L1ATTN_OK otherwise.
  */
 int l1attn_device_status(void);
@@ -77,8 +77,8 @@ int l1attn_device_status(void);
 int l1attn_device_status_async(int *host_word, void *stream);
 
 /* The current device's word in pinned host memory that a kernel of this library sets to 1 when it gives up a bounded wait: nothing
- * to enqueue, the caller looks at it when it likes and clears it (l1attn_device_status() clears the device's word).  NULL
- * when it cannot be set up at that moment; every later call may try again. */
+ * to enqueue, the caller looks at it when it likes and clears both words by l1attn_device_status().  It starts at 1 when a kernel has
+ * given up a wait that nobody has asked about yet.  NULL when it cannot be set up at that moment; every later call may try again. */
 int *l1attn_device_status_word(void);
 /*
  * Test hook, not an operator: launches one warp that waits at most limit_us (1..100000) microseconds on a

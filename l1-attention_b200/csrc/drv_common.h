@@ -53,14 +53,14 @@ inline void *l1b_stream() { return static_cast<void *>(at::cuda::getCurrentCUDAS
 // A kernel of the library that gives up a bounded wait sets a sticky word on the device and a word in pinned host memory,
 // and returns; its outputs are then garbage.  The drivers never synchronise, so they learn of it at a later call: every call
 // looks at the host word first (l1b_check_pending) and raises if it is set.  (A copy of the device's word behind every
-// launch, as this was done before, cost a call two microseconds of GPU time and five of the host's.)  A caller that needs
+// launch would cost a call two microseconds of GPU time and five of the host's.)  A caller that needs
 // the answer at once can call l1attn_device_status() through the C ABI, which synchronises.
 inline void l1b_check_pending(const char *fn)
 {
 	int *w = l1attn_device_status_word();
 	if (w && *reinterpret_cast<volatile int *>(w) != 0) {
 		*reinterpret_cast<volatile int *>(w) = 0;
-		(void)l1attn_device_status(); // synchronises and clears the device word
+		(void)l1attn_device_status(); // synchronises and clears both words
 		TORCH_CHECK(false, fn, ": an earlier kernel of this library gave up a bounded wait on an asynchronous copy; "
 				       "the results of the calls made since the previous successful call are invalid");
 	}

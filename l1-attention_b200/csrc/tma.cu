@@ -93,16 +93,19 @@ int multiprocessors(int *out)
 
 } // namespace l1b
 
-// Reads (and clears) the sticky error word set by a kernel whose bounded wait ran out.
+// Reads (and clears, with the host's copy of it) the sticky error word set by a kernel whose bounded wait ran out.
 extern "C" int l1attn_device_status(void)
 {
-	int v = 0;
+	int v = 0, dev = 0;
 	int *p = l1b::device_error_word();
 	if (!p)
 		return L1ATTN_ERR_CUDA;
 	L1B_CUDA(cudaMemcpy(&v, p, sizeof(int), cudaMemcpyDeviceToHost));
 	if (v) {
 		L1B_CUDA(cudaMemset(p, 0, sizeof(int)));
+		L1B_CUDA(cudaGetDevice(&dev)); // (device_error_word() has found it in range)
+		if (volatile int *host = l1b::g_error_host[dev].load(std::memory_order_acquire))
+			*host = 0; // reported: the next look at the host word must not report it again
 		return L1ATTN_ERR_TIMEOUT;
 	}
 	return L1ATTN_OK;
@@ -130,10 +133,13 @@ extern "C" int *l1attn_device_status_word(void)
 	}
 	bool ok = cudaHostAlloc(reinterpret_cast<void **>(&host), 64, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess;
 	if (ok) {
-		*host = 0;
+		host[0] = host[1] = 0;
 		ok = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess &&
 		     cudaMemcpyAsync(err + ERROR_HOST_WORD, &host, sizeof host, cudaMemcpyHostToDevice, st) == cudaSuccess &&
+		     cudaMemcpyAsync(&host[1], err, sizeof(int), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
 		     cudaStreamSynchronize(st) == cudaSuccess;
+		if (ok && host[1])
+			*reinterpret_cast<volatile int *>(host) = 1; // a kernel has given up before there was a host word
 		if (st)
 			(void)cudaStreamDestroy(st);
 		if (!ok)

@@ -5,7 +5,7 @@ Tolerances (norm-wise, see conftest.rel_err): fp64 1e-12, fp32 1e-5 -- the bars 
 import numpy as np
 import pytest
 
-from conftest import assert_close
+from conftest import PKG, assert_close
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -412,7 +412,7 @@ def test_bounded_wait_gives_up_and_is_reported():
 
 
 def test_driver_raises_on_a_pending_timeout():
-    """The pybind driver never synchronises; it polls the error word through pinned memory and raises at the next
+    """The pybind driver never synchronises; it looks at the error word in pinned memory and raises at the next
     call after a kernel gave up a wait."""
     import l1attn_cuda_drv
     cabi = _cabi()
@@ -423,7 +423,6 @@ def test_driver_raises_on_a_pending_timeout():
     l1attn_cuda_drv.forward(q, q)  # nothing pending: fine
     returned = torch.zeros(2, dtype=torch.int32, device="cuda")
     assert lib.l1attn_test_wait_timeout(2000, returned.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
-    l1attn_cuda_drv.forward(q, q)  # enqueued behind the probe; copies the (now set) word to the pinned word
     torch.cuda.synchronize()
     with pytest.raises(RuntimeError, match="bounded wait"):
         l1attn_cuda_drv.forward(q, q)
@@ -431,3 +430,31 @@ def test_driver_raises_on_a_pending_timeout():
     out = l1attn_cuda_drv.forward(q, q)[0]
     torch.cuda.synchronize()
     assert torch.isfinite(out).all()
+
+
+def test_a_timeout_is_reported_once():
+    """Whoever learns of a timeout first clears it for everyone: the status through the C ABI, then no error from the driver."""
+    import l1attn_cuda_drv
+    lib = _cabi().lib()
+    q = torch.randn(1, 32, 8, 64, device="cuda")
+    l1attn_cuda_drv.forward(q, q)  # (the host word exists from here on)
+    returned = torch.zeros(2, dtype=torch.int32, device="cuda")
+    assert lib.l1attn_test_wait_timeout(2000, returned.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert lib.l1attn_device_status() == -7
+    l1attn_cuda_drv.forward(q, q)
+    assert lib.l1attn_device_status() == 0
+
+
+def test_a_timeout_before_the_first_driver_call_is_reported():
+    """In a process of its own: the wait runs out before any driver call has set the host word up."""
+    import subprocess
+    import sys
+    code = ("import torch, l1attn_cabi, l1attn_cuda_drv\n"
+            "lib, q, r = l1attn_cabi.lib(), torch.randn(1, 32, 8, 64, device='cuda'), torch.zeros(2, dtype=torch.int32, device='cuda')\n"
+            "assert lib.l1attn_test_wait_timeout(2000, r.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0\n"
+            "torch.cuda.synchronize()\n"
+            "try:\n    l1attn_cuda_drv.forward(q, q)\nexcept RuntimeError as e:\n    assert 'bounded wait' in str(e)\nelse:\n    raise SystemExit('not reported')\n"
+            "l1attn_cuda_drv.forward(q, q)\n"
+            "assert lib.l1attn_device_status() == 0\n")
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=PKG, timeout=300)
