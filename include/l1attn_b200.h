@@ -113,7 +113,7 @@ int l1attn_dense_fwd(const void *q, const void *k, void *attn,
  * single-visit kernels leave per block of 128 (256, 512) query rows: ceil(n_tok / 128) * sizeof(d_k) bytes, i.e.
  * about width / 128 times the size of d_attn (plus 2, 4 or 8 times sizeof(d_q) for shapes whose work items
  * split their source rows: long context with a small batch).  With NULL every tile takes the exact loop and no scratch is
- * needed (same results, about 2.7 times the time in fp32).  Sets of at most 32 tokens, and fp64, take an exact kernel in any case.  Contents need no initialisation and mean
+ * needed (same results, about 2.7 times the time in fp32).  Sets of at most 48 tokens, and fp64, take an exact kernel in any case.  Contents need no initialisation and mean
  * nothing after the call; calls that share a scratch buffer must not overlap on the GPU.  A smaller batch may need more
  * (its source rows may be split over more ranges): a buffer that serves several batch sizes has the largest of their sizes.
  * Replaces l1attn_cuda_drv.backward (cuda/l1attn_cuda_drv.cpp:67-104) and

@@ -277,7 +277,7 @@ int dense_bwd_launch(const void *d_attn, const void *q, const void *k, void *d_q
 {
 	if (bs == 0 || n_tok == 0 || n_heads == 0 || width == 0)
 		return L1ATTN_OK;
-	if (n_tok <= BWD_SMALL_TOK)
+	if (n_tok <= bwd_small_tokens(dtype == L1ATTN_F32))
 		return dense_bwd_small_launch(d_attn, q, k, d_q, d_k, bs, n_tok, n_heads, width, dtype, st);
 	static const bool no_tma = getenv("L1ATTN_NO_TMA") != nullptr; // debugging aid: force the generic kernel
 	static const bool no_sv = getenv("L1ATTN_NO_SV") != nullptr;   // debugging aid: force the two-pass kernel

@@ -1,11 +1,12 @@
-// Dense L1 scores, backward, for sets of at most 32 tokens (fp32 and fp64, any width, head count and alignment).
+// Dense L1 scores, backward, for sets of at most 48 tokens (fp32) or 32 (fp64), any width, head count and alignment.
 //
 // A warp owns one head and 32 width columns (a lane each) of one batch item and holds every query row of its column in
 // registers: both gradients of a term come from ONE visit, d_k of a source row is complete at the end of its row, and the
 // sign is exact (zero where q == k), so there is no tie list, no scratch and no second kernel.  The head's scores'
 // gradients lie [s][t] in shared memory and are read as broadcasts, 16 bytes at a time.
 //
-// Bound by instruction issue, and by its one launch where the batch is small: [512,16,8,32] 18 us, [200,30,8,64] 41 us.  The
+// Bound by instruction issue, and by its one launch where the batch is small: [512,16,8,32] 18 us, [200,30,8,64] 41 us, [200,48,6,33]
+// 91 us (the tiled kernels 224).  The
 // tiled kernels spent their time on padding (an item is 128 query rows), on the tie detector and, with padded sets, on the exact
 // two-pass kernel: 1.3 ms (padded) and 225 us for the same.
 #include "common.cuh"
@@ -14,9 +15,8 @@
 namespace l1b {
 namespace {
 
-constexpr int NW = 8; // warps per CTA: consecutive (head, 32 columns) units of one batch item
-
-template <typename T, int TN> // TN >= n_tok query rows per thread
+// TN >= n_tok query rows per thread; NW warps per CTA: consecutive (head, 32 columns) units of one batch item
+template <typename T, int TN, int NW>
 __global__ void __launch_bounds__(NW * 32)
 dense_bwd_small_kernel(const T *__restrict__ g, const T *__restrict__ q, const T *__restrict__ k, T *__restrict__ d_q,
 		       T *__restrict__ d_k, int n_tok, int n_heads, int width, T scale, int nws, int cpb)
@@ -77,7 +77,7 @@ dense_bwd_small_kernel(const T *__restrict__ g, const T *__restrict__ q, const T
 			d_q[off + t * row] = scale * acc[t];
 }
 
-template <typename T, int TN>
+template <typename T, int TN, int NW = 8>
 int launch(const T *g, const T *q, const T *k, T *d_q, T *d_k, int bs, int n_tok, int n_heads, int width, cudaStream_t st)
 {
 	const int nws = (width + 31) / 32;
@@ -85,7 +85,7 @@ int launch(const T *g, const T *q, const T *k, T *d_q, T *d_k, int bs, int n_tok
 	if (nu > 0x7fffffffLL || grid > 0x7fffffffLL)
 		return L1ATTN_ERR_SHAPE;
 	const size_t smem = NW * ((size_t(n_tok) * TN + 31) / 32 * 32 + 16 / sizeof(T)) * sizeof(T);
-	auto kern = dense_bwd_small_kernel<T, TN>;
+	auto kern = dense_bwd_small_kernel<T, TN, NW>;
 	L1B_SHARED_MEMORY(kern, int(smem));
 	kern<<<unsigned(grid), NW * 32, smem, st>>>(g, q, k, d_q, d_k, n_tok, n_heads, width, T(-1.0 / sqrt(double(width))), nws, int(cpb));
 	L1B_LAUNCH_CHECK();
@@ -97,6 +97,12 @@ int pick(const void *g, const void *q, const void *k, void *d_q, void *d_k, int 
 {
 	if (n_tok <= 16)
 		return launch<T, 16>((const T *)g, (const T *)q, (const T *)k, (T *)d_q, (T *)d_k, bs, n_tok, n_heads, width, st);
+	if (sizeof(T) == 4 && n_tok > 32) {
+		// two warps per CTA while eight would leave SMs without one ([4,48,8,64] 28 us, 37 with eight)
+		const bool few = (long long)bs * n_heads * ((width + 31) / 32) < 8 * 148;
+		auto go = few ? launch<float, 48, 2> : launch<float, 48, 8>;
+		return go((const float *)g, (const float *)q, (const float *)k, (float *)d_q, (float *)d_k, bs, n_tok, n_heads, width, st);
+	}
 	return launch<T, 32>((const T *)g, (const T *)q, (const T *)k, (T *)d_q, (T *)d_k, bs, n_tok, n_heads, width, st);
 }
 

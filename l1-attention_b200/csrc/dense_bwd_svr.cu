@@ -13,7 +13,7 @@
 // d_k: the row groups' partial sums of a tile meet in shared memory one tile behind the math, in a fixed order; an
 // item's share goes to scratch and the shares are added in order (no atomics: bit-reproducible).
 //
-// Bound by instruction issue, as dense_bwd_sv.cu.  [48,201,6,65]: 261 us (any-shape kernel 1247), [8,512,1,64]: 55 us (736).
+// Bound by instruction issue, as dense_bwd_sv.cu.  [48,201,6,65]: 268 us (any-shape kernel 1247), [8,512,1,64]: 57 us (736).
 #include "common.cuh"
 #include "dense_bwd_tiles.h"
 
@@ -25,20 +25,41 @@ constexpr int XR = 32;      // query rows per thread
 constexpr int NTHREADS = TY * 32;
 constexpr int G_FLOATS = TY * (512 + 32);
 constexpr int NSTAGE = 3;
-// d_q goes to memory every so many tiles, twice per item at least: 2 sum p g - sum g rounds like a sum of twice the terms, and in
-// blocks d_q stays closer to its exact value than one signed sum over all source rows ([48,201,6,65]: error 2.0e-7 with
-// four tiles, 3.4e-7 in one block, 2.6e-7 for the signed sum).
-constexpr int FLUSH_MAX = 16;
+// The sums of d_q are folded every 4 to 32 source rows: acc - (sum of g) / 2, half the signed sum so far.  A plain sum of the g where
+// q > k grows with the rows even where the signed sum does not, and rounds accordingly; short sets are folded more often, where a
+// tile is most of the sum.  Error of d_q against float64, relative to that of one signed sum over all source rows (the exact
+// kernel), k N(0,1), q N(0,1) / q 0.3 N(0,1) with gradients 1 + 0.1 N(0,1), without the folding in brackets: 64 tokens
+// 0.97 / 1.00 (2.1), 100 tokens 0.92 / 0.96 (2.5), 201 tokens 0.86 / 0.90 (2.6), 333 tokens 0.84 / 0.91 (2.8), 1040 tokens
+// 0.37 / 0.22 (0.40).  It costs 1 to 3 % of this kernel.  d_k is such a difference per group of 32 query rows: 0.97 / 0.88,
+// 0.79 / 0.56, 0.57 / 0.32, 0.46 / 0.23, 0.27 / 0.13.
+__device__ __forceinline__ int fold_mask(int n_tok) { return n_tok <= 64 ? 0 : n_tok <= 128 ? 1 : n_tok <= 256 ? 3 : 7; } // fold behind the quarters of tiles whose number has these bits
 template <int HG> struct Stage {
 	static constexpr int TX = 512 / HG, PITCH = 544 / HG, B_FLOATS = TY * HG * 32, FLOATS = G_FLOATS + B_FLOATS;
 };
 constexpr int PK_FLOATS = TY * TY * 32; // [warp][s][lane]
-template <int HG> constexpr size_t smem_bytes() { return sizeof(float) * (NSTAGE * Stage<HG>::FLOATS + 2 * PK_FLOATS + 2 * TY * HG + TY * 32); }
+template <int HG> constexpr size_t smem_bytes() { return sizeof(float) * (NSTAGE * Stage<HG>::FLOATS + 2 * PK_FLOATS + 2 * TY * TY + TY * 32); }
 
 struct Items {
 	unsigned nws, ntb, nhg, ns;
 	int nt; // tiles of TY source rows per item
 };
+
+struct Item {
+	int b, h0, tb, sh, w0; // batch item, first head, block of query rows, range of source rows, first column
+};
+template <int HG> __device__ __forceinline__ Item item_at(unsigned r, const Items &wk)
+{
+	Item x;
+	x.w0 = int(r % wk.nws) * 32;
+	r /= wk.nws;
+	x.sh = int(r % wk.ns);
+	r /= wk.ns;
+	x.tb = int(r % wk.ntb);
+	r /= wk.ntb;
+	x.h0 = int(r % wk.nhg) * HG;
+	x.b = int(r / wk.nhg);
+	return x;
+}
 
 __device__ __forceinline__ size_t opaque(size_t x)
 {
@@ -74,19 +95,12 @@ dense_bwd_svr_kernel(const float *__restrict__ g, int g_pitch, const float *__re
 		return; // too many ties to list: the exact kernel computes this call (or dense_bwd_sv_kernel has)
 	extern __shared__ __align__(16) float sm[];
 	float *pk = sm + NSTAGE * St::FLOATS;   // [tile & 1][warp][s][lane]
-	float *cs = pk + 2 * PK_FLOATS;          // [tile & 1][s][h]: sum over the item's query rows of g
-	float *rowsum = cs + 2 * TY * HG;        // [warp][lane]
+	float *cs = pk + 2 * PK_FLOATS;          // [tile & 1][s][h][group]: sum over the group's query rows of g
+	float *rowsum = cs + 2 * TY * TY;        // [warp][lane]
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int xg = warp / HG, h = warp % HG;  // math: group of 32 query rows, head
-	unsigned r = blockIdx.x;
-	const int w0 = int(r % wk.nws) * 32;
-	r /= wk.nws;
-	const int sh = int(r % wk.ns);
-	r /= wk.ns;
-	const int tb = int(r % wk.ntb);
-	r /= wk.ntb;
-	const int h0 = int(r % wk.nhg) * HG;
-	const int b = int(r / wk.nhg);
+	const Item it = item_at<HG>(blockIdx.x, wk);
+	const int w0 = it.w0, sh = it.sh, tb = it.tb, h0 = it.h0, b = it.b;
 	const int t0 = tb * St::TX, s_first = sh * wk.nt * TY;
 	const size_t row = size_t(n_heads) * width;
 	const size_t tok0 = size_t(b) * n_tok;
@@ -165,42 +179,37 @@ dense_bwd_svr_kernel(const float *__restrict__ g, int g_pitch, const float *__re
 		float *out = part + ((size_t(tb) * bs + b) * n_tok + s) * row + size_t(h0) * width + w0 + lane;
 #pragma unroll
 		for (int j = 0; j < HG; j++) {
-			float v = P[j * (TY * 32)];
+			const float4 *C = reinterpret_cast<const float4 *>(cs + ((m & 1) * TY + warp) * TY + j * (TY / HG));
+			float v = 0.f;
 #pragma unroll
-			for (int x = 1; x < TY / HG; x++)
-				v += P[(x * HG + j) * (TY * 32)];
+			for (int x = 0; x < TY / HG; x += 4) {
+				const float4 c = C[x / 4];
+				v += (fmaf(2.f, P[(x * HG + j) * (TY * 32)], -c.x) + fmaf(2.f, P[((x + 1) * HG + j) * (TY * 32)], -c.y)) +
+				     (fmaf(2.f, P[((x + 2) * HG + j) * (TY * 32)], -c.z) + fmaf(2.f, P[((x + 3) * HG + j) * (TY * 32)], -c.w));
+			}
 			if (s < n_tok && h0 + j < n_heads && w0 + lane < width)
-				out[size_t(j) * width] = fmaf(2.f, v, -cs[((m & 1) * TY + warp) * HG + j]);
+				out[size_t(j) * width] = v;
 		}
 	};
 
-	// d_q += scale * (2 acc - row sum) over the tiles since the last call; the row sum of query row i sits in lane i.  The
-	// addresses are formed one after the other (opaque) and the accesses stay in program order (volatile): formed up front
-	// they would take the hot loop's registers.  After the first time the sum is added in memory, without waiting for the old value
-	// (every element has one writer, so the order of its additions is the program's: reproducible).
-	auto flush = [&](bool first) {
-		volatile float *rs = rowsum + warp * 32;
+	// acc -= (row sum) / 2 over the source rows since the last call; the row sum of query row i sits in lane i
+	auto fold = [&]() {
+		float *rs = rowsum + warp * 32;
 		rs[lane] = rsq;
 		__syncwarp();
-		size_t off = opaque(size_t(sh) * dq_stride + qoff);
 #pragma unroll
-		for (int i = 0; i < XR; i++) {
-			if (i < rows_ok) {
-				const float x = scale * fmaf(2.f, acc[i], -rs[i]);
-				if (first)
-					*reinterpret_cast<volatile float *>(d_q + off) = x;
-				else
-					asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(d_q + off), "f"(x) : "memory");
-			}
-			off = opaque(off + row);
-			acc[i] = 0.f;
+		for (int i4 = 0; i4 < XR / 4; i4++) {
+			const float4 x = reinterpret_cast<const float4 *>(rs)[i4];
+			acc[i4 * 4] = fmaf(-0.5f, x.x, acc[i4 * 4]);
+			acc[i4 * 4 + 1] = fmaf(-0.5f, x.y, acc[i4 * 4 + 1]);
+			acc[i4 * 4 + 2] = fmaf(-0.5f, x.z, acc[i4 * 4 + 2]);
+			acc[i4 * 4 + 3] = fmaf(-0.5f, x.w, acc[i4 * 4 + 3]);
 		}
 		rsq = 0.f;
 		__syncwarp();
 	};
+	const int fold_at = fold_mask(n_tok);
 
-	const int every = min(FLUSH_MAX, (wk.nt + 1) / 2);
-	int next = every;
 	for (int m = 0; m < wk.nt; m++) {
 		cp_async_wait<1>(); // this thread's copies of tile m have landed ...
 		__syncthreads();     // ... everyone's have; and all are done with the math of tile m - 1 and the sums of tile m - 2
@@ -212,45 +221,58 @@ dense_bwd_svr_kernel(const float *__restrict__ g, int g_pitch, const float *__re
 		const float *GL = st + h * St::PITCH + xg * XR + lane;
 		const float *B = st + G_FLOATS + h * 32 + lane;
 		float *pkw = pk + (m & 1) * PK_FLOATS + warp * (TY * 32) + lane;
-#pragma unroll 4
-		for (int s = 0; s < TY; s++) {
-			const float bv = B[s * (HG * 32)];
-			float p = 0.f;
+#pragma unroll 1
+		for (int quarter = 0; quarter < 4; quarter++) {
 #pragma unroll
-			for (int i4 = 0; i4 < XR / 4; i4++) {
-				const float4 gv = GT[s * (HG * St::PITCH / 4) + i4];
-				bwd_sv_terms(acc[i4 * 4], acc[i4 * 4 + 1], acc[i4 * 4 + 2], acc[i4 * 4 + 3], p, a[i4 * 4], a[i4 * 4 + 1], a[i4 * 4 + 2],
-					     a[i4 * 4 + 3], bv, gv);
+			for (int sq = 0; sq < TY / 4; sq++) {
+				const int s = quarter * (TY / 4) + sq;
+				const float bv = B[s * (HG * 32)];
+				float p = 0.f;
+#pragma unroll
+				for (int i4 = 0; i4 < XR / 4; i4++) {
+					const float4 gv = GT[s * (HG * St::PITCH / 4) + i4];
+					bwd_sv_terms(acc[i4 * 4], acc[i4 * 4 + 1], acc[i4 * 4 + 2], acc[i4 * 4 + 3], p, a[i4 * 4], a[i4 * 4 + 1],
+						     a[i4 * 4 + 2], a[i4 * 4 + 3], bv, gv);
+				}
+				pkw[s * 32] = p;
+				rsq += GL[s * (HG * St::PITCH)]; // lane l sums g of query row l of the group
 			}
-			pkw[s * 32] = p;
-			rsq += GL[s * (HG * St::PITCH)]; // lane l sums g of query row l of the group
+			if (((m * 4 + quarter) & fold_at) == fold_at)
+				fold();
 		}
 		if (m > 0)
 			reduce(m - 1);
-		// sum over the item's query rows of source row `warp`, per head
+		// sums over groups of 32 query rows of source row `warp`, per head: eight lanes hold a group
 		const float4 *R = reinterpret_cast<const float4 *>(st + warp * HG * St::PITCH);
 #pragma unroll
-		for (int j = 0; j < HG; j++) {
-			float c = 0.f;
+		for (int j = 0; j < HG; j++)
 #pragma unroll
 			for (int i = 0; i < St::TX / 128; i++) {
 				const float4 x = R[j * (St::PITCH / 4) + i * 32 + lane];
-				c += (x.x + x.y) + (x.z + x.w);
-			}
+				float c = (x.x + x.y) + (x.z + x.w);
 #pragma unroll
-			for (int o = 16; o > 0; o >>= 1)
-				c += __shfl_xor_sync(0xffffffffu, c, o);
-			if (lane == 0)
-				cs[((m & 1) * TY + warp) * HG + j] = c;
-		}
-		if (m + 1 == next && m + 1 < wk.nt) {
-			flush(next == every);
-			next += every;
-		}
+				for (int o = 4; o > 0; o >>= 1)
+					c += __shfl_xor_sync(0xffffffffu, c, o);
+				if (lane % 8 == 0)
+					cs[((m & 1) * TY + warp) * TY + j * (TY / HG) + i * 4 + lane / 8] = c;
+			}
 	}
+	fold();
 	__syncthreads();
 	reduce(wk.nt - 1);
-	flush(next == every);
+	// (the item is decoded anew, and the 32 addresses one after the other: what is kept over the hot loop spills)
+	unsigned block;
+	asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(block));
+	const Item o = item_at<HG>(block, wk);
+	const int first = o.tb * St::TX + xg * XR, left = o.h0 + h < n_heads && o.w0 + lane < width ? n_tok - first : 0;
+	size_t off = opaque(size_t(o.sh) * dq_stride + (size_t(o.b) * n_tok + first) * row + size_t(o.h0 + h) * width + o.w0 + lane);
+#pragma unroll
+	for (int i = 0; i < XR; i++) {
+		if (i < left) {
+			*reinterpret_cast<volatile float *>(d_q + off) = 2.f * scale * acc[i];
+		}
+		off = opaque(off + row);
+	}
 }
 
 template <int HG, bool HST, bool K16>

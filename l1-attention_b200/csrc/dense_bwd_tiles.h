@@ -164,7 +164,10 @@ inline size_t bwd_bitmap_bytes(int n_tok) { return size_t(BWD_TIE_COLS) << bwd_b
 inline size_t bwd_zero_mask_bytes(int n_tok) { return (2 * size_t(n_tok) + 7) / 8 * 8; }
 inline bool bwd_zeros_apart(int n_tok) { return bwd_zero_mask_bytes(n_tok) <= bwd_bitmap_bytes(n_tok); }
 
-constexpr int BWD_SMALL_TOK = 32; // token counts up to here: one exact kernel without scratch (dense_bwd_small.cu)
+// Token counts that take one exact kernel without scratch (dense_bwd_small.cu).  fp32, 33 to 48 tokens: the single-visit kernels' sums
+// of up to 32 gradients, of which half the total is taken away, round up to 1.7 times as much as one signed sum of so few (33 tokens,
+// gradients 1 + 0.1 N(0,1)), and most of an item of 128 query rows is padding.  With fp64 more rows do not fit the registers.
+inline int bwd_small_tokens(bool f32) { return f32 ? 48 : 32; }
 
 #ifdef __CUDACC__
 // Four terms of the single-visit backward: four compares, then the eight predicated adds they feed -- the query rows'

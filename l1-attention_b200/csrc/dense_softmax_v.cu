@@ -966,7 +966,7 @@ int dense_softmax_v_bwd_launch(const void *q, const void *k, const void *v, cons
 		return L1ATTN_OK;
 	static const bool no_tma = getenv("L1ATTN_NO_TMA") != nullptr, no_sv = getenv("L1ATTN_NO_SV") != nullptr;
 	void *scratch = static_cast<unsigned char *>(work) + sv_dx_bytes(bs, n_tok, n_heads, dtype);
-	if (dtype == L1ATTN_F32 && !no_tma && !no_sv && n_tok > BWD_SMALL_TOK && n_tok < (1 << 24)) {
+	if (dtype == L1ATTN_F32 && !no_tma && !no_sv && n_tok > bwd_small_tokens(true) && n_tok < (1 << 24)) {
 		const int pitch = (n_tok + 3) / 4 * 4;
 		int rc = softmax_v_bwd_tile((const float *)q, (const float *)k, (const float *)v, (const float *)dvo, (const float *)lse,
 					    (const float *)delta, (float *)work, pitch, (float *)dv, bs, n_tok, n_heads, width, v_width, st);
