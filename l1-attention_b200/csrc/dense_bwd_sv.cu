@@ -348,14 +348,23 @@ dense_bwd_sv_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_const
 	}
 }
 
+// Sums that are not finite: the exact kernel behind this one computes the call.  (Threads that see the word in time leave their
+// elements to it too.)
+__device__ __forceinline__ void hand_over(int *tie_hdr)
+{
+	if (blockIdx.x == 0 && threadIdx.x == 0 && tie_hdr[BWD_HDR_NOT_FINITE] != 0)
+		tie_hdr[BWD_HDR_OVERFLOW] = 1;
+}
+
 // d_k = -scale * sum over the query-row blocks of their shares, in block order; and, when the source rows were
 // split over ns items, d_q = sum of the ns partial d_q (already scaled), in order.  n4 = float4 count of d_k (= of d_q).
 __global__ void __launch_bounds__(256)
 dense_bwd_sv_partsum_kernel(const float4 *__restrict__ part, float4 *__restrict__ d_k, const float4 *__restrict__ dq_part,
-			    float4 *__restrict__ d_q, const int *__restrict__ tie_hdr, size_t n4, int ntb, int ns, float scale)
+			    float4 *__restrict__ d_q, int *tie_hdr, size_t n4, int ntb, int ns, float scale)
 {
 	if (tie_hdr[BWD_HDR_OVERFLOW] != 0)
 		return;
+	hand_over(tie_hdr);
 	for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += size_t(gridDim.x) * blockDim.x) {
 		float4 s = part[i];
 		for (int r = 1; r < ntb; r++) {
@@ -383,10 +392,11 @@ dense_bwd_sv_partsum_kernel(const float4 *__restrict__ part, float4 *__restrict_
 // As dense_bwd_sv_partsum_kernel, element by element.
 __global__ void __launch_bounds__(256)
 dense_bwd_svr_partsum_kernel(const float *__restrict__ part, float *__restrict__ d_k, const float *__restrict__ dq_part,
-			     float *__restrict__ d_q, const int *__restrict__ tie_hdr, size_t n, int ntb, int ns, float scale)
+			     float *__restrict__ d_q, int *tie_hdr, size_t n, int ntb, int ns, float scale)
 {
 	if (tie_hdr[BWD_HDR_OVERFLOW] != 0)
 		return;
+	hand_over(tie_hdr);
 	for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
 		float s = part[i];
 		for (int r = 1; r < ntb; r++)
@@ -461,8 +471,8 @@ int dense_bwd_sv_launch(const void *d_attn, const void *q, const void *k, void *
 int dense_bwd_partsum_launch(void *d_q, void *d_k, void *scratch, int bs, int n_tok, int n_heads, int width, cudaStream_t st)
 {
 	const BwdScratchLayout sl = bwd_scratch_layout(bs, n_tok, n_heads, width);
-	const unsigned char *sc = static_cast<const unsigned char *>(scratch);
-	const int *tie_hdr = reinterpret_cast<const int *>(sc + sl.hdr);
+	unsigned char *sc = static_cast<unsigned char *>(scratch);
+	int *tie_hdr = reinterpret_cast<int *>(sc + sl.hdr);
 	const float scale = float(-1.0 / sqrt(double(width)));
 	const size_t n = size_t(bs) * n_tok * n_heads * width;
 	const bool vec = n % 4 == 0 && aligned(d_q, 16) && aligned(d_k, 16); // (shares and partial sums start on 256 bytes)

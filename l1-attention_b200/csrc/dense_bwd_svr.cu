@@ -12,6 +12,9 @@
 // A CTA walks ONE item (or one of its ns ranges of source rows); three operand stages, one CTA barrier per tile.
 // d_k: the row groups' partial sums of a tile meet in shared memory one tile behind the math, in a fixed order; an
 // item's share goes to scratch and the shares are added in order (no atomics: bit-reproducible).
+// A gradient that is not finite makes 2 sum p g - sum g NaN where a signed sum would be infinite.  A sum that is not finite sets a word of
+// its own in the header (this kernel's CTAs must agree on the overflow word); dense_bwd_partsum_launch() turns it into the overflow
+// word, and the exact kernel behind it computes the call.
 //
 // Bound by instruction issue, as dense_bwd_sv.cu.  [48,201,6,65]: 268 us (any-shape kernel 1247), [8,512,1,64]: 57 us (736).
 #include "common.cuh"
@@ -86,7 +89,7 @@ __device__ __forceinline__ void copy16(float *dst, const float *src, int n)
 template <int HG, bool HST, bool K16>
 __global__ void __launch_bounds__(NTHREADS, 1)
 dense_bwd_svr_kernel(const float *__restrict__ g, int g_pitch, const float *__restrict__ q, const float *__restrict__ k, float *__restrict__ d_q,
-		     size_t dq_stride, float *__restrict__ part, const int *__restrict__ tie_hdr,
+		     size_t dq_stride, float *__restrict__ part, int *__restrict__ tie_hdr,
 		     const unsigned char *__restrict__ zero_q, const unsigned char *__restrict__ zero_k, int bs, int n_tok, int n_heads, int width, float scale, Items wk, int only_zeros)
 {
 	using St = Stage<HG>;
@@ -177,6 +180,7 @@ dense_bwd_svr_kernel(const float *__restrict__ g, int g_pitch, const float *__re
 		const float *P = pk + (m & 1) * PK_FLOATS + warp * 32 + lane;
 		const int s = s_first + m * TY + warp;
 		float *out = part + ((size_t(tb) * bs + b) * n_tok + s) * row + size_t(h0) * width + w0 + lane;
+		float all = 0.f; // (rows and columns that do not exist add zeros)
 #pragma unroll
 		for (int j = 0; j < HG; j++) {
 			const float4 *C = reinterpret_cast<const float4 *>(cs + ((m & 1) * TY + warp) * TY + j * (TY / HG));
@@ -189,7 +193,10 @@ dense_bwd_svr_kernel(const float *__restrict__ g, int g_pitch, const float *__re
 			}
 			if (s < n_tok && h0 + j < n_heads && w0 + lane < width)
 				out[size_t(j) * width] = v;
+			all += v;
 		}
+		if (!(fabsf(all) < INFINITY))
+			tie_hdr[BWD_HDR_NOT_FINITE] = 1;
 	};
 
 	// acc -= (row sum) / 2 over the source rows since the last call; the row sum of query row i sits in lane i
@@ -269,7 +276,10 @@ dense_bwd_svr_kernel(const float *__restrict__ g, int g_pitch, const float *__re
 #pragma unroll
 	for (int i = 0; i < XR; i++) {
 		if (i < left) {
-			*reinterpret_cast<volatile float *>(d_q + off) = 2.f * scale * acc[i];
+			const float x = 2.f * scale * acc[i];
+			*reinterpret_cast<volatile float *>(d_q + off) = x;
+			if (!(fabsf(x) < INFINITY))
+				tie_hdr[BWD_HDR_NOT_FINITE] = 1;
 		}
 		off = opaque(off + row);
 	}
@@ -288,7 +298,7 @@ int launch(const float *g, int g_pitch, int only_zeros, const float *q, const fl
 	const long long total = (long long)bs * wk.nhg * wk.ntb * wk.nws * wk.ns;
 	if (total > 0x7fffffffLL)
 		return 1;
-	const int *hdr = reinterpret_cast<const int *>(scratch + sl.hdr);
+	int *hdr = reinterpret_cast<int *>(scratch + sl.hdr);
 	float *part = reinterpret_cast<float *>(scratch + sl.part), *dqp = reinterpret_cast<float *>(scratch + sl.dqpart);
 	const size_t n = size_t(bs) * n_tok * n_heads * width;
 	const float scale = float(-1.0 / sqrt(double(width)));

@@ -89,8 +89,9 @@ inline int bwd_heads_per_item(int n_tok, int n_heads, int width)
 	return best;
 }
 
-// The tie header: listed ties; set when not every tie is listed; set when some q (k) row is zero in every column
-constexpr int BWD_HDR_COUNT = 0, BWD_HDR_OVERFLOW = 1, BWD_HDR_ZERO_Q = 2, BWD_HDR_ZERO_K = 3;
+// The tie header: listed ties; set when not every tie is listed; set when some q (k) row is zero in every column; set by
+// dense_bwd_svr_kernel when a sum of its is not finite
+constexpr int BWD_HDR_COUNT = 0, BWD_HDR_OVERFLOW = 1, BWD_HDR_ZERO_Q = 2, BWD_HDR_ZERO_K = 3, BWD_HDR_NOT_FINITE = 4;
 
 // Caller-provided scratch of the dense backward, in this order (every part 256-byte aligned):
 //   tie flags | tie header | tie list uint4[BWD_TIE_CAP] | shares of d_k | partial d_q (if split)

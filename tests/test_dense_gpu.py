@@ -202,6 +202,25 @@ def test_zero_rows_beside_zero_values(shape):
         assert_close(dk, rk, 1e-5, "dk")
 
 
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 3e38])
+@pytest.mark.parametrize("shape", [(2, 201, 6, 65), (1, 130, 3, 33), (1, 520, 1, 17), (1, 270, 2, 47), (1, 48, 9, 20)])
+def test_ragged_rows_with_gradients_that_are_not_finite(shape, bad):
+    """Infinities, NaN and sums that overflow give what the exact kernel gives, which takes the sign of every term (3e38 four
+    times on one query and one source row, with both signs)."""
+    cabi = _cabi()
+    q, k, g = (_dev(a) for a in _rand(shape, np.float32, 38))
+    b, n, h = shape[0] - 1, shape[1], shape[2] - 1
+    if np.isfinite(bad):
+        g[b, 3, 2:n:n // 4, h], g[b, 5:n:n // 4, n - 1, h] = bad, bad
+        g[b, 3, 3, h] = -bad
+    else:
+        g[b, 3, n - 1, h] = bad
+    got, want = cabi.dense_bwd(g, q, k), cabi.dense_bwd(g, q, k, scratch=None)
+    for x, r in zip(got, want):
+        assert torch.equal(x.nan_to_num(0.5, 2e38, -2e38), r.nan_to_num(0.5, 2e38, -2e38))
+    assert not all(torch.isfinite(r).all() for r in want)
+
+
 @pytest.mark.parametrize("mean", [0.0, 1.0])
 @pytest.mark.parametrize("spread", [1.0, 0.3])
 @pytest.mark.parametrize("shape", [(20, 64, 5, 33), (20, 100, 6, 33), (8, 201, 6, 65), (4, 333, 5, 33), (2, 1040, 1, 66)])
