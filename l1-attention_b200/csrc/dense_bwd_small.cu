@@ -15,6 +15,14 @@
 namespace l1b {
 namespace {
 
+// sign(d) * g with the reference's sign: also a difference of equal infinities (NaN in fp32) has none, as where ties are listed
+__device__ __forceinline__ float term(float d, float g)
+{
+	const float sg = __uint_as_float(__float_as_uint(g) ^ (__float_as_uint(d) & 0x80000000u));
+	return fabsf(d) > 0.f ? sg : 0.f;
+}
+__device__ __forceinline__ double term(double d, double g) { return sign_apply(d, g); }
+
 // TN >= n_tok query rows per thread; NW warps per CTA: consecutive (head, 32 columns) units of one batch item
 template <typename T, int TN, int NW>
 __global__ void __launch_bounds__(NW * 32)
@@ -63,7 +71,7 @@ dense_bwd_small_kernel(const T *__restrict__ g, const T *__restrict__ q, const T
 			const V gv = Gh[s * (TN / VEC) + i];
 #pragma unroll
 			for (int e = 0; e < VEC; e++) {
-				const T x = sign_apply(a[i * VEC + e] - kv, gv.v[e]);
+				const T x = term(a[i * VEC + e] - kv, gv.v[e]);
 				acc[i * VEC + e] += x;
 				sum += x;
 			}

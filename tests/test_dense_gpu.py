@@ -221,6 +221,23 @@ def test_ragged_rows_with_gradients_that_are_not_finite(shape, bad):
     assert not all(torch.isfinite(r).all() for r in want)
 
 
+@pytest.mark.parametrize("shape", [(3, 12, 8, 32), (2, 30, 3, 33), (2, 45, 8, 64), (2, 70, 3, 33), (2, 130, 8, 64)])
+def test_equal_infinities_are_ties(shape):
+    """sign(inf - inf) is 0 in the reference (NaN compares as neither), in every kernel that fp32 takes with scratch."""
+    from oracle import oracle
+    cabi = _cabi()
+    q, k, g = _rand(shape, np.float32, 40)
+    n = shape[1]
+    for b, h, w, x in ((0, 0, 0, np.inf), (1, 2, 31, -np.inf), (1, 1, 4, np.inf)):
+        q[b, n - 2, h, w] = k[b, 3, h, w] = x
+        q[b, 1, h, w] = -x
+    with np.errstate(invalid="ignore"):
+        rq, rk = oracle.dense_bwd(g.astype(np.float64), q.astype(np.float64), k.astype(np.float64))
+    dq, dk = (x.cpu().numpy() for x in cabi.dense_bwd(_dev(g), _dev(q), _dev(k)))
+    assert_close(dq, rq, 1e-5, "dq")
+    assert_close(dk, rk, 1e-5, "dk")
+
+
 @pytest.mark.parametrize("mean", [0.0, 1.0])
 @pytest.mark.parametrize("spread", [1.0, 0.3])
 @pytest.mark.parametrize("shape", [(20, 64, 5, 33), (20, 100, 6, 33), (8, 201, 6, 65), (4, 333, 5, 33), (2, 1040, 1, 66)])
