@@ -315,17 +315,18 @@ softmax_v_tile_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
 				x[j] = (m * TS + j * 16 + sg < sh.n_tok) ? acc[i][j] * sh.scale : -INFINITY; // keys past the end weigh nothing
 				mx = fmaxf(mx, x[j]);
 			}
-			float mnew = mrow[i];
+			float mnew = mrow[i], shift = mnew;
 			if (softmax) {
 #pragma unroll
 				for (int d = 8; d > 0; d >>= 1)
 					mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
 				mnew = fmaxf(mrow[i], mx);
+				shift = mnew == -INFINITY ? 0.f : mnew; // all keys so far infinitely far (masked): they weigh nothing
 			}
 			float ps = 0.f;
 #pragma unroll
 			for (int j = 0; j < 4; j++) {
-				const float p = expf(x[j] - mnew);
+				const float p = expf(x[j] - shift);
 				Pw[i * (2 * NW) * PP + j * 16 + sg] = p;
 				ps += p;
 			}
@@ -333,7 +334,7 @@ softmax_v_tile_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
 			for (int d = 8; d > 0; d >>= 1)
 				ps += __shfl_xor_sync(0xffffffffu, ps, d);
 			if (softmax) {
-				const float alpha = expf(mrow[i] - mnew); // exp(-inf) = 0 on the first tile
+				const float alpha = expf(mrow[i] - shift); // exp(-inf) = 0 on the first tile
 				lrow[i] = lrow[i] * alpha + ps;
 #pragma unroll
 				for (int e = 0; e < NV; e++)

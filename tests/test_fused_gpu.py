@@ -167,6 +167,29 @@ def test_backward_chunks_over_the_batch(monkeypatch):
         assert torch.equal(a, b.grad)
 
 
+@pytest.mark.parametrize("value", [-np.inf, float(np.finfo(np.float32).min)])
+@pytest.mark.parametrize("dims", [(1, 200, 2, 33, 21), (1, 200, 2, 64, 64), (2, 150, 1, 100, 7)])
+def test_masked_keys(dims, value):
+    """Keys at the type's lowest value or at infinity are infinitely far from every query (the distance overflows): they weigh nothing,
+    also where whole tiles of them come first, and get no gradient."""
+    import l1attn_fused_cuda
+    torch.manual_seed(5)
+    bs, n, h, w, wv = dims
+    q, k, v, g = (torch.randn(bs, n, h, x, device="cuda") for x in (w, w, wv, wv))
+    k[:, :130] = value
+    leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    out = l1attn_fused_cuda.L1AttnSoftmaxV()(*leaves)
+    out.backward(g)
+    ref = [t.clone().double().requires_grad_(True) for t in (q, k[:, 130:], v[:, 130:])]
+    x = -(ref[0][:, None] - ref[1][:, :, None]).abs().sum(-1) / w ** 0.5
+    rout = torch.einsum("bsdh,bshw->bdhw", torch.softmax(x, 1), ref[2])
+    rout.backward(g.double())
+    for name, a, r in (("vo", out, rout), ("dq", leaves[0].grad, ref[0].grad), ("dk", leaves[1].grad[:, 130:], ref[1].grad),
+                       ("dv", leaves[2].grad[:, 130:], ref[2].grad)):
+        assert_close(a.detach().cpu().numpy(), r.detach().cpu().numpy(), 1e-5, name)
+    assert not leaves[1].grad[:, :130].any() and not leaves[2].grad[:, :130].any()
+
+
 @pytest.mark.parametrize("dims,step", [((18, 520, 1, 33, 33), 10), ((21, 600, 16, 64, 64), 11)])
 def test_smaller_last_chunk(monkeypatch, dims, step):
     """A last chunk of fewer items splits its source rows over more ranges than the others: every item's gradients are what
