@@ -174,11 +174,12 @@ __device__ __forceinline__ int next_slots(const int32_t *slots, int rb, int dm, 
 // ---- forward, dst pass: scores -> exp -> (+1)-softmax -> attn, vo[dst] = sum_r a_r v[src_r] ----
 // With NX > 0 ONE walk over the slots does all of it: k[src] and v[src] of a slot are gathered together.  The weights
 // have no maximum to subtract, so vo = (sum_r e_r v[src_r]) / denom needs no second walk (two walks: the v rows waited
-// for the last score, and every weight went through memory).
+// for the last score, and every weight went through memory).  That sum is up to denom times as large as vo: `share`, a power of two of at
+// most 1 / (dm + 1), keeps it in range for values close to the type's largest (1 without the softmax).
 template <typename S, typename T, int VEC, int LPHC, int NX, bool EX>
 __global__ void __launch_bounds__(CTA) sparse_fwd_dst_kernel(SparseArgs a, const S *__restrict__ v,
 							      const S *__restrict__ q, const S *__restrict__ k,
-							      S *__restrict__ vo, S *attn, T scale)
+							      S *__restrict__ vo, S *attn, T scale, T share)
 {
 	Who w;
 	if (!decode<LPHC>(a, w))
@@ -228,7 +229,7 @@ __global__ void __launch_bounds__(CTA) sparse_fwd_dst_kernel(SparseArgs a, const
 					for (int i = 0; i < VEC; i++)
 						part += absdiff(qv[it].v[i], kr[u][it].v[i]);
 				part = group_sum<LPHC>(part, lph);
-				const T e = src[u] >= 0 ? exp_t(part * scale) : T(0);
+				const T e = src[u] >= 0 ? exp_t(part * scale) : T(0), es = e * share;
 				denom += e;
 				if (w.li == 0 && w.head_ok && r0 + u < dm)
 					st1<S, T>(arow + size_t(r0 + u) * H, e);
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(CTA) sparse_fwd_dst_kernel(SparseArgs a, const
 					for (int it = 0; it < NX; it++)
 #pragma unroll
 						for (int i = 0; i < VEC; i++)
-							acc[it].v[i] += e * vr[u][it].v[i];
+							acc[it].v[i] += es * vr[u][it].v[i];
 			}
 		}
 		__syncwarp();
@@ -245,7 +246,7 @@ __global__ void __launch_bounds__(CTA) sparse_fwd_dst_kernel(SparseArgs a, const
 			return;
 		T inv = T(1);
 		if (a.use_softmax) {
-			inv = T(1) / denom;
+			inv = T(1) / (denom * share);
 			for (int r = w.li; r < dm; r += lph)
 				st1<S, T>(arow + size_t(r) * H, ld1<S, T>(arow + size_t(r) * H) / denom);
 		}
@@ -862,9 +863,12 @@ int fwd_t(SparseArgs a, const S *v, const S *vb, const S *q, const S *k, S *vo, 
 	if (!g.ok)
 		return L1ATTN_ERR_SHAPE;
 	const T scale = T(-1.0 / sqrt(double(a.width)));
+	T share = T(1);
+	for (double n = 1.0; a.use_softmax && n < a.dm + 1.0; n *= 2.0)
+		share *= T(0.5);
 #define L1B_RUN(LP, NXV, EX)                                                                                         \
 	do {                                                                                                         \
-		sparse_fwd_dst_kernel<S, T, VEC, LP, NXV, EX><<<g.blocks, CTA, 0, st>>>(a, v, q, k, vo, attn, scale); \
+		sparse_fwd_dst_kernel<S, T, VEC, LP, NXV, EX><<<g.blocks, CTA, 0, st>>>(a, v, q, k, vo, attn, scale, share); \
 		L1B_LAUNCH_CHECK();                                                                                  \
 		if (a.bidi) {                                                                                        \
 			sparse_fwd_src_kernel<S, T, VEC, LP, NXV, EX><<<g.blocks, CTA, 0, st>>>(a, vb, attn, vo);     \

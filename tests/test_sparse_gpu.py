@@ -359,6 +359,34 @@ def test_long_and_short_lists_vs_oracle(case, bidi):
         assert_close(x, r, 1e-5, "gradients")
 
 
+@pytest.mark.parametrize("tdtype", ["float32", "float64", "bfloat16"])
+@pytest.mark.parametrize("case", [(1, 40, 8, 64, 64, 30), (2, 24, 2, 33, 20, 20), (1, 24, 3, 32, 32, 12)])
+def test_values_near_the_largest(case, tdtype):
+    """The weights of a destination sum to less than one: values close to the type's largest give finite outputs, although their sum
+    with the weights not yet divided is not.  An infinite value reaches its own destinations only."""
+    import l1attn_sparse_cuda
+    bs, n, h, w, wv, deg = case
+    gen = torch.Generator().manual_seed(7)
+    dt = getattr(torch, tdtype)
+    q, k = (0.01 * torch.randn(bs, n, h, w, generator=gen, dtype=torch.float64) for _ in range(2))
+    big = 2.0 ** (1023 if tdtype == "float64" else 127)  # half the largest, and a power of two
+    v = ((1 + torch.rand(bs, n, h, wv, generator=gen, dtype=torch.float64)) * big * 0.9).to(dt)
+    co = torch.stack([torch.arange(n).repeat_interleave(deg), (torch.arange(n)[:, None] + torch.arange(deg)[None]).reshape(-1) % n], 1)
+    coo, dm, _ = l1attn_sparse_cuda.expandCoo(co)
+    q, k = q.to(dt).cuda(), k.to(dt).cuda()
+    module = l1attn_sparse_cuda.L1AttnSparse()
+    out = module(v.cuda(), q, k, coo.cuda(), dm, True)
+    assert torch.isfinite(out).all()
+    scaled = module((v.double() / big).to(dt).cuda(), q, k, coo.cuda(), dm, True)
+    assert_close(out.double().cpu().numpy() / big, scaled.double().cpu().numpy(), {"float32": 1e-5, "float64": 1e-12, "bfloat16": 1e-2}[tdtype], "vo")
+    v[0, 5] = float("inf")
+    out = module(v.cuda(), q, k, coo.cuda(), dm, True)
+    reached = torch.zeros(bs, n, dtype=torch.bool)
+    reached[0, co[co[:, 1] == 5, 0]] = True
+    assert torch.equal(~torch.isfinite(out).all(-1).all(-1).cpu(), reached)
+    assert torch.isinf(out.cpu()[reached]).all()
+
+
 # ------------------------------------------------------------------ expandCoo
 
 def test_expandcoo_golden(golden):
