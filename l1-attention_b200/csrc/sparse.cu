@@ -175,7 +175,8 @@ __device__ __forceinline__ int next_slots(const int32_t *slots, int rb, int dm, 
 // With NX > 0 ONE walk over the slots does all of it: k[src] and v[src] of a slot are gathered together.  The weights
 // have no maximum to subtract, so vo = (sum_r e_r v[src_r]) / denom needs no second walk (two walks: the v rows waited
 // for the last score, and every weight went through memory).  That sum is up to denom times as large as vo: `share`, a power of two of at
-// most 1 / (dm + 1), keeps it in range for values close to the type's largest (1 without the softmax).
+// most 1 / (dm + 1), keeps it in range for values close to the type's largest (1 without the softmax).  It changes nothing else while a
+// weight times it is no subnormal number.
 template <typename S, typename T, int VEC, int LPHC, int NX, bool EX>
 __global__ void __launch_bounds__(CTA) sparse_fwd_dst_kernel(SparseArgs a, const S *__restrict__ v,
 							      const S *__restrict__ q, const S *__restrict__ k,
@@ -814,10 +815,10 @@ int pow2_ceil(int x)
 // least (idle_den - 1) / idle_den of them would.  Measured at 4096 tokens, 131072 edges, width 64, one batch item:
 // forward 4 heads 0.038 ms against 0.055 ms, 2 heads 0.030 / 0.050; backward 4 heads 0.124 against 0.107 (the
 // unrolled four-vector walk wins although half its lanes idle), 2 heads 0.073 / 0.104 -- so the forward asks
-// with idle_den 2 and the backward with 4.  Rows that are not whole lanes of vectors used to take the generic walk, once
-// per vector and quantity; forward + backward, start and now: 256 tokens, 17 edges each, 64 items of 8 x 32 columns,
-// bidirectional 629 / 259 us; 3001 tokens, 75000 edges, 2 items of 6 x 40 columns (values 24), a new list in
-// every pass (its index included) 718 / 502 us.
+// with idle_den 2 and the backward with 4.  Rows that are not whole lanes of vectors take the same walks with their ends
+// masked: with the generic walk, once per vector and quantity, forward + backward take 629 us instead of 259 (256 tokens,
+// 17 edges each, 64 items of 8 x 32 columns, bidirectional) and 718 instead of 502 (3001 tokens, 75000 edges, 2 items of
+// 6 x 40 columns, values 24, a new list and index in every pass).
 struct RowPlan {
 	int lph, nx;
 	bool exact; // width == v_width == nx * lph vectors: no vector of any lane lies past the end of a row

@@ -341,8 +341,8 @@ def test_full_size_config(bidi, qk_scale):
 @pytest.mark.parametrize("bidi", [False, True])
 @pytest.mark.parametrize("case", [(2, 70, 8, 64, 64), (1, 60, 2, 32, 32), (1, 40, 5, 33, 9), (1, 50, 3, 40, 24)])
 def test_long_and_short_lists_vs_oracle(case, bidi):
-    """Sources with 64, 65 and several hundred incoming edges beside sources with none (long lists are shared by the warps of a
-    CTA), destinations whose slots end early, and a hole in the middle of a list."""
+    """Sources with 64, 65 and several hundred incoming edges beside sources with none (one warp walks a whole list, 32
+    entries' indices at a time), destinations whose slots end early, and a hole in the middle of a list."""
     bs, n, h, w, wv = case
     rng = np.random.RandomState(sum(case))
     rows = [[rng.randint(n), s] for s, c in ((0, 64), (1, 65), (2, 333), (n - 1, 130)) for _ in range(c)] + [[5, s] for s in range(3, 40)]
@@ -357,6 +357,23 @@ def test_long_and_short_lists_vs_oracle(case, bidi):
     assert_close(attn, rattn, 1e-5, "attn")
     for x, r in zip(grads, rgrads):
         assert_close(x, r, 1e-5, "gradients")
+
+
+@pytest.mark.parametrize("tdtype,digits", [("bfloat16", 9), ("float16", 12)])
+@pytest.mark.parametrize("wv", [64, 20])
+def test_16bit_output_is_rounded_once(wv, tdtype, digits):
+    """Weights and sums are float32 up to the output, whose rounding alone is left: 2^-9 of the value in bfloat16, 2^-12 (half
+    of 2^-11) in float16 (weights rounded first: 1.4 times that and more), and 1e-5 for the float32 arithmetic."""
+    from oracle import oracle
+    import l1attn_sparse_cuda
+    rng = np.random.RandomState(8)
+    coo, dm, _ = oracle.expand_coo(random_graph(rng, 60, 20))
+    dt = getattr(torch, tdtype)
+    q, k, v = (torch.from_numpy(s * rng.standard_normal((2, 60, 4, x))).to(dt) for s, x in ((0.3, 64), (0.3, 64), (1, wv)))
+    out = l1attn_sparse_cuda.L1AttnSparse()(v.cuda(), q.cuda(), k.cuda(), torch.from_numpy(coo.astype(np.int32)).cuda(), dm, True)
+    ref, _ = oracle.sparse_fwd(*(x.double().numpy() for x in (v, q, k)), coo, dm, True)
+    err = np.linalg.norm(out.double().cpu().numpy() - ref) / np.linalg.norm(ref)
+    assert err <= 2.0 ** -digits + 1e-5, err
 
 
 @pytest.mark.parametrize("tdtype", ["float32", "float64", "bfloat16"])
