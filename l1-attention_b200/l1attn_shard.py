@@ -223,9 +223,10 @@ class DenseGridShard:
 
     def backward(self, d_attn_loc, q_loc, k_loc, out=None):
         """Returns (d_q of the rank's query rows, d_k of its key rows), complete after the two all-reduces."""
-        if self._scratch is None or self._scratch_for != tuple(q_loc.shape):
+        wanted = (tuple(q_loc.shape), q_loc.dtype, q_loc.device)  # (float64 needs less scratch than float32)
+        if self._scratch is None or self._scratch_for != wanted:
             self._scratch = self.ops.scratch(q_loc)
-            self._scratch_for = tuple(q_loc.shape)
+            self._scratch_for = wanted
         d_q, d_k = self.ops.backward(d_attn_loc, q_loc, k_loc, out, self._scratch)
         if self.row_group is not None:
             dist.all_reduce(d_q, group=self.row_group)

@@ -163,6 +163,26 @@ class _TorchDenseOps:
         return None
 
 
+def test_grid_shard_scratch_follows_the_dtype():
+    """One plan, first in float64 and then in float32 at the same shape: the second needs scratch of its own."""
+    import torch
+    sys.path.insert(0, PKG)
+    import l1attn_shard as sh
+
+    class Ops(_TorchDenseOps):
+        def scratch(self, q):
+            return q.dtype
+
+        def backward(self, d_attn, q, k, out, scratch):
+            assert scratch == q.dtype
+            return super().backward(d_attn, q, k, out, scratch)
+
+    plan = sh.DenseGridShard(1, 6, 2, 0, 1, ops=Ops())
+    for dtype in (torch.float64, torch.float32, torch.float32, torch.float64):
+        q, k = torch.randn(1, 6, 2, 4, dtype=dtype), torch.randn(1, 6, 2, 4, dtype=dtype)
+        plan.backward(torch.randn(1, 6, 6, 2, dtype=dtype), q, k)
+
+
 def _grid_worker(rank, world, port, shape, q):
     sys.path.insert(0, PKG)
     import l1attn_shard as sh
