@@ -22,6 +22,7 @@
 #include <stdlib.h>
 #include "common.cuh"
 #include "tma.cuh"
+#include "tcgen05.cuh"
 #include "dense_bwd_tiles.h"
 
 namespace l1b {
@@ -401,6 +402,379 @@ softmax_v_tile_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_con
 	}
 }
 
+// acc += |q row - k row| over one slice of 32 columns: TI query rows (i * 2 NW + tg) x 4 keys (j * 16 + sg), nc 16-byte chunks of it
+template <int TI, int NW, bool FULL>
+__device__ __forceinline__ void score_slice(const unsigned char *Qslice, const unsigned char *Kslice, int tg, int sg, int nc, float (&acc)[TI][4])
+{
+	const ulonglong2 *Qb = reinterpret_cast<const ulonglong2 *>(Qslice);
+	const ulonglong2 *Kb = reinterpret_cast<const ulonglong2 *>(Kslice);
+#pragma unroll 2
+	for (int c = 0; c < (FULL ? 8 : nc); c++) {
+		ulonglong2 kv[4];
+#pragma unroll
+		for (int j = 0; j < 4; j++) // row j*16+sg, chunk c ^ (row & 7)
+			kv[j] = Kb[(j * 16 + sg) * 8 + (c ^ (sg & 7))];
+#pragma unroll
+		for (int i = 0; i < TI; i++) {
+			const ulonglong2 qv = Qb[(i * (2 * NW) + tg) * 8 + (c ^ (tg & 7))];
+#pragma unroll
+			for (int j = 0; j < 4; j++) {
+				unsigned long long d0, d1;
+				float x0, x1, x2, x3;
+				asm("sub.f32x2 %0, %1, %2;" : "=l"(d0) : "l"(qv.x), "l"(kv[j].x));
+				asm("sub.f32x2 %0, %1, %2;" : "=l"(d1) : "l"(qv.y), "l"(kv[j].y));
+				asm("mov.b64 {%0, %1}, %2;" : "=f"(x0), "=f"(x1) : "l"(d0));
+				asm("mov.b64 {%0, %1}, %2;" : "=f"(x2), "=f"(x3) : "l"(d1));
+				acc[i][j] += fabsf(x0);
+				acc[i][j] += fabsf(x1);
+				acc[i][j] += fabsf(x2);
+				acc[i][j] += fabsf(x3);
+			}
+		}
+	}
+}
+
+// ------------------------------------------------------------------------------------------------
+// Forward with the value product on the tensor cores (fp32, 128-row CTAs, width <= 96, v_width <= 64)
+// ------------------------------------------------------------------------------------------------
+// The scores, the softmax and who owns what are those of softmax_v_tile_kernel<.., 4, 16, ..>; the value product -- a third of that
+// kernel's instructions -- is done by tcgen05.mma.  Weights and values are written as sums of three bf16 each (exact: 3 x 8 bits
+// of 24), nine products with fp32 accumulators per key tile, smallest first; the sums of a tile are read back, rescaled and added in
+// fp32 registers, a tile behind the scores.  Warps:
+//   0-15   scores and weights; the weights' pieces to shared memory (A, [query row][key]), keys in the order 4 * (s % 16) + s / 16, so
+//          that a lane's four weights are neighbours; sums of the tile before: warp = 32 rows x v_width / 4 columns
+//   16     issues the MMAs       17, 18  values' pieces to shared memory (B, [column][key])        19  nothing
+// [16,1024,16,64], values 64 wide: 2.01 ms, softmax_v_tile_kernel 2.24; error against float64 0.85-1.0 of that kernel's.  Bound: FP32 pipe
+// of the scores (two lane-cycles per term) with the shared loads of a 4 x 4 tile beside it.
+// Values that are not finite have no such pieces (inf - inf): a CTA that meets one computes its rows once more, plainly.
+constexpr int TC_NW = 16, TC_ROWS = 128, TC_THREADS = (TC_NW + 4) * 32;
+constexpr int TC_REGS = 104, TC_REGS_REST = 64; // registers per thread, from 96 at the launch: 4 x 104 + 64 <= 5 x 96
+static_assert(4 * TC_REGS + TC_REGS_REST <= 5 * 96, "more than the block was launched with");
+constexpr int TC_A_PIECE = TC_ROWS * 128;          // 64 bf16 a row
+constexpr size_t TC_SMEM = 227 * 1024 - 3072;      // per CTA, less the static part
+
+struct TcBars {
+	uint64_t own, full[MAX_STAGE], empty[MAX_STAGE], p_full, v_full, done, done2;
+	uint32_t tmem;
+	int bad; // something is not finite
+};
+
+// this lane's four weights of row r (keys 4 sg .. in the order above), as three pieces
+__device__ __forceinline__ void store_weights(unsigned char *pieces, int r, int sg, const float (&p)[4])
+{
+	uint32_t a[3], b[3];
+	split_bf16(p[0], p[1], a);
+	split_bf16(p[2], p[3], b);
+	unsigned char *d = pieces + r * 128 + (((sg >> 1) ^ (r & 7)) << 4) + (sg & 1) * 8;
+#pragma unroll
+	for (int i = 0; i < 3; i++)
+		*reinterpret_cast<uint2 *>(d + i * TC_A_PIECE) = make_uint2(a[i], b[i]);
+}
+
+// all products of the pieces, smallest first; steps of 16 k
+template <int STEPS> __device__ __forceinline__ void mma_pieces(uint32_t d, uint64_t a, uint32_t a_piece, uint64_t b, uint32_t b_piece, uint32_t b_step, uint32_t idesc)
+{
+	bool more = false;
+#pragma unroll 1
+	for (int i = 8; i >= 0; i--) { // i = 3 * piece of a + piece of b: (2,2), (2,1), ... (0,0)
+		const uint64_t ai = a + i / 3 * (a_piece >> 4), bi = b + i % 3 * (b_piece >> 4);
+#pragma unroll
+		for (int k = 0; k < STEPS; k++) {
+			tc_mma_bf16_ss(d, ai + k * 2, bi + k * (b_step >> 4), idesc, more);
+			more = true;
+		}
+	}
+}
+
+template <int NV, bool TMA, bool FULL>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
+		    const __grid_constant__ CUtensorMap vmap, const float *__restrict__ q, const float *__restrict__ k,
+		    const float *__restrict__ v, float *__restrict__ vo, float *__restrict__ lse, SvShape sh, int *err)
+{
+	constexpr int NW = TC_NW, TI = 4, TT = TC_ROWS, VW = 16 * NV, V_BYTES = TS * VW * 4, NO = VW / 4;
+	constexpr int V_PIECE = VW * 128;
+	extern __shared__ __align__(1024) unsigned char smem_raw[];
+	unsigned char *base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+	__shared__ __align__(8) TcBars bars;
+	__shared__ float row_corr[2][TT], row_inv[TT], row_max[TT];
+	const int q_bytes = sh.nwb * TT * 128, k_bytes = sh.nwb * TS * 128, stage_bytes = k_bytes + V_BYTES;
+	unsigned char *Pp = base, *Vp = Pp + 3 * TC_A_PIECE, *Qs = Vp + 3 * V_PIECE, *stages = Qs + q_bytes;
+
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	unsigned r = blockIdx.x;
+	const int t0 = int(r % unsigned(sh.ntt)) * TT;
+	r /= unsigned(sh.ntt);
+	const int h = int(r % unsigned(sh.n_heads));
+	const int b = int(r / unsigned(sh.n_heads));
+	const int ns = (sh.n_tok + TS - 1) / TS;
+
+	if (warp == 16)
+		tmem_alloc(&bars.tmem, 64);
+	if (tid == 0) {
+		mbar_init(&bars.own, TMA ? 1 : NW * 32);
+		for (int s = 0; s < MAX_STAGE; s++) {
+			mbar_init(&bars.full[s], TMA ? 1 : NW * 32);
+			mbar_init(&bars.empty[s], NW + 2);
+		}
+		mbar_init(&bars.p_full, NW);
+		mbar_init(&bars.v_full, 2);
+		mbar_init(&bars.done, 1);
+		bars.bad = 0;
+		mbar_fence_init();
+	}
+	tc_fence_before();
+	__syncthreads();
+	tc_fence_after();
+	const uint32_t tmem = bars.tmem;
+	const size_t krow = size_t(sh.n_heads) * sh.width, vrow = size_t(sh.n_heads) * sh.v_width;
+	const size_t qk0 = size_t(b) * sh.n_tok * krow + size_t(h) * sh.width, v0 = size_t(b) * sh.n_tok * vrow + size_t(h) * sh.v_width;
+
+	if (warp < NW) {
+		asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TC_REGS));
+		auto load_tile = [&](int m) {
+			const int st = m % sh.nstage;
+			unsigned char *dst = stages + size_t(st) * stage_bytes;
+			if (!TMA) {
+				copy_rows<NW, true>(dst, k + qk0, krow, m * TS, TS, sh.nwb, sh.width, sh.n_tok);
+				copy_rows<NW, false>(dst + k_bytes, v + v0, vrow, m * TS, TS, VW / 32, sh.v_width, sh.n_tok);
+				copy_arrive(&bars.full[st]);
+				return;
+			}
+			mbar_expect_tx(&bars.full[st], uint32_t(stage_bytes));
+			for (int wb = 0; wb < sh.nwb; wb++)
+				tma_load_4d(dst + wb * TS * 128, &kmap, &bars.full[st], wb * 32, h, m * TS, b);
+			tma_load_4d(dst + k_bytes, &vmap, &bars.full[st], 0, h, m * TS, b);
+		};
+		if (!TMA || tid == 0) {
+			if (TMA) {
+				mbar_expect_tx(&bars.own, uint32_t(q_bytes));
+				for (int wb = 0; wb < sh.nwb; wb++)
+					tma_load_4d(Qs + wb * TT * 128, &qmap, &bars.own, wb * 32, h, t0, b);
+			} else {
+				copy_rows<NW, true>(Qs, q + qk0, krow, t0, TT, sh.nwb, sh.width, sh.n_tok);
+				copy_arrive(&bars.own);
+			}
+			for (int m = 0; m < sh.nstage - 1 && m < ns; m++)
+				load_tile(m);
+		}
+
+		const int sg = lane & 15, tg = warp * 2 + (lane >> 4);
+		const int orow = (warp & 3) * 32 + lane, ocol = (warp >> 2) * NO; // this thread's part of the output
+		const uint32_t d_at = tmem + (uint32_t((warp & 3) * 32) << 16) + ocol;
+		const bool softmax = sh.mode == L1ATTN_SV_SOFTMAX;
+		float o[NO], mrow[TI], lrow[TI];
+#pragma unroll
+		for (int i = 0; i < TI; i++) {
+			mrow[i] = softmax ? -INFINITY : 0.f;
+			lrow[i] = sh.mode == L1ATTN_SV_SOFTMAX_PLUS_ONE ? 1.f : 0.f; // the extra all-zero row weighs exp(0)
+		}
+#pragma unroll
+		for (int e = 0; e < NO; e++)
+			o[e] = 0.f;
+		bool dead = !mbar_wait_inline(&bars.own, 0, err);
+		// the sums of tile m, once its MMAs are done, onto the output, which goes to that tile's shift first
+		auto collect = [&](int m) {
+			if (!dead && !(mbar_wait_inline(&bars.p_full, m & 1, err) && mbar_wait_inline(&bars.done, m & 1, err)))
+				dead = true;
+			tc_fence_after();
+			float d[NO];
+			tmem_load(d_at, d);
+			const float c = row_corr[m & 1][orow];
+#pragma unroll
+			for (int e = 0; e < NO; e++)
+				o[e] = fmaf(o[e], c, d[e]);
+		};
+
+		for (int m = 0; m < ns; m++) {
+			if ((!TMA || (warp == m % NW && lane == 0)) && m + sh.nstage - 1 < ns && !dead) {
+				const int mm = m + sh.nstage - 1;
+				if (mbar_wait_inline(&bars.empty[mm % sh.nstage], ((unsigned(mm) / unsigned(sh.nstage)) & 1u) ^ 1u, err))
+					load_tile(mm);
+				else
+					dead = true;
+			}
+			__syncwarp();
+			const int st = m % sh.nstage;
+			if (!dead && !mbar_wait_inline(&bars.full[st], (unsigned(m) / unsigned(sh.nstage)) & 1u, err))
+				dead = true; // keep walking without waiting; the error word reports the failure
+			const unsigned char *Ks = stages + size_t(st) * stage_bytes;
+
+			float acc[TI][4];
+#pragma unroll
+			for (int i = 0; i < TI; i++)
+#pragma unroll
+				for (int j = 0; j < 4; j++)
+					acc[i][j] = 0.f;
+			for (int wb = 0; wb < sh.nwb; wb++) {
+				const int nc = FULL ? 8 : min(8, ((sh.width - wb * 32 + 7) >> 3) * 2);
+				score_slice<TI, NW, FULL>(Qs + wb * TT * 128, Ks + wb * TS * 128, tg, sg, nc, acc);
+			}
+			__syncwarp();
+			if (lane == 0)
+				mbar_arrive(&bars.empty[st]);
+
+			float corr[TI];
+#pragma unroll
+			for (int i = 0; i < TI; i++) {
+				float mx = -INFINITY;
+#pragma unroll
+				for (int j = 0; j < 4; j++) {
+					acc[i][j] = (m * TS + j * 16 + sg < sh.n_tok) ? acc[i][j] * sh.scale : -INFINITY; // keys past the end weigh nothing
+					mx = fmaxf(mx, acc[i][j]);
+				}
+				float shift = mrow[i];
+				corr[i] = 1.f;
+				if (softmax) {
+#pragma unroll
+					for (int d = 8; d > 0; d >>= 1)
+						mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+					const float mnew = fmaxf(mrow[i], mx);
+					shift = mnew == -INFINITY ? 0.f : mnew; // all keys so far infinitely far (masked): they weigh nothing
+					corr[i] = expf(mrow[i] - shift);        // exp(-inf) = 0 on the first tile
+					mrow[i] = mnew;
+				}
+				float ps = 0.f;
+#pragma unroll
+				for (int j = 0; j < 4; j++) {
+					acc[i][j] = expf(acc[i][j] - shift);
+					ps += acc[i][j];
+				}
+#pragma unroll
+				for (int d = 8; d > 0; d >>= 1)
+					ps += __shfl_xor_sync(0xffffffffu, ps, d);
+				lrow[i] = lrow[i] * corr[i] + ps;
+			}
+			if (m > 0)
+				collect(m - 1); // (and the pieces of tile m - 1 are read)
+#pragma unroll
+			for (int i = 0; i < TI; i++) {
+				store_weights(Pp, i * (2 * NW) + tg, sg, acc[i]);
+				if (sg == 0)
+					row_corr[m & 1][i * (2 * NW) + tg] = corr[i];
+			}
+			fence_proxy_async_smem();
+			tc_fence_before();
+			__syncwarp();
+			if (lane == 0)
+				mbar_arrive(&bars.p_full);
+		}
+		collect(ns - 1);
+#pragma unroll
+		for (int i = 0; i < TI; i++) {
+			const int row = i * (2 * NW) + tg, t = t0 + row;
+			if (sg == 0) {
+				row_inv[row] = sh.mode == L1ATTN_SV_EXP ? 1.f : 1.f / lrow[i];
+				row_max[row] = mrow[i];
+				if (lse && t < sh.n_tok) // weight of (s, t) = exp(x - lse)
+					lse[(size_t(b) * sh.n_tok + t) * sh.n_heads + h] = sh.mode == L1ATTN_SV_EXP ? 0.f : mrow[i] + logf(lrow[i]);
+			}
+		}
+		named_barrier(1, NW * 32);
+		if (*reinterpret_cast<volatile int *>(&bars.bad) == 0) {
+			if (t0 + orow < sh.n_tok) {
+				float *op = vo + v0 + size_t(t0 + orow) * vrow + ocol;
+				const float inv = row_inv[orow];
+#pragma unroll
+				for (int e = 0; e < NO; e++)
+					if (FULL || ocol + e < sh.v_width)
+						op[e] = o[e] * inv;
+			}
+		} else { // a row per warp, 32 keys at a time
+#pragma unroll 1
+			for (int row = warp; row < TT && t0 + row < sh.n_tok; row += NW) {
+				const float *qr = q + qk0 + size_t(t0 + row) * krow;
+				const float shift = row_max[row] == -INFINITY ? 0.f : row_max[row];
+				float sum[VW / 32] = {};
+#pragma unroll 1
+				for (int s0 = 0; s0 < sh.n_tok; s0 += 32) {
+					float x = 0.f;
+					if (s0 + lane < sh.n_tok)
+						for (int w = 0; w < sh.width; w++)
+							x += fabsf(qr[w] - k[qk0 + size_t(s0 + lane) * krow + w]);
+					const float p = expf(x * sh.scale - shift);
+#pragma unroll 1
+					for (int e = 0; e < 32 && s0 + e < sh.n_tok; e++) {
+						const float pe = __shfl_sync(0xffffffffu, p, e);
+#pragma unroll
+						for (int c = 0; c < VW / 32; c++)
+							if (c * 32 + lane < sh.v_width)
+								sum[c] = fmaf(pe, v[v0 + size_t(s0 + e) * vrow + c * 32 + lane], sum[c]);
+					}
+				}
+#pragma unroll
+				for (int c = 0; c < VW / 32; c++)
+					if (c * 32 + lane < sh.v_width)
+						vo[v0 + size_t(t0 + row) * vrow + c * 32 + lane] = sum[c] * row_inv[row];
+			}
+		}
+	} else {
+		asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TC_REGS_REST));
+		if (warp == 16 && lane == 0) {
+			const uint64_t a = tc_desc(smem_u32(Pp)), bd = tc_desc(smem_u32(Vp));
+			bool dead = false;
+			for (int m = 0; m < ns && !dead; m++) {
+				dead = !(mbar_wait_inline(&bars.v_full, m & 1, err) && mbar_wait_inline(&bars.p_full, m & 1, err));
+				tc_fence_after();
+				if (!dead)
+					mma_pieces<4>(tmem, a, TC_A_PIECE, bd, V_PIECE, 32, tc_idesc_bf16(VW, false));
+				tc_commit(&bars.done);
+			}
+		}
+		if (warp == 17 || warp == 18) { // a column per thread (VW 32: half of the threads)
+			const int c = (warp - 17) * 32 + lane;
+			bool dead = false;
+			for (int m = 0; m < ns; m++) {
+				const int st = m % sh.nstage;
+				if (!dead && !mbar_wait_inline(&bars.full[st], (unsigned(m) / unsigned(sh.nstage)) & 1u, err))
+					dead = true;
+				if (m > 0 && !dead && !mbar_wait_inline(&bars.done, (m - 1) & 1, err))
+					dead = true;
+				const float *Vs = reinterpret_cast<const float *>(stages + size_t(st) * stage_bytes + k_bytes);
+				float chk = 0.f;
+				if (c < VW) {
+#pragma unroll 2
+					for (int g = 0; g < 8; g++) { // keys at places 8 g .. 8 g + 7
+						uint32_t o[3][4];
+#pragma unroll
+						for (int e = 0; e < 4; e++) {
+							const int s = (e & 1) * 32 + 2 * g + (e >> 1); // places 8 g + 2 e, + 1: keys s, s + 16
+							const float x = Vs[s * VW + c], y = Vs[(s + 16) * VW + c];
+							chk = fmaf(x, 0.f, fmaf(y, 0.f, chk));
+							uint32_t pc[3];
+							split_bf16(x, y, pc);
+#pragma unroll
+							for (int i = 0; i < 3; i++)
+								o[i][e] = pc[i];
+						}
+#pragma unroll
+						for (int i = 0; i < 3; i++)
+							*reinterpret_cast<uint4 *>(Vp + i * V_PIECE + c * 128 + ((g ^ (c & 7)) << 4)) = make_uint4(o[i][0], o[i][1], o[i][2], o[i][3]);
+					}
+				}
+				if (!(chk == 0.f))
+					*reinterpret_cast<volatile int *>(&bars.bad) = 1;
+				fence_proxy_async_smem();
+				__syncwarp();
+				if (lane == 0) {
+					mbar_arrive(&bars.v_full);
+					mbar_arrive(&bars.empty[st]);
+				}
+			}
+		}
+		__syncwarp();
+	}
+	tc_fence_before();
+	__syncthreads();
+	if (warp == 16)
+		tmem_free(tmem, 64);
+}
+
+size_t sv_tc_smem(int nwb, int nv, int nstage)
+{
+	return size_t(3) * TC_A_PIECE + size_t(3) * nv * 16 * 128 + size_t(nwb) * TC_ROWS * 128 + size_t(nstage) * (size_t(nwb) * TS * 128 + size_t(TS) * nv * 64) + 1024;
+}
+
 template <int NV, int TI, int NW, bool TMA, bool FULL>
 int launch_tile(const float *q, const float *k, const float *v, float *vo, float *lse, int bs, int n_tok, int n_heads,
 		int width, int v_width, int mode, int nstage, size_t smem, cudaStream_t st)
@@ -432,6 +806,18 @@ int launch_tile(const float *q, const float *k, const float *v, float *vo, float
 	const long long grid = (long long)bs * n_heads * sh.ntt;
 	if (grid > 0x7fffffffLL)
 		return L1ATTN_ERR_SHAPE;
+	if constexpr (NW == TC_NW && NV <= 4) { // 128-row CTAs
+		const int tc_stages = sv_tc_smem(sh.nwb, NV, 3) <= TC_SMEM ? 3 : 2;
+		const size_t tc_smem = sv_tc_smem(sh.nwb, NV, tc_stages);
+		if (tc_smem <= TC_SMEM) {
+			sh.nstage = tc_stages;
+			auto kern = softmax_v_tc_kernel<NV, TMA, FULL>;
+			L1B_SHARED_MEMORY(kern, int(tc_smem));
+			kern<<<unsigned(grid), TC_THREADS, tc_smem, st>>>(qmap, kmap, vmap, q, k, v, vo, lse, sh, err);
+			L1B_LAUNCH_CHECK();
+			return L1ATTN_OK;
+		}
+	}
 	auto kern = softmax_v_tile_kernel<NV, TI, NW, TMA, FULL>;
 	L1B_SHARED_MEMORY(kern, int(smem));
 	kern<<<unsigned(grid), NTH, smem, st>>>(qmap, kmap, vmap, q, k, v, vo, lse, sh, err);
@@ -829,6 +1215,316 @@ softmax_v_bwd_tile_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
 	}
 }
 
+
+// The same with both products on the tensor cores (128-row CTAs, width and v_width <= 64): dp = <v, dvo> in D1, dv in D2, operands as
+// three bf16 pieces each (see softmax_v_tc_kernel).  The pieces of dvo lie [query][column], queries in the order 4 * (t % 16) + t / 16:
+// for dp that is B with its columns along k, for dv B with its queries along k (n contiguous).  Per tile: dp is computed as soon as its
+// pieces are there, beside the scores; it goes through shared memory from the tensor memory's rows to the lanes that hold the scores, in
+// the place of the weights' pieces, which are written behind it.  [4,1024,16,64], values 64 wide: 632 us, softmax_v_bwd_tile_kernel 909.
+template <int NV, bool TMA, bool FULL>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
+			const __grid_constant__ CUtensorMap gmap, const float *__restrict__ q, const float *__restrict__ k,
+			const float *__restrict__ v, const float *__restrict__ dvo, const float *__restrict__ lse,
+			const float *__restrict__ delta, float *__restrict__ dx, float *__restrict__ dv, SvShape sh, int *err)
+{
+	constexpr int NW = TC_NW, TI = 4, TT = TC_ROWS, VW = 16 * NV, NVB = VW / 32, NO = VW / 4;
+	constexpr int G_PIECE = TS * 128; // 64 queries of 64 bf16 (VW 32: half of them unused)
+	extern __shared__ __align__(1024) unsigned char smem_raw[];
+	unsigned char *base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+	__shared__ __align__(8) TcBars bars;
+	const int k_bytes = sh.nwb * TT * 128, q_bytes = sh.nwb * TS * 128, g_bytes = NVB * TS * 128, stage_bytes = q_bytes + g_bytes;
+	unsigned char *Vp = base, *Pp = Vp + 3 * TC_A_PIECE, *Gp = Pp + 3 * TC_A_PIECE, *Ks = Gp + 3 * G_PIECE, *stages = Ks + k_bytes;
+
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	unsigned r = blockIdx.x;
+	const int s0 = int(r % unsigned(sh.ntt)) * TT;
+	r /= unsigned(sh.ntt);
+	const int h = int(r % unsigned(sh.n_heads));
+	const int b = int(r / unsigned(sh.n_heads));
+	const int nt = (sh.n_tok + TS - 1) / TS;
+	const size_t krow = size_t(sh.n_heads) * sh.width, vrow = size_t(sh.n_heads) * sh.v_width;
+	const size_t qk0 = size_t(b) * sh.n_tok * krow + size_t(h) * sh.width, v0 = size_t(b) * sh.n_tok * vrow + size_t(h) * sh.v_width;
+
+	if (warp == 16)
+		tmem_alloc(&bars.tmem, 128);
+	if (tid == 0) {
+		mbar_init(&bars.own, TMA ? 1 : NW * 32);
+		for (int s = 0; s < MAX_STAGE; s++) {
+			mbar_init(&bars.full[s], TMA ? 1 : NW * 32);
+			mbar_init(&bars.empty[s], NW + 2);
+		}
+		mbar_init(&bars.p_full, NW);
+		mbar_init(&bars.v_full, 2); // (the pieces of dvo)
+		mbar_init(&bars.done, 1);   // D1
+		mbar_init(&bars.done2, 1);  // D2
+		bars.bad = 0;
+		mbar_fence_init();
+	}
+	__syncthreads();
+	// the CTA's own value rows as pieces [source row][column]
+	for (int i = tid; i < TT * (VW / 2); i += TC_THREADS) {
+		const int row = i / (VW / 2), c = i % (VW / 2) * 2;
+		const float *vp = v + v0 + size_t(s0 + row < sh.n_tok ? s0 + row : 0) * vrow + c;
+		const float x = s0 + row < sh.n_tok && c < sh.v_width ? vp[0] : 0.f, y = s0 + row < sh.n_tok && c + 1 < sh.v_width ? vp[1] : 0.f;
+		if (!(fmaf(x, 0.f, y * 0.f) == 0.f))
+			*reinterpret_cast<volatile int *>(&bars.bad) = 1;
+		uint32_t pc[3];
+		split_bf16(x, y, pc);
+		unsigned char *d = Vp + row * 128 + (((c >> 3) ^ (row & 7)) << 4) + (c & 7) * 2;
+#pragma unroll
+		for (int e = 0; e < 3; e++)
+			*reinterpret_cast<uint32_t *>(d + e * TC_A_PIECE) = pc[e];
+	}
+	fence_proxy_async_smem();
+	tc_fence_before();
+	__syncthreads();
+	tc_fence_after();
+	const uint32_t tmem = bars.tmem, D1 = 0, D2 = 64;
+	const size_t hstride = size_t(sh.n_heads);
+	const size_t dx_t = sh.dx_pitch > 0 ? 1 : hstride, dx_s = sh.dx_pitch > 0 ? size_t(sh.dx_pitch) : hstride * sh.n_tok;
+	const size_t dx0 = sh.dx_pitch > 0 ? (size_t(b) * sh.n_heads + h) * sh.n_tok * sh.dx_pitch : size_t(b) * sh.n_tok * sh.n_tok * hstride + h;
+
+	if (warp < NW) {
+		asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TC_REGS));
+		auto load_tile = [&](int m) {
+			const int st = m % sh.nstage;
+			unsigned char *dst = stages + size_t(st) * stage_bytes;
+			if (!TMA) {
+				copy_rows<NW, true>(dst, q + qk0, krow, m * TS, TS, sh.nwb, sh.width, sh.n_tok);
+				copy_rows<NW, true>(dst + q_bytes, dvo + v0, vrow, m * TS, TS, NVB, sh.v_width, sh.n_tok);
+				copy_arrive(&bars.full[st]);
+				return;
+			}
+			mbar_expect_tx(&bars.full[st], uint32_t(stage_bytes));
+			for (int wb = 0; wb < sh.nwb; wb++)
+				tma_load_4d(dst + wb * TS * 128, &qmap, &bars.full[st], wb * 32, h, m * TS, b);
+			for (int vb = 0; vb < NVB; vb++)
+				tma_load_4d(dst + q_bytes + vb * TS * 128, &gmap, &bars.full[st], vb * 32, h, m * TS, b);
+		};
+		if (!TMA || tid == 0) {
+			if (TMA) {
+				mbar_expect_tx(&bars.own, uint32_t(k_bytes));
+				for (int wb = 0; wb < sh.nwb; wb++)
+					tma_load_4d(Ks + wb * TT * 128, &kmap, &bars.own, wb * 32, h, s0, b);
+			} else {
+				copy_rows<NW, true>(Ks, k + qk0, krow, s0, TT, sh.nwb, sh.width, sh.n_tok);
+				copy_arrive(&bars.own);
+			}
+			for (int m = 0; m < sh.nstage - 1 && m < nt; m++)
+				load_tile(m);
+		}
+
+		const int sg = lane & 15, tg = warp * 2 + (lane >> 4);
+		const int orow = (warp & 3) * 32 + lane, part = warp >> 2; // this thread's part of D1 and D2: a row, a quarter of the columns
+		const uint32_t d_at = tmem + (uint32_t((warp & 3) * 32) << 16);
+		float o[NO];
+#pragma unroll
+		for (int e = 0; e < NO; e++)
+			o[e] = 0.f;
+		bool dead = !mbar_wait_inline(&bars.own, 0, err);
+		auto collect = [&](int m) { // dv of tile m
+			if (!dead && !mbar_wait_inline(&bars.done2, m & 1, err))
+				dead = true;
+			tc_fence_after();
+			float d[NO];
+			tmem_load(d_at + D2 + part * NO, d);
+#pragma unroll
+			for (int e = 0; e < NO; e++)
+				o[e] += d[e];
+		};
+
+		for (int m = 0; m < nt; m++) {
+			if ((!TMA || (warp == m % NW && lane == 0)) && m + sh.nstage - 1 < nt && !dead) {
+				const int mm = m + sh.nstage - 1;
+				if (mbar_wait_inline(&bars.empty[mm % sh.nstage], ((unsigned(mm) / unsigned(sh.nstage)) & 1u) ^ 1u, err))
+					load_tile(mm);
+				else
+					dead = true;
+			}
+			__syncwarp();
+			const int st = m % sh.nstage;
+			if (!dead && !mbar_wait_inline(&bars.full[st], (unsigned(m) / unsigned(sh.nstage)) & 1u, err))
+				dead = true;
+			const unsigned char *Qs = stages + size_t(st) * stage_bytes;
+			float acc[TI][4];
+#pragma unroll
+			for (int i = 0; i < TI; i++)
+#pragma unroll
+				for (int j = 0; j < 4; j++)
+					acc[i][j] = 0.f;
+			for (int wb = 0; wb < sh.nwb; wb++) {
+				const int nc = FULL ? 8 : min(8, ((sh.width - wb * 32 + 7) >> 3) * 2);
+				score_slice<TI, NW, FULL>(Ks + wb * TT * 128, Qs + wb * TS * 128, tg, sg, nc, acc);
+			}
+			__syncwarp();
+			if (lane == 0)
+				mbar_arrive(&bars.empty[st]);
+			// per-query statistics of this lane's 4 columns (in flight while the products are collected)
+			float lj[4], dj[4];
+#pragma unroll
+			for (int j = 0; j < 4; j++) {
+				const int t = m * TS + j * 16 + sg;
+				const bool ok = t < sh.n_tok;
+				const size_t at = (size_t(b) * sh.n_tok + (ok ? t : 0)) * hstride + h;
+				lj[j] = ok ? lse[at] : INFINITY; // exp(x - inf) = 0: query rows past the end weigh nothing
+				dj[j] = ok ? delta[at] : 0.f;
+			}
+			if (m > 0)
+				collect(m - 1); // (and the weights' pieces of tile m - 1 are read)
+			if (!dead && !mbar_wait_inline(&bars.done, m & 1, err))
+				dead = true;
+			tc_fence_after();
+			{ // dp: a row and 16 places of it per thread to [row][place], 16-byte chunk ^= row & 15
+				float d[16];
+				tmem_load(d_at + D1 + part * 16, d);
+#pragma unroll
+				for (int e = 0; e < 4; e++)
+					*reinterpret_cast<float4 *>(Pp + orow * 256 + (((part * 4 + e) ^ (orow & 15)) << 4)) =
+						make_float4(d[e * 4], d[e * 4 + 1], d[e * 4 + 2], d[e * 4 + 3]);
+			}
+			named_barrier(1, NW * 32);
+#pragma unroll
+			for (int i = 0; i < TI; i++) {
+				const int row = i * (2 * NW) + tg, s = s0 + row;
+				const float4 dp = *reinterpret_cast<const float4 *>(Pp + row * 256 + ((sg ^ (row & 15)) << 4));
+				float *dxr = dx + dx0 + size_t(s < sh.n_tok ? s : 0) * dx_s;
+				const float dpj[4] = {dp.x, dp.y, dp.z, dp.w};
+#pragma unroll
+				for (int j = 0; j < 4; j++) {
+					const int t = m * TS + j * 16 + sg;
+					const float p = expf(acc[i][j] * sh.scale - lj[j]);
+					// (equal rows: the distance has no slope in any column, so its gradient reaches neither)
+					if (s < sh.n_tok && t < sh.n_tok)
+						dxr[size_t(t) * dx_t] = sh.dx_pitch > 0 && acc[i][j] == 0.f ? 0.f : p * (dpj[j] - dj[j]);
+					acc[i][j] = p;
+				}
+			}
+			named_barrier(1, NW * 32); // (dp is read)
+#pragma unroll
+			for (int i = 0; i < TI; i++)
+				store_weights(Pp, i * (2 * NW) + tg, sg, acc[i]);
+			fence_proxy_async_smem();
+			tc_fence_before();
+			__syncwarp();
+			if (lane == 0)
+				mbar_arrive(&bars.p_full);
+		}
+		collect(nt - 1);
+		if (*reinterpret_cast<volatile int *>(&bars.bad) == 0) {
+			if (s0 + orow < sh.n_tok) {
+				float *op = dv + v0 + size_t(s0 + orow) * vrow + part * NO;
+#pragma unroll
+				for (int e = 0; e < NO; e++)
+					if (FULL || part * NO + e < sh.v_width)
+						op[e] = o[e];
+			}
+		} else { // a source row per warp, 32 queries at a time
+			named_barrier(1, NW * 32);
+#pragma unroll 1
+			for (int row = warp; row < TT && s0 + row < sh.n_tok; row += NW) {
+				const float *kr = k + qk0 + size_t(s0 + row) * krow, *vr = v + v0 + size_t(s0 + row) * vrow;
+				float sum[NVB] = {};
+#pragma unroll 1
+				for (int t0 = 0; t0 < sh.n_tok; t0 += 32) {
+					const int t = t0 + lane;
+					float x = 0.f, p = 0.f, d = 0.f;
+					if (t < sh.n_tok) {
+						for (int w = 0; w < sh.width; w++)
+							x += fabsf(kr[w] - q[qk0 + size_t(t) * krow + w]);
+						for (int c = 0; c < sh.v_width; c++)
+							d = fmaf(vr[c], dvo[v0 + size_t(t) * vrow + c], d);
+						const size_t at = (size_t(b) * sh.n_tok + t) * hstride + h;
+						p = expf(x * sh.scale - lse[at]);
+						dx[dx0 + size_t(s0 + row) * dx_s + size_t(t) * dx_t] = sh.dx_pitch > 0 && x == 0.f ? 0.f : p * (d - delta[at]);
+					}
+#pragma unroll 1
+					for (int e = 0; e < 32 && t0 + e < sh.n_tok; e++) {
+						const float pe = __shfl_sync(0xffffffffu, p, e);
+#pragma unroll
+						for (int c = 0; c < NVB; c++)
+							if (c * 32 + lane < sh.v_width)
+								sum[c] = fmaf(pe, dvo[v0 + size_t(t0 + e) * vrow + c * 32 + lane], sum[c]);
+					}
+				}
+#pragma unroll
+				for (int c = 0; c < NVB; c++)
+					if (c * 32 + lane < sh.v_width)
+						dv[v0 + size_t(s0 + row) * vrow + c * 32 + lane] = sum[c];
+			}
+		}
+	} else {
+		asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TC_REGS_REST));
+		if (warp == 16 && lane == 0) {
+			const uint64_t va = tc_desc(smem_u32(Vp)), pa = tc_desc(smem_u32(Pp)), gk = tc_desc(smem_u32(Gp)), gn = tc_desc_mn(smem_u32(Gp));
+			bool dead = false;
+			for (int m = 0; m < nt && !dead; m++) {
+				dead = !mbar_wait_inline(&bars.v_full, m & 1, err);
+				tc_fence_after();
+				if (!dead)
+					mma_pieces<VW / 16>(tmem + D1, va, TC_A_PIECE, gk, G_PIECE, 32, tc_idesc_bf16(TS, false));
+				tc_commit(&bars.done);
+				dead = dead || !mbar_wait_inline(&bars.p_full, m & 1, err);
+				tc_fence_after();
+				if (!dead)
+					mma_pieces<TS / 16>(tmem + D2, pa, TC_A_PIECE, gn, G_PIECE, 2048, tc_idesc_bf16(VW, true));
+				tc_commit(&bars.done2);
+			}
+		}
+		if (warp == 17 || warp == 18) { // a query row per thread
+			const int t = (warp - 17) * 32 + lane, place = 4 * (t % 16) + t / 16;
+			bool dead = false;
+			for (int m = 0; m < nt; m++) {
+				const int st = m % sh.nstage;
+				if (!dead && !mbar_wait_inline(&bars.full[st], (unsigned(m) / unsigned(sh.nstage)) & 1u, err))
+					dead = true;
+				if (m > 0 && !dead && !mbar_wait_inline(&bars.done2, (m - 1) & 1, err))
+					dead = true;
+				const unsigned char *Gs = stages + size_t(st) * stage_bytes + q_bytes;
+				float chk = 0.f;
+#pragma unroll 2
+				for (int g = 0; g < VW / 8; g++) { // columns 8 g .. 8 g + 7: two chunks of the row's 128-byte slice
+					uint32_t o[3][4];
+#pragma unroll
+					for (int e = 0; e < 2; e++) {
+						const float4 x = *reinterpret_cast<const float4 *>(Gs + (g >> 2) * TS * 128 + t * 128 + ((((g & 3) * 2 + e) ^ (t & 7)) << 4));
+						chk = fmaf(x.x, 0.f, fmaf(x.y, 0.f, fmaf(x.z, 0.f, fmaf(x.w, 0.f, chk))));
+						uint32_t pa[3], pb[3];
+						split_bf16(x.x, x.y, pa);
+						split_bf16(x.z, x.w, pb);
+#pragma unroll
+						for (int i = 0; i < 3; i++) {
+							o[i][e * 2] = pa[i];
+							o[i][e * 2 + 1] = pb[i];
+						}
+					}
+#pragma unroll
+					for (int i = 0; i < 3; i++)
+						*reinterpret_cast<uint4 *>(Gp + i * G_PIECE + place * 128 + ((g ^ (place & 7)) << 4)) = make_uint4(o[i][0], o[i][1], o[i][2], o[i][3]);
+				}
+				if (!(chk == 0.f))
+					*reinterpret_cast<volatile int *>(&bars.bad) = 1;
+				fence_proxy_async_smem();
+				__syncwarp();
+				if (lane == 0) {
+					mbar_arrive(&bars.v_full);
+					mbar_arrive(&bars.empty[st]);
+				}
+			}
+		}
+		__syncwarp();
+	}
+	tc_fence_before();
+	__syncthreads();
+	if (warp == 16)
+		tmem_free(tmem, 128);
+}
+
+size_t sv_bwd_tc_smem(int nwb, int nv, int nstage)
+{
+	return size_t(6) * TC_A_PIECE + size_t(3) * TS * 128 + size_t(nwb) * TC_ROWS * 128 + size_t(nstage) * (size_t(nwb) + nv / 2) * TS * 128 + 1024;
+}
+
 size_t sv_bwd_smem(int nwb, int nv, int tt_rows, int nstage)
 {
 	const size_t tt = size_t(tt_rows), nvb = size_t(nv) / 2;
@@ -869,6 +1565,18 @@ int launch_bwd_tile(const float *q, const float *k, const float *v, const float 
 	const long long grid = (long long)bs * n_heads * sh.ntt;
 	if (grid > 0x7fffffffLL)
 		return L1ATTN_ERR_SHAPE;
+	if constexpr (NW == TC_NW && NV <= 4) { // 128-row CTAs
+		const int tc_stages = sv_bwd_tc_smem(sh.nwb, NV, 3) <= TC_SMEM ? 3 : 2;
+		const size_t tc_smem = sv_bwd_tc_smem(sh.nwb, NV, tc_stages);
+		if (tc_smem <= TC_SMEM) {
+			sh.nstage = tc_stages;
+			auto kern = softmax_v_bwd_tc_kernel<NV, TMA, FULL>;
+			L1B_SHARED_MEMORY(kern, int(tc_smem));
+			kern<<<unsigned(grid), TC_THREADS, tc_smem, st>>>(qmap, kmap, gmap, q, k, v, dvo, lse, delta, dx, dv, sh, err);
+			L1B_LAUNCH_CHECK();
+			return L1ATTN_OK;
+		}
+	}
 	auto kern = softmax_v_bwd_tile_kernel<NV, TI, NW, TMA, FULL>;
 	L1B_SHARED_MEMORY(kern, int(smem));
 	kern<<<unsigned(grid), NTH, smem, st>>>(qmap, kmap, vmap, gmap, q, k, v, dvo, lse, delta, dx, dv, sh, err);

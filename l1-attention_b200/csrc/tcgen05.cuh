@@ -43,6 +43,49 @@ __device__ __forceinline__ void tc_mma_s8(uint32_t d, uint32_t a, uint64_t b, ui
 		     : "memory");
 }
 
+// The same for bf16 operands that both lie in shared memory (16 k a step, 32 bytes) and fp32 accumulators.  b_mn: B lies with its n
+// contiguous -- rows of k, 128 bytes of n each, swizzled alike; k advances by 2048 bytes per 16 rows.
+constexpr uint32_t tc_idesc_bf16(int n, bool b_mn)
+{
+	return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn ? 1u << 16 : 0u) | (uint32_t(n / 8) << 17) | (uint32_t(128 / 16) << 24);
+}
+__device__ __forceinline__ uint64_t tc_desc_mn(uint32_t addr) // one block of 64 n; groups of eight k rows 1024 bytes apart
+{
+	return uint64_t((addr & 0x3ffffu) >> 4) | (uint64_t(1024 >> 4) << 16) | (uint64_t(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ void tc_mma_bf16_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate)
+{
+	asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+		     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(uint32_t(accumulate))
+		     : "memory");
+}
+// a and b as three bf16 each, exactly (but for what lies below 2^-133): truncations of the value and of what they leave
+__device__ __forceinline__ void split_bf16(float a, float b, uint32_t (&piece)[3])
+{
+#pragma unroll
+	for (int i = 0; i < 3; i++) {
+		asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(piece[i]) : "r"(__float_as_uint(a)), "r"(__float_as_uint(b)));
+		a -= __uint_as_float(__float_as_uint(a) & 0xffff0000u);
+		b -= __uint_as_float(__float_as_uint(b) & 0xffff0000u);
+	}
+}
+__device__ __forceinline__ void tmem_load(uint32_t t, float (&r)[16])
+{
+	asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+		     "tcgen05.wait::ld.sync.aligned;"
+		     : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]), "=f"(r[9]),
+		       "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
+		     : "r"(t)
+		     : "memory");
+}
+__device__ __forceinline__ void tmem_load(uint32_t t, float (&r)[8])
+{
+	asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\ttcgen05.wait::ld.sync.aligned;"
+		     : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
+		     : "r"(t)
+		     : "memory");
+}
+
 // 32 columns of the calling warp's 32 lanes
 __device__ __forceinline__ void tmem_store32(uint32_t t, const uint32_t (&r)[32])
 {
