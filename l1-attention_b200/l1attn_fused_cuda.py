@@ -15,14 +15,16 @@ Forward: one kernel (`l1attn_dense_softmax_v_fwd`), nothing of size n x n is sto
 of every query row's normaliser ([bs, n, h]) for the backward.
 Backward, a few batch items at a time (`l1attn_dense_softmax_v_bwd`): one kernel recomputes the weights and
 writes the score gradients dx and dv; the library's dense backward turns dx into dq, dk.
-The only n x n tensor alive is that one chunk of dx (256 MB by default).
+The only n x n tensor alive is that one chunk of dx (512 MB by default).
 """
 import torch
 
 import l1attn_cabi as _c
 
 MODES = tuple(_c.SV_MODES)
-_CHUNK_BYTES = 256 << 20  # score tensor of one backward chunk
+# Score tensor of one backward chunk.  The kernel that makes it runs a CTA per 128 rows and head: at [16,1024,16,64] 256 MB are 512 CTAs,
+# 3.46 waves of 148 SMs (86 % of four), 512 MB are 6.92 (99 % of seven).
+_CHUNK_BYTES = 512 << 20
 
 
 class L1AttnSoftmaxVFn(torch.autograd.Function):
