@@ -671,7 +671,7 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 			}
 		}
 		named_barrier(1, NW * 32);
-		if (*reinterpret_cast<volatile int *>(&bars.bad) == 0) {
+		if (__shfl_sync(0xffffffffu, *reinterpret_cast<volatile int *>(&bars.bad), 0) == 0) {
 			if (t0 + orow < sh.n_tok) {
 				float *op = vo + v0 + size_t(t0 + orow) * vrow + ocol;
 				const float inv = row_inv[orow];
@@ -713,13 +713,15 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 		if (warp == 16 && lane == 0) {
 			const uint64_t a = tc_desc(smem_u32(Pp)), bd = tc_desc(smem_u32(Vp));
 			bool dead = false;
-			for (int m = 0; m < ns && !dead; m++) {
+			int m = 0;
+			for (; m < ns && !dead; m++) {
 				dead = !(mbar_wait_inline(&bars.v_full, m & 1, err) && mbar_wait_inline(&bars.p_full, m & 1, err));
 				tc_fence_after();
 				if (!dead)
 					mma_pieces<4>(tmem, a, TC_A_PIECE, bd, V_PIECE, 32, tc_idesc_bf16(VW, false));
 				tc_commit(&bars.done);
 			}
+			mbar_wait_inline(&bars.done, (m - 1) & 1, err); // no product is in flight when the tensor memory goes, also after a timeout
 		}
 		if (warp == 17 || warp == 18) { // a column per thread (VW 32: half of the threads)
 			const int c = (warp - 17) * 32 + lane;
@@ -1411,7 +1413,10 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 				mbar_arrive(&bars.p_full);
 		}
 		collect(nt - 1);
-		if (*reinterpret_cast<volatile int *>(&bars.bad) == 0) {
+		// (dx of every row is written before a row of it is written again.  The barrier stands before the look at `bad`: when a wait has
+		// run out, warps may see different values of it)
+		named_barrier(1, NW * 32);
+		if (__shfl_sync(0xffffffffu, *reinterpret_cast<volatile int *>(&bars.bad), 0) == 0) {
 			if (s0 + orow < sh.n_tok) {
 				float *op = dv + v0 + size_t(s0 + orow) * vrow + part * NO;
 #pragma unroll
@@ -1420,7 +1425,6 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 						op[e] = o[e];
 			}
 		} else { // a source row per warp, 32 queries at a time
-			named_barrier(1, NW * 32);
 #pragma unroll 1
 			for (int row = warp; row < TT && s0 + row < sh.n_tok; row += NW) {
 				const float *kr = k + qk0 + size_t(s0 + row) * krow, *vr = v + v0 + size_t(s0 + row) * vrow;
@@ -1458,7 +1462,8 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 		if (warp == 16 && lane == 0) {
 			const uint64_t va = tc_desc(smem_u32(Vp)), pa = tc_desc(smem_u32(Pp)), gk = tc_desc(smem_u32(Gp)), gn = tc_desc_mn(smem_u32(Gp));
 			bool dead = false;
-			for (int m = 0; m < nt && !dead; m++) {
+			int m = 0;
+			for (; m < nt && !dead; m++) {
 				dead = !mbar_wait_inline(&bars.v_full, m & 1, err);
 				tc_fence_after();
 				if (!dead)
@@ -1470,6 +1475,7 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 					mma_pieces<TS / 16>(tmem + D2, pa, TC_A_PIECE, gn, G_PIECE, 2048, tc_idesc_bf16(VW, true));
 				tc_commit(&bars.done2);
 			}
+			mbar_wait_inline(&bars.done2, (m - 1) & 1, err); // no product is in flight when the tensor memory goes, also after a timeout
 		}
 		if (warp == 17 || warp == 18) { // a query row per thread
 			const int t = (warp - 17) * 32 + lane, place = 4 * (t % 16) + t / 16;

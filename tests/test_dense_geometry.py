@@ -48,3 +48,28 @@ def test_cluster_barrier_before_remote_shared_memory(name):
     assert bodies
     for body in bodies:
         assert "cluster.sync()" in body[:body.index("map_shared_rank")], body[:300]
+
+
+def test_barriers_of_the_fused_kernels_are_unconditional():
+    """A barrier of several warps stands only under conditions that no wait that ran out can make different for some of them (which warp
+    it is, the tile's number): under any other -- a word of shared memory, say -- some warps could wait for others that never come."""
+    source = re.sub(r"//.*", "", open(os.path.join(PKG, "csrc", "dense_softmax_v.cu")).read())
+    uniform = [r"if \(warp < NW\)", r"for \(int m = 0; m < n[st]; m\+\+\)"]
+    found = 0
+    for kernel in re.findall(r"^softmax_v\w*_kernel\(.*?^}", source, re.S | re.M):
+        stack, start, depth = [], 0, 0
+        for i, c in enumerate(kernel):
+            depth += (c == "(") - (c == ")")
+            if c in "{;}" and depth == 0:
+                head = kernel[start:i].strip()
+                if re.match(r"(named_barrier|__syncthreads|if\s*\(.*\)\s*(named_barrier|__syncthreads))\b", head, re.S):
+                    found += 1
+                    assert re.match("named_barrier|__syncthreads", head), head  # not the statement of an `if` without braces
+                    for h in stack[1:]:
+                        assert any(re.fullmatch(u, h) for u in uniform), (h, head)
+                if c == "{":
+                    stack.append(head)
+                elif c == "}":
+                    stack.pop()
+                start = i + 1
+    assert found >= 10
