@@ -52,6 +52,20 @@ struct SharedMemoryLimit {
 			return rc__;                                                            \
 	} while (0)
 
+// Refuses to launch `kern` unless it was built with at least `regs` registers per thread.  For kernels that move registers between their
+// warps (setmaxnreg): warps that ask for more than the block was launched with wait for them without any limit.
+#define L1B_REGISTERS(kern, regs)                                                       \
+	do {                                                                            \
+		static std::atomic<int> built__{0};                                     \
+		if (built__.load(std::memory_order_relaxed) == 0) {                     \
+			cudaFuncAttributes at__;                                        \
+			L1B_CUDA(cudaFuncGetAttributes(&at__, kern));                   \
+			built__.store(at__.numRegs, std::memory_order_relaxed);         \
+		}                                                                       \
+		if (built__.load(std::memory_order_relaxed) < (regs))                   \
+			return ::l1b::cuda_fail(cudaErrorLaunchOutOfResources);         \
+	} while (0)
+
 // Multiprocessors of the current device (asked for once per device).
 int multiprocessors(int *out);
 

@@ -448,8 +448,8 @@ __device__ __forceinline__ void score_slice(const unsigned char *Qslice, const u
 // of the scores (two lane-cycles per term) with the shared loads of a 4 x 4 tile beside it.
 // Values that are not finite have no such pieces (inf - inf): a CTA that meets one computes its rows once more, plainly.
 constexpr int TC_NW = 16, TC_ROWS = 128, TC_THREADS = (TC_NW + 4) * 32;
-constexpr int TC_REGS = 104, TC_REGS_REST = 64; // registers per thread, from 96 at the launch: 4 x 104 + 64 <= 5 x 96
-static_assert(4 * TC_REGS + TC_REGS_REST <= 5 * 96, "more than the block was launched with");
+constexpr int TC_REGS = 104, TC_REGS_REST = 64, TC_REGS_LAUNCH = 96; // registers per thread; the launcher asks whether the kernel was built with the last
+static_assert(4 * TC_REGS + TC_REGS_REST <= 5 * TC_REGS_LAUNCH, "more than the block was launched with");
 constexpr int TC_A_PIECE = TC_ROWS * 128;          // 64 bf16 a row
 constexpr size_t TC_SMEM = 227 * 1024 - 3072;      // per CTA, less the static part
 
@@ -815,6 +815,7 @@ int launch_tile(const float *q, const float *k, const float *v, float *vo, float
 			sh.nstage = tc_stages;
 			auto kern = softmax_v_tc_kernel<NV, TMA, FULL>;
 			L1B_SHARED_MEMORY(kern, int(tc_smem));
+			L1B_REGISTERS(kern, TC_REGS_LAUNCH);
 			kern<<<unsigned(grid), TC_THREADS, tc_smem, st>>>(qmap, kmap, vmap, q, k, v, vo, lse, sh, err);
 			L1B_LAUNCH_CHECK();
 			return L1ATTN_OK;
@@ -1578,6 +1579,7 @@ int launch_bwd_tile(const float *q, const float *k, const float *v, const float 
 			sh.nstage = tc_stages;
 			auto kern = softmax_v_bwd_tc_kernel<NV, TMA, FULL>;
 			L1B_SHARED_MEMORY(kern, int(tc_smem));
+			L1B_REGISTERS(kern, TC_REGS_LAUNCH);
 			kern<<<unsigned(grid), TC_THREADS, tc_smem, st>>>(qmap, kmap, gmap, q, k, v, dvo, lse, delta, dx, dv, sh, err);
 			L1B_LAUNCH_CHECK();
 			return L1ATTN_OK;

@@ -73,3 +73,15 @@ def test_barriers_of_the_fused_kernels_are_unconditional():
                     stack.pop()
                 start = i + 1
     assert found >= 10
+
+
+def test_kernels_that_move_registers_are_asked_what_they_were_built_with():
+    """setmaxnreg.inc waits without a limit when the block was launched with fewer registers than its warps ask for in all, and a
+    launch has as many as the compiler gave the kernel: whoever launches such a kernel asks for them first."""
+    for name in os.listdir(os.path.join(PKG, "csrc")):
+        source = re.sub(r"//.*", "", open(os.path.join(PKG, "csrc", name), errors="replace").read()) if name.endswith((".cu", ".cuh")) else ""
+        kernels = [re.search(r"(\w+_kernel)\(", b).group(1) for b in source.split("__global__")[1:] if "setmaxnreg.inc" in b]
+        for kernel in kernels:
+            launches = re.findall(r"auto kern = %s<.*?<<<" % kernel, source, re.S)
+            assert launches and all("L1B_REGISTERS(kern, TC_REGS_LAUNCH)" in x for x in launches), (name, kernel)
+        assert not kernels or "4 * TC_REGS + TC_REGS_REST <= 5 * TC_REGS_LAUNCH" in source
