@@ -88,6 +88,8 @@ int *l1attn_device_status_word(void);
  * Nothing faults or hangs.  No counterpart in the reference.
  */
 int l1attn_test_wait_timeout(int limit_us, int *returned_dev, void *stream);
+/* The same of the wait that gives up after a number of failed polls (1..100000) instead of a time. */
+int l1attn_test_wait_polls(int polls, int *returned_dev, void *stream);
 
 /* ------------------------------------------------------------------ dense --------------- */
 

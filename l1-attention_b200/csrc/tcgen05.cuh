@@ -76,11 +76,11 @@ __device__ __forceinline__ void tmem_load(uint32_t t, float (&r)[8])
 }
 
 // mbar_wait() without its call of the clocked loop: a call keeps what lives across it in half of the registers, and warps that hold
-// a whole tile of operands have none to spare.  2 FAST_POLLS failed polls, a second or two, then it gives up the same way.
-__device__ __forceinline__ bool mbar_wait_inline(uint64_t *bar, uint32_t parity, int *err)
+// a whole tile of operands have none to spare.  `polls` failed polls (2 FAST_POLLS: a second or two), then it gives up the same way.
+__device__ __forceinline__ bool mbar_wait_inline(uint64_t *bar, uint32_t parity, int *err, uint32_t polls = 2 * FAST_POLLS)
 {
 	const uint32_t a = smem_u32(bar);
-	for (uint32_t i = 0; i < 2 * FAST_POLLS; i++)
+	for (uint32_t i = 0; i < polls; i++)
 		if (mbar_try(a, parity))
 			return true;
 	*reinterpret_cast<volatile int *>(err) = 1;

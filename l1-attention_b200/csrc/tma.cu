@@ -5,6 +5,7 @@
 #include <mutex>
 #include "common.cuh"
 #include "tma.cuh"
+#include "tcgen05.cuh"
 
 namespace l1b {
 
@@ -170,8 +171,8 @@ namespace l1b {
 namespace {
 // One warp waits on a barrier that nothing ever completes, with a short limit: the wait runs out, the error word
 // is set and the kernel returns.  Nothing faults and nothing hangs; it exists so that the give-up path of
-// mbar_wait and the error word's set / read / clear cycle can be exercised.
-__global__ void wait_timeout_probe_kernel(unsigned long long limit_ns, int *err, int *returned)
+// mbar_wait and the error word's set / read / clear cycle can be exercised.  limit_polls: the wait that counts its polls instead.
+__global__ void wait_timeout_probe_kernel(unsigned long long limit_ns, unsigned limit_polls, int *err, int *returned)
 { // returned[0]: 1 = the wait gave up, 2 = it succeeded (cannot happen); returned[1]: failed polls of thread 0
 	__shared__ __align__(8) uint64_t bar;
 	if (threadIdx.x == 0) {
@@ -179,8 +180,8 @@ __global__ void wait_timeout_probe_kernel(unsigned long long limit_ns, int *err,
 		mbar_fence_init();
 	}
 	__syncthreads();
-	unsigned polls = 0;
-	const bool ok = mbar_wait_timed(&bar, 0, err, limit_ns, &polls);
+	unsigned polls = limit_polls;
+	const bool ok = limit_polls ? mbar_wait_inline(&bar, 0, err, limit_polls) : mbar_wait_timed(&bar, 0, err, limit_ns, &polls);
 	if (threadIdx.x == 0) {
 		returned[0] = ok ? 2 : 1;
 		returned[1] = int(polls);
@@ -189,14 +190,17 @@ __global__ void wait_timeout_probe_kernel(unsigned long long limit_ns, int *err,
 } // namespace
 } // namespace l1b
 
-extern "C" int l1attn_test_wait_timeout(int limit_us, int *returned_dev, void *stream)
+static int wait_timeout_probe(int limit_us, int limit_polls, int *returned_dev, void *stream)
 {
-	if (limit_us < 1 || limit_us > 100000 || !returned_dev)
+	const int limit = limit_us + limit_polls; // one of them is 0
+	if (limit < 1 || limit > 100000 || !returned_dev)
 		return L1ATTN_ERR_ARG;
 	int *err = l1b::device_error_word();
 	if (!err)
 		return L1ATTN_ERR_CUDA;
-	l1b::wait_timeout_probe_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(1000ull * limit_us, err, returned_dev);
+	l1b::wait_timeout_probe_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(1000ull * limit_us, unsigned(limit_polls), err, returned_dev);
 	L1B_LAUNCH_CHECK();
 	return L1ATTN_OK;
 }
+extern "C" int l1attn_test_wait_timeout(int limit_us, int *returned_dev, void *stream) { return wait_timeout_probe(limit_us, 0, returned_dev, stream); }
+extern "C" int l1attn_test_wait_polls(int polls, int *returned_dev, void *stream) { return wait_timeout_probe(0, polls, returned_dev, stream); }

@@ -6,8 +6,8 @@
 //    offsets that are multiples of the 64-byte stage row, and 0 for the head/row axes that are
 //    innermost in their tensors);
 //  * every wait is bounded: after FAST_POLLS failed polls the waiter goes on by the global nanosecond
-//    timer for at most WAIT_LIMIT_NS, then records an error code in the device error word and gives
-//    up, so a lost copy cannot hang the GPU.
+//    timer for at most WAIT_LIMIT_NS (mbar_wait_inline of tcgen05.cuh: by a limit of polls alone), then
+//    records an error code in the device error word and gives up, so a lost copy cannot hang the GPU.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>

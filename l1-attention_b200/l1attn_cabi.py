@@ -28,6 +28,7 @@ SIGNATURES = {
     "l1attn_device_status_async": (_i, [_vp, _vp]),
     "l1attn_device_status_word": (_vp, []),
     "l1attn_test_wait_timeout": (_i, [_i, _vp, _vp]),
+    "l1attn_test_wait_polls": (_i, [_i, _vp, _vp]),
     "l1attn_dense_fwd": (_i, [_vp] * 3 + [_i] * 5 + [_vp]),
     "l1attn_dense_softmax_v_fwd": (_i, [_vp] * 5 + [_i] * 7 + [_vp]),
     "l1attn_dense_softmax_v_bwd_bytes": (_sz, [_i] * 6),

@@ -50,3 +50,18 @@ def test_values_that_are_not_finite(bad):
         fine = x.isfinite() & r.isfinite()
         assert_close(x[fine].detach().cpu().numpy(), r[fine].detach().cpu().numpy(), 1e-5, name)
         assert torch.isfinite(x[7]).all()
+
+
+def test_wait_that_counts_polls_gives_up_and_is_reported():
+    """The wait of these kernels is bounded by its polls: 500 of them on a barrier that nothing completes, then the kernel returns and the
+    status reports a timeout, once.  More polls than a hundred thousand are refused."""
+    import l1attn_cabi
+    lib = l1attn_cabi.lib()
+    torch.cuda.synchronize()
+    assert lib.l1attn_device_status() == 0
+    returned = torch.zeros(2, dtype=torch.int32, device="cuda")
+    assert lib.l1attn_test_wait_polls(500, returned.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert returned.tolist() == [1, 500]
+    assert lib.l1attn_device_status() == -7 and lib.l1attn_device_status() == 0
+    assert lib.l1attn_test_wait_polls(0, returned.data_ptr(), None) == lib.l1attn_test_wait_polls(100001, returned.data_ptr(), None) == -1
