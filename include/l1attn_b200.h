@@ -170,6 +170,11 @@ int l1attn_dense_softmax_v_bwd(const void *q, const void *k, const void *v, cons
 			       const void *lse, const void *delta, void *dq, void *dk, void *dv, void *work,
 			       int bs, int n_tok, int n_heads, int width, int v_width,
 			       int dtype, void *stream);
+/*
+ * Test hook, not an operator: which kernel a float32 call of these sizes takes (backward: the one that makes dx and dv).  0: one for any shape;
+ * else the query (source) rows of a CTA, 64 or 128, plus 1 where the value products are done by the tensor cores.
+ */
+int l1attn_test_softmax_v_form(int bs, int n_tok, int n_heads, int width, int v_width, int backward);
 
 /* ------------------------------------------------------------------ sparse -------------- */
 

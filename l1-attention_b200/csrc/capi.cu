@@ -236,6 +236,13 @@ extern "C" int l1attn_dense_softmax_v_bwd_dx(const void *q, const void *k, const
 					     static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int l1attn_test_softmax_v_form(int bs, int n_tok, int n_heads, int width, int v_width, int backward)
+{
+	if (bs < 1 || n_tok < 1 || n_heads < 1 || width < 1 || v_width < 1)
+		return L1ATTN_ERR_ARG;
+	return dense_softmax_v_form(bs, n_tok, n_heads, width, v_width, backward);
+}
+
 extern "C" size_t l1attn_dense_softmax_v_bwd_bytes(int bs, int n_tok, int n_heads, int width, int v_width, int dtype)
 {
 	if (bs < 1 || n_tok < 1 || n_heads < 1 || width < 1 || v_width < 1 || (dtype != L1ATTN_F32 && dtype != L1ATTN_F64))

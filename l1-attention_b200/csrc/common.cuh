@@ -150,6 +150,7 @@ int dense_softmax_v_launch(const void *q, const void *k, const void *v, void *vo
 int dense_softmax_v_bwd_dx_launch(const void *q, const void *k, const void *v, const void *dvo, const void *lse,
 				  const void *delta, void *dx, void *dv, int bs, int n_tok, int n_heads, int width, int v_width,
 				  int dtype, cudaStream_t st);
+int dense_softmax_v_form(int bs, int n_tok, int n_heads, int width, int v_width, int backward);
 // the whole backward; work: dense_softmax_v_bwd_bytes() bytes of device memory, 256-byte aligned
 size_t dense_softmax_v_bwd_bytes(int bs, int n_tok, int n_heads, int width, int v_width, int dtype);
 int dense_softmax_v_bwd_launch(const void *q, const void *k, const void *v, const void *dvo, const void *lse, const void *delta,

@@ -777,9 +777,52 @@ size_t sv_tc_smem(int nwb, int nv, int nstage)
 	return size_t(3) * TC_A_PIECE + size_t(3) * nv * 16 * 128 + size_t(nwb) * TC_ROWS * 128 + size_t(nstage) * (size_t(nwb) * TS * 128 + size_t(TS) * nv * 64) + 1024;
 }
 
+// (query rows per half-warp, warps, ring stages) of the tiled kernels.  4 x 16 and 8 x 8 make a 128-row CTA, 4 x 8 a 64-row
+// one.  Sixteen warps of 128 registers measured 7 % faster than eight of 168 (four warps per scheduler hide the
+// shared-memory and arithmetic latencies); with 128 value columns the thread state does not fit 128 registers.  A 64-row CTA
+// takes SHORT_CTA of the time of a 128-row one (forward 41 / 66 us at [4,333,6,64], 97 / 164 at [1,1024,8,64]; 56 / 88 with 128 value
+// columns; two waves of it against one 1.13-1.17); it is taken where the rows do not fit shared memory otherwise, or where its
+// finer grid fills the SMs better (few rows in all, or few left over for the last wave).
+struct TilePlan {
+	int ti, nw, nstage; // nstage 0: no form fits
+	size_t smem;
+	bool tc; // products on the tensor cores
+};
+constexpr double SHORT_CTA = 0.6;
+template <typename F, typename G> TilePlan plan_tile(int nv, long long groups, int n_tok, F smem_of, G tc_smem_of)
+{
+	const size_t limit = 227 * 1024 - 256; // per-CTA maximum minus the static barriers
+	const bool nw16 = nv <= 4;
+	const int cand[2][2] = {{nw16 ? 4 : 8, nw16 ? TC_NW : 8}, {4, 8}};
+	TilePlan best{0, 0, 0, 0, false};
+	double best_cost = 0;
+	for (const auto &c : cand)
+		for (int ns : {3, 2}) {
+			const int tt = 2 * c[0] * c[1];
+			const size_t smem = smem_of(tt, ns);
+			if (smem > limit)
+				continue;
+			const long long ctas = groups * ((n_tok + tt - 1) / tt);
+			const double cost = double((ctas + 147) / 148) * (tt == 64 ? SHORT_CTA : 1.0);
+			if (!best.nstage || cost < best_cost) {
+				best = {c[0], c[1], ns, smem, false};
+				best_cost = cost;
+			}
+			break; // the deeper ring that fits
+		}
+	if (best.nw == TC_NW)
+		for (int ns : {2, 3}) // (the deeper ring that fits)
+			if (tc_smem_of(ns) <= TC_SMEM) {
+				best.nstage = ns;
+				best.smem = tc_smem_of(ns);
+				best.tc = true;
+			}
+	return best;
+}
+
 template <int NV, int TI, int NW, bool TMA, bool FULL>
 int launch_tile(const float *q, const float *k, const float *v, float *vo, float *lse, int bs, int n_tok, int n_heads,
-		int width, int v_width, int mode, int nstage, size_t smem, cudaStream_t st)
+		int width, int v_width, int mode, const TilePlan &plan, cudaStream_t st)
 {
 	constexpr int TT = 2 * NW * TI, VW = 16 * NV, NTH = NW * 32;
 	const uint64_t dims[4] = {uint64_t(width), uint64_t(n_heads), uint64_t(n_tok), uint64_t(bs)};
@@ -801,29 +844,25 @@ int launch_tile(const float *q, const float *k, const float *v, float *vo, float
 	sh.width = width;
 	sh.v_width = v_width;
 	sh.nwb = (width + 31) / 32;
-	sh.nstage = nstage;
+	sh.nstage = plan.nstage;
 	sh.ntt = (n_tok + TT - 1) / TT;
 	sh.mode = mode;
 	sh.scale = float(-1.0 / sqrt(double(width)));
 	const long long grid = (long long)bs * n_heads * sh.ntt;
 	if (grid > 0x7fffffffLL)
 		return L1ATTN_ERR_SHAPE;
-	if constexpr (NW == TC_NW && NV <= 4) { // 128-row CTAs
-		const int tc_stages = sv_tc_smem(sh.nwb, NV, 3) <= TC_SMEM ? 3 : 2;
-		const size_t tc_smem = sv_tc_smem(sh.nwb, NV, tc_stages);
-		if (tc_smem <= TC_SMEM) {
-			sh.nstage = tc_stages;
+	if constexpr (NW == TC_NW)
+		if (plan.tc) {
 			auto kern = softmax_v_tc_kernel<NV, TMA, FULL>;
-			L1B_SHARED_MEMORY(kern, int(tc_smem));
+			L1B_SHARED_MEMORY(kern, int(plan.smem));
 			L1B_REGISTERS(kern, TC_REGS_LAUNCH);
-			kern<<<unsigned(grid), TC_THREADS, tc_smem, st>>>(qmap, kmap, vmap, q, k, v, vo, lse, sh, err);
+			kern<<<unsigned(grid), TC_THREADS, plan.smem, st>>>(qmap, kmap, vmap, q, k, v, vo, lse, sh, err);
 			L1B_LAUNCH_CHECK();
 			return L1ATTN_OK;
 		}
-	}
 	auto kern = softmax_v_tile_kernel<NV, TI, NW, TMA, FULL>;
-	L1B_SHARED_MEMORY(kern, int(smem));
-	kern<<<unsigned(grid), NTH, smem, st>>>(qmap, kmap, vmap, q, k, v, vo, lse, sh, err);
+	L1B_SHARED_MEMORY(kern, int(plan.smem));
+	kern<<<unsigned(grid), NTH, plan.smem, st>>>(qmap, kmap, vmap, q, k, v, vo, lse, sh, err);
 	L1B_LAUNCH_CHECK();
 	return L1ATTN_OK;
 }
@@ -835,55 +874,27 @@ size_t sv_smem(int nwb, int nv, int tt_rows, int nstage)
 	return size_t(nwb) * tt * 128 + size_t(nstage) * (size_t(nwb) * TS * 128 + size_t(TS) * nv * 64) + tt * PP * 4 + 1024;
 }
 
-// (query rows per half-warp, warps, ring stages) of the tiled kernels.  4 x 16 and 8 x 8 make a 128-row CTA, 4 x 8 a 64-row
-// one.  Sixteen warps of 128 registers measured 7 % faster than eight of 168 (four warps per scheduler hide the
-// shared-memory and arithmetic latencies); with 128 value columns the thread state does not fit 128 registers.  A 64-row CTA
-// takes SHORT_CTA of the time of a 128-row one (forward 41 / 66 us at [4,333,6,64], 97 / 164 at [1,1024,8,64]; 56 / 88 with 128 value
-// columns; two waves of it against one 1.13-1.17); it is taken where the rows do not fit shared memory otherwise, or where its
-// finer grid fills the SMs better (few rows in all, or few left over for the last wave).
-struct TilePlan {
-	int ti, nw, nstage; // nstage 0: no form fits
-	size_t smem;
-};
-constexpr double SHORT_CTA = 0.6;
-template <typename F> TilePlan plan_tile(int nv, long long groups, int n_tok, F smem_of)
+int sv_nv(int v_width) { return v_width <= 32 ? 2 : v_width <= 64 ? 4 : 8; } // value columns per lane
+TilePlan sv_plan(int bs, int n_tok, int n_heads, int width, int v_width)
 {
-	const size_t limit = 227 * 1024 - 256; // per-CTA maximum minus the static barriers
-	const bool nw16 = nv <= 4;
-	const int cand[2][2] = {{nw16 ? 4 : 8, nw16 ? 16 : 8}, {4, 8}};
-	TilePlan best{0, 0, 0, 0};
-	double best_cost = 0;
-	for (const auto &c : cand)
-		for (int ns : {3, 2}) {
-			const int tt = 2 * c[0] * c[1];
-			const size_t smem = smem_of(tt, ns);
-			if (smem > limit)
-				continue;
-			const long long ctas = groups * ((n_tok + tt - 1) / tt);
-			const double cost = double((ctas + 147) / 148) * (tt == 64 ? SHORT_CTA : 1.0);
-			if (!best.nstage || cost < best_cost) {
-				best = {c[0], c[1], ns, smem};
-				best_cost = cost;
-			}
-			break; // the deeper ring that fits
-		}
-	return best;
+	if (width < 1 || width > 128 || v_width < 1 || v_width > 128)
+		return {0, 0, 0, 0, false};
+	const int nwb = (width + 31) / 32, nv = sv_nv(v_width);
+	return plan_tile(nv, (long long)bs * n_heads, n_tok, [&](int tt, int ns) { return sv_smem(nwb, nv, tt, ns); }, [&](int ns) { return sv_tc_smem(nwb, nv, ns); });
 }
 
 // Returns L1ATTN_OK, a negative error, or 1 when the shape is outside this kernel's set.
 int softmax_v_tile(const float *q, const float *k, const float *v, float *vo, float *lse, int bs, int n_tok, int n_heads,
 		   int width, int v_width, int mode, cudaStream_t st)
 {
-	if (width > 128 || v_width > 128)
-		return 1;
-	const bool tma = width % 4 == 0 && v_width % 4 == 0 && aligned(q, 16) && aligned(k, 16) && aligned(v, 16);
-	const int nwb = (width + 31) / 32, nv = v_width <= 32 ? 2 : v_width <= 64 ? 4 : 8;
-	const bool full = width % 32 == 0 && v_width == 16 * nv; // no padded columns
-	const TilePlan p = plan_tile(nv, (long long)bs * n_heads, n_tok, [&](int tt, int ns) { return sv_smem(nwb, nv, tt, ns); });
+	const TilePlan p = sv_plan(bs, n_tok, n_heads, width, v_width);
 	if (!p.nstage)
 		return 1;
+	const bool tma = width % 4 == 0 && v_width % 4 == 0 && aligned(q, 16) && aligned(k, 16) && aligned(v, 16);
+	const int nv = sv_nv(v_width);
+	const bool full = width % 32 == 0 && v_width == 16 * nv; // no padded columns
 #define L1B_SV_RUN(NV_, TI_, NW_, TMA_, FULL_) \
-	launch_tile<NV_, TI_, NW_, TMA_, FULL_>(q, k, v, vo, lse, bs, n_tok, n_heads, width, v_width, mode, p.nstage, p.smem, st)
+	launch_tile<NV_, TI_, NW_, TMA_, FULL_>(q, k, v, vo, lse, bs, n_tok, n_heads, width, v_width, mode, p, st)
 #define L1B_SV(NV_, TI_, NW_)                                                                                                  \
 	if (nv == NV_ && p.ti == TI_ && p.nw == NW_) {                                                                         \
 		const int rc = !tma ? 1 : full ? L1B_SV_RUN(NV_, TI_, NW_, true, true) : L1B_SV_RUN(NV_, TI_, NW_, true, false); \
@@ -1540,8 +1551,7 @@ size_t sv_bwd_smem(int nwb, int nv, int tt_rows, int nstage)
 
 template <int NV, int TI, int NW, bool TMA, bool FULL>
 int launch_bwd_tile(const float *q, const float *k, const float *v, const float *dvo, const float *lse, const float *delta,
-		    float *dx, int dx_pitch, float *dv, int bs, int n_tok, int n_heads, int width, int v_width, int nstage, size_t smem,
-		    cudaStream_t st)
+		    float *dx, int dx_pitch, float *dv, int bs, int n_tok, int n_heads, int width, int v_width, const TilePlan &plan, cudaStream_t st)
 {
 	constexpr int TT = 2 * NW * TI, NTH = NW * 32;
 	const uint64_t dims[4] = {uint64_t(width), uint64_t(n_heads), uint64_t(n_tok), uint64_t(bs)};
@@ -1564,7 +1574,7 @@ int launch_bwd_tile(const float *q, const float *k, const float *v, const float 
 	sh.width = width;
 	sh.v_width = v_width;
 	sh.nwb = (width + 31) / 32;
-	sh.nstage = nstage;
+	sh.nstage = plan.nstage;
 	sh.ntt = (n_tok + TT - 1) / TT;
 	sh.mode = 0;
 	sh.dx_pitch = dx_pitch;
@@ -1572,39 +1582,41 @@ int launch_bwd_tile(const float *q, const float *k, const float *v, const float 
 	const long long grid = (long long)bs * n_heads * sh.ntt;
 	if (grid > 0x7fffffffLL)
 		return L1ATTN_ERR_SHAPE;
-	if constexpr (NW == TC_NW && NV <= 4) { // 128-row CTAs
-		const int tc_stages = sv_bwd_tc_smem(sh.nwb, NV, 3) <= TC_SMEM ? 3 : 2;
-		const size_t tc_smem = sv_bwd_tc_smem(sh.nwb, NV, tc_stages);
-		if (tc_smem <= TC_SMEM) {
-			sh.nstage = tc_stages;
+	if constexpr (NW == TC_NW)
+		if (plan.tc) {
 			auto kern = softmax_v_bwd_tc_kernel<NV, TMA, FULL>;
-			L1B_SHARED_MEMORY(kern, int(tc_smem));
+			L1B_SHARED_MEMORY(kern, int(plan.smem));
 			L1B_REGISTERS(kern, TC_REGS_LAUNCH);
-			kern<<<unsigned(grid), TC_THREADS, tc_smem, st>>>(qmap, kmap, gmap, q, k, v, dvo, lse, delta, dx, dv, sh, err);
+			kern<<<unsigned(grid), TC_THREADS, plan.smem, st>>>(qmap, kmap, gmap, q, k, v, dvo, lse, delta, dx, dv, sh, err);
 			L1B_LAUNCH_CHECK();
 			return L1ATTN_OK;
 		}
-	}
 	auto kern = softmax_v_bwd_tile_kernel<NV, TI, NW, TMA, FULL>;
-	L1B_SHARED_MEMORY(kern, int(smem));
-	kern<<<unsigned(grid), NTH, smem, st>>>(qmap, kmap, vmap, gmap, q, k, v, dvo, lse, delta, dx, dv, sh, err);
+	L1B_SHARED_MEMORY(kern, int(plan.smem));
+	kern<<<unsigned(grid), NTH, plan.smem, st>>>(qmap, kmap, vmap, gmap, q, k, v, dvo, lse, delta, dx, dv, sh, err);
 	L1B_LAUNCH_CHECK();
 	return L1ATTN_OK;
+}
+
+TilePlan sv_bwd_plan(int bs, int n_tok, int n_heads, int width, int v_width)
+{
+	if (width < 1 || width > 128 || v_width < 1 || v_width > 128)
+		return {0, 0, 0, 0, false};
+	const int nwb = (width + 31) / 32, nv = sv_nv(v_width);
+	return plan_tile(nv, (long long)bs * n_heads, n_tok, [&](int tt, int ns) { return sv_bwd_smem(nwb, nv, tt, ns); }, [&](int ns) { return sv_bwd_tc_smem(nwb, nv, ns); });
 }
 
 int softmax_v_bwd_tile(const float *q, const float *k, const float *v, const float *dvo, const float *lse, const float *delta,
 		       float *dx, int dx_pitch, float *dv, int bs, int n_tok, int n_heads, int width, int v_width, cudaStream_t st)
 {
-	if (width > 128 || v_width > 128)
-		return 1;
-	const bool tma = width % 4 == 0 && v_width % 4 == 0 && aligned(q, 16) && aligned(k, 16) && aligned(v, 16) && aligned(dvo, 16);
-	const int nwb = (width + 31) / 32, nv = v_width <= 32 ? 2 : v_width <= 64 ? 4 : 8;
-	const bool full = width % 32 == 0 && v_width == 16 * nv; // no padded columns
-	const TilePlan p = plan_tile(nv, (long long)bs * n_heads, n_tok, [&](int tt, int ns) { return sv_bwd_smem(nwb, nv, tt, ns); });
+	const TilePlan p = sv_bwd_plan(bs, n_tok, n_heads, width, v_width);
 	if (!p.nstage)
 		return 1;
+	const bool tma = width % 4 == 0 && v_width % 4 == 0 && aligned(q, 16) && aligned(k, 16) && aligned(v, 16) && aligned(dvo, 16);
+	const int nv = sv_nv(v_width);
+	const bool full = width % 32 == 0 && v_width == 16 * nv; // no padded columns
 #define L1B_SVB_RUN(NV_, TI_, NW_, TMA_, FULL_) \
-	launch_bwd_tile<NV_, TI_, NW_, TMA_, FULL_>(q, k, v, dvo, lse, delta, dx, dx_pitch, dv, bs, n_tok, n_heads, width, v_width, p.nstage, p.smem, st)
+	launch_bwd_tile<NV_, TI_, NW_, TMA_, FULL_>(q, k, v, dvo, lse, delta, dx, dx_pitch, dv, bs, n_tok, n_heads, width, v_width, p, st)
 #define L1B_SVB(NV_, TI_, NW_)                                                                                                   \
 	if (nv == NV_ && p.ti == TI_ && p.nw == NW_) {                                                                           \
 		const int rc = !tma ? 1 : full ? L1B_SVB_RUN(NV_, TI_, NW_, true, true) : L1B_SVB_RUN(NV_, TI_, NW_, true, false); \
@@ -1617,6 +1629,13 @@ int softmax_v_bwd_tile(const float *q, const float *k, const float *v, const flo
 }
 
 } // namespace
+
+// The kernel that a float32 call of these sizes takes: 0 one for any shape, else the rows of a CTA, and one more where the products are on the tensor cores
+int dense_softmax_v_form(int bs, int n_tok, int n_heads, int width, int v_width, int backward)
+{
+	const TilePlan p = backward ? sv_bwd_plan(bs, n_tok, n_heads, width, v_width) : sv_plan(bs, n_tok, n_heads, width, v_width);
+	return p.nstage ? 2 * p.ti * p.nw + p.tc : 0;
+}
 
 int dense_softmax_v_launch(const void *q, const void *k, const void *v, void *vo, void *lse, int bs, int n_tok, int n_heads,
 			   int width, int v_width, int mode, int dtype, cudaStream_t st)

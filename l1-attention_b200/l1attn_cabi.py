@@ -33,6 +33,7 @@ SIGNATURES = {
     "l1attn_dense_softmax_v_fwd": (_i, [_vp] * 5 + [_i] * 7 + [_vp]),
     "l1attn_dense_softmax_v_bwd_bytes": (_sz, [_i] * 6),
     "l1attn_dense_softmax_v_bwd": (_i, [_vp] * 10 + [_i] * 6 + [_vp]),
+    "l1attn_test_softmax_v_form": (_i, [_i] * 6),
     "l1attn_dense_softmax_v_bwd_dx": (_i, [_vp] * 8 + [_i] * 6 + [_vp]),
     "l1attn_dense_bwd_scratch_bytes": (_sz, [_i] * 5),
     "l1attn_dense_bwd": (_i, [_vp] * 6 + [_i] * 5 + [_vp]),

@@ -1,6 +1,6 @@
 """The fused operator's 128-row kernels with the value products on the tensor cores (csrc/dense_softmax_v.cu): ragged ends of the tiles of 128
-rows, 64 keys, 32 columns and 64 value columns, rows with and without TMA, and values that are not finite.  148 (batch, head) pairs
-make those kernels the ones that fill the GPU."""
+rows, 64 keys, 32 columns and 64 value columns, rows with and without TMA, masked keys, ties, and values that are not finite.  Every
+test asserts that its sizes take the kernels it is about (148 (batch, head) pairs fill the GPU with 128-row CTAs)."""
 import numpy as np
 import pytest
 import torch
@@ -8,55 +8,132 @@ import torch
 from conftest import assert_close
 
 pytestmark = pytest.mark.gpu
-SHAPES = [(65, 64, 64), (100, 33, 21), (127, 32, 32), (128, 64, 33), (200, 17, 64), (256, 64, 64), (193, 48, 40), (130, 96, 64), (128, 4, 1)]
+SHAPES = [(65, 64, 64), (100, 33, 21), (127, 32, 32), (128, 64, 33), (200, 17, 64), (256, 64, 64), (193, 48, 40), (128, 4, 1)]
+WIDE = [(128, 96, 64), (128, 65, 7), (200, 128, 32), (128, 97, 21)]  # (rows of three and four slices: the forward alone)
+MODES = ["softmax", "softmax_plus_one", "exp"]
+BS, HEADS = 37, 4
+
+
+def _cabi():
+    import l1attn_cabi
+    return l1attn_cabi
+
+
+def _assert_form(n, w, wv, forward=129, backward=129):
+    form = _cabi().lib().l1attn_test_softmax_v_form
+    assert (form(BS, n, HEADS, w, wv, 0), form(BS, n, HEADS, w, wv, 1)) == (forward, backward)
 
 
 def _inputs(n, w, wv, seed=60):
     gen = torch.Generator(device="cuda").manual_seed(seed)
-    return [torch.randn(37, n, 4, x, generator=gen, device="cuda") for x in (w, w, wv, wv)]
+    return [torch.randn(BS, n, HEADS, x, generator=gen, device="cuda") for x in (w, w, wv, wv)]
 
 
-@pytest.mark.parametrize("mode", ["softmax", "softmax_plus_one", "exp"])
-@pytest.mark.parametrize("n,w,wv", SHAPES)
+def _run(q, k, v, g, mode):
+    """vo, dq, dk, dv in float32, and the float64 kernels' on the same values"""
+    import l1attn_fused_cuda
+    res = []
+    for dt in (torch.float32, torch.float64):
+        t = [x.to(dt).requires_grad_(True) for x in (q, k, v)]
+        out = l1attn_fused_cuda.L1AttnSoftmaxV(mode)(*t)
+        res.append([out.detach(), *torch.autograd.grad(out, t, g.to(dt))])
+    return list(zip(("vo", "dq", "dk", "dv"), *res))
+
+
+def _close(x, r, tol, name):
+    assert_close(x.cpu().numpy(), r.cpu().numpy(), tol, name)
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("n,w,wv", SHAPES + WIDE)
 def test_output_and_gradients(n, w, wv, mode):
-    import l1attn_fused_cuda
-    q, k, v, g = _inputs(n, w, wv)
-    m = l1attn_fused_cuda.L1AttnSoftmaxV(mode)
-    res = []
-    for dt in (torch.float32, torch.float64):
-        t = [x.to(dt).requires_grad_(True) for x in (q, k, v)]
-        out = m(*t)
-        res.append([out, *torch.autograd.grad(out, t, g.to(dt))])
+    _assert_form(n, w, wv, backward=129 if w <= 64 else 128)
     # pieces hold the operands exactly; what is left are fp32 sums and the rounding of scores of about sqrt(w), which exp() makes relative
-    for x, r, name in zip(*res, ("vo", "dq", "dk", "dv")):
-        assert_close(x.detach().cpu().numpy(), r.detach().cpu().numpy(), 1e-5, name)
+    for name, x, r in _run(*_inputs(n, w, wv), mode):
+        _close(x, r, 1e-5, name)
 
 
-@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
-def test_values_that_are_not_finite(bad):
-    """A value that is not finite has no pieces: the CTA computes its rows plainly, and the others are as ever."""
-    import l1attn_fused_cuda
-    q, k, v, g = _inputs(130, 64, 64)
-    m = l1attn_fused_cuda.L1AttnSoftmaxV()
-    v[3, 128, 2, 5] = g[5, 70, 1, 63] = bad
+@pytest.mark.parametrize("n,w,wv", [(65, 64, 64), (193, 48, 40), (200, 33, 21)])
+def test_score_gradients_in_the_order_of_d_attn(n, w, wv):
+    """The first half of the backward alone (l1attn_dense_softmax_v_bwd_dx): dx [b][s][t][h], equal rows among them."""
+    _assert_form(n, w, wv)
+    q, k, v, g = _inputs(n, w, wv)
+    k[:, 3:9] = q[:, 5:11]
     res = []
     for dt in (torch.float32, torch.float64):
-        t = [x.to(dt).requires_grad_(True) for x in (q, k, v)]
-        out = m(*t)
-        res.append([out, *torch.autograd.grad(out, t, g.to(dt))])
-    for i, (x, r, name) in enumerate(zip(*res, ("vo", "dq", "dk", "dv"))):
-        if i in (0, 3):  # (in dq and dk everything of the pair is NaN)
-            assert torch.equal(x.isfinite(), r.isfinite()) and torch.equal(x.isnan(), r.isnan()), name
-        fine = x.isfinite() & r.isfinite()
-        assert_close(x[fine].detach().cpu().numpy(), r[fine].detach().cpu().numpy(), 1e-5, name)
-        assert torch.isfinite(x[7]).all()
+        a = [x.to(dt) for x in (q, k, v, g)]
+        lse = torch.empty(q.shape[:3], dtype=dt, device="cuda")
+        vo = _cabi().dense_softmax_v_fwd(*a[:3], lse=lse)
+        dx, dv = torch.full((BS, n, n, HEADS), np.nan, dtype=dt, device="cuda"), torch.empty_like(a[2])
+        _cabi().dense_softmax_v_bwd_dx(*a, lse, (vo * a[3]).sum(-1), dx, dv)
+        res.append((lse, dx, dv))
+    for name, x, r in zip(("lse", "dx", "dv"), *res):
+        _close(x, r, 1e-5, name)
+
+
+@pytest.mark.parametrize("value", [-np.inf, float(np.finfo(np.float32).min)])
+@pytest.mark.parametrize("n,w,wv", [(200, 64, 64), (200, 33, 21)])
+def test_masked_keys_in_front(n, w, wv, value):
+    """Two whole tiles of keys that are infinitely far, and two keys more: they weigh nothing and get no gradient."""
+    _assert_form(n, w, wv)
+    q, k, v, g = _inputs(n, w, wv)
+    k[:, :130] = value
+    got = [x for _, x, _ in _run(q, k, v, g, "softmax")]
+    ref = [t.double().requires_grad_(True) for t in (q, k[:, 130:], v[:, 130:])]
+    out = []
+    for b in range(BS):
+        x = -(ref[0][b][None] - ref[1][b][:, None]).abs().sum(-1) / w ** 0.5
+        out.append(torch.einsum("sdh,shw->dhw", torch.softmax(x, 0), ref[2][b]))
+    out = torch.stack(out)
+    grads = torch.autograd.grad(out, ref, g.double())
+    for name, x, r in (("vo", got[0], out.detach()), ("dq", got[1], grads[0]), ("dk", got[2][:, 130:], grads[1]), ("dv", got[3][:, 130:], grads[2])):
+        _close(x, r, 1e-5, name)
+    assert not got[2][:, :130].any() and not got[3][:, :130].any()
+
+
+@pytest.mark.parametrize("kind", ["equal_rows", "grid"])
+def test_ties(kind):
+    """Equal rows (their score has no slope) and ties everywhere, against torch's own chain in float64, whose |x| has slope 0 at 0."""
+    n, w, wv = 100, 32, 40
+    _assert_form(n, w, wv)
+    q, k, v, g = _inputs(n, w, wv)
+    if kind == "equal_rows":
+        k[:, 3:9] = q[:, 5:11]
+    else:
+        q, k = (q * 4).round() / 4, (k * 4).round() / 4
+    got = [x for _, x, _ in _run(q, k, v, g, "softmax")]
+    for b in (0, 36):
+        ref = [t[b].double().requires_grad_(True) for t in (q, k, v)]
+        x = -(ref[0][None] - ref[1][:, None]).abs().sum(-1) / w ** 0.5
+        out = torch.einsum("sdh,shw->dhw", torch.softmax(x, 0), ref[2])
+        for name, x, r in zip(("vo", "dq", "dk", "dv"), got, (out.detach(), *torch.autograd.grad(out, ref, g[b].double()))):
+            _close(x[b], r, 1e-5, name)
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("where", ["v", "dvo", "both"])
+@pytest.mark.parametrize("n,w,wv,bad", [(128, 64, 64, np.inf), (128, 64, 64, np.nan), (200, 33, 21, -np.inf), (193, 48, 32, np.inf)])
+def test_values_that_are_not_finite(n, w, wv, bad, where, mode):
+    """A value that is not finite has no pieces: what it reaches is what float64 says, of the same sign, and the others are as ever."""
+    _assert_form(n, w, wv)
+    q, k, v, g = _inputs(n, w, wv)
+    if where != "dvo":
+        v[3, n - 2, 2, 5] = bad
+    if where != "v":
+        g[5, 70, 1, wv - 1] = bad
+    hit = torch.zeros(BS, 1, HEADS, 1, dtype=torch.bool, device="cuda")
+    hit[3, 0, 2, 0], hit[5, 0, 1, 0] = where != "dvo", where != "v"
+    for name, x, r in _run(q, k, v, g, mode):
+        assert torch.isfinite(x[~hit.expand_as(x)]).all(), name
+        assert torch.equal(x.isnan(), r.isnan()) and torch.equal(x.isposinf(), r.isposinf()) and torch.equal(x.isneginf(), r.isneginf()), name
+        fine = x.isfinite()
+        _close(x[fine], r[fine], 1e-5, name)
 
 
 def test_wait_that_counts_polls_gives_up_and_is_reported():
     """The wait of these kernels is bounded by its polls: 500 of them on a barrier that nothing completes, then the kernel returns and the
     status reports a timeout, once.  More polls than a hundred thousand are refused."""
-    import l1attn_cabi
-    lib = l1attn_cabi.lib()
+    lib = _cabi().lib()
     torch.cuda.synchronize()
     assert lib.l1attn_device_status() == 0
     returned = torch.zeros(2, dtype=torch.int32, device="cuda")
