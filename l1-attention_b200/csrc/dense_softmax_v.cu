@@ -444,9 +444,10 @@ __device__ __forceinline__ void score_slice(const unsigned char *Qslice, const u
 //   0-15   scores and weights; the weights' pieces to shared memory (A, [query row][key]), keys in the order 4 * (s % 16) + s / 16, so
 //          that a lane's four weights are neighbours; sums of the tile before: warp = 32 rows x v_width / 4 columns
 //   16     issues the MMAs       17, 18  values' pieces to shared memory (B, [column][key])        19  nothing
-// [16,1024,16,64], values 64 wide: 2.01 ms, softmax_v_tile_kernel 2.24; error against float64 0.85-1.0 of that kernel's.  Bound: FP32 pipe
+// [16,1024,16,64], values 64 wide: 2.09 ms, softmax_v_tile_kernel 2.27; error against float64 0.85-1.0 of that kernel's.  Bound: FP32 pipe
 // of the scores (two lane-cycles per term) with the shared loads of a 4 x 4 tile beside it.
-// Values that are not finite have no such pieces (inf - inf): a CTA that meets one computes its rows once more, plainly.
+// Values without pieces (not finite) are added by FMAs to the sums of their tile, from the weights' pieces and the values in global memory (one such
+// value in every head: 2.12 ms).
 constexpr int TC_NW = 16, TC_ROWS = 128, TC_THREADS = (TC_NW + 4) * 32;
 constexpr int TC_REGS = 104, TC_REGS_REST = 64, TC_REGS_LAUNCH = 96; // registers per thread; the launcher asks whether the kernel was built with the last
 static_assert(4 * TC_REGS + TC_REGS_REST <= 5 * TC_REGS_LAUNCH, "more than the block was launched with");
@@ -454,10 +455,54 @@ constexpr int TC_A_PIECE = TC_ROWS * 128;          // 64 bf16 a row
 constexpr size_t TC_SMEM = 227 * 1024 - 3072;      // per CTA, less the static part
 
 struct TcBars {
-	uint64_t own, full[MAX_STAGE], empty[MAX_STAGE], p_full, v_full, done, done2;
+	uint64_t own, full[MAX_STAGE], empty[MAX_STAGE], p_full, v_full, done, done2, patched;
 	uint32_t tmem;
-	int bad; // something is not finite
+	uint32_t own_without[TC_ROWS / 32];           // rows of the CTA's own values that hold some without pieces
+	__align__(16) uint32_t without[2][2][2];      // [tile & 1][warp - 17]: tokens of the streamed tile that do, by 32
 };
+
+// Values that are not finite have no pieces (inf - inf).  The products are done without them, and the tile is marked.
+__device__ __forceinline__ bool has_pieces(float x) { return fabsf(x) < INFINITY; }
+__device__ __forceinline__ float take(float x, bool &all)
+{
+	const bool ok = has_pieces(x);
+	all = all && ok;
+	return ok ? x : 0.f;
+}
+__device__ __forceinline__ unsigned long long tile_without(const TcBars &bars, int m)
+{
+	uint32_t a, b, c, d;
+	asm volatile("ld.volatile.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(smem_u32(bars.without[m & 1])) : "memory");
+	return (unsigned long long)(b | d) << 32 | (a | c);
+}
+// o[e] += weight x rows[token][e], e < left, for the values of tile m without pieces; they are of the tokens in `which`.  The weights come from their
+// pieces, so all sixteen warps wait for one another before any of them writes the next tile's.  False: a wait has run out.
+template <int NO> __device__ __forceinline__ bool add_without(float (&o)[NO], unsigned long long which, const unsigned char *pieces, int row, const float *rows,
+							      size_t pitch, int m, int n_tok, int left, TcBars &bars, int &patches, int *err)
+{
+	bool ok = mbar_wait_inline(&bars.p_full, m & 1, err); // (the weights are there: complete already, and seen by this thread)
+#pragma unroll 1
+	for (; which; which &= which - 1) {
+		const int i = __ffsll(which) - 1, place = 4 * (i % 16) + i / 16;
+		const unsigned char *a = pieces + row * 128 + (((place >> 3) ^ (row & 7)) << 4) + (place & 7) * 2;
+		float p = 0.f;
+#pragma unroll
+		for (int j = 2; j >= 0; j--)
+			p += __uint_as_float(uint32_t(*reinterpret_cast<const unsigned short *>(a + j * TC_A_PIECE)) << 16);
+#pragma unroll
+		for (int e = 0; e < NO; e++) {
+			const float x = e < left && m * TS + i < n_tok ? rows[size_t(m * TS + i) * pitch + e] : 0.f;
+			if (!has_pieces(x))
+				o[e] = fmaf(p, x, o[e]);
+		}
+	}
+	__syncwarp();
+	if ((threadIdx.x & 31) == 0)
+		mbar_arrive(&bars.patched);
+	ok = ok && mbar_wait_inline(&bars.patched, patches & 1, err);
+	patches++;
+	return ok;
+}
 
 // this lane's four weights of row r (keys 4 sg .. in the order above), as three pieces
 __device__ __forceinline__ void store_weights(unsigned char *pieces, int r, int sg, const float (&p)[4])
@@ -497,7 +542,7 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 	extern __shared__ __align__(1024) unsigned char smem_raw[];
 	unsigned char *base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
 	__shared__ __align__(8) TcBars bars;
-	__shared__ float row_corr[2][TT], row_inv[TT], row_max[TT];
+	__shared__ float row_corr[2][TT], row_inv[TT];
 	const int q_bytes = sh.nwb * TT * 128, k_bytes = sh.nwb * TS * 128, stage_bytes = k_bytes + V_BYTES;
 	unsigned char *Pp = base, *Vp = Pp + 3 * TC_A_PIECE, *Qs = Vp + 3 * V_PIECE, *stages = Qs + q_bytes;
 
@@ -520,7 +565,7 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 		mbar_init(&bars.p_full, NW);
 		mbar_init(&bars.v_full, 2);
 		mbar_init(&bars.done, 1);
-		bars.bad = 0;
+		mbar_init(&bars.patched, NW);
 		mbar_fence_init();
 	}
 	tc_fence_before();
@@ -573,6 +618,7 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 		for (int e = 0; e < NO; e++)
 			o[e] = 0.f;
 		bool dead = !mbar_wait_inline(&bars.own, 0, err);
+		int patches = 0;
 		// the sums of tile m, once its MMAs are done, onto the output, which goes to that tile's shift first
 		auto collect = [&](int m) {
 			if (!dead && !(mbar_wait_inline(&bars.p_full, m & 1, err) && mbar_wait_inline(&bars.done, m & 1, err)))
@@ -584,6 +630,9 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 #pragma unroll
 			for (int e = 0; e < NO; e++)
 				o[e] = fmaf(o[e], c, d[e]);
+			const unsigned long long which = tile_without(bars, m);
+			if (__all_sync(0xffffffffu, which != 0 && !dead)) // (a warp as one, also after a timeout)
+				dead = !add_without(o, which, Pp, orow, v + v0 + ocol, vrow, m, sh.n_tok, sh.v_width - ocol, bars, patches, err);
 		};
 
 		for (int m = 0; m < ns; m++) {
@@ -665,48 +714,18 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 			const int row = i * (2 * NW) + tg, t = t0 + row;
 			if (sg == 0) {
 				row_inv[row] = sh.mode == L1ATTN_SV_EXP ? 1.f : 1.f / lrow[i];
-				row_max[row] = mrow[i];
 				if (lse && t < sh.n_tok) // weight of (s, t) = exp(x - lse)
 					lse[(size_t(b) * sh.n_tok + t) * sh.n_heads + h] = sh.mode == L1ATTN_SV_EXP ? 0.f : mrow[i] + logf(lrow[i]);
 			}
 		}
 		named_barrier(1, NW * 32);
-		if (__shfl_sync(0xffffffffu, *reinterpret_cast<volatile int *>(&bars.bad), 0) == 0) {
-			if (t0 + orow < sh.n_tok) {
-				float *op = vo + v0 + size_t(t0 + orow) * vrow + ocol;
-				const float inv = row_inv[orow];
+		if (t0 + orow < sh.n_tok) {
+			float *op = vo + v0 + size_t(t0 + orow) * vrow + ocol;
+			const float inv = row_inv[orow];
 #pragma unroll
-				for (int e = 0; e < NO; e++)
-					if (FULL || ocol + e < sh.v_width)
-						op[e] = o[e] * inv;
-			}
-		} else { // a row per warp, 32 keys at a time
-#pragma unroll 1
-			for (int row = warp; row < TT && t0 + row < sh.n_tok; row += NW) {
-				const float *qr = q + qk0 + size_t(t0 + row) * krow;
-				const float shift = row_max[row] == -INFINITY ? 0.f : row_max[row];
-				float sum[VW / 32] = {};
-#pragma unroll 1
-				for (int s0 = 0; s0 < sh.n_tok; s0 += 32) {
-					float x = 0.f;
-					if (s0 + lane < sh.n_tok)
-						for (int w = 0; w < sh.width; w++)
-							x += fabsf(qr[w] - k[qk0 + size_t(s0 + lane) * krow + w]);
-					const float p = expf(x * sh.scale - shift);
-#pragma unroll 1
-					for (int e = 0; e < 32 && s0 + e < sh.n_tok; e++) {
-						const float pe = __shfl_sync(0xffffffffu, p, e);
-#pragma unroll
-						for (int c = 0; c < VW / 32; c++)
-							if (c * 32 + lane < sh.v_width)
-								sum[c] = fmaf(pe, v[v0 + size_t(s0 + e) * vrow + c * 32 + lane], sum[c]);
-					}
-				}
-#pragma unroll
-				for (int c = 0; c < VW / 32; c++)
-					if (c * 32 + lane < sh.v_width)
-						vo[v0 + size_t(t0 + row) * vrow + c * 32 + lane] = sum[c] * row_inv[row];
-			}
+			for (int e = 0; e < NO; e++)
+				if (FULL || ocol + e < sh.v_width)
+					op[e] = o[e] * inv;
 		}
 	} else {
 		asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TC_REGS_REST));
@@ -733,7 +752,7 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 				if (m > 0 && !dead && !mbar_wait_inline(&bars.done, (m - 1) & 1, err))
 					dead = true;
 				const float *Vs = reinterpret_cast<const float *>(stages + size_t(st) * stage_bytes + k_bytes);
-				float chk = 0.f;
+				bool all = true;
 				if (c < VW) {
 #pragma unroll 2
 					for (int g = 0; g < 8; g++) { // keys at places 8 g .. 8 g + 7
@@ -741,10 +760,8 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 #pragma unroll
 						for (int e = 0; e < 4; e++) {
 							const int s = (e & 1) * 32 + 2 * g + (e >> 1); // places 8 g + 2 e, + 1: keys s, s + 16
-							const float x = Vs[s * VW + c], y = Vs[(s + 16) * VW + c];
-							chk = fmaf(x, 0.f, fmaf(y, 0.f, chk));
 							uint32_t pc[3];
-							split_bf16(x, y, pc);
+							split_bf16(take(Vs[s * VW + c], all), take(Vs[(s + 16) * VW + c], all), pc);
 #pragma unroll
 							for (int i = 0; i < 3; i++)
 								o[i][e] = pc[i];
@@ -754,11 +771,15 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 							*reinterpret_cast<uint4 *>(Vp + i * V_PIECE + c * 128 + ((g ^ (c & 7)) << 4)) = make_uint4(o[i][0], o[i][1], o[i][2], o[i][3]);
 					}
 				}
-				if (!(chk == 0.f))
-					*reinterpret_cast<volatile int *>(&bars.bad) = 1;
+				uint32_t which[2] = {0, 0};
+				if (!__all_sync(0xffffffffu, all))
+					for (int s = 0; s < TS; s++)
+						which[s >> 5] |= uint32_t(__any_sync(0xffffffffu, c < VW && !has_pieces(Vs[s * VW + c]))) << (s & 31);
 				fence_proxy_async_smem();
 				__syncwarp();
 				if (lane == 0) {
+					bars.without[m & 1][warp - 17][0] = which[0];
+					bars.without[m & 1][warp - 17][1] = which[1];
 					mbar_arrive(&bars.v_full);
 					mbar_arrive(&bars.empty[st]);
 				}
@@ -1272,7 +1293,9 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 		mbar_init(&bars.v_full, 2); // (the pieces of dvo)
 		mbar_init(&bars.done, 1);   // D1
 		mbar_init(&bars.done2, 1);  // D2
-		bars.bad = 0;
+		mbar_init(&bars.patched, NW);
+		for (int i = 0; i < TT / 32; i++)
+			bars.own_without[i] = 0;
 		mbar_fence_init();
 	}
 	__syncthreads();
@@ -1280,9 +1303,10 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 	for (int i = tid; i < TT * (VW / 2); i += TC_THREADS) {
 		const int row = i / (VW / 2), c = i % (VW / 2) * 2;
 		const float *vp = v + v0 + size_t(s0 + row < sh.n_tok ? s0 + row : 0) * vrow + c;
-		const float x = s0 + row < sh.n_tok && c < sh.v_width ? vp[0] : 0.f, y = s0 + row < sh.n_tok && c + 1 < sh.v_width ? vp[1] : 0.f;
-		if (!(fmaf(x, 0.f, y * 0.f) == 0.f))
-			*reinterpret_cast<volatile int *>(&bars.bad) = 1;
+		bool all = true;
+		const float x = take(s0 + row < sh.n_tok && c < sh.v_width ? vp[0] : 0.f, all), y = take(s0 + row < sh.n_tok && c + 1 < sh.v_width ? vp[1] : 0.f, all);
+		if (!all)
+			atomicOr(&bars.own_without[row >> 5], 1u << (row & 31));
 		uint32_t pc[3];
 		split_bf16(x, y, pc);
 		unsigned char *d = Vp + row * 128 + (((c >> 3) ^ (row & 7)) << 4) + (c & 7) * 2;
@@ -1337,6 +1361,8 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 		for (int e = 0; e < NO; e++)
 			o[e] = 0.f;
 		bool dead = !mbar_wait_inline(&bars.own, 0, err);
+		const bool any_own = (bars.own_without[0] | bars.own_without[1] | bars.own_without[2] | bars.own_without[3]) != 0;
+		int patches = 0;
 		auto collect = [&](int m) { // dv of tile m
 			if (!dead && !mbar_wait_inline(&bars.done2, m & 1, err))
 				dead = true;
@@ -1346,6 +1372,9 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 #pragma unroll
 			for (int e = 0; e < NO; e++)
 				o[e] += d[e];
+			const unsigned long long which = tile_without(bars, m);
+			if (__all_sync(0xffffffffu, which != 0 && !dead)) // (a warp as one, also after a timeout)
+				dead = !add_without(o, which, Pp, orow, dvo + v0 + part * NO, vrow, m, sh.n_tok, sh.v_width - part * NO, bars, patches, err);
 		};
 
 		for (int m = 0; m < nt; m++) {
@@ -1396,6 +1425,31 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 				for (int e = 0; e < 4; e++)
 					*reinterpret_cast<float4 *>(Pp + orow * 256 + (((part * 4 + e) ^ (orow & 15)) << 4)) =
 						make_float4(d[e * 4], d[e * 4 + 1], d[e * 4 + 2], d[e * 4 + 3]);
+				const unsigned long long which = tile_without(bars, m);
+				if (which != 0 || any_own) { // this thread's part again: the terms with a factor that has no pieces
+					const float *vr = v + v0 + size_t(s0 + orow) * vrow, *gr = dvo + v0 + size_t(m) * TS * vrow;
+					auto token = [&](int i) { return i % 4 * 16 + part * 4 + i / 4; }; // of place part * 16 + i
+					auto add = [&](int i, float x, float y) {
+						float *cell = reinterpret_cast<float *>(Pp + orow * 256 + (((part * 4 + i / 4) ^ (orow & 15)) << 4)) + i % 4;
+						*cell = fmaf(x, y, *cell);
+					};
+					if (bars.own_without[orow >> 5] >> (orow & 31) & 1) // the factor of v
+#pragma unroll 1
+						for (int c = 0; c < sh.v_width; c++)
+							if (!has_pieces(vr[c]))
+#pragma unroll 1
+								for (int i = 0; i < 16; i++)
+									if (m * TS + token(i) < sh.n_tok)
+										add(i, vr[c], gr[size_t(token(i)) * vrow + c]);
+					if (which != 0 && s0 + orow < sh.n_tok) // the factor of dvo alone
+#pragma unroll 1
+						for (int i = 0; i < 16; i++)
+							if ((which >> token(i) & 1) && m * TS + token(i) < sh.n_tok)
+#pragma unroll 1
+								for (int c = 0; c < sh.v_width; c++)
+									if (!has_pieces(gr[size_t(token(i)) * vrow + c]) && has_pieces(vr[c]))
+										add(i, vr[c], gr[size_t(token(i)) * vrow + c]);
+				}
 			}
 			named_barrier(1, NW * 32);
 #pragma unroll
@@ -1425,49 +1479,12 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 				mbar_arrive(&bars.p_full);
 		}
 		collect(nt - 1);
-		// (dx of every row is written before a row of it is written again.  The barrier stands before the look at `bad`: when a wait has
-		// run out, warps may see different values of it)
-		named_barrier(1, NW * 32);
-		if (__shfl_sync(0xffffffffu, *reinterpret_cast<volatile int *>(&bars.bad), 0) == 0) {
-			if (s0 + orow < sh.n_tok) {
-				float *op = dv + v0 + size_t(s0 + orow) * vrow + part * NO;
+		if (s0 + orow < sh.n_tok) {
+			float *op = dv + v0 + size_t(s0 + orow) * vrow + part * NO;
 #pragma unroll
-				for (int e = 0; e < NO; e++)
-					if (FULL || part * NO + e < sh.v_width)
-						op[e] = o[e];
-			}
-		} else { // a source row per warp, 32 queries at a time
-#pragma unroll 1
-			for (int row = warp; row < TT && s0 + row < sh.n_tok; row += NW) {
-				const float *kr = k + qk0 + size_t(s0 + row) * krow, *vr = v + v0 + size_t(s0 + row) * vrow;
-				float sum[NVB] = {};
-#pragma unroll 1
-				for (int t0 = 0; t0 < sh.n_tok; t0 += 32) {
-					const int t = t0 + lane;
-					float x = 0.f, p = 0.f, d = 0.f;
-					if (t < sh.n_tok) {
-						for (int w = 0; w < sh.width; w++)
-							x += fabsf(kr[w] - q[qk0 + size_t(t) * krow + w]);
-						for (int c = 0; c < sh.v_width; c++)
-							d = fmaf(vr[c], dvo[v0 + size_t(t) * vrow + c], d);
-						const size_t at = (size_t(b) * sh.n_tok + t) * hstride + h;
-						p = expf(x * sh.scale - lse[at]);
-						dx[dx0 + size_t(s0 + row) * dx_s + size_t(t) * dx_t] = sh.dx_pitch > 0 && x == 0.f ? 0.f : p * (d - delta[at]);
-					}
-#pragma unroll 1
-					for (int e = 0; e < 32 && t0 + e < sh.n_tok; e++) {
-						const float pe = __shfl_sync(0xffffffffu, p, e);
-#pragma unroll
-						for (int c = 0; c < NVB; c++)
-							if (c * 32 + lane < sh.v_width)
-								sum[c] = fmaf(pe, dvo[v0 + size_t(t0 + e) * vrow + c * 32 + lane], sum[c]);
-					}
-				}
-#pragma unroll
-				for (int c = 0; c < NVB; c++)
-					if (c * 32 + lane < sh.v_width)
-						dv[v0 + size_t(s0 + row) * vrow + c * 32 + lane] = sum[c];
-			}
+			for (int e = 0; e < NO; e++)
+				if (FULL || part * NO + e < sh.v_width)
+					op[e] = o[e];
 		}
 	} else {
 		asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TC_REGS_REST));
@@ -1499,17 +1516,16 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 				if (m > 0 && !dead && !mbar_wait_inline(&bars.done2, (m - 1) & 1, err))
 					dead = true;
 				const unsigned char *Gs = stages + size_t(st) * stage_bytes + q_bytes;
-				float chk = 0.f;
+				bool all = true;
 #pragma unroll 2
 				for (int g = 0; g < VW / 8; g++) { // columns 8 g .. 8 g + 7: two chunks of the row's 128-byte slice
 					uint32_t o[3][4];
 #pragma unroll
 					for (int e = 0; e < 2; e++) {
 						const float4 x = *reinterpret_cast<const float4 *>(Gs + (g >> 2) * TS * 128 + t * 128 + ((((g & 3) * 2 + e) ^ (t & 7)) << 4));
-						chk = fmaf(x.x, 0.f, fmaf(x.y, 0.f, fmaf(x.z, 0.f, fmaf(x.w, 0.f, chk))));
 						uint32_t pa[3], pb[3];
-						split_bf16(x.x, x.y, pa);
-						split_bf16(x.z, x.w, pb);
+						split_bf16(take(x.x, all), take(x.y, all), pa);
+						split_bf16(take(x.z, all), take(x.w, all), pb);
 #pragma unroll
 						for (int i = 0; i < 3; i++) {
 							o[i][e * 2] = pa[i];
@@ -1520,11 +1536,12 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 					for (int i = 0; i < 3; i++)
 						*reinterpret_cast<uint4 *>(Gp + i * G_PIECE + place * 128 + ((g ^ (place & 7)) << 4)) = make_uint4(o[i][0], o[i][1], o[i][2], o[i][3]);
 				}
-				if (!(chk == 0.f))
-					*reinterpret_cast<volatile int *>(&bars.bad) = 1;
+				const uint32_t which = __ballot_sync(0xffffffffu, !all);
 				fence_proxy_async_smem();
 				__syncwarp();
 				if (lane == 0) {
+					bars.without[m & 1][warp - 17][warp - 17] = which;
+					bars.without[m & 1][warp - 17][18 - warp] = 0;
 					mbar_arrive(&bars.v_full);
 					mbar_arrive(&bars.empty[st]);
 				}
