@@ -438,16 +438,16 @@ __device__ __forceinline__ void score_slice(const unsigned char *Qslice, const u
 // Forward with the value product on the tensor cores (fp32, 128-row CTAs, width <= 96, v_width <= 64)
 // ------------------------------------------------------------------------------------------------
 // The scores, the softmax and who owns what are those of softmax_v_tile_kernel<.., 4, 16, ..>; the value product -- a third of that
-// kernel's instructions -- is done by tcgen05.mma.  Weights and values are written as sums of three bf16 each (exact: 3 x 8 bits
-// of 24), nine products with fp32 accumulators per key tile, smallest first; the sums of a tile are read back, rescaled and added in
-// fp32 registers, a tile behind the scores.  Warps:
+// kernel's instructions -- is done by tcgen05.mma.  Weights and values, times 2^24, are written as sums of three bf16 each (exact: 3 x 8
+// bits of 24, none of them subnormal), nine products with fp32 accumulators per key tile, smallest first; the sums of a tile are read back,
+// rescaled and added in fp32 registers, a tile behind the scores.  Warps:
 //   0-15   scores and weights; the weights' pieces to shared memory (A, [query row][key]), keys in the order 4 * (s % 16) + s / 16, so
 //          that a lane's four weights are neighbours; sums of the tile before: warp = 32 rows x v_width / 4 columns
 //   16     issues the MMAs       17, 18  values' pieces to shared memory (B, [column][key])        19  nothing
 // [16,1024,16,64], values 64 wide: 2.09 ms, softmax_v_tile_kernel 2.27; error against float64 0.85-1.0 of that kernel's.  Bound: FP32 pipe
 // of the scores (two lane-cycles per term) with the shared loads of a 4 x 4 tile beside it.
-// Values without pieces (not finite) are added by FMAs to the sums of their tile, from the weights' pieces and the values in global memory (one such
-// value in every head: 2.12 ms).
+// Values without pieces (not finite, or 2^36 and more) are added by FMAs to the sums of their tile, from the weights' pieces and the values in
+// global memory (one such value in every head: 2.12 ms).
 constexpr int TC_NW = 16, TC_ROWS = 128, TC_THREADS = (TC_NW + 4) * 32;
 constexpr int TC_REGS = 104, TC_REGS_REST = 64, TC_REGS_LAUNCH = 96; // registers per thread; the launcher asks whether the kernel was built with the last
 static_assert(4 * TC_REGS + TC_REGS_REST <= 5 * TC_REGS_LAUNCH, "more than the block was launched with");
@@ -461,13 +461,14 @@ struct TcBars {
 	__align__(16) uint32_t without[2][2][2];      // [tile & 1][warp - 17]: tokens of the streamed tile that do, by 32
 };
 
-// Values that are not finite have no pieces (inf - inf).  The products are done without them, and the tile is marked.
-__device__ __forceinline__ bool has_pieces(float x) { return fabsf(x) < INFINITY; }
+// Values that are not finite have no pieces (inf - inf), and very large ones get none, for the range of the sums.  The products are
+// done without them, and the tile is marked.
+__device__ __forceinline__ bool has_pieces(float x) { return fabsf(x) < PIECE_LIMIT; }
 __device__ __forceinline__ float take(float x, bool &all)
 {
 	const bool ok = has_pieces(x);
 	all = all && ok;
-	return ok ? x : 0.f;
+	return ok ? x * PIECE_SCALE : 0.f;
 }
 __device__ __forceinline__ unsigned long long tile_without(const TcBars &bars, int m)
 {
@@ -493,7 +494,7 @@ template <int NO> __device__ __forceinline__ bool add_without(float (&o)[NO], un
 		for (int e = 0; e < NO; e++) {
 			const float x = e < left && m * TS + i < n_tok ? rows[size_t(m * TS + i) * pitch + e] : 0.f;
 			if (!has_pieces(x))
-				o[e] = fmaf(p, x, o[e]);
+				o[e] = fmaf(p * (1.f / PIECE_SCALE), x, o[e]);
 		}
 	}
 	__syncwarp();
@@ -508,8 +509,8 @@ template <int NO> __device__ __forceinline__ bool add_without(float (&o)[NO], un
 __device__ __forceinline__ void store_weights(unsigned char *pieces, int r, int sg, const float (&p)[4])
 {
 	uint32_t a[3], b[3];
-	split_bf16(p[0], p[1], a);
-	split_bf16(p[2], p[3], b);
+	split_bf16(p[0] * PIECE_SCALE, p[1] * PIECE_SCALE, a);
+	split_bf16(p[2] * PIECE_SCALE, p[3] * PIECE_SCALE, b);
 	unsigned char *d = pieces + r * 128 + (((sg >> 1) ^ (r & 7)) << 4) + (sg & 1) * 8;
 #pragma unroll
 	for (int i = 0; i < 3; i++)
@@ -629,7 +630,7 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 			const float c = row_corr[m & 1][orow];
 #pragma unroll
 			for (int e = 0; e < NO; e++)
-				o[e] = fmaf(o[e], c, d[e]);
+				o[e] = fmaf(o[e], c, d[e] * PIECE_UNSCALE);
 			const unsigned long long which = tile_without(bars, m);
 			if (__all_sync(0xffffffffu, which != 0 && !dead)) // (a warp as one, also after a timeout)
 				dead = !add_without(o, which, Pp, orow, v + v0 + ocol, vrow, m, sh.n_tok, sh.v_width - ocol, bars, patches, err);
@@ -1371,7 +1372,7 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 			tmem_load(d_at + D2 + part * NO, d);
 #pragma unroll
 			for (int e = 0; e < NO; e++)
-				o[e] += d[e];
+				o[e] = fmaf(d[e], PIECE_UNSCALE, o[e]);
 			const unsigned long long which = tile_without(bars, m);
 			if (__all_sync(0xffffffffu, which != 0 && !dead)) // (a warp as one, also after a timeout)
 				dead = !add_without(o, which, Pp, orow, dvo + v0 + part * NO, vrow, m, sh.n_tok, sh.v_width - part * NO, bars, patches, err);
@@ -1421,6 +1422,9 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 			{ // dp: a row and 16 places of it per thread to [row][place], 16-byte chunk ^= row & 15
 				float d[16];
 				tmem_load(d_at + D1 + part * 16, d);
+#pragma unroll
+				for (int e = 0; e < 16; e++)
+					d[e] *= PIECE_UNSCALE;
 #pragma unroll
 				for (int e = 0; e < 4; e++)
 					*reinterpret_cast<float4 *>(Pp + orow * 256 + (((part * 4 + e) ^ (orow & 15)) << 4)) =

@@ -47,7 +47,10 @@ __device__ __forceinline__ void tc_mma_bf16_ss(uint32_t d, uint64_t a, uint64_t 
 		     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(uint32_t(accumulate))
 		     : "memory");
 }
-// a and b as three bf16 each, exactly (but for what lies below 2^-126): truncations of the value and of what they leave
+// Operands of the products are split times 2^24.  The last bit of a float lies at 2^-149 or above, that of its 2^24-fold at 2^-125: no
+// piece is subnormal and none is lost.  Below 2^36 the sum of 64 products of two such operands stays below 2^126; larger ones have no pieces.
+constexpr float PIECE_SCALE = 0x1p24f, PIECE_LIMIT = 0x1p36f, PIECE_UNSCALE = 0x1p-48f;
+// a and b (times PIECE_SCALE) as three bf16 each, exactly: truncations of the value and of what they leave
 __device__ __forceinline__ void split_bf16(float a, float b, uint32_t (&piece)[3])
 {
 #pragma unroll

@@ -158,6 +158,46 @@ def test_values_that_are_not_finite_cost_little():
     assert took[1][0] < 3 * took[0][0] and took[1][1] < 3 * took[0][1], took
 
 
+@pytest.mark.parametrize("n,w,wv", [(65, 64, 64), (200, 33, 21)])
+def test_small_values(n, w, wv):
+    """Values and gradients down to the smallest normal floats keep their 24 bits in the products (what is left are the roundings of scores and of
+    subnormal outputs): v and dvo at 2^-119 one at a time, so that <v, dvo> does not leave the range."""
+    _assert_form(n, w, wv)
+    for i in (2, 3):
+        t = _inputs(n, w, wv)
+        t[i] *= 2.0 ** -119
+        for name, x, r in _run(*t, "softmax"):
+            _close(x, r, 1e-5, name)
+
+
+@pytest.mark.parametrize("mode", ["softmax_plus_one", "exp"])
+def test_small_weights(mode):
+    """Scores of -84, unshifted: weights of 2^-121 keep their 24 bits.  q and k on a grid of 1/4 and a width of 64: scores without rounding, so the
+    bound is that of exp() and of the sums alone."""
+    n, w, wv = 100, 64, 64
+    _assert_form(n, w, wv)
+    q, k, v, g = _inputs(n, w, wv)
+    q, k = (q.clamp(-3, 3) * 4).round() / 4, (k.clamp(-3, 3) * 4).round() / 4 + 10.5
+    for name, x, r in _run(q, k, v, g, mode):
+        if name in ("vo", "dv"):
+            _close(x, r, 1e-6, name)
+
+
+@pytest.mark.parametrize("mode", MODES)
+def test_large_values(mode):
+    """Values up to 1e36 beside ordinary ones stay in range, and each column keeps its precision."""
+    n, w, wv = 128, 48, 40
+    _assert_form(n, w, wv)
+    q, k, v, g = _inputs(n, w, wv)
+    v[..., 3] *= 1e36
+    v[:, 5, :, 7] *= 1e20
+    g[..., 3] = 0
+    for name, x, r in _run(q, k, v, g, mode):
+        for c in range(wv if name in ("vo", "dv") else 0):
+            _close(x[..., c], r[..., c], 1e-5, (name, c))
+        _close(x, r, 1e-5, name)
+
+
 def test_wait_that_counts_polls_gives_up_and_is_reported():
     """The wait of these kernels is bounded by its polls: 500 of them on a barrier that nothing completes, then the kernel returns and the
     status reports a timeout, once.  More polls than a hundred thousand are refused."""
