@@ -435,24 +435,30 @@ __device__ __forceinline__ void score_slice(const unsigned char *Qslice, const u
 }
 
 // ------------------------------------------------------------------------------------------------
-// Forward with the value product on the tensor cores (fp32, 128-row CTAs, width <= 96, v_width <= 64)
+// Forward with the value product on the tensor cores (fp32, 128-row CTAs, width <= 64, v_width <= 64)
 // ------------------------------------------------------------------------------------------------
 // The scores, the softmax and who owns what are those of softmax_v_tile_kernel<.., 4, 16, ..>; the value product -- a third of that
 // kernel's instructions -- is done by tcgen05.mma.  Weights and values, times 2^24, are written as sums of three bf16 each (exact: 3 x 8
-// bits of 24, none of them subnormal), nine products with fp32 accumulators per key tile, smallest first; the sums of a tile are read back,
+// bits of 24, none of them subnormal), nine products in three fp32 sums per key tile (see mma_pieces); they are read back,
 // rescaled and added in fp32 registers, a tile behind the scores.  Warps:
 //   0-15   scores and weights; the weights' pieces to shared memory (A, [query row][key]), keys in the order 4 * (s % 16) + s / 16, so
 //          that a lane's four weights are neighbours; sums of the tile before: warp = 32 rows x v_width / 4 columns
 //   16     issues the MMAs       17, 18  values' pieces to shared memory (B, [column][key])        19  nothing
-// [16,1024,16,64], values 64 wide: 2.09 ms, softmax_v_tile_kernel 2.27; error against float64 0.85-1.0 of that kernel's.  Bound: FP32 pipe
+// [16,1024,16,64], values 64 wide: 2.11 ms, softmax_v_tile_kernel 2.27; error against float64 0.85-1.0 of that kernel's.  Bound: FP32 pipe
 // of the scores (two lane-cycles per term) with the shared loads of a 4 x 4 tile beside it.
 // Values without pieces (not finite, or 2^36 and more) are added by FMAs to the sums of their tile, from the weights' pieces and the values in
-// global memory (one such value in every head: 2.12 ms).
+// global memory (one such value in every head: 2.14 ms).
 constexpr int TC_NW = 16, TC_ROWS = 128, TC_THREADS = (TC_NW + 4) * 32;
 constexpr int TC_REGS = 104, TC_REGS_REST = 64, TC_REGS_LAUNCH = 96; // registers per thread; the launcher asks whether the kernel was built with the last
 static_assert(4 * TC_REGS + TC_REGS_REST <= 5 * TC_REGS_LAUNCH, "more than the block was launched with");
+constexpr int TC_MAINS = 2;                        // sums of the leading products (see mma_pieces), each 64 columns of tensor memory
+constexpr int TC_SUM = 64 * (1 + TC_MAINS), TC_COLUMNS = 256, TC_BWD_COLUMNS = 512;
+static_assert(TC_SUM <= TC_COLUMNS && 2 * TC_SUM <= TC_BWD_COLUMNS, "tensor memory");
 constexpr int TC_A_PIECE = TC_ROWS * 128;          // 64 bf16 a row
 constexpr size_t TC_SMEM = 227 * 1024 - 3072;      // per CTA, less the static part
+// Widest rows of q, k.  More do not fit the backward; a forward on the tensor cores before a backward that is not gained nothing ([1,512,37,96], values
+// 64 wide: 120 us either way) and cost precision: dp - delta no longer cancels what is left of the adder's one-sided error in vo.
+constexpr int TC_WIDTH = 64;
 
 struct TcBars {
 	uint64_t own, full[MAX_STAGE], empty[MAX_STAGE], p_full, v_full, done, done2, patched;
@@ -517,12 +523,15 @@ __device__ __forceinline__ void store_weights(unsigned char *pieces, int r, int 
 		*reinterpret_cast<uint2 *>(d + i * TC_A_PIECE) = make_uint2(a[i], b[i]);
 }
 
-// all products of the pieces, smallest first; steps of 16 k
+// All products of the pieces, STEPS of 16 k.  The tensor core adds to its fp32 sums by truncation, which for values of one sign is an error of one
+// sign.  So the leading products go to two sums of their own, a half of the k each (at d + 64, d + 128), the eight others, 2^-6 of them and less,
+// to a third (at d, smallest first), and the three are added with rounding.  (All in one sum: vo and dv of positive values 4.5e-8 too small.)
 template <int STEPS> __device__ __forceinline__ void mma_pieces(uint32_t d, uint64_t a, uint32_t a_piece, uint64_t b, uint32_t b_piece, uint32_t b_step, uint32_t idesc)
 {
+	static_assert(STEPS % TC_MAINS == 0, "every sum gets products");
 	bool more = false;
 #pragma unroll 1
-	for (int i = 8; i >= 0; i--) { // i = 3 * piece of a + piece of b: (2,2), (2,1), ... (0,0)
+	for (int i = 8; i > 0; i--) { // i = 3 * piece of a + piece of b: (2,2), (2,1), ... (0,1)
 		const uint64_t ai = a + i / 3 * (a_piece >> 4), bi = b + i % 3 * (b_piece >> 4);
 #pragma unroll
 		for (int k = 0; k < STEPS; k++) {
@@ -530,6 +539,18 @@ template <int STEPS> __device__ __forceinline__ void mma_pieces(uint32_t d, uint
 			more = true;
 		}
 	}
+#pragma unroll
+	for (int k = 0; k < STEPS; k++)
+		tc_mma_bf16_ss(d + 64 * (1 + k * TC_MAINS / STEPS), a + k * 2, b + k * (b_step >> 4), idesc, k * TC_MAINS % STEPS != 0);
+}
+// this lane's row of them: d + 64, d + 128 and d
+template <int N> __device__ __forceinline__ void load_sums(uint32_t d, float (&r)[N])
+{
+	float x[N], y[N];
+	tmem_load3(d + 64, d + 128, d, r, x, y);
+#pragma unroll
+	for (int e = 0; e < N; e++)
+		r[e] = r[e] + x[e] + y[e];
 }
 
 template <int NV, bool TMA, bool FULL>
@@ -556,7 +577,7 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 	const int ns = (sh.n_tok + TS - 1) / TS;
 
 	if (warp == 16)
-		tmem_alloc(&bars.tmem, 64);
+		tmem_alloc(&bars.tmem, TC_COLUMNS);
 	if (tid == 0) {
 		mbar_init(&bars.own, TMA ? 1 : NW * 32);
 		for (int s = 0; s < MAX_STAGE; s++) {
@@ -626,7 +647,7 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 				dead = true;
 			tc_fence_after();
 			float d[NO];
-			tmem_load(d_at, d);
+			load_sums(d_at, d);
 			const float c = row_corr[m & 1][orow];
 #pragma unroll
 			for (int e = 0; e < NO; e++)
@@ -762,7 +783,7 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 						for (int e = 0; e < 4; e++) {
 							const int s = (e & 1) * 32 + 2 * g + (e >> 1); // places 8 g + 2 e, + 1: keys s, s + 16
 							uint32_t pc[3];
-							split_bf16(take(Vs[s * VW + c], all), take(Vs[(s + 16) * VW + c], all), pc);
+							split_bf16_short(take(Vs[s * VW + c], all), take(Vs[(s + 16) * VW + c], all), pc);
 #pragma unroll
 							for (int i = 0; i < 3; i++)
 								o[i][e] = pc[i];
@@ -791,7 +812,7 @@ softmax_v_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
 	tc_fence_before();
 	__syncthreads();
 	if (warp == 16)
-		tmem_free(tmem, 64);
+		tmem_free(tmem, TC_COLUMNS);
 }
 
 size_t sv_tc_smem(int nwb, int nv, int nstage)
@@ -902,7 +923,7 @@ TilePlan sv_plan(int bs, int n_tok, int n_heads, int width, int v_width)
 	if (width < 1 || width > 128 || v_width < 1 || v_width > 128)
 		return {0, 0, 0, 0, false};
 	const int nwb = (width + 31) / 32, nv = sv_nv(v_width);
-	return plan_tile(nv, (long long)bs * n_heads, n_tok, [&](int tt, int ns) { return sv_smem(nwb, nv, tt, ns); }, [&](int ns) { return sv_tc_smem(nwb, nv, ns); });
+	return plan_tile(nv, (long long)bs * n_heads, n_tok, [&](int tt, int ns) { return sv_smem(nwb, nv, tt, ns); }, [&](int ns) { return width <= TC_WIDTH ? sv_tc_smem(nwb, nv, ns) : TC_SMEM + 1; });
 }
 
 // Returns L1ATTN_OK, a negative error, or 1 when the shape is outside this kernel's set.
@@ -1283,7 +1304,7 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 	const size_t qk0 = size_t(b) * sh.n_tok * krow + size_t(h) * sh.width, v0 = size_t(b) * sh.n_tok * vrow + size_t(h) * sh.v_width;
 
 	if (warp == 16)
-		tmem_alloc(&bars.tmem, 128);
+		tmem_alloc(&bars.tmem, TC_BWD_COLUMNS);
 	if (tid == 0) {
 		mbar_init(&bars.own, TMA ? 1 : NW * 32);
 		for (int s = 0; s < MAX_STAGE; s++) {
@@ -1309,7 +1330,7 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 		if (!all)
 			atomicOr(&bars.own_without[row >> 5], 1u << (row & 31));
 		uint32_t pc[3];
-		split_bf16(x, y, pc);
+		split_bf16_short(x, y, pc);
 		unsigned char *d = Vp + row * 128 + (((c >> 3) ^ (row & 7)) << 4) + (c & 7) * 2;
 #pragma unroll
 		for (int e = 0; e < 3; e++)
@@ -1319,7 +1340,7 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 	tc_fence_before();
 	__syncthreads();
 	tc_fence_after();
-	const uint32_t tmem = bars.tmem, D1 = 0, D2 = 64;
+	const uint32_t tmem = bars.tmem, D1 = 0, D2 = TC_SUM;
 	const size_t hstride = size_t(sh.n_heads);
 	const size_t dx_t = sh.dx_pitch > 0 ? 1 : hstride, dx_s = sh.dx_pitch > 0 ? size_t(sh.dx_pitch) : hstride * sh.n_tok;
 	const size_t dx0 = sh.dx_pitch > 0 ? (size_t(b) * sh.n_heads + h) * sh.n_tok * sh.dx_pitch : size_t(b) * sh.n_tok * sh.n_tok * hstride + h;
@@ -1369,7 +1390,7 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 				dead = true;
 			tc_fence_after();
 			float d[NO];
-			tmem_load(d_at + D2 + part * NO, d);
+			load_sums(d_at + D2 + part * NO, d);
 #pragma unroll
 			for (int e = 0; e < NO; e++)
 				o[e] = fmaf(d[e], PIECE_UNSCALE, o[e]);
@@ -1421,7 +1442,7 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 			tc_fence_after();
 			{ // dp: a row and 16 places of it per thread to [row][place], 16-byte chunk ^= row & 15
 				float d[16];
-				tmem_load(d_at + D1 + part * 16, d);
+				load_sums(d_at + D1 + part * 16, d);
 #pragma unroll
 				for (int e = 0; e < 16; e++)
 					d[e] *= PIECE_UNSCALE;
@@ -1528,8 +1549,8 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 					for (int e = 0; e < 2; e++) {
 						const float4 x = *reinterpret_cast<const float4 *>(Gs + (g >> 2) * TS * 128 + t * 128 + ((((g & 3) * 2 + e) ^ (t & 7)) << 4));
 						uint32_t pa[3], pb[3];
-						split_bf16(take(x.x, all), take(x.y, all), pa);
-						split_bf16(take(x.z, all), take(x.w, all), pb);
+						split_bf16_short(take(x.x, all), take(x.y, all), pa);
+						split_bf16_short(take(x.z, all), take(x.w, all), pb);
 #pragma unroll
 						for (int i = 0; i < 3; i++) {
 							o[i][e * 2] = pa[i];
@@ -1556,7 +1577,7 @@ softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 	tc_fence_before();
 	__syncthreads();
 	if (warp == 16)
-		tmem_free(tmem, 128);
+		tmem_free(tmem, TC_BWD_COLUMNS);
 }
 
 size_t sv_bwd_tc_smem(int nwb, int nv, int nstage)

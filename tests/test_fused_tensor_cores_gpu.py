@@ -9,7 +9,7 @@ from conftest import assert_close
 
 pytestmark = pytest.mark.gpu
 SHAPES = [(65, 64, 64), (100, 33, 21), (127, 32, 32), (128, 64, 33), (200, 17, 64), (256, 64, 64), (193, 48, 40), (128, 4, 1)]
-WIDE = [(128, 96, 64), (128, 65, 7), (200, 128, 32), (128, 97, 21)]  # (rows of three and four slices: the forward alone)
+WIDE = [(128, 96, 64), (128, 65, 7), (200, 128, 32), (128, 97, 21)]  # (wider rows: the same CTAs without the tensor cores)
 MODES = ["softmax", "softmax_plus_one", "exp"]
 BS, HEADS = 37, 4
 
@@ -47,7 +47,7 @@ def _close(x, r, tol, name):
 @pytest.mark.parametrize("mode", MODES)
 @pytest.mark.parametrize("n,w,wv", SHAPES + WIDE)
 def test_output_and_gradients(n, w, wv, mode):
-    _assert_form(n, w, wv, backward=129 if w <= 64 else 128)
+    _assert_form(n, w, wv, *((129, 129) if w <= 64 else (128, 128)))
     # pieces hold the operands exactly; what is left are fp32 sums and the rounding of scores of about sqrt(w), which exp() makes relative
     for name, x, r in _run(*_inputs(n, w, wv), mode):
         _close(x, r, 1e-5, name)
@@ -196,6 +196,27 @@ def test_large_values(mode):
         for c in range(wv if name in ("vo", "dv") else 0):
             _close(x[..., c], r[..., c], 1e-5, (name, c))
         _close(x, r, 1e-5, name)
+
+
+@pytest.mark.parametrize("n", [65, 128, 256])
+def test_sums_of_one_sign(n):
+    """The tensor core adds by truncation.  Of values of one sign the sums must not come out systematically small: on scores without rounding the
+    mean relative error stays within half of what one truncated sum per tile gives (2^-24 x 3/4 or so, 4.5e-8)."""
+    w, wv = 64, 64
+    _assert_form(n, w, wv)
+    q, k, v, g = _inputs(n, w, wv)
+    q, k, v, g = (q * 4).round() / 4, (k * 4).round() / 4, v.abs() + 0.01, g.abs() + 0.01
+    res = []
+    for dt in (torch.float32, torch.float64):
+        a = [x.to(dt) for x in (q, k, v, g)]
+        lse = torch.empty(q.shape[:3], dtype=dt, device="cuda")
+        vo = _cabi().dense_softmax_v_fwd(*a[:3], "exp", lse=lse)
+        dx, dv = torch.empty((BS, n, n, HEADS), dtype=dt, device="cuda"), torch.empty_like(a[2])
+        _cabi().dense_softmax_v_bwd_dx(*a, lse, torch.zeros_like(lse), dx, dv)
+        res.append((vo, dx, dv))
+    for name, x, r in zip(("vo", "dx", "dv"), *res):
+        bias = float(((x.double() - r) / r).mean())
+        assert abs(bias) < 2.25e-8, (name, bias)
 
 
 def test_wait_that_counts_polls_gives_up_and_is_reported():
