@@ -822,17 +822,20 @@ size_t sv_tc_smem(int nwb, int nv, int nstage)
 
 // (query rows per half-warp, warps, ring stages) of the tiled kernels.  4 x 16 and 8 x 8 make a 128-row CTA, 4 x 8 a 64-row
 // one.  Sixteen warps of 128 registers measured 7 % faster than eight of 168 (four warps per scheduler hide the
-// shared-memory and arithmetic latencies); with 128 value columns the thread state does not fit 128 registers.  A 64-row CTA
-// takes SHORT_CTA of the time of a 128-row one (forward 41 / 66 us at [4,333,6,64], 97 / 164 at [1,1024,8,64]; 56 / 88 with 128 value
-// columns; two waves of it against one 1.13-1.17); it is taken where the rows do not fit shared memory otherwise, or where its
-// finer grid fills the SMs better (few rows in all, or few left over for the last wave).
+// shared-memory and arithmetic latencies); with 128 value columns the thread state does not fit 128 registers.  A 64-row CTA is taken
+// where the rows do not fit shared memory otherwise, or where its finer grid fills the SMs better (few rows in all, or few left over for the
+// last wave): its waves count `short_cta` each.  Measured, a wave of 64-row CTAs (half of two) against one of 128-row CTAs, us at [1,512,37,w]:
+// forward, width 64 50 / 86, 48 (values 40) 45 / 71, 33 (21) 39 / 70, 96 (64) 61 / 106, 32 (32) 28 / 57; backward on the tensor cores 64 / 94,
+// 53 / 79, 51 / 76, -, 38 / 61, without (width 96) 75 / 140.  From 36 to 450 CTAs of 128 rows, ten widths, the rule is within 6 % of the better form in
+// the forward, 3 % in the backward.
 struct TilePlan {
 	int ti, nw, nstage; // nstage 0: no form fits
 	size_t smem;
 	bool tc; // products on the tensor cores
 };
-constexpr double SHORT_CTA = 0.6;
-template <typename F, typename G> TilePlan plan_tile(int nv, long long groups, int n_tok, F smem_of, G tc_smem_of)
+double sv_short_cta(int width, int v_width) { return width <= 32 && v_width <= 32 ? 0.48 : 0.6; }
+double sv_bwd_short_cta(bool tc) { return tc ? 0.67 : 0.54; }
+template <typename F, typename G> TilePlan plan_tile(int nv, long long groups, int n_tok, double short_cta, F smem_of, G tc_smem_of)
 {
 	const size_t limit = 227 * 1024 - 256; // per-CTA maximum minus the static barriers
 	const bool nw16 = nv <= 4;
@@ -846,7 +849,7 @@ template <typename F, typename G> TilePlan plan_tile(int nv, long long groups, i
 			if (smem > limit)
 				continue;
 			const long long ctas = groups * ((n_tok + tt - 1) / tt);
-			const double cost = double((ctas + 147) / 148) * (tt == 64 ? SHORT_CTA : 1.0);
+			const double cost = double((ctas + 147) / 148) * (tt == 64 ? short_cta : 1.0);
 			if (!best.nstage || cost < best_cost) {
 				best = {c[0], c[1], ns, smem, false};
 				best_cost = cost;
@@ -923,7 +926,8 @@ TilePlan sv_plan(int bs, int n_tok, int n_heads, int width, int v_width)
 	if (width < 1 || width > 128 || v_width < 1 || v_width > 128)
 		return {0, 0, 0, 0, false};
 	const int nwb = (width + 31) / 32, nv = sv_nv(v_width);
-	return plan_tile(nv, (long long)bs * n_heads, n_tok, [&](int tt, int ns) { return sv_smem(nwb, nv, tt, ns); }, [&](int ns) { return width <= TC_WIDTH ? sv_tc_smem(nwb, nv, ns) : TC_SMEM + 1; });
+	return plan_tile(nv, (long long)bs * n_heads, n_tok, sv_short_cta(width, v_width), [&](int tt, int ns) { return sv_smem(nwb, nv, tt, ns); },
+			 [&](int ns) { return width <= TC_WIDTH ? sv_tc_smem(nwb, nv, ns) : TC_SMEM + 1; });
 }
 
 // Returns L1ATTN_OK, a negative error, or 1 when the shape is outside this kernel's set.
@@ -1645,7 +1649,8 @@ TilePlan sv_bwd_plan(int bs, int n_tok, int n_heads, int width, int v_width)
 	if (width < 1 || width > 128 || v_width < 1 || v_width > 128)
 		return {0, 0, 0, 0, false};
 	const int nwb = (width + 31) / 32, nv = sv_nv(v_width);
-	return plan_tile(nv, (long long)bs * n_heads, n_tok, [&](int tt, int ns) { return sv_bwd_smem(nwb, nv, tt, ns); }, [&](int ns) { return sv_bwd_tc_smem(nwb, nv, ns); });
+	return plan_tile(nv, (long long)bs * n_heads, n_tok, sv_bwd_short_cta(nv <= 4 && width <= TC_WIDTH), [&](int tt, int ns) { return sv_bwd_smem(nwb, nv, tt, ns); },
+			 [&](int ns) { return width <= TC_WIDTH ? sv_bwd_tc_smem(nwb, nv, ns) : TC_SMEM + 1; });
 }
 
 int softmax_v_bwd_tile(const float *q, const float *k, const float *v, const float *dvo, const float *lse, const float *delta,

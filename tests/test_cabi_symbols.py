@@ -113,6 +113,23 @@ def test_workspace_of_a_chunk_serves_smaller_chunks():
     assert larger > 100  # (such counts are among them)
 
 
+@pytest.mark.parametrize("n,h,w,wv,forward,backward", [
+    (512, 9, 64, 64, 64, 64),      # 36 CTAs of 128 rows: half of the SMs, 72 of 64 rows fill them
+    (512, 37, 64, 64, 129, 129),   # 148: one wave
+    (512, 46, 64, 64, 64, 129),    # 184: two waves against three of 64 rows (160 against 179 us forward; 402, 396 backward)
+    (512, 46, 48, 40, 64, 129), (512, 56, 64, 64, 129, 129),
+    (512, 80, 32, 32, 64, 129),    # 320: three waves against five (144 against 175 us forward; 393, 388 backward)
+    (512, 37, 32, 32, 64, 129),    # (67 against 69)
+    (512, 80, 96, 64, 128, 64),    # without the tensor cores (804 against 848 us backward)
+    (512, 37, 96, 64, 128, 128), (512, 37, 65, 33, 128, 128), (512, 37, 128, 64, 128, 64), (512, 37, 64, 128, 128, 64), (512, 37, 128, 128, 64, 64),
+    (64, 148, 64, 64, 64, 64), (65, 148, 64, 64, 129, 129), (130, 148, 64, 64, 64, 129), (128, 148, 33, 1, 129, 129),
+    (100, 37, 129, 64, 0, 0), (100, 37, 64, 129, 0, 0)])
+def test_forms_of_the_fused_kernels(n, h, w, wv, forward, backward):
+    """Rows of a CTA (+ 1: products on the tensor cores) at both sides of every line of the rule, measured times beside it."""
+    form = l1attn_cabi.lib().l1attn_test_softmax_v_form
+    assert (form(1, n, h, w, wv, 0), form(1, n, h, w, wv, 1)) == (forward, backward)
+
+
 def test_no_cpu_fallback_in_product():
     """The shipped package must never import the oracle."""
     pkg = os.path.join(ROOT, "l1-attention_b200")

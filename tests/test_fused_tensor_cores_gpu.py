@@ -8,7 +8,7 @@ import torch
 from conftest import assert_close
 
 pytestmark = pytest.mark.gpu
-SHAPES = [(65, 64, 64), (100, 33, 21), (127, 32, 32), (128, 64, 33), (200, 17, 64), (256, 64, 64), (193, 48, 40), (128, 4, 1)]
+SHAPES = [(65, 64, 64), (100, 33, 21), (127, 32, 32), (128, 64, 33), (200, 17, 64), (256, 64, 64), (193, 48, 40), (128, 4, 1), (128, 64, 32)]
 WIDE = [(128, 96, 64), (128, 65, 7), (200, 128, 32), (128, 97, 21)]  # (wider rows: the same CTAs without the tensor cores)
 MODES = ["softmax", "softmax_plus_one", "exp"]
 BS, HEADS = 37, 4
@@ -47,7 +47,7 @@ def _close(x, r, tol, name):
 @pytest.mark.parametrize("mode", MODES)
 @pytest.mark.parametrize("n,w,wv", SHAPES + WIDE)
 def test_output_and_gradients(n, w, wv, mode):
-    _assert_form(n, w, wv, *((129, 129) if w <= 64 else (128, 128)))
+    _assert_form(n, w, wv, *((128, 128) if w > 64 else (64, 129) if max(w, wv) <= 32 else (129, 129)))  # (narrow rows: the backward alone)
     # pieces hold the operands exactly; what is left are fp32 sums and the rounding of scores of about sqrt(w), which exp() makes relative
     for name, x, r in _run(*_inputs(n, w, wv), mode):
         _close(x, r, 1e-5, name)
