@@ -11,13 +11,16 @@
 // (README.md:64-66: F.softmax(a, 1) then einsum 'bsdh,bshw->bdhw'); the "+1" forms are the dense
 // equivalents of the sparse operator's normalisation (python/l1attn_sparse.py:491-502).
 //
-// Two kernels:
+// Three kernels forward (and as many, with the roles swapped, for the first step of the backward):
 //   * softmax_v_kernel: any shape, fp32/fp64.  One CTA per (b, t, h) keeps the n_tok scores of its row
 //     in shared memory: scores, max, exp/sum, value product, each in a fixed order.
 //   * softmax_v_tile_kernel (fp32, width and v_width up to 128): one CTA per (b, h, tile of 64 or 128 query
 //     rows) streams the keys and values of its head in tiles of 64 through a ring and keeps running
 //     max / sum / output rows in registers (online softmax).  The ring is filled by TMA where rows are whole
 //     16-byte vectors, else by 4-byte asynchronous copies of all threads; columns past the end of a row read as zeros.
+//   * softmax_v_tc_kernel (fp32, width and v_width up to 64, where CTAs of 128 rows fill the SMs well): the same with the value product
+//     on the tensor cores.
+// sv_plan() and sv_bwd_plan() choose.
 #include <math.h>
 #include <stdlib.h>
 #include "common.cuh"
@@ -826,8 +829,8 @@ size_t sv_tc_smem(int nwb, int nv, int nstage)
 // where the rows do not fit shared memory otherwise, or where its finer grid fills the SMs better (few rows in all, or few left over for the
 // last wave): its waves count `short_cta` each.  Measured, a wave of 64-row CTAs (half of two) against one of 128-row CTAs, us at [1,512,37,w]:
 // forward, width 64 50 / 86, 48 (values 40) 45 / 71, 33 (21) 39 / 70, 96 (64) 61 / 106, 32 (32) 28 / 57; backward on the tensor cores 64 / 94,
-// 53 / 79, 51 / 76, -, 38 / 61, without (width 96) 75 / 140.  From 36 to 450 CTAs of 128 rows, ten widths, the rule is within 6 % of the better form in
-// the forward, 3 % in the backward.
+// 53 / 79, 51 / 76, -, 38 / 61, without (width 96) 75 / 140.  From 36 to 450 CTAs of 128 rows, ten widths, the rule is within 7 % of the better form in
+// the forward, 4 % in the backward.
 struct TilePlan {
 	int ti, nw, nstage; // nstage 0: no form fits
 	size_t smem;
@@ -1281,7 +1284,8 @@ softmax_v_bwd_tile_kernel(const __grid_constant__ CUtensorMap qmap, const __grid
 // three bf16 pieces each (see softmax_v_tc_kernel).  The pieces of dvo lie [query][column], queries in the order 4 * (t % 16) + t / 16:
 // for dp that is B with its columns along k, for dv B with its queries along k (n contiguous).  Per tile: dp is computed as soon as its
 // pieces are there, beside the scores; it goes through shared memory from the tensor memory's rows to the lanes that hold the scores, in
-// the place of the weights' pieces, which are written behind it.  [4,1024,16,64], values 64 wide: 632 us, softmax_v_bwd_tile_kernel 909.
+// the place of the weights' pieces, which are written behind it.  Whole backward of [8,1024,16,64], values 64 wide, d_q and d_k included: 2.56 ms,
+// with softmax_v_bwd_tile_kernel 3.00.  Bound: FP32 pipe of the scores (55 % of the active cycles, issue 64 %), the two barriers per tile beside it.
 template <int NV, bool TMA, bool FULL>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 softmax_v_bwd_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,

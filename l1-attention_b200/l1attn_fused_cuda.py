@@ -15,15 +15,18 @@ Forward: one kernel (`l1attn_dense_softmax_v_fwd`), nothing of size n x n is sto
 of every query row's normaliser ([bs, n, h]) for the backward.
 Backward, a few batch items at a time (`l1attn_dense_softmax_v_bwd`): one kernel recomputes the weights and
 writes the score gradients dx and dv; the library's dense backward turns dx into dq, dk.
-The only n x n tensor alive is that one chunk of dx (512 MB by default).
+The only n x n tensor alive is that one chunk of dx (512 MB by default); the dense backward's scratch for the same items comes on top.
 """
 import torch
 
 import l1attn_cabi as _c
 
 MODES = tuple(_c.SV_MODES)
-# Score tensor of one backward chunk.  The kernel that makes it runs a CTA per 128 rows and head: at [16,1024,16,64] 256 MB are 512 CTAs,
-# 3.46 waves of 148 SMs (86 % of four), 512 MB are 6.92 (99 % of seven).
+# Score tensor of one backward chunk.  The kernel that makes it runs a CTA per 128 rows and head, and every chunk ends in a wave that is partly empty;
+# memory pays for fewer chunks.  Forward and backward in ms, and peak memory beyond the inputs in MiB, with 256 / 512 MB:
+# [16,1024,16,64] 7.81 / 7.33, 706 / 1154; [16,1024,8,96] (values 64) 5.81 / 5.53, 801 / 1249; [24,700,16,64] 6.42 / 6.18, 722 / 1210; [64,300,12,48] 2.85 / 2.75,
+# 627 / 635; [8,2048,8,64] 7.53 / 7.35, 577 / 961; [2,4096,8,128], where one item fills it, 17.7, 1216 either way.  1024 MB take 1.5 to 6 % less
+# at four of them, for 290 to 1020 MiB.
 _CHUNK_BYTES = 512 << 20
 
 
